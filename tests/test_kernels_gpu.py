@@ -597,3 +597,35 @@ def test_attention_on_tcgen05_waits_for_its_products(K, q_len):
         del junk
         torch.testing.assert_close(out.cpu().float(), ref.float(), rtol=1.6e-2, atol=1.6e-2)
     K.check_device_errors()
+
+
+# The plain float32 product adds an output's terms in eight parts of the k range, whatever the number of rows: at every
+# edge of its two kernels (8 rows of x or 8 and 32 of w per CTA; tiles of 64 x 64 from 17 rows on; copies of 16 bytes or of one
+# float; parts that are short or empty) a row has the same bits in the batch and alone.  A chain of k / 16 products and the
+# adds of the parts round by at most (k / 16 + 4) * 2^-24 of the sum of the products' sizes.
+@pytest.mark.parametrize("n,o,k", [(1, 8, 16), (1, 16385, 36), (2, 33, 64), (4, 9, 130), (8, 16384, 20), (9, 31, 128), (16, 40, 1000),
+                                   (17, 64, 272), (64, 65, 37), (65, 129, 2048), (200, 63, 1), (130, 128, 129)])
+@pytest.mark.parametrize("epilogue", ["none", "silu_gate", "tanh"])
+def test_plain_product_of_a_row_is_the_same_in_every_batch(K, n, o, k, epilogue):
+    gated = epilogue == "silu_gate"
+    x, w = rnd((n, k), torch.float32, 91).cuda(), rnd((2 * o if gated else o, k), torch.float32, 92, scale=k ** -0.5).cuda()
+    bias = None if gated else rnd((o,), torch.float32, 93).cuda()
+    out = torch.full((n, o), float("nan"), device="cuda")
+    K.linear(x, w, out, epilogue, bias=bias)
+    y, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    bound = (k / 16 + 4) * 2.0 ** -24 * size + 1e-7
+    if gated:
+        ref = torch.nn.functional.silu(y[:, :o]) * y[:, o:]
+        bound = 1.1 * bound[:, :o] * y[:, o:].abs() + bound[:, o:] * y[:, :o].abs() + 1e-6 * ref.abs() + 1e-7      # |silu'| <= 1.1
+    else:
+        ref = y + bias.double()
+        bound = bound + 2.0 ** -23 * ref.abs()
+        if epilogue == "tanh":
+            ref = torch.tanh(ref)
+            bound = bound + 4e-7
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    for row in {0, n // 2, n - 1}:
+        alone = torch.empty((1, o), device="cuda")
+        K.linear(x[row:row + 1].contiguous(), w, alone, epilogue, bias=bias)
+        assert torch.equal(alone[0], out[row])
+
