@@ -629,3 +629,27 @@ def test_plain_product_of_a_row_is_the_same_in_every_batch(K, n, o, k, epilogue)
         K.linear(x[row:row + 1].contiguous(), w, alone, epilogue, bias=bias)
         assert torch.equal(alone[0], out[row])
 
+
+# Plain attention in float32 storage: a query's bits do not depend on the other queries of the step, and rows that it may
+# not see (stale pages, later tokens, here NaN) never reach it.
+@pytest.mark.parametrize("nq,nkv,d,ps,window", [(16, 8, 128, 16, 0), (4, 2, 16, 16, 0), (9, 1, 36, 8, 33), (20, 1, 4, 1, 0), (6, 3, 200, 5, 40),
+                                                (2, 2, 256, 32, 0)])
+def test_plain_attention_of_a_query_is_the_same_in_every_step(K, nq, nkv, d, ps, window):
+    q_lens, seq_lens = [40, 1, 3, 67], [40, 300, 65, 97]
+    qkv, kv, bt, cu, sl = _attention_case(torch.float32, nq, nkv, d, ps, window, q_lens, seq_lens, 19)
+    args = (nq, nkv, d, kv.cuda(), bt.cuda())
+    out = torch.empty((qkv.shape[0], nq * d), device="cuda")
+    K.paged_attention(qkv.cuda(), *args, cu.cuda(), sl.cuda(), out, d ** -0.5, window, max(q_lens), max(seq_lens))
+    ref = torch.empty_like(out, device="cpu")
+    REF.paged_attention(qkv, nq, nkv, d, kv, bt, cu, sl, ref, d ** -0.5, window, max(q_lens), max(seq_lens))
+    torch.testing.assert_close(out.cpu(), ref, rtol=1e-4, atol=1e-5)
+    for r, at in [(0, 0), (0, 31), (1, 0), (2, 1), (3, 66)]:
+        row, p = int(cu[r]) + at, seq_lens[r] - q_lens[r] + at
+        later = kv.clone()
+        for q in range(p + 1, seq_lens[r]):                      # the request's later tokens are not there yet
+            later[int(bt[r, q // ps]), :, :, q % ps] = float("nan")
+        alone = torch.empty((1, nq * d), device="cuda")
+        K.paged_attention(qkv[row:row + 1].cuda(), nq, nkv, d, later.cuda(), bt[r:r + 1].cuda(), torch.tensor([0, 1], dtype=torch.int32).cuda(),
+                          torch.tensor([p + 1], dtype=torch.int32).cuda(), alone, d ** -0.5, window, 1, p + 1)
+        assert torch.equal(alone[0], out[row])
+
