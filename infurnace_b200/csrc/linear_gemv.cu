@@ -92,7 +92,8 @@ __device__ __forceinline__ void gv_cluster_barrier() {
 // 2: a warp walks a long k range and keeps the memory pipe full while it multiplies (large models, where the
 // bytes count).
 template <int NB, int EPI, int WARPS, typename TO, int STAGES>
-__global__ void __launch_bounds__(WARPS * 32, (EPI == 4 && WARPS == 8) ? 2 : (EPI == 0 && WARPS == 8 && STAGES == 1 && NB == 1) ? IFB_GV_LM_BLOCKS : 0)
+__global__ void __launch_bounds__(WARPS * 32, (EPI == 4 && WARPS == 8) ? 2 : (EPI == 0 && WARPS == 8 && STAGES == 1 && NB == 1) ? IFB_GV_LM_BLOCKS
+                                  : (EPI == 2 && NB == 1 && WARPS <= 16 && (WARPS == 16 || STAGES == 2)) ? 2 : 0)
 linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* __restrict__ out, int n_rows, int o_out,
                    int k_dim, GvRowScale rs, GvResidual res, GvQkv qk) {
   extern __shared__ float gv_red[];                 // [WARPS][NE][NB*8][GV_ROWS], then [NB*8] row factors
@@ -136,6 +137,31 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
 #pragma unroll
     for (int j = 0; j < NB; ++j) acc[e][j][0] = acc[e][j][1] = acc[e][j][2] = acc[e][j][3] = 0.f;
 
+  // What the epilogue reads for this thread's (first) item is requested with the operands, not after the products: norm
+  // weights (constants, which come from memory behind the weights of this and the next kernel) before the wait, the
+  // stream's element, the angles and the place in the pages after it.
+  const int item_n = tid / GV_ROWS, item_m = tid % GV_ROWS, item_tok = n0 + item_n, item_o = o0 + item_m;
+  const bool item = tid < NB * 8 * GV_ROWS && item_tok < n_rows;
+  float pre_a = 1.f, pre_b = 1.f, pre_x = 0.f;
+  float2 pre_cs = make_float2(1.f, 0.f);
+  int pre_slot = -1;
+  const bool qk_is_v = EPI == 3 && qk_head >= qk.nq + qk.nkv, qk_is_k = EPI == 3 && qk_head >= qk.nq && !qk_is_v;
+  const void* qk_nw = EPI != 3 || qk_is_v ? nullptr : qk_is_k ? qk.kw : qk.qw;
+  auto request_constants = [&]() {
+    if (EPI == 2 && item && item_o < o_out && (!half_tile || item_m < 8)) pre_a = load_as_f32(res.g, res.g_dtype, item_o);
+    if (EPI == 3 && item && qk_nw) {
+      pre_a = load_as_f32(qk_nw, qk.w_dtype, qk_c * GV_ROWS + item_m);
+      pre_b = load_as_f32(qk_nw, qk.w_dtype, qk_c * GV_ROWS + item_m + qk.head_dim / 2);
+    }
+  };
+  auto request_item = [&]() {
+    if (EPI == 2 && item && item_o < o_out && (!half_tile || item_m < 8)) pre_x = res.x[(size_t)item_tok * o_out + item_o];
+    if (EPI == 3 && item) {
+      if (!qk_is_v && qk.rope) pre_cs = qk.rope[(size_t)item_tok * (qk.head_dim / 2) + qk_c * GV_ROWS + item_m];
+      if ((qk_is_v || qk_is_k) && qk.slots) pre_slot = qk.slots[item_tok];
+    }
+  };
+
   if constexpr (STAGES == 1) {
     // every warp's k range is (mostly) one step: weights requested, then the wait for whoever writes x, then the products
     bool waited = false;
@@ -152,9 +178,11 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
         }
       }
       if (!waited) {           // the weights are on their way; now wait for whoever writes x
+        request_constants();
         ifb_pdl_wait();
         ifb_pdl_trigger();
         waited = true;
+        request_item();
         if (rs.partials) {     // the rows' factors, requested now and used after the products
           for (int n = warp; n < NB * 8; n += WARPS) {
             float ssum = 0.f;
@@ -240,7 +268,9 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
     // the first weights are on their way before this kernel waits for whoever writes x
   #pragma unroll
     for (int st = 0; st < STAGES; ++st) load_w(st, kbeg + st * 128);
+    request_constants();
     ifb_pdl_wait();
+    request_item();
   #pragma unroll
     for (int st = 0; st < STAGES; ++st) load_x(st, kbeg + st * 128);
     if (rs.partials) {     // the rows' factors, requested now and used after the products
@@ -315,9 +345,9 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
     if (EPI == 2) {
       float v = 0.f;
       if (valid) {
-        v = res.x[(size_t)tok * o_out + o] + r;
+        v = (idx == tid ? pre_x : res.x[(size_t)tok * o_out + o]) + r;
         res.x[(size_t)tok * o_out + o] = v;
-        out[(size_t)tok * o_out + o] = from_f32<TO>(v * load_as_f32(res.g, res.g_dtype, o));
+        out[(size_t)tok * o_out + o] = from_f32<TO>(v * (idx == tid ? pre_a : load_as_f32(res.g, res.g_dtype, o)));
       }
       float sq = v * v;                              // the sum over this CTA's 16 features, in a fixed order
       sq += __shfl_xor_sync(0xffffffffu, sq, 8);
@@ -333,9 +363,8 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
   if (EPI == 3) {
     __shared__ float qk_ssq[8][NB * 8];                 // [CTA of the head][token]: sums of squares over 32 features
     const bool mine = tid < NB * 8 * GV_ROWS;           // this thread holds the pair (m, m + head_dim/2) of token n
-    const int n = tid / GV_ROWS, m = tid % GV_ROWS, tok = n0 + n;
-    const bool is_v = qk_head >= qk.nq + qk.nkv, is_k = qk_head >= qk.nq && !is_v;
-    const void* nw = is_v ? nullptr : (is_k ? qk.kw : qk.qw);
+    const int n = item_n, m = item_m, tok = item_tok;
+    const bool is_v = qk_is_v;
     const uint32_t rank = gv_cluster_rank(), peers = gv_cluster_size();
     float sq = mine ? qk_y0 * qk_y0 + qk_y1 * qk_y1 : 0.f;
     sq += __shfl_xor_sync(0xffffffffu, sq, 8);
@@ -348,15 +377,15 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
     if (!mine || tok >= n_rows) return;
     const int D = qk.head_dim, half = D / 2, i = qk_c * GV_ROWS + m;
     float a = qk_y0, b = qk_y1;
-    if (nw) {
+    if (qk_nw) {
       float total = 0.f;
       for (uint32_t p = 0; p < peers; ++p) total += qk_ssq[p][n];      // in a fixed order
       const float rn = rsqrtf(total / (float)D + qk.eps);
-      a *= rn * load_as_f32(nw, qk.w_dtype, i);
-      b *= rn * load_as_f32(nw, qk.w_dtype, i + half);
+      a *= rn * pre_a;
+      b *= rn * pre_b;
     }
     if (!is_v && qk.rope) {
-      const float2 cs = qk.rope[(size_t)tok * half + i];
+      const float2 cs = pre_cs;
       const float ra = a * cs.x - b * cs.y, rb = b * cs.x + a * cs.y;
       a = ra; b = rb;
     }
@@ -365,7 +394,7 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
     row[i] = oa;
     row[i + half] = ob;
     if (qk_head >= qk.nq && qk.slots) {
-      const int slot = qk.slots[tok];
+      const int slot = pre_slot;
       if (slot >= 0) {
         const int kvh = is_v ? qk_head - qk.nq - qk.nkv : qk_head - qk.nq;
         bf16* dst = qk.pages + ((((size_t)(slot / qk.page_size) * 2 + (is_v ? 1 : 0)) * qk.nkv + kvh) * qk.page_size +
