@@ -46,6 +46,7 @@ template <int EPI_, int MH_, int NACC_, int STAGES_> struct GemmCfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int TMEM_COLS = MH * NACC;                 // 128, 256 or 512 columns of 32 bits
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /* alignment */ + 256 /* barriers */;
+  static constexpr bool SHARED_K = MH == 1 && 2 * SMEM_BYTES > 226 * 1024;      // the deep shapes: the k range may be shared by a cluster
   // float32 accumulator, bfloat16 a and b, both K-major, M = 128, N = NACC
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NACC >> 3) << 17) | ((uint32_t)(G_BM >> 4) << 24);
 };
@@ -138,6 +139,8 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, int rank) {
   return v;
 }
 
+template <int N> struct TcInt { static constexpr int value = N; };
+
 // Shared-memory matrix descriptor of a K-major tile in the 128-byte swizzle: rows of 128 bytes, groups of 8
 // rows 1024 bytes apart (stride byte offset), leading byte offset unused (1), descriptor version 1.
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
@@ -166,9 +169,10 @@ struct TcFold {
   float* res_partials;        // [parts][n_rows], written; what a part covers depends on the launch (tc_fold_parts)
   int unary;                  // without res_x: the function of common.cuh applied to every element (0: none), or to the gates (0: silu)
   const float* bias;          // plain epilogue: [o_out], added to the product before the unary function (null: none)
-  // The product is the fused q | k | v projection of an attention layer with heads of 128, in the shared-k form, whose
-  // tile of 128 features is one head: the sum over the cluster finishes what follows the projection (RMSNorm over the q
-  // and k heads, rotation in the half-split pairing, q to its row, k and v to the token's place in the pages).
+  // The product is the fused q | k | v projection of an attention layer with heads of 128; a tile's 128 features (or each
+  // 128 of its 256) are one head: the epilogue, or the sum over the cluster in the shared-k form, finishes what follows the
+  // projection (RMSNorm over the q and k heads, rotation in the half-split pairing, q to its row, k and v to the token's
+  // place in the pages).
   int qk_nq, qk_nkv;          // qk_nq > 0: on
   const void* qk_qw;          // [128] norm weights (null: no norm)
   const void* qk_kw;
@@ -221,8 +225,174 @@ __device__ __forceinline__ float tc_residual_chunk(const TcFold& f, float (&y)[3
   return ss;
 }
 
+// 32 columns of the accumulator (a lane's row of them) times `f`, as float32 at `dst`.
+__device__ __forceinline__ void tc_stage_rows(uint32_t taddr, unsigned char* dst, float f) {
+  uint32_t v[32];
+  tmem_ld32(taddr, v);
+  tmem_ld_wait();
+#pragma unroll
+  for (int j = 0; j < 32; j += 4)
+    *reinterpret_cast<float4*>(dst + j * 4) = make_float4(__uint_as_float(v[j]) * f, __uint_as_float(v[j + 1]) * f,
+                                                          __uint_as_float(v[j + 2]) * f, __uint_as_float(v[j + 3]) * f);
+}
+// The end of a product with the residual addition, for a warp's 32 rows of CW features: v = x + y goes back to x, v * g to
+// `out`, the sum of v^2 over the CW features to its part.  CW / 4 lanes share a row, so every access of the stream is a whole
+// row segment (a lane with a row of its own touches 32 rows per instruction: for a prompt of 2,048 rows that epilogue cost
+// what the separate norm did).  Eight warps per SM hide no latency by themselves, so the stream's rows are requested AHEAD
+// passes at a time, the first of them before the product is there.
+template <int CW, int AHEAD>
+__device__ __forceinline__ void tc_residual_load(const TcFold& f, int row0, int n_rows, int col0, int o_out, int lane, float4 (&xv)[AHEAD]) {
+  constexpr int LPR = CW / 4, RPP = 32 / LPR;
+#pragma unroll
+  for (int a = 0; a < AHEAD; ++a) {
+    const int row = row0 + a * RPP + lane / LPR;
+    xv[a] = row < n_rows ? *reinterpret_cast<const float4*>(f.res_x + (size_t)row * o_out + col0 + (lane % LPR) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+}
+// `xv`: the first AHEAD passes' rows, requested by the caller before it waited for the product.
+template <int CW, int PITCH, int AHEAD, typename TO>
+__device__ __forceinline__ void tc_finish_residual(const TcFold& f, const unsigned char* rows32, TO* out, int row0, int n_rows, int col0,
+                                                   int o_out, int part, int lane, float4 (&xv)[AHEAD]) {
+  constexpr int LPR = CW / 4, RPP = 32 / LPR;
+  static_assert(32 % (RPP * AHEAD) == 0, "whole batches of passes");
+  const int sub = lane / LPR, c = (lane % LPR) * 4;
+  const bool whole = (((uintptr_t)out) & (4 * sizeof(TO) - 1)) == 0;
+  float g[4], bias[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    g[j] = load_as_f32(f.res_g, f.res_g_dtype, col0 + c + j);
+    bias[j] = f.bias ? __ldg(f.bias + col0 + c + j) : 0.f;
+  }
+  constexpr int GROUP = 4;                                       // passes whose reads precede all their stores
+  static_assert(AHEAD % GROUP == 0, "whole groups");
+#pragma unroll 1
+  for (int r0 = 0; r0 < 32; r0 += RPP * AHEAD) {
+    if (row0 + r0 >= n_rows) break;                              // warp-uniform
+    if (r0) tc_residual_load<CW, AHEAD>(f, row0 + r0, n_rows, col0, o_out, lane, xv);
+#pragma unroll
+    for (int a0 = 0; a0 < AHEAD; a0 += GROUP) {
+      float4 v[GROUP];
+      float ss[GROUP];
+#pragma unroll
+      for (int a = 0; a < GROUP; ++a) v[a] = *reinterpret_cast<const float4*>(rows32 + (r0 + (a0 + a) * RPP + sub) * PITCH + c * 4);
+#pragma unroll
+      for (int a = 0; a < GROUP; ++a) {
+        const float4 x = xv[a0 + a];
+        v[a] = make_float4(x.x + (v[a].x + bias[0]), x.y + (v[a].y + bias[1]), x.z + (v[a].z + bias[2]), x.w + (v[a].w + bias[3]));
+        ss[a] = v[a].x * v[a].x + v[a].y * v[a].y + v[a].z * v[a].z + v[a].w * v[a].w;
+      }
+#pragma unroll
+      for (int d = LPR / 2; d > 0; d >>= 1)
+#pragma unroll
+        for (int a = 0; a < GROUP; ++a) ss[a] += __shfl_xor_sync(0xffffffffu, ss[a], d);
+#pragma unroll
+      for (int a = 0; a < GROUP; ++a) {
+        const int row = row0 + r0 + (a0 + a) * RPP + sub;
+        if (row < n_rows) {
+          *reinterpret_cast<float4*>(f.res_x + (size_t)row * o_out + col0 + c) = v[a];
+          TO* dst = out + (size_t)row * o_out + col0 + c;
+          const float h[4] = {v[a].x * g[0], v[a].y * g[1], v[a].z * g[2], v[a].w * g[3]};
+          if (!whole) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dst[j] = from_f32<TO>(h[j]);
+          } else if (sizeof(TO) == 2) {
+            __nv_bfloat162 lo = __floats2bfloat162_rn(h[0], h[1]), hi = __floats2bfloat162_rn(h[2], h[3]);
+            *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+          } else {
+            *reinterpret_cast<float4*>(dst) = make_float4(h[0], h[1], h[2], h[3]);
+          }
+          if (lane % LPR == 0) f.res_partials[(size_t)part * n_rows + row] = ss[a];
+        }
+      }
+    }
+  }
+}
+// The end of the fused q | k | v projection for a warp's 32 tokens and NP of the 64 rotation pairs of one head (elements
+// i0 .. i0 + NP - 1 and their partners 64 further on, staged one after the other, already divided by the head's rms): norm
+// weight, rotation, the head's row of `out`, and for k and v heads the token's place in the pages.  NP / 4 lanes share a token.
+template <int NP, int AHEAD>
+__device__ __forceinline__ void tc_heads_load(const TcFold& f, int row0, int n_rows, int i0, bool rotate, bool store, int lane,
+                                              float4 (&cs)[AHEAD][2], int (&slot)[AHEAD]) {
+  constexpr int LPR = NP / 4, RPP = 32 / LPR;
+#pragma unroll
+  for (int a = 0; a < AHEAD; ++a) {
+    const int row = row0 + a * RPP + lane / LPR;
+    const float4* t = reinterpret_cast<const float4*>(f.qk_rope + (size_t)row * 64 + i0 + (lane % LPR) * 4);
+    const bool in = rotate && row < n_rows;
+    cs[a][0] = in ? __ldg(t) : make_float4(1.f, 0.f, 1.f, 0.f);
+    cs[a][1] = in ? __ldg(t + 1) : make_float4(1.f, 0.f, 1.f, 0.f);
+    slot[a] = store && row < n_rows ? __ldg(f.qk_slots + row) : -1;
+  }
+}
+// `cs`, `slot`: the first AHEAD passes' angles and places, requested by the caller before it waited for the product.
+template <int NP, int PITCH, int AHEAD>
+__device__ __forceinline__ void tc_finish_heads(const TcFold& f, const unsigned char* rows32, bf16* out, int row0, int n_rows, int head,
+                                                int i0, int o_out, const void* wn, bool is_v, bool rotate, bool store, int lane,
+                                                float4 (&cs)[AHEAD][2], int (&slot)[AHEAD]) {
+  constexpr int LPR = NP / 4, RPP = 32 / LPR, GROUP = 2;         // passes whose reads precede all their stores
+  static_assert(32 % (RPP * AHEAD) == 0 && AHEAD % GROUP == 0, "whole batches of passes, whole groups");
+  const int sub = lane / LPR, p = (lane % LPR) * 4, i = i0 + p;
+  float wa[4] = {1.f, 1.f, 1.f, 1.f}, wb[4] = {1.f, 1.f, 1.f, 1.f};
+  if (wn) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { wa[j] = load_as_f32(wn, f.qk_w_dtype, i + j); wb[j] = load_as_f32(wn, f.qk_w_dtype, 64 + i + j); }
+  }
+  const int kvh = is_v ? head - f.qk_nq - f.qk_nkv : head - f.qk_nq;
+  const int ps_shift = (f.qk_page_size & (f.qk_page_size - 1)) ? -1 : __ffs(f.qk_page_size) - 1;
+#pragma unroll 1
+  for (int r0 = 0; r0 < 32; r0 += RPP * AHEAD) {
+    if (row0 + r0 >= n_rows) break;                              // warp-uniform
+    if (r0) tc_heads_load<NP, AHEAD>(f, row0 + r0, n_rows, i0, rotate, store, lane, cs, slot);
+#pragma unroll
+    for (int a0 = 0; a0 < AHEAD; a0 += GROUP) {
+      float4 x[GROUP], y[GROUP];
+#pragma unroll
+      for (int a = 0; a < GROUP; ++a) {
+        const unsigned char* at = rows32 + (r0 + (a0 + a) * RPP + sub) * PITCH + p * 4;
+        x[a] = *reinterpret_cast<const float4*>(at);
+        y[a] = *reinterpret_cast<const float4*>(at + NP * 4);
+      }
+      uint2 lo[GROUP], hi[GROUP];
+#pragma unroll
+      for (int a = 0; a < GROUP; ++a) {
+        const float4 c0 = cs[a0 + a][0], c1 = cs[a0 + a][1];
+        const float u[4] = {x[a].x * wa[0], x[a].y * wa[1], x[a].z * wa[2], x[a].w * wa[3]};
+        const float v[4] = {y[a].x * wb[0], y[a].y * wb[1], y[a].z * wb[2], y[a].w * wb[3]};
+        const float co[4] = {c0.x, c0.z, c1.x, c1.z}, si[4] = {c0.y, c0.w, c1.y, c1.w};
+        float s[4], t[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s[j] = rotate ? u[j] * co[j] - v[j] * si[j] : u[j];
+          t[j] = rotate ? v[j] * co[j] + u[j] * si[j] : v[j];
+        }
+        const __nv_bfloat162 s0 = __floats2bfloat162_rn(s[0], s[1]), s1 = __floats2bfloat162_rn(s[2], s[3]);
+        const __nv_bfloat162 t0 = __floats2bfloat162_rn(t[0], t[1]), t1 = __floats2bfloat162_rn(t[2], t[3]);
+        lo[a] = make_uint2(*reinterpret_cast<const uint32_t*>(&s0), *reinterpret_cast<const uint32_t*>(&s1));
+        hi[a] = make_uint2(*reinterpret_cast<const uint32_t*>(&t0), *reinterpret_cast<const uint32_t*>(&t1));
+      }
+#pragma unroll
+      for (int a = 0; a < GROUP; ++a) {
+        const int row = row0 + r0 + (a0 + a) * RPP + sub, sl = slot[a0 + a];
+        if (row < n_rows) {
+          bf16* dst = out + (size_t)row * o_out + head * 128 + i;
+          *reinterpret_cast<uint2*>(dst) = lo[a];
+          *reinterpret_cast<uint2*>(dst + 64) = hi[a];
+        }
+        if (sl >= 0) {
+          const int page = ps_shift >= 0 ? sl >> ps_shift : sl / f.qk_page_size;
+          const size_t at = ((size_t)page * 2 + (is_v ? 1 : 0)) * f.qk_nkv + kvh;
+          bf16* pg = f.qk_pages + (at * f.qk_page_size + sl - page * f.qk_page_size) * 128 + i;
+          *reinterpret_cast<uint2*>(pg) = lo[a];
+          *reinterpret_cast<uint2*>(pg + 64) = hi[a];
+        }
+      }
+    }
+  }
+}
+
+// (CTAs per SM by shared memory: left to itself the compiler aims for more and takes 64 registers, with spills)
 template <typename Cfg, typename TO>
-__global__ void __launch_bounds__(G_THREADS)
+__global__ void __launch_bounds__(G_THREADS, 2 * Cfg::SMEM_BYTES <= 226 * 1024 ? 2 : 1)
 linear_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                       TO* __restrict__ out, int n_rows, int o_out, int k_dim, int* __restrict__ err,
                       int splits, TcFold fold) {
@@ -265,6 +435,21 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+
+  // What the sum over the cluster multiplies and adds per feature (a lane's four, the same for every row) is requested here:
+  // requested behind the products it would come from memory after the weights of the next kernel.
+  const int sum_c = lane * 4, qk_head = blockIdx.x;
+  const bool qk_v = qk_head >= fold.qk_nq + fold.qk_nkv, qk_k = qk_head >= fold.qk_nq && !qk_v;
+  const void* wn = fold.res_x ? fold.res_g : !fold.qk_nq || qk_v ? nullptr : qk_k ? fold.qk_kw : fold.qk_qw;
+  float wv[4] = {1.f, 1.f, 1.f, 1.f}, bv[4] = {0.f, 0.f, 0.f, 0.f};
+  if (Cfg::SHARED_K && !EPI && splits > 1) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (wn && n0 + sum_c + j < o_out)
+        wv[j] = load_as_f32(wn, fold.res_x ? fold.res_g_dtype : fold.qk_w_dtype, (size_t)(fold.res_x ? n0 : 0) + sum_c + j);
+      if (fold.bias && n0 + sum_c + j < o_out) bv[j] = __ldg(fold.bias + n0 + sum_c + j);
+    }
+  }
 
   if (warp == 0) {
     // The first fill of the stages: the w tiles, which no kernel of the step writes, are requested before this kernel
@@ -337,16 +522,85 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
     static_assert(8 * 32 * PITCH <= Cfg::STAGES * Cfg::STAGE_BYTES, "the staging rows must fit in the stages");
     const int q = warp & 3;                                      // this warp's quarter of the 128 lanes
     const int c_lo = ((warp - 2) >> 2) * CW;                     // and its half of the tile's features
+    // What reads or finishes whole rows of float32 (tc_finish_residual, tc_finish_heads) gets its piece in float32 rows.
+    const bool finish_res = !EPI && splits == 1 && fold.res_x && (o_out & 3) == 0 && n0 + c_lo + CW <= o_out;
+    const bool finish_qk = !EPI && sizeof(TO) == 2 && splits == 1 && fold.qk_nq;
+    constexpr int FPITCH = CW * 4 + 16;                          // bytes of a float32 row, padded
+    static_assert(EPI || 8 * 32 * FPITCH <= Cfg::STAGES * Cfg::STAGE_BYTES, "the float32 rows must fit in the stages");
+    // What the epilogue reads beside the product is requested while the product is being made.
+    constexpr int AHEAD = (CW == 64 && Cfg::STAGES == 3) ? 8 : 16;       // (two CTAs per SM: half the registers)
+    constexpr int AHEAD_H = AHEAD / 2;                           // passes over heads: twice the angles each
+    float rfac_of[MH];
+    float4 ahead[EPI ? 1 : AHEAD], angles[EPI ? 1 : AHEAD_H][2];      // rows of the stream, or angles
+    int slot_of[EPI ? 1 : AHEAD_H];
+    // finish_qk: CW 128: the warp has a head of its own; CW 64: the pairs [32 c, 32 c + 32) of the tile's one head
+    const int qk_base = CW == 128 ? c_lo : 0, qk_i0 = CW == 128 ? 0 : c_lo / 2, qk_head = (n0 + qk_base) / 128;
+    const bool qk_v = qk_head >= fold.qk_nq + fold.qk_nkv, qk_k = qk_head >= fold.qk_nq && !qk_v;
+    const bool qk_rotate = finish_qk && !qk_v && fold.qk_rope, qk_store = finish_qk && (qk_v || qk_k) && fold.qk_slots;
+    if (fold.rs_partials || fold.res_x || fold.qk_nq) ifb_pdl_wait();             // what the predecessor wrote is read here directly
+#pragma unroll
+    for (int hf = 0; hf < MH; ++hf) rfac_of[hf] = tc_row_factor(fold, m0 + hf * G_BM + q * 32 + lane, n_rows);
+    if constexpr (!EPI) {
+      if (finish_res) tc_residual_load<CW, AHEAD>(fold, m0 + q * 32, n_rows, n0 + c_lo, o_out, lane, ahead);
+      else if (finish_qk) tc_heads_load<CW / 2, AHEAD_H>(fold, m0 + q * 32, n_rows, qk_i0, qk_rotate, qk_store, lane, angles, slot_of);
+    }
     if (kblocks > 0 && mbar_wait(accum, 0, abort_flag, err, 3)) {
       tc_fence_after();
-      if (fold.rs_partials || fold.res_x) ifb_pdl_wait();         // what the predecessor wrote is read here directly
+     if constexpr (!EPI) {
+      if (finish_res || finish_qk) {
+        unsigned char* rows32 = smem + (warp - 2) * (32 * FPITCH);
+#pragma unroll
+        for (int hf = 0; hf < MH; ++hf) {
+          const int row0 = m0 + hf * G_BM + q * 32;
+          if (row0 >= n_rows) break;                             // warp-uniform
+          const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16) + hf * NACC;
+          float rfac = rfac_of[hf];
+          if (finish_res) {
+            if (hf) tc_residual_load<CW, AHEAD>(fold, row0, n_rows, n0 + c_lo, o_out, lane, ahead);
+#pragma unroll 1
+            for (int c0 = 0; c0 < CW; c0 += 32) tc_stage_rows(lane_base + c_lo + c0, rows32 + lane * FPITCH + c0 * 4, rfac);
+            __syncwarp();
+            tc_finish_residual<CW, FPITCH, AHEAD, TO>(fold, rows32, out, row0, n_rows, n0 + c_lo, o_out,
+                                                      blockIdx.x * 2 + (c_lo ? 1 : 0), lane, ahead);
+          } else if constexpr (sizeof(TO) == 2) {
+            if (n0 + qk_base < o_out) {
+              if (hf) tc_heads_load<CW / 2, AHEAD_H>(fold, row0, n_rows, qk_i0, qk_rotate, qk_store, lane, angles, slot_of);
+              const void* wn = qk_v ? nullptr : qk_k ? fold.qk_kw : fold.qk_qw;
+              if (wn) {
+                float ss = 0.f;
+#pragma unroll 1
+                for (int c0 = 0; c0 < 128; c0 += 32) {
+                  uint32_t v[32];
+                  tmem_ld32(lane_base + qk_base + c0, v);
+                  tmem_ld_wait();
+#pragma unroll
+                  for (int j = 0; j < 32; ++j) { const float f = __uint_as_float(v[j]) * rfac; ss = fmaf(f, f, ss); }
+                }
+                rfac *= rsqrtf(ss * (1.f / 128.f) + fold.qk_eps);
+              }
+              constexpr int NP = CW / 2;                         // pairs of the warp
+#pragma unroll 1
+              for (int c0 = 0; c0 < NP; c0 += 32) {
+                tc_stage_rows(lane_base + qk_base + qk_i0 + c0, rows32 + lane * FPITCH + c0 * 4, rfac);
+                tc_stage_rows(lane_base + qk_base + 64 + qk_i0 + c0, rows32 + lane * FPITCH + (NP + c0) * 4, rfac);
+              }
+              __syncwarp();
+              tc_finish_heads<NP, FPITCH, AHEAD_H>(fold, rows32, reinterpret_cast<bf16*>(out), row0, n_rows, qk_head, qk_i0, o_out, wn, qk_v,
+                                                   qk_rotate, qk_store, lane, angles, slot_of);
+            }
+          }
+          __syncwarp();                                          // before the next rows overwrite the buffer
+        }
+      }
+     }
+     if (!finish_res && !finish_qk) {
       const bool vec = ((size_t)o_out * sizeof(TO)) % 16 == 0 && (((uintptr_t)out) & 15) == 0 && n0 + c_lo + CW <= o_out;
       unsigned char* buf = smem + (warp - 2) * (32 * PITCH);
 #pragma unroll 1
       for (int hf = 0; hf < MH; ++hf) {
         const int row0 = m0 + hf * G_BM + q * 32;
         const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16) + hf * NACC;
-        const float rfac = tc_row_factor(fold, row0 + lane, n_rows);
+        const float rfac = MH == 1 || hf == 0 ? rfac_of[0] : rfac_of[MH - 1];
         float ss = 0.f;                                          // this row's v^2 over this warp's features
 #pragma unroll 1
        for (int p0 = c_lo; p0 < c_lo + CW; p0 += PW) {
@@ -439,113 +693,163 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
        if (!EPI && splits == 1 && fold.res_x && row0 + lane < n_rows)
          fold.res_partials[(size_t)(blockIdx.x * 2 + (c_lo ? 1 : 0)) * n_rows + row0 + lane] = ss;
       }
+     }
     }
   }
-  if (splits > 1) {
-    cluster_sync_all();                        // every CTA's part is in its shared memory
-    if (fold.res_x || fold.qk_nq) ifb_pdl_wait();
-    const int rows = min(G_BM, n_rows - m0), cols = min(FO, o_out - n0);
-    const int used = (kb_all + kb_per - 1) / kb_per;                       // CTAs that had k blocks
-    const int per = (rows + splits - 1) / splits;
-    const int r_lo = blockIdx.z * per, r_hi = min(rows, r_lo + per);
-    const bool vec = ((size_t)o_out * sizeof(TO)) % 16 == 0 && (((uintptr_t)out) & 15) == 0 && cols == FO;
-    const uint32_t tile_addr = g_smem_u32(smem);
-    for (int i = threadIdx.x; i < (r_hi - r_lo) * (FO / 4); i += G_THREADS) {
-      const int r = r_lo + i / (FO / 4), c = (i % (FO / 4)) * 4;
-      const uint32_t at = tile_addr + (uint32_t)((r * RED_PITCH + c) * 4);
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int z = 0; z < used; ++z) {
-        const float4 v = ld_cluster_f4(at, z);
-        acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-      }
-      if (EPI) {
-        float4 up = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int z = 0; z < used; ++z) {
-          const float4 v = ld_cluster_f4(at + FO * 4, z);
-          up.x += v.x; up.y += v.y; up.z += v.z; up.w += v.w;
-        }
-        acc.x = tc_gate(acc.x, fold.unary) * up.x; acc.y = tc_gate(acc.y, fold.unary) * up.y;
-        acc.z = tc_gate(acc.z, fold.unary) * up.z; acc.w = tc_gate(acc.w, fold.unary) * up.w;
-      }
-      TO* dst = out + (size_t)(m0 + r) * o_out + n0 + c;
-      if (!EPI && fold.bias) {
-        const float* bp = fold.bias + n0 + c;
-        if (c < cols) acc.x += __ldg(bp);
-        if (c + 1 < cols) acc.y += __ldg(bp + 1);
-        if (c + 2 < cols) acc.z += __ldg(bp + 2);
-        if (c + 3 < cols) acc.w += __ldg(bp + 3);
-      }
-      if (!EPI && fold.unary) {
-        acc.x = ifb_unary(acc.x, fold.unary); acc.y = ifb_unary(acc.y, fold.unary);
-        acc.z = ifb_unary(acc.z, fold.unary); acc.w = ifb_unary(acc.w, fold.unary);
-      }
-      if (!EPI && fold.res_x) {
-        // a warp holds one row of the tile: v = x + y, x <- v, the output becomes v * g, the warp's sum of v^2 one part
-        float* xr = fold.res_x + (size_t)(m0 + r) * o_out + n0 + c;
-        float yv[4] = {acc.x, acc.y, acc.z, acc.w}, ss = 0.f;
+  if constexpr (Cfg::SHARED_K) {
+    if (splits > 1) {
+      // The sum over the cluster: a warp adds a row of the tile at a time (a lane four features), from the row of each CTA
+      // that had k blocks.  What bounds it is the round trip to the other CTAs' shared memory and the code's first run: the parts
+      // of a row, and what else the epilogue reads for it, are requested before the first is used, but no more than two rows
+      // at a time (with two and four rows unrolled a decode step of 64 rows of the 0.6B sizes took 1.73 ms, with one and two 1.64;
+      // with the parts added one round trip after the other 1.67, and a prompt of 131 tokens 1.50 ms for 1.24).
+      static_assert(FO == 128, "a lane of the sum has four of a row's features");
+      constexpr int PARTS = EPI ? 2 : 1, ROWS_OF_8 = 1, ROWS_OF_4 = 2, WARPS = G_THREADS / 32;
+      const int c = sum_c;
+      const int rows = min(G_BM, n_rows - m0), cols = min(FO, o_out - n0);
+      const int used = (kb_all + kb_per - 1) / kb_per;                     // CTAs that had k blocks
+      const int per = (rows + splits - 1) / splits;
+      const int r_lo = blockIdx.z * per + warp, r_hi = min(rows, ((int)blockIdx.z + 1) * per);
+      const bool vec = ((size_t)o_out * sizeof(TO)) % 16 == 0 && (((uintptr_t)out) & 15) == 0 && cols == FO;
+      cluster_sync_all();                      // every CTA's part is in its shared memory
+      if (fold.res_x || fold.qk_nq) ifb_pdl_wait();
+      const uint32_t tile_addr = g_smem_u32(smem);
+      auto run = [&](auto z_max, auto rows_ahead) {
+        constexpr int Z = decltype(z_max)::value, B = decltype(rows_ahead)::value;
+        for (int rb = r_lo;; rb += B * WARPS) {
+          float4 v[B][PARTS][Z], xr[EPI ? 1 : B], cs[EPI ? 1 : B][2];
+          int slot[EPI ? 1 : B];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (c + j < cols) {
-            const float v = xr[j] + yv[j];
-            xr[j] = v;
-            ss += v * v;
-            yv[j] = v * load_as_f32(fold.res_g, fold.res_g_dtype, n0 + c + j);
+          for (int b = 0; b < B; ++b) {
+            const int r = rb + b * WARPS;
+            const uint32_t at = tile_addr + (uint32_t)((r * RED_PITCH + c) * 4);
+#pragma unroll
+            for (int e = 0; e < PARTS; ++e)
+#pragma unroll
+              for (int z = 0; z < Z; ++z)
+                v[b][e][z] = r < r_hi && z < used ? ld_cluster_f4(at + e * FO * 4, z) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (!EPI && fold.res_x) {
+              const float* x = fold.res_x + (size_t)(m0 + r) * o_out + n0 + c;
+              if (r >= r_hi) xr[b] = make_float4(0.f, 0.f, 0.f, 0.f);
+              else if (cols == FO && (o_out & 3) == 0) xr[b] = *reinterpret_cast<const float4*>(x);
+              else xr[b] = make_float4(c < cols ? x[0] : 0.f, c + 1 < cols ? x[1] : 0.f, c + 2 < cols ? x[2] : 0.f, c + 3 < cols ? x[3] : 0.f);
+            }
+            if (!EPI && fold.qk_nq) {
+              const bool turn = !qk_v && fold.qk_rope && r < r_hi;
+              const float4* t = reinterpret_cast<const float4*>(fold.qk_rope + (size_t)(m0 + r) * 64 + (c & 63));
+              cs[b][0] = turn ? __ldg(t) : make_float4(1.f, 0.f, 1.f, 0.f);
+              cs[b][1] = turn ? __ldg(t + 1) : make_float4(1.f, 0.f, 1.f, 0.f);
+              slot[b] = (qk_v || qk_k) && fold.qk_slots && r < r_hi ? __ldg(fold.qk_slots + m0 + r) : -1;
+            }
+          }
+          float4 sum[B][PARTS];
+#pragma unroll
+          for (int b = 0; b < B; ++b)
+#pragma unroll
+            for (int e = 0; e < PARTS; ++e) {
+              float4 t = make_float4(0.f, 0.f, 0.f, 0.f);                  // in the order of the CTAs
+#pragma unroll
+              for (int z = 0; z < Z; ++z)
+                if (z < used) { t.x += v[b][e][z].x; t.y += v[b][e][z].y; t.z += v[b][e][z].z; t.w += v[b][e][z].w; }
+              sum[b][e] = t;
+            }
+          const bool last = rb + B * WARPS >= r_hi;
+          // this warp has read all it reads of the other CTAs' shared memory (and has stored nothing of its own yet that the
+          // release would have to wait for, where one batch of rows is all)
+          if (last) {
+            // (the vote makes the arrival wait for every value read; it needs no release, which would wait for more)
+            float all = 0.f;
+#pragma unroll
+            for (int b = 0; b < B; ++b)
+#pragma unroll
+              for (int e = 0; e < PARTS; ++e) all += sum[b][e].x;
+            const int votes = __popc(__ballot_sync(0xffffffffu, all != 0.f));
+            asm volatile("{\n .reg .pred p;\n setp.ge.s32 p, %0, 0;\n @p barrier.cluster.arrive.relaxed.aligned;\n}\n" ::"r"(votes) : "memory");
           }
 #pragma unroll
-        for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-        if ((threadIdx.x & 31) == 0) fold.res_partials[(size_t)blockIdx.x * n_rows + m0 + r] = ss;
-        acc = make_float4(yv[0], yv[1], yv[2], yv[3]);
-      }
-      if (!EPI && sizeof(TO) == 2 && fold.qk_nq) {
-        // a warp holds one head of one token (lane l its elements 4l .. 4l + 3; the rotation partner 16 lanes on)
-        const int head = blockIdx.x, ln = threadIdx.x & 31;
-        const bool is_v = head >= fold.qk_nq + fold.qk_nkv, is_k = head >= fold.qk_nq && !is_v;
-        float yv[4] = {acc.x, acc.y, acc.z, acc.w};
-        const void* wn = is_k ? fold.qk_kw : fold.qk_qw;
-        if (!is_v && wn) {
-          float ss = yv[0] * yv[0] + yv[1] * yv[1] + yv[2] * yv[2] + yv[3] * yv[3];
+          for (int b = 0; b < B; ++b) {
+            const int r = rb + b * WARPS;
+            if (r >= r_hi) break;                                          // warp-uniform
+            float yv[4] = {sum[b][0].x, sum[b][0].y, sum[b][0].z, sum[b][0].w};
+            if (EPI) {
+              const float4 up = sum[b][PARTS - 1];
+              yv[0] = tc_gate(yv[0], fold.unary) * up.x; yv[1] = tc_gate(yv[1], fold.unary) * up.y;
+              yv[2] = tc_gate(yv[2], fold.unary) * up.z; yv[3] = tc_gate(yv[3], fold.unary) * up.w;
+            } else {
+              if (fold.bias) {
 #pragma unroll
-          for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
-          const float rn = rsqrtf(ss * (1.f / 128.f) + fold.qk_eps);
+                for (int j = 0; j < 4; ++j) yv[j] += bv[j];
+              }
+              if (fold.unary) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) yv[j] = yv[j] * rn * load_as_f32(wn, fold.qk_w_dtype, c + j);
-        }
-        if (!is_v && fold.qk_rope) {
-          const float2* t = fold.qk_rope + (size_t)(m0 + r) * 64 + (c & 63);
+                for (int j = 0; j < 4; ++j) yv[j] = ifb_unary(yv[j], fold.unary);
+              }
+            }
+            TO* dst = out + (size_t)(m0 + r) * o_out + n0 + c;
+            if (!EPI && fold.res_x) {
+              // v = x + y, x <- v, the output becomes v * g, the warp's sum of v^2 one part
+              float* x = fold.res_x + (size_t)(m0 + r) * o_out + n0 + c;
+              const float xo[4] = {xr[b].x, xr[b].y, xr[b].z, xr[b].w};
+              float ss = 0.f;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float o = __shfl_xor_sync(0xffffffffu, yv[j], 16);
-            const float2 cs = t[j];
-            yv[j] = ln < 16 ? yv[j] * cs.x - o * cs.y : yv[j] * cs.x + o * cs.y;
+              for (int j = 0; j < 4; ++j)
+                if (c + j < cols) {
+                  const float t = xo[j] + yv[j];
+                  x[j] = t;
+                  ss += t * t;
+                  yv[j] = t * wv[j];
+                }
+#pragma unroll
+              for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+              if ((threadIdx.x & 31) == 0) fold.res_partials[(size_t)blockIdx.x * n_rows + m0 + r] = ss;
+            }
+            if (!EPI && sizeof(TO) == 2 && fold.qk_nq) {
+              // the warp holds one head of one token (lane l its elements 4l .. 4l + 3; the rotation partner 16 lanes on)
+              if (wn) {
+                float ss = yv[0] * yv[0] + yv[1] * yv[1] + yv[2] * yv[2] + yv[3] * yv[3];
+#pragma unroll
+                for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+                const float rn = rsqrtf(ss * (1.f / 128.f) + fold.qk_eps);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) yv[j] = yv[j] * rn * wv[j];
+              }
+              if (!qk_v && fold.qk_rope) {
+                const float co[4] = {cs[b][0].x, cs[b][0].z, cs[b][1].x, cs[b][1].z}, si[4] = {cs[b][0].y, cs[b][0].w, cs[b][1].y, cs[b][1].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float o = __shfl_xor_sync(0xffffffffu, yv[j], 16);
+                  yv[j] = (threadIdx.x & 31) < 16 ? yv[j] * co[j] - o * si[j] : yv[j] * co[j] + o * si[j];
+                }
+              }
+              const __nv_bfloat162 lo = __floats2bfloat162_rn(yv[0], yv[1]), hi = __floats2bfloat162_rn(yv[2], yv[3]);
+              const uint2 pk = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+              *reinterpret_cast<uint2*>(dst) = pk;
+              if (slot[b] >= 0) {
+                const int kvh = qk_v ? qk_head - fold.qk_nq - fold.qk_nkv : qk_head - fold.qk_nq;
+                const size_t row = ((size_t)(slot[b] / fold.qk_page_size) * 2 + (qk_v ? 1 : 0)) * fold.qk_nkv + kvh;
+                *reinterpret_cast<uint2*>(fold.qk_pages + (row * fold.qk_page_size + slot[b] % fold.qk_page_size) * 128 + c) = pk;
+              }
+              continue;
+            }
+            if (vec) {
+              if (sizeof(TO) == 4) {
+                *reinterpret_cast<float4*>(dst) = make_float4(yv[0], yv[1], yv[2], yv[3]);
+              } else {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(yv[0], yv[1]), hi = __floats2bfloat162_rn(yv[2], yv[3]);
+                *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+              }
+            } else {
+              for (int j = 0; j < 4; ++j)
+                if (c + j < cols) dst[j] = from_f32<TO>(yv[j]);
+            }
           }
+          if (last) break;
         }
-        __nv_bfloat162 lo = __floats2bfloat162_rn(yv[0], yv[1]), hi = __floats2bfloat162_rn(yv[2], yv[3]);
-        const uint2 pk = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-        *reinterpret_cast<uint2*>(dst) = pk;
-        if (head >= fold.qk_nq && fold.qk_slots) {
-          const int slot = fold.qk_slots[m0 + r];
-          if (slot >= 0) {
-            const int kvh = is_v ? head - fold.qk_nq - fold.qk_nkv : head - fold.qk_nq;
-            const size_t row = ((size_t)(slot / fold.qk_page_size) * 2 + (is_v ? 1 : 0)) * fold.qk_nkv + kvh;
-            *reinterpret_cast<uint2*>(fold.qk_pages + (row * fold.qk_page_size + slot % fold.qk_page_size) * 128 + c) = pk;
-          }
-        }
-        continue;
-      }
-      if (vec) {
-        if (sizeof(TO) == 4) {
-          *reinterpret_cast<float4*>(dst) = acc;
-        } else {
-          __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x, acc.y), hi = __floats2bfloat162_rn(acc.z, acc.w);
-          *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-        }
-      } else {
-        const float y[4] = {acc.x, acc.y, acc.z, acc.w};
-        for (int j = 0; j < 4; ++j)
-          if (c + j < cols) dst[j] = from_f32<TO>(y[j]);
-      }
+      };
+      if (used > 4) run(TcInt<8>{}, TcInt<ROWS_OF_8>{});
+      else run(TcInt<4>{}, TcInt<ROWS_OF_4>{});
+      asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");      // nobody leaves while its shared memory is being read
     }
-    cluster_sync_all();                        // nobody leaves while its shared memory is being read
   }
   if (*abort_flag) {                         // a wait gave up: let copies in flight land before the CTA goes away
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
@@ -585,6 +889,55 @@ template <int EPI_, int NACC_, int STAGES_> struct PersistCfg {
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 1024 /* alignment */ + 256 /* barriers */;
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NACC >> 3) << 17) | ((uint32_t)(G_BM >> 4) << 24);
 };
+
+// 32 columns of an accumulator (a lane's row of them) through the epilogue: y.  FO: columns from a gate to its up.
+template <int EPI>
+__device__ __forceinline__ void tc_epilogue_row(const TcFold& fold, uint32_t taddr, int fo, float rfac, int col, int o_out, float (&y)[32]) {
+  uint32_t v[32];
+  tmem_ld32(taddr, v);
+  if (EPI) {
+    uint32_t u[32];
+    tmem_ld32(taddr + fo, u);
+    tmem_ld_wait();
+    if (fold.unary) {                                    // warp-uniform: another function than silu on the gate
+#pragma unroll
+      for (int j = 0; j < 32; ++j) y[j] = tc_gate(__uint_as_float(v[j]) * rfac, fold.unary) * (__uint_as_float(u[j]) * rfac);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) y[j] = tc_gate(__uint_as_float(v[j]) * rfac, 0) * (__uint_as_float(u[j]) * rfac);
+    }
+  } else {
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(v[j]) * rfac;
+    if (fold.bias) {                                     // warp-uniform; every lane holds the same 32 features
+#pragma unroll
+      for (int j = 0; j < 32; ++j) y[j] += col + j < o_out ? __ldg(fold.bias + col + j) : 0.f;
+    }
+    if (fold.unary) {                                    // warp-uniform
+#pragma unroll
+      for (int j = 0; j < 32; ++j) y[j] = ifb_unary(y[j], fold.unary);
+    }
+  }
+}
+// 32 values in the output type at 16-byte aligned `dst`.
+template <typename TO>
+__device__ __forceinline__ void tc_pack_row(unsigned char* dst, const float (&y)[32]) {
+  if (sizeof(TO) == 2) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) {
+      uint4 pk;
+      __nv_bfloat162 h0 = __floats2bfloat162_rn(y[j], y[j + 1]), h1 = __floats2bfloat162_rn(y[j + 2], y[j + 3]);
+      __nv_bfloat162 h2 = __floats2bfloat162_rn(y[j + 4], y[j + 5]), h3 = __floats2bfloat162_rn(y[j + 6], y[j + 7]);
+      pk.x = *reinterpret_cast<uint32_t*>(&h0); pk.y = *reinterpret_cast<uint32_t*>(&h1);
+      pk.z = *reinterpret_cast<uint32_t*>(&h2); pk.w = *reinterpret_cast<uint32_t*>(&h3);
+      *reinterpret_cast<uint4*>(dst + j * 2) = pk;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j * 4) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
+  }
+}
 
 template <typename Cfg, typename TO>
 __global__ void __launch_bounds__(G_THREADS, 1)
@@ -714,50 +1067,10 @@ linear_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, con
         if (n0 + p0 >= o_out) break;                             // warp-uniform
 #pragma unroll
         for (int c0 = p0; c0 < p0 + PW; c0 += 32) {
-          uint32_t v[32];
           float y[32];
-          tmem_ld32(lane_base + c0, v);
-          if (EPI) {
-            uint32_t u[32];
-            tmem_ld32(lane_base + FO + c0, u);
-            tmem_ld_wait();
-            if (fold.unary) {                                    // warp-uniform: another function than silu on the gate
-#pragma unroll
-              for (int j = 0; j < 32; ++j) y[j] = tc_gate(__uint_as_float(v[j]) * rfac, fold.unary) * (__uint_as_float(u[j]) * rfac);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) y[j] = tc_gate(__uint_as_float(v[j]) * rfac, 0) * (__uint_as_float(u[j]) * rfac);
-            }
-          } else {
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; ++j) y[j] = __uint_as_float(v[j]) * rfac;
-            if (fold.bias) {                                     // warp-uniform; every lane holds the same 32 features
-#pragma unroll
-              for (int j = 0; j < 32; ++j) y[j] += n0 + c0 + j < o_out ? __ldg(fold.bias + n0 + c0 + j) : 0.f;
-            }
-            if (fold.unary) {                                    // warp-uniform
-#pragma unroll
-              for (int j = 0; j < 32; ++j) y[j] = ifb_unary(y[j], fold.unary);
-            }
-          }
+          tc_epilogue_row<EPI>(fold, lane_base + c0, FO, rfac, n0 + c0, o_out, y);
           if (vec) {
-            unsigned char* dst = buf + lane * PITCH + (c0 - p0) * (int)sizeof(TO);
-            if (sizeof(TO) == 2) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                uint4 pk;
-                __nv_bfloat162 h0 = __floats2bfloat162_rn(y[j], y[j + 1]), h1 = __floats2bfloat162_rn(y[j + 2], y[j + 3]);
-                __nv_bfloat162 h2 = __floats2bfloat162_rn(y[j + 4], y[j + 5]), h3 = __floats2bfloat162_rn(y[j + 6], y[j + 7]);
-                pk.x = *reinterpret_cast<uint32_t*>(&h0); pk.y = *reinterpret_cast<uint32_t*>(&h1);
-                pk.z = *reinterpret_cast<uint32_t*>(&h2); pk.w = *reinterpret_cast<uint32_t*>(&h3);
-                *reinterpret_cast<uint4*>(dst + j * 2) = pk;
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4*>(dst + j * 4) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
-            }
+            tc_pack_row<TO>(buf + lane * PITCH + (c0 - p0) * (int)sizeof(TO), y);
           } else if (row0 + lane < n_rows) {
             TO* dst = out + (size_t)(row0 + lane) * o_out + n0 + c0;
 #pragma unroll
@@ -789,6 +1102,343 @@ linear_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, con
   tc_fence_before();
   __syncthreads();
   if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, Cfg::TMEM_COLS); }
+}
+
+// ---------------------------------------------------------------------------------------------------
+// The persistent form over pairs of SMs, for prompts.  A cluster of two CTAs takes a tile of 256 tokens x NACC accumulator
+// columns: each CTA loads its own 128 rows of x and HALF of the tile's rows of w (with the silu_gate epilogue: one CTA the gate
+// rows, the other the up rows), and one tcgen05.mma of the pair (cta_group::2, M = 256), issued by the first CTA, multiplies out
+// of both CTAs' shared memory into both tensor memories, where each CTA finds its 128 tokens' full rows.  What bounds these
+// products is the bytes that reach an SM from L2 (57 a cycle measured): per product of 128 x 256 the pair brings 32 KB to an SM
+// per 64 of k where a CTA alone brings 48 KB, the same as a 256 x 256 tile of one CTA, but with a tile half as large, so that the other
+// half of tensor memory holds a second accumulator and a tile's epilogue runs beside the next tile's products.
+// Stages, barriers and epilogue are those of the persistent kernel above, except: the "full" barriers are the first CTA's and
+// count both CTAs' bytes, the "empty" and "accumulator ready" barriers are each CTA's own and get a multicast commit, and the
+// "accumulator read" barriers are the first CTA's and count both CTAs' epilogue warps.
+// Measured at 2,048 rows against the best shape of one CTA: gate and up of 12,288 x 4,096 338 to 257 us (1.6 PFLOP/s),
+// q | k | v of 6,144 x 4,096 82 to 70, gate and up of 3,072 x 1,024 22.4 to 20.3, 1,024 x 3,072 14.9 to 13.8.
+// ROWS32: the epilogue stages 64 float32 features of a row at a time (tc_finish_residual, tc_finish_heads).
+// ---------------------------------------------------------------------------------------------------
+template <int EPI_, int NACC_, int STAGES_, bool ROWS32_> struct PairCfg {
+  static constexpr int EPI = EPI_, NACC = NACC_, STAGES = STAGES_;
+  static constexpr bool ROWS32 = ROWS32_;
+  static constexpr int FO = EPI ? NACC / 2 : NACC;            // output features per tile
+  static constexpr int W_ROWS = NACC / 2;                     // rows of w of a CTA's stage
+  static constexpr int A_BYTES = G_TILE_BYTES, B_BYTES = W_ROWS * G_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int TMEM_COLS = 2 * NACC;                  // two accumulators: 256 or 512 columns
+  static constexpr int STAGING_PITCH = (ROWS32 ? 256 : 128) + 16;
+  static constexpr int STAGING_BYTES = 8 * 32 * STAGING_PITCH;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 1024 /* alignment */ + 256 /* barriers */;
+  // float32 accumulator, bfloat16 a and b, both K-major, M = 256 over the pair, N = NACC
+  static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NACC >> 3) << 17) | ((uint32_t)(2 * G_BM >> 4) << 24);
+  static_assert(SMEM_BYTES <= 227 * 1024, "stages and staging rows must fit in shared memory");
+};
+
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(a) : "r"(g_smem_u32(p)), "r"(rank));
+  return a;
+}
+// Into this CTA's shared memory; the bytes are counted by the barrier at `bar`, an address in the cluster (either CTA's).
+__device__ __forceinline__ void tma_load_2d_pair(void* smem, const CUtensorMap* map, uint32_t bar, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
+               ::"r"(g_smem_u32(smem)), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+               ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Arrives at the barrier of this address in both CTAs once the products issued so far are done.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+               ::"r"(g_smem_u32(bar)), "h"((uint16_t)3) : "memory");
+}
+
+template <typename Cfg, typename TO>
+__global__ void __launch_bounds__(G_THREADS, 1)
+linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
+                           TO* __restrict__ out, int n_rows, int o_out, int k_dim, int tiles_m, int tiles_total,
+                           int* __restrict__ err, TcFold fold) {
+  constexpr int EPI = Cfg::EPI, NACC = Cfg::NACC, FO = Cfg::FO, STAGES = Cfg::STAGES;
+  extern __shared__ unsigned char g_smem_raw[];
+  const uint32_t raw = g_smem_u32(g_smem_raw);
+  unsigned char* smem = g_smem_raw + (((raw + 1023u) & ~1023u) - raw);      // the same offset in both CTAs
+  unsigned char* staging = smem + STAGES * Cfg::STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(staging + Cfg::STAGING_BYTES);
+  uint64_t* empty = full + STAGES;
+  uint64_t* acc_full = empty + STAGES;                         // [2]: a tile's products are in accumulator b
+  uint64_t* acc_empty = acc_full + 2;                          // [2], the first CTA's: the sixteen epilogue warps have read it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform
+  const int rank = blockIdx.x & 1;                             // the cluster is two neighbours along x
+  const int kblocks = (k_dim + G_BK - 1) / G_BK;
+  // this pair's tiles: first, first + step, ...; tile t covers tokens (t % tiles_m) * 256 and features (t / tiles_m) * FO
+  const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 16); }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(g_smem_u32(tmem_slot)), "r"(Cfg::TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                                          // both CTAs' barriers exist before either CTA's copies count on them
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ---- producer, in both CTAs.  The w tiles of the first stages are requested before the wait for the predecessor.
+    int g = 0;                                                  // k blocks issued so far, over all tiles
+    bool waited = false, ok = true;
+    for (int t = first; t < tiles_total && ok; t += step) {
+      const int m0 = (t % tiles_m) * (2 * G_BM) + rank * G_BM, n0 = (t / tiles_m) * FO;
+      const int w0 = EPI ? rank * o_out + n0 : n0 + rank * Cfg::W_ROWS;
+      for (int kb = 0; kb < kblocks; ++kb, ++g) {
+        const int s = g % STAGES;
+        if (g >= STAGES && !mbar_wait(&empty[s], ((g / STAGES) - 1) & 1, abort_flag, err, 1)) { ok = false; break; }
+        unsigned char* stage = smem + s * Cfg::STAGE_BYTES;
+        const uint32_t bar = cluster_addr(&full[s], 0);
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(&full[s], 2 * Cfg::STAGE_BYTES);
+          tma_load_2d_pair(stage + Cfg::A_BYTES, &tmap_w, bar, kb * G_BK, w0);
+        }
+        __syncwarp();
+        if (!waited && (g == STAGES - 1 || (kb == kblocks - 1 && t + step >= tiles_total))) {
+          // the ring is full of w tiles (or there are no more): now the predecessor, then the x tiles held back
+          ifb_pdl_wait();
+          ifb_pdl_trigger();
+          waited = true;
+          int gg = 0;
+          for (int tt = first; tt < tiles_total && gg <= g; tt += step)
+            for (int kk = 0; kk < kblocks && gg <= g; ++kk, ++gg) {
+              const uint32_t bb = cluster_addr(&full[gg % STAGES], 0);
+              if (elect_one())
+                tma_load_2d_pair(smem + (gg % STAGES) * Cfg::STAGE_BYTES, &tmap_x, bb, kk * G_BK, (tt % tiles_m) * (2 * G_BM) + rank * G_BM);
+              __syncwarp();
+            }
+        } else if (waited) {
+          if (elect_one()) tma_load_2d_pair(stage, &tmap_x, bar, kb * G_BK, m0);
+          __syncwarp();
+        }
+      }
+    }
+    if (!waited) { ifb_pdl_wait(); ifb_pdl_trigger(); }         // a CTA without tiles still orders itself behind the predecessor
+  } else if (warp == 1) {
+    // ---- issuer, in the first CTA: tile i of this pair accumulates in accumulator i & 1
+    int g = 0, it = 0;
+    bool ok = rank == 0;
+    for (int t = first; t < tiles_total && ok; t += step, ++it) {
+      const int b = it & 1;
+      if (it >= 2) ok = mbar_wait(&acc_empty[b], ((it >> 1) - 1) & 1, abort_flag, err, 4);
+      if (!ok) break;
+      tc_fence_after();
+      for (int kb = 0; kb < kblocks && ok; ++kb, ++g) {
+        const int s = g % STAGES;
+        ok = mbar_wait(&full[s], (g / STAGES) & 1, abort_flag, err, 2);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+          const uint32_t a_addr = g_smem_u32(smem + s * Cfg::STAGE_BYTES);
+          const uint64_t a_desc = make_smem_desc(a_addr), b_desc = make_smem_desc(a_addr + Cfg::A_BYTES);
+#pragma unroll
+          for (int k = 0; k < G_BK / G_UK; ++k) {
+            const uint64_t kstep = (uint64_t)((k * G_UK * 2) >> 4);          // 32 bytes per k step, in 16-byte units
+            umma_bf16_pair(tmem_base + b * NACC, a_desc + kstep, b_desc + kstep, Cfg::IDESC, (kb | k) != 0);
+          }
+          umma_commit_pair(&empty[s]);
+          if (kb == kblocks - 1) umma_commit_pair(&acc_full[b]);
+        }
+        __syncwarp();
+      }
+    }
+  } else {
+    // ---- epilogue, in both CTAs, each its own 128 tokens.  A warp's piece of a tile is 32 tokens (its lanes) by CW features.
+    constexpr int CW = FO / 2;
+    constexpr int PITCH = Cfg::STAGING_PITCH;
+    const int q = warp & 3;                                      // this warp's quarter of the 128 lanes
+    const int c_lo = ((warp - 2) >> 2) * CW;                     // and its half of the tile's features
+    unsigned char* buf = staging + (warp - 2) * (32 * PITCH);
+    int it = 0;
+    bool ok = true;
+    if (fold.rs_partials || Cfg::ROWS32) ifb_pdl_wait();         // what the predecessors wrote is read here directly
+    for (int t = first; t < tiles_total && ok; t += step, ++it) {
+      const int b = it & 1;
+      const int row0 = (t % tiles_m) * (2 * G_BM) + rank * G_BM + q * 32, n0 = (t / tiles_m) * FO;
+      const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16) + b * NACC;
+      float rfac = tc_row_factor(fold, row0 + lane, n_rows);
+      if constexpr (Cfg::ROWS32) {
+        // whole rows of float32, 64 features at a time: the residual addition, or heads of 128
+        constexpr int AHEAD = 16;
+        float4 ahead[AHEAD], angles[AHEAD / 2][2];
+        int slot_of[AHEAD / 2];
+        const int head = (n0 + c_lo) / 128;
+        const bool qk_v = head >= fold.qk_nq + fold.qk_nkv, qk_k = head >= fold.qk_nq && !qk_v;
+        const bool heads = CW == 128 && sizeof(TO) == 2 && fold.qk_nq > 0;
+        const bool rotate = !qk_v && fold.qk_rope, store = (qk_v || qk_k) && fold.qk_slots;
+        if (heads) tc_heads_load<32, AHEAD / 2>(fold, row0, n_rows, 0, rotate, store, lane, angles, slot_of);
+        else if (n0 + c_lo < o_out) tc_residual_load<64, AHEAD>(fold, row0, n_rows, n0 + c_lo, o_out, lane, ahead);
+        ok = mbar_wait(&acc_full[b], (it >> 1) & 1, abort_flag, err, 3);
+        if (!ok) break;
+        tc_fence_after();
+        if (row0 < n_rows && n0 + c_lo < o_out) {                // warp-uniform
+          if (heads) {
+            if constexpr (sizeof(TO) == 2 && CW == 128) {
+              const void* wn = qk_v ? nullptr : qk_k ? fold.qk_kw : fold.qk_qw;
+              if (wn) {
+                float ss[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+                for (int c0 = 0; c0 < 128; c0 += 32) {
+                  uint32_t v[32];
+                  tmem_ld32(lane_base + c_lo + c0, v);
+                  tmem_ld_wait();
+#pragma unroll
+                  for (int j = 0; j < 32; ++j) { const float f = __uint_as_float(v[j]) * rfac; ss[j & 3] = fmaf(f, f, ss[j & 3]); }
+                }
+                rfac *= rsqrtf(((ss[0] + ss[1]) + (ss[2] + ss[3])) * (1.f / 128.f) + fold.qk_eps);
+              }
+#pragma unroll 1
+              for (int i0 = 0; i0 < 64; i0 += 32) {
+                if (i0) tc_heads_load<32, AHEAD / 2>(fold, row0, n_rows, i0, rotate, store, lane, angles, slot_of);
+                tc_stage_rows(lane_base + c_lo + i0, buf + lane * PITCH, rfac);
+                tc_stage_rows(lane_base + c_lo + 64 + i0, buf + lane * PITCH + 128, rfac);
+                __syncwarp();
+                tc_finish_heads<32, PITCH, AHEAD / 2>(fold, buf, reinterpret_cast<bf16*>(out), row0, n_rows, head, i0, o_out, wn, qk_v, rotate,
+                                                      store, lane, angles, slot_of);
+                __syncwarp();
+              }
+            }
+          } else {
+#pragma unroll 1
+            for (int c0 = c_lo; c0 < c_lo + CW && n0 + c0 < o_out; c0 += 64) {
+              if (c0 != c_lo) tc_residual_load<64, AHEAD>(fold, row0, n_rows, n0 + c0, o_out, lane, ahead);
+              tc_stage_rows(lane_base + c0, buf + lane * PITCH, rfac);
+              tc_stage_rows(lane_base + c0 + 32, buf + lane * PITCH + 128, rfac);
+              __syncwarp();
+              tc_finish_residual<64, PITCH, AHEAD, TO>(fold, buf, out, row0, n_rows, n0 + c0, o_out, (n0 + c0) / 64, lane, ahead);
+              __syncwarp();
+            }
+          }
+        }
+      } else {
+        constexpr int PW = 128 / (int)sizeof(TO);                // features per staged row segment
+        static_assert(CW % PW == 0, "a warp's features are whole row segments");
+        ok = mbar_wait(&acc_full[b], (it >> 1) & 1, abort_flag, err, 3);
+        if (!ok) break;
+        tc_fence_after();
+        const bool vec = ((size_t)o_out * sizeof(TO)) % 16 == 0 && (((uintptr_t)out) & 15) == 0 && n0 + c_lo + CW <= o_out;
+#pragma unroll 1
+        for (int p0 = c_lo; p0 < c_lo + CW; p0 += PW) {
+          if (n0 + p0 >= o_out || row0 >= n_rows) break;         // warp-uniform
+#pragma unroll
+          for (int c0 = p0; c0 < p0 + PW; c0 += 32) {
+            float y[32];
+            tc_epilogue_row<EPI>(fold, lane_base + c0, FO, rfac, n0 + c0, o_out, y);
+            if (vec) tc_pack_row<TO>(buf + lane * PITCH + (c0 - p0) * (int)sizeof(TO), y);
+            else if (row0 + lane < n_rows) {
+              TO* dst = out + (size_t)(row0 + lane) * o_out + n0 + c0;
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                if (n0 + c0 + j < o_out) dst[j] = from_f32<TO>(y[j]);
+            }
+          }
+          if (vec) {
+            __syncwarp();
+            unsigned char* obase = reinterpret_cast<unsigned char*>(out + (size_t)row0 * o_out + n0 + p0);
+#pragma unroll
+            for (int off = lane * 16; off < 32 * 128; off += 512) {
+              const int r = off >> 7, cb = off & 127;
+              if (row0 + r < n_rows)
+                *reinterpret_cast<uint4*>(obase + (size_t)r * o_out * sizeof(TO) + cb) = *reinterpret_cast<const uint4*>(buf + r * PITCH + cb);
+            }
+            __syncwarp();                                        // before the next segment overwrites the rows
+          }
+        }
+      }
+      // this warp has read its part of accumulator b: the issuer may overwrite it (with the tile after next)
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr(&acc_empty[b], 0)) : "memory");
+    }
+  }
+  if (*abort_flag) {                         // a wait gave up: let copies in flight land before the CTA goes away
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();                        // neither CTA leaves while the other's products or arrivals need its memory
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(Cfg::TMEM_COLS) : "memory");
+  }
+}
+
+// How many pairs of a kernel the device runs at a time (known once per device and kernel; 0 if it cannot say).
+template <typename Cfg, typename TO>
+static int tc_pairs() {
+  static int known[IFB_MAX_DEVICES] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= IFB_MAX_DEVICES) return 0;
+  if (!known[dev]) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2);
+    cfg.blockDim = dim3(G_THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(linear_tcgen05_pair_kernel<Cfg, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM_BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, linear_tcgen05_pair_kernel<Cfg, TO>, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      return 0;
+    }
+    known[dev] = n;
+  }
+  return known[dev];
+}
+
+template <typename Cfg, typename TO>
+static int tc_launch_pair(const void* x, const void* w, void* out, int n, int o, int k, int* err, cudaStream_t s, const TcFold& fold) {
+  CUtensorMap mx, mw;
+  int st = make_map(&mx, x, n, k, G_BM);
+  if (st) return st;
+  st = make_map(&mw, w, Cfg::EPI ? 2 * o : o, k, Cfg::W_ROWS);
+  if (st) return st;
+  const int pairs = tc_pairs<Cfg, TO>();
+  if (!pairs) return IFB_ERR_ARG;
+  IFB_ALLOW_SMEM((linear_tcgen05_pair_kernel<Cfg, TO>), Cfg::SMEM_BYTES);
+  const long long tiles_m = (n + 2 * G_BM - 1) / (2 * G_BM), tiles_n = (o + Cfg::FO - 1) / Cfg::FO;
+  if (tiles_m * tiles_n > 0x7fffffffLL) return IFB_ERR_SIZE;
+  const int total = (int)(tiles_m * tiles_n);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (total < pairs ? total : pairs));
+  cfg.blockDim = dim3(G_THREADS);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ifb_pdl_enabled() ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, linear_tcgen05_pair_kernel<Cfg, TO>, mx, mw, (TO*)out, n, o, k, (int)tiles_m, total, err, fold);
+  if (e != cudaSuccess) { cudaGetLastError(); return -(int)e; }
+  return IFB_OK;
 }
 
 template <typename Cfg, typename TO>
@@ -843,7 +1493,7 @@ static int tc_launch_cfg(const void* x, const void* w, void* out, int n, int o, 
 
 // The shape of the tiles: a wave of wide tiles does four 128 x 128 products per SM in little more time than a wave of
 // narrow tiles (two CTAs per SM) does two, but only if there are enough wide tiles to fill the SMs.  shape: 0 chooses
-// (see below), 1 narrow, 2 deep, 3 wide, 4 and 5 persistent (for tests and measurements).
+// (see below), 1 narrow, 2 deep, 3 wide, 4 and 5 persistent, 6 the pairs (for tests and measurements).
 static int tc_sm_count() {
   static int sm_count = 0;
   if (!sm_count) {
@@ -867,6 +1517,23 @@ static int tc_pick_shape(int epi, int n, int o) {
   return (n > G_BM && cost_wide < cost_narrow) ? 3 : (tn <= sm_count ? 2 : 1);
 }
 
+// Whether the kernel over pairs of SMs takes a product (a rule on sizes alone, as the parts of a folded norm must agree with the
+// launch): from 513 rows on (up to 512 few tiles share their k range in clusters), where the tiles of its last round, of 256 x 256
+// or 256 x 128, keep most pairs busy (four fifths over all rounds).  Narrow tiles take 0.7 of a wide one's time: an SM gets 24 KB
+// per 64 of k where it gets 32 (2,048 x 1,024 x 2,048: one round of 64 narrow tiles 10.9 us).
+static int tc_pair_rounds(int n, int o, int features) {
+  const int pairs = tc_sm_count() / 2;
+  const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
+  return (int)((tiles + pairs - 1) / pairs);
+}
+static bool tc_pair_narrow(int n, int o) { return 0.7 * tc_pair_rounds(n, o, 128) < tc_pair_rounds(n, o, 256); }
+static bool tc_pick_pair(int epi, int n, int o) {
+  if (o % 64 || n <= 512) return false;
+  const int features = epi || tc_pair_narrow(n, o) ? 128 : 256;
+  const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
+  return tiles * 10 >= (long long)tc_sm_count() / 2 * 8 * tc_pair_rounds(n, o, features);
+}
+
 template <int EPI, typename TO>
 static int tc_launch(const void* x, const void* w, void* out, int n, int o, int k, int* err, int shape, int splits, const TcFold& fold,
                      cudaStream_t s) {
@@ -878,13 +1545,29 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
   if (splits > 1) {
     static_assert(G_BM * (Deep::NACC + 4) * 4 <= Deep::STAGES * Deep::STAGE_BYTES, "the float32 tile must fit in the stages");
     if (splits > 8) return IFB_ERR_ARG;
-    // one tile of rows: a CTA per SM with a deep ring; more: two CTAs per SM, one's sum beside the other's products
-    if ((n <= G_BM && shape != 1) || G_BM * (Narrow::NACC + 4) * 4 > Narrow::STAGES * Narrow::STAGE_BYTES)
-      return tc_launch_cfg<Deep, TO>(x, w, out, n, o, k, err, s, fold, splits);
-    return tc_launch_cfg<Narrow, TO>(x, w, out, n, o, k, err, s, fold, splits);
+    return tc_launch_cfg<Deep, TO>(x, w, out, n, o, k, err, s, fold, splits);
   }
-  if (shape == 0) shape = tc_pick_shape(EPI, n, o);
-  if (fold.res_x && (EPI || shape > 3)) return IFB_ERR_ARG;        // the making side is the one-tile kernel's
+  if (shape == 0) {
+    shape = tc_pick_shape(EPI, n, o);
+    if (tc_pick_pair(EPI, n, o)) shape = 6;
+  }
+  if (EPI && fold.res_x) return IFB_ERR_ARG;
+  if (shape == 6) {
+    using Pair = PairCfg<EPI, 256, 5, false>;
+    if constexpr (!EPI) {
+      using Rows256 = PairCfg<0, 256, 4, true>;
+      using Rows128 = PairCfg<0, 128, 6, true>;
+      using Pair128 = PairCfg<0, 128, 7, false>;
+      const bool narrow = !fold.qk_nq && tc_pair_narrow(n, o);
+      if (fold.qk_nq || fold.res_x) {
+        if (o % 64) return IFB_ERR_ARG;                              // (a forced shape: the rule asks for it)
+        return narrow ? tc_launch_pair<Rows128, TO>(x, w, out, n, o, k, err, s, fold) : tc_launch_pair<Rows256, TO>(x, w, out, n, o, k, err, s, fold);
+      }
+      if (narrow) return tc_launch_pair<Pair128, TO>(x, w, out, n, o, k, err, s, fold);
+    }
+    return tc_launch_pair<Pair, TO>(x, w, out, n, o, k, err, s, fold);
+  }
+  if (fold.res_x && shape > 3) return IFB_ERR_ARG;        // the making side is the one-tile kernel's
   if (shape == 5 && !EPI) return tc_launch_persistent<P256, TO>(x, w, out, n, o, k, err, tc_sm_count(), s, fold);
   if (shape == 4 || shape == 5) return tc_launch_persistent<P128, TO>(x, w, out, n, o, k, err, tc_sm_count(), s, fold);
   if (shape == 3) return tc_launch_cfg<Wide, TO>(x, w, out, n, o, k, err, s, fold);
@@ -896,7 +1579,7 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
 // 1 + 16 * u: gated with u in silu's place.
 // x [n_rows, k] and w [out_features (x2 for the silu_gate epilogue), k] bfloat16, 16-byte aligned, k a multiple of 8;
 // out bfloat16 or float32.  `err` points to a device int that stays 0 unless a bounded wait gave up.  shape: 0 lets the
-// library choose, 1-3 force the one-tile-per-CTA kernel narrow, deep or wide, 4 and 5 the persistent kernel with tiles
+// library choose, 1-3 force the one-tile-per-CTA kernel narrow, deep or wide, 6 the kernel over pairs of SMs, 4 and 5 the persistent kernel with tiles
 // of 128 or 256 features.  splits 2 to 8: the k range of a tile of 128 x 128 is shared by a cluster of
 // that many CTAs, whose parts are added in a fixed order; for few tiles of a long k (a step of some tens of tokens).
 // scale_partials (may be null): [scale_parts][n_rows] sums of squares; output row n is multiplied by
@@ -915,7 +1598,7 @@ IFB_EXPORT int ifb_linear_tcgen05_ex(const void* x, const void* w, void* out, in
   epilogue &= 15;
   if (epilogue > 1 || unary < 0 || unary > IFB_UNARY_LAST || (unary && res_x) || (bias && epilogue))
     return IFB_ERR_ARG;
-  if (shape < 0 || shape > 5 || splits < 0 || splits > 8) return IFB_ERR_ARG;
+  if (shape < 0 || shape > 6 || splits < 0 || splits > 8) return IFB_ERR_ARG;
   if (scale_partials && (scale_parts < 1 || scale_width < 1)) return IFB_ERR_ARG;
   if (res_x && (!res_g || !res_partials || ((uintptr_t)res_x & 15))) return IFB_ERR_ARG;
   TcFold fold = {};
@@ -967,18 +1650,18 @@ IFB_EXPORT int ifb_linear_tcgen05(const void* x, const void* w, void* out, int o
                                nullptr, 0, nullptr, nullptr, err, stream);
 }
 
-// The fused q | k | v projection of an attention layer in the shared-k form with what follows it in the sum over the
-// cluster (see TcFold): qkv [n_rows, (nq + 2 nkv) * 128] bfloat16 gets the normalised and rotated q heads (and the k and
+// The fused q | k | v projection of an attention layer with what follows it (see TcFold) in the epilogue of the one-tile
+// kernel (splits 1) or in the sum over the cluster of the shared-k form (splits 2 to 8): qkv [n_rows, (nq + 2 nkv) * 128] bfloat16 gets the normalised and rotated q heads (and the k and
 // v heads as they are stored), the pages get k and v at slots[n].  Heads of 128, rotated whole in the half-split pairing
-// (rope: [n_rows][64] pairs of cos and sin, or null); splits 2 to 8.  scale_*: as in ifb_linear_tcgen05_ex.
+// (rope: [n_rows][64] pairs of cos and sin, or null).  scale_*: as in ifb_linear_tcgen05_ex.
 IFB_EXPORT int ifb_linear_tcgen05_qkv(const void* x, const void* w, void* qkv, int n_rows, int nq, int nkv, int head_dim, int k_dim,
                                       int splits, const float* scale_partials, int scale_parts, float scale_eps, int scale_width,
                                       const void* q_weight, const void* k_weight, int w_dtype, float eps, const float* rope,
                                       const int* slots, void* pages, int page_size, int* err, cudaStream_t stream) {
   if (n_rows <= 0) return IFB_OK;
-  if (head_dim != 128 || nq < 1 || nkv < 1 || splits < 2 || splits > 8) return IFB_ERR_SIZE;
+  if (head_dim != 128 || nq < 1 || nkv < 1 || splits < 1 || splits > 8) return IFB_ERR_SIZE;
   if (k_dim < 8 || k_dim % 8) return IFB_ERR_SIZE;
-  if (((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)qkv & 15) || ((uintptr_t)pages & 15) || ((uintptr_t)rope & 7))
+  if (((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)qkv & 15) || ((uintptr_t)pages & 15) || ((uintptr_t)rope & 15))
     return IFB_ERR_ALIGN;
   if ((q_weight || k_weight) && w_dtype != IFB_F32 && w_dtype != IFB_BF16) return IFB_ERR_DTYPE;
   if (scale_partials && (scale_parts < 1 || scale_width < 1)) return IFB_ERR_ARG;
@@ -995,6 +1678,7 @@ IFB_EXPORT int ifb_linear_tcgen05_qkv(const void* x, const void* w, void* qkv, i
 // Parts of sums of squares that a product with res_x writes per row (the launch with shape 0 and these splits).
 IFB_EXPORT int ifb_linear_tcgen05_fold_parts(int n_rows, int out_features, int splits) {
   if (splits > 1) return (out_features + 127) / 128;
+  if (tc_pick_pair(0, n_rows, out_features)) return (out_features + 63) / 64;
   return tc_pick_shape(0, n_rows, out_features) == 3 ? 2 * ((out_features + 255) / 256) : 2 * ((out_features + 127) / 128);
 }
 

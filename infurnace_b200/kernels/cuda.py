@@ -149,6 +149,8 @@ class CudaKernels:
         self.fused_qkv_tc = os.environ.get("INFURNACE_FUSED_QKV_TC", "1") != "0"
         self.tc_split_min_rows = int(os.environ.get("INFURNACE_TC_SPLIT_MIN_ROWS", "0"))     # 0: by the matrix
         self.tc_fold_max_rows = int(os.environ.get("INFURNACE_TC_FOLD_MAX_ROWS", "128"))
+        # matrices from this many elements on fold the norms for any number of rows (unless the most rows are given)
+        self.tc_fold_large = 1 << (62 if "INFURNACE_TC_FOLD_MAX_ROWS" in os.environ else 20)
         self._tc_clusters = {}         # CTAs per cluster -> clusters of the split product that run at a time
         self._route_memo = {}          # what _on_tcgen05 and tcgen05_splits answered (asked several times per launch)
         self._splits_memo = {}
@@ -292,7 +294,7 @@ class CudaKernels:
         return 9 if w.numel() >= (1 << 23) else 17
 
     def _linear_tcgen05(self, x, w, out, n, o, k, epi, shape=0, splits=1, row_scale=None, residual=None, bias=None):
-        """shape: 0 lets the library choose its tile shape; 1 narrow, 2 deep, 3 wide, 4 and 5 persistent.
+        """shape: 0 lets the library choose its tile shape; 1 narrow, 2 deep, 3 wide, 4 and 5 persistent, 6 over pairs of SMs.
         splits > 1: the k range of a tile is shared by a cluster of that many CTAs.  row_scale: as in
         :meth:`linear`.  residual (x, norm_weight, partials): as in :meth:`linear_residual_norm`."""
         partials, parts, eps, width = row_scale if row_scale is not None else (None, 0, 0.0, 0)
@@ -373,14 +375,15 @@ class CudaKernels:
     # makes v writes v * g and partial sums of v^2, and the product that reads it multiplies by r at its end.
     def can_fold_norm(self, n, dtype, w, epilogue="none"):
         """Whether a product of ``n`` rows of ``dtype`` against ``w`` (with that epilogue) takes or makes a
-        folded norm: on the tcgen05 kernel up to ``tc_fold_max_rows`` rows (one tile of rows: with many
-        rows the longer epilogue costs what the norm's own launch did), on the few-rows kernel up to
-        ``fold_max_rows``."""
+        folded norm: on the tcgen05 kernel up to ``tc_fold_max_rows`` rows (one tile of rows), or for any number of them where
+        the matrix has ``tc_fold_large`` elements (a norm's own launch costs 5 to 6 us at 2,048 rows of 1,024, the longer
+        epilogue of the product before it 2 to 3, and a step of 131 rows of the 0.6B sizes is a quarter shorter without its
+        three launches per layer), on the few-rows kernel up to ``fold_max_rows``."""
         if not (dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.shape[1] % 8 == 0 and n > 0
                 and self.fold_max_rows > 0):
             return False
         if self._on_tcgen05(n, w, epilogue):
-            return n <= self.tc_fold_max_rows
+            return n <= self.tc_fold_max_rows or w.numel() >= self.tc_fold_large
         return n <= min(self.gemv_max_rows, self.fold_max_rows)
 
     def fold_parts(self, out_features, n=None, w=None):
@@ -444,7 +447,7 @@ class CudaKernels:
     def can_fuse_qkv(self, n, dtype, w_qkv, head_dim, rotary_dim, interleaved, kv_pages):
         """Whether :meth:`linear_qkv_rope_store` takes a step of ``n`` rows: bfloat16, heads rotated whole in
         the half-split pairing (or not rotated); up to 16 rows on the few-rows kernel (heads of 64, 128 or
-        256), or up to 128 rows on the tcgen05 kernel in its shared-k form (heads of 128)."""
+        256), or on the tcgen05 kernel (heads of 128; up to 128 rows in its shared-k form only)."""
         if not (self.fused_qkv and n > 0 and dtype == torch.bfloat16 and w_qkv.dtype == torch.bfloat16
                 and w_qkv.shape[1] % 8 == 0 and (rotary_dim == 0 or (rotary_dim == head_dim and not interleaved))
                 and (kv_pages is None or kv_pages.dtype == torch.bfloat16)):
@@ -455,8 +458,8 @@ class CudaKernels:
         """"gemv", "tcgen05" or None for the fused q | k | v product of ``n`` rows."""
         if n <= 16 and head_dim in (64, 128, 256) and not self._on_tcgen05(n, w_qkv, shared_k=False):
             return "gemv"
-        if n <= 128 and head_dim == 128 and self.fused_qkv_tc and self._on_tcgen05(n, w_qkv) \
-                and self.tcgen05_splits(n, w_qkv.shape[0], w_qkv.shape[1]) > 1:
+        if head_dim == 128 and self.fused_qkv_tc and self._on_tcgen05(n, w_qkv) \
+                and (n > 128 or self.tcgen05_splits(n, w_qkv.shape[0], w_qkv.shape[1]) > 1):
             return "tcgen05"
         return None
 
@@ -497,11 +500,12 @@ class CudaKernels:
             raise KernelError("linear_qkv_rope_store: no kernel takes these sizes (see can_fuse_qkv)")
         if route == "tcgen05":
             self._err_armed = True
-            self.tc_shared_k_calls += 1
+            # (more than one tile of rows: the cluster's sum would take longer over the heads than the shorter k range saves)
+            splits = self.tcgen05_splits(n, width, k) if n <= 128 else 1
+            self.tc_shared_k_calls += splits > 1
             self.tc_folded_calls += partials is not None
             _check(self._tc_lib().ifb_linear_tcgen05_qkv(
-                x.data_ptr(), w_qkv.data_ptr(), qkv.data_ptr(), n, num_heads, num_kv_heads, head_dim, k,
-                self.tcgen05_splits(n, width, k), _ptr(partials), int(parts), float(seps), int(swidth), _ptr(q_weight),
+                x.data_ptr(), w_qkv.data_ptr(), qkv.data_ptr(), n, num_heads, num_kv_heads, head_dim, k, splits, _ptr(partials), int(parts), float(seps), int(swidth), _ptr(q_weight),
                 _ptr(k_weight), wd, float(eps), _ptr(rope_table), _ptr(slot_mapping),
                 _ptr(kv_pages) if slot_mapping is not None else 0, page_size, self._dev_err.data_ptr(), self._stream()),
                 "linear_qkv_rope_store")

@@ -653,3 +653,66 @@ def test_plain_attention_of_a_query_is_the_same_in_every_step(K, nq, nkv, d, ps,
                           torch.tensor([p + 1], dtype=torch.int32).cuda(), alone, d ** -0.5, window, 1, p + 1)
         assert torch.equal(alone[0], out[row])
 
+
+# More than one tile of rows: the shared-k form again (129), then the epilogue of the one-tile kernel with one head per tile
+# (deep stages, then two CTAs per SM) and with two, the last tile's second one missing where the heads are odd.
+@pytest.mark.parametrize("n", [129, 300, 700, 1300])
+@pytest.mark.parametrize("nq,nkv,d,k,ps", [(16, 8, 128, 1024, 16), (25, 1, 128, 520, 32)])
+@pytest.mark.parametrize("norm,rotate,scaled", [(True, True, False), (True, True, True), (False, True, False), (True, False, False)])
+def test_qkv_product_of_a_prompt_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, d, k, ps, norm, rotate, scaled):
+    test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, d, k, ps, norm, rotate, scaled)
+
+
+# A prompt's product with the residual addition by whole row segments (one tile per CTA: deep, narrow; wide is tested above), and
+# with rows of features that are not whole (by single features).
+@pytest.mark.parametrize("n,hidden,inner", [(700, 1024, 520), (1300, 2304, 264), (513, 1096, 136), (700, 1026, 136)])
+@pytest.mark.parametrize("gdt", [torch.bfloat16, torch.float32])
+def test_linear_with_a_folded_norm_on_prompts(K, n, hidden, inner, gdt, monkeypatch):
+    monkeypatch.setattr(K, "tc_fold_max_rows", 1 << 20)
+    if hidden % 8 == 0:
+        return _folded_norm_case(K, n, hidden, inner, 200, "silu_gate", gdt)
+    a, w = rnd((n, inner), torch.bfloat16, 1), rnd((hidden, inner), torch.bfloat16, 2, scale=inner ** -0.5)
+    x, g = rnd((n, hidden), torch.float32, 3), (1 + rnd((hidden,), torch.float32, 4, scale=0.1)).to(gdt)
+    ref = x.double() + a.double() @ w.double().t()
+    vals = torch.full((n, hidden), float("nan"), dtype=torch.bfloat16, device="cuda")
+    partials = torch.full((K.fold_parts(hidden, n, w.cuda()), n), float("nan"), dtype=torch.float32, device="cuda")
+    xd = x.cuda()
+    K.linear_residual_norm(a.cuda(), w.cuda(), xd, g.cuda(), vals, partials)
+    torch.testing.assert_close(xd.cpu().double(), ref, rtol=2e-4, atol=1e-4)
+    torch.testing.assert_close(partials.sum(dim=0).cpu().double(), (ref ** 2).sum(dim=1), rtol=1e-5, atol=1e-6)
+    torch.testing.assert_close(vals.cpu().double(), ref * g.double(), rtol=1e-2, atol=1e-3)
+
+
+# The kernel over pairs of SMs: one and several tiles per pair, ragged rows, features and k, both output types and every epilogue.
+@pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,o,k", [(1, 72, 72), (257, 256, 64), (513, 1000, 136), (2048, 4096, 200), (300, 20000, 1032)])
+@pytest.mark.parametrize("epilogue", ["none", "silu_gate", "gelu_gate", "relu2"])
+def test_linear_tcgen05_over_pairs(K, od, n, o, k, epilogue):
+    gated = epilogue.endswith("_gate")
+    x, w = rnd((n, k), torch.bfloat16, 4).cuda(), rnd((2 * o if gated else o, k), torch.bfloat16, 5, scale=k ** -0.5).cuda()
+    bias = None if gated else rnd((o,), torch.float32, 6).cuda()
+    y = x.double() @ w.double().t()
+    if gated:
+        g = torch.nn.functional.silu(y[:, :o]) if epilogue == "silu_gate" else torch.nn.functional.gelu(y[:, :o], approximate="tanh")
+        ref = g * y[:, o:]
+    else:
+        ref = y + bias.double()
+        ref = ref.relu() ** 2 if epilogue == "relu2" else ref
+    out = torch.full((n, o), float("nan"), dtype=od, device="cuda")
+    from infurnace_b200.kernels.cuda import EPILOGUES
+    K._linear_tcgen05(x, w, out, n, o, k, EPILOGUES[epilogue], shape=6, bias=bias)
+    K.check_device_errors()
+    torch.testing.assert_close(out.double(), ref, rtol=1.6e-2 if od == torch.bfloat16 else 2e-3, atol=1e-2 if od == torch.bfloat16 else 1e-3)
+
+
+# Folded norms and heads on pairs of SMs: tiles of 256 x 128 (1,900 rows of 1,024 features) and of 256 x 256, the reading side behind them.
+@pytest.mark.parametrize("n,hidden,inner,epilogue", [(1900, 1024, 520, "silu_gate"), (1300, 4160, 264, "none"), (4000, 2048, 72, "silu_gate")])
+def test_linear_with_a_folded_norm_over_pairs(K, n, hidden, inner, epilogue, monkeypatch):
+    monkeypatch.setattr(K, "tc_fold_max_rows", 1 << 20)
+    _folded_norm_case(K, n, hidden, inner, 1024, epilogue, torch.bfloat16)
+
+
+@pytest.mark.parametrize("n,nq,nkv", [(1500, 17, 4), (2500, 16, 8)])
+@pytest.mark.parametrize("norm,rotate,scaled", [(True, True, True), (False, True, False), (True, False, False)])
+def test_qkv_product_over_pairs_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, norm, rotate, scaled):
+    test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, 128, 520, 16, norm, rotate, scaled)
