@@ -327,22 +327,38 @@ __device__ __forceinline__ void load_q_frags(uint32_t (&qf)[KB][4], const bf16* 
 }
 
 constexpr int NO_ROW = -1000000000;
+constexpr int ATT_MAX_CLUSTER = 8;      // splits of a context that may be a cluster (the portable cluster size)
+
+// The float at this CTA's shared address `p`, read from the CTA of rank `rank` of the cluster.
+__device__ __forceinline__ float ld_cluster_f32(const float* p, int rank) {
+  uint32_t remote;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(remote) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(v) : "r"(remote) : "memory");
+  return v;
+}
 
 // The end of a small-q CTA: its four consumer warps' (m, l, o) are merged through shared memory (`scratch`, at least
 // 4*16*VD + 128 floats, free by now); then the output row is written, or with several splits the partial sums go to
-// global memory and the CTA that arrives last for its (request, key/value head) merges the splits in split order.
+// global memory and the CTA that arrives last for its (request, key/value head) merges the splits in split order; or, where
+// the splits are a thread-block cluster (`clustered`), they stay in shared memory and each CTA merges its share of the output
+// from all of them, in split order (no scratch, no atomic, one round trip through the cluster instead of four through L2).
 // The sink (base-2 score; -inf: none) joins the denominator where it is last summed.
 // Every thread of the CTA calls this (threads of warps above 3 only keep the barriers company).
 __device__ __forceinline__ void small_q_finish(float* scratch, float (&m)[2], float (&l)[2], float (&o)[VD / 8][4], int rows,
                                                int G, int q0, int kvh, int r, int split, int num_splits, int nq, int nkv,
                                                bf16* __restrict__ out, float* __restrict__ part_o,
-                                               float* __restrict__ part_ml, int* __restrict__ counters, int* is_last_p, float sink) {
+                                               float* __restrict__ part_ml, int* __restrict__ counters, int* is_last_p, float sink,
+                                               bool clustered = false) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nthreads = blockDim.x;
   const int rowA = lane >> 2, rowB = rowA + 8;
   float* sm_o = scratch;                                     // [4][16][VD]
   float* sm_m = sm_o + 4 * 16 * VD;                          // [4][16]
   float* sm_l = sm_m + 64;                                   // [4][16]
+  float* mg_o = sm_l + 64;                                   // clustered: this CTA's sums [16][VD], maxima [16], denominators [16]
+  float* mg_m = mg_o + 16 * VD;
+  float* mg_l = mg_m + 16;
   if (warp < 4) {
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
@@ -379,6 +395,9 @@ __device__ __forceinline__ void small_q_finish(float* scratch, float (&m)[2], fl
     if (num_splits == 1) {
       den += exp2f(sink - U);
       out[((size_t)tok * nq + head) * VD + dim] = __float2bfloat16_rn(den > 0.f ? acc / den : 0.f);
+    } else if (clustered) {
+      mg_o[idx] = acc;
+      if (dim == 0) { mg_m[row] = M; mg_l[row] = den; }
     } else {
       const size_t base = ((size_t)tok * nq + head) * num_splits + split;
       part_o[base * VD + dim] = acc;
@@ -386,6 +405,41 @@ __device__ __forceinline__ void small_q_finish(float* scratch, float (&m)[2], fl
     }
   }
   if (num_splits == 1) return;
+  if (clustered) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+    const int total = rows * VD, step = num_splits * nthreads;      // VD is a multiple of 64 here: whole warps have items
+    for (int idx = split * nthreads + tid;; idx += step) {
+      const bool have = idx < total, last = idx + step >= total;
+      const int row = have ? idx / VD : 0;
+      float pm[ATT_MAX_CLUSTER], pl[ATT_MAX_CLUSTER], po[ATT_MAX_CLUSTER];
+#pragma unroll
+      for (int sp = 0; sp < ATT_MAX_CLUSTER; ++sp) {
+        const bool in = have && sp < num_splits;
+        pm[sp] = in ? ld_cluster_f32(mg_m + row, sp) : -INFINITY;
+        pl[sp] = in ? ld_cluster_f32(mg_l + row, sp) : 0.f;
+        po[sp] = in ? ld_cluster_f32(mg_o + idx, sp) : 0.f;
+      }
+      float M = sink;
+#pragma unroll
+      for (int sp = 0; sp < ATT_MAX_CLUSTER; ++sp) M = fmaxf(M, pm[sp]);
+      const float U = M == -INFINITY ? 0.f : M;
+      float den = exp2f(sink - U), acc = 0.f;
+#pragma unroll
+      for (int sp = 0; sp < ATT_MAX_CLUSTER; ++sp) {
+        if (sp >= num_splits) continue;
+        const float f = exp2f(pm[sp] - U);
+        den += pl[sp] * f;
+        acc += po[sp] * f;
+      }
+      // (warp-uniform) nothing of the other CTAs' shared memory is read after this
+      if (last) asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
+      if (have) out[((size_t)(q0 + row / G) * nq + kvh * G + row % G) * VD + idx % VD] = __float2bfloat16_rn(den > 0.f ? acc / den : 0.f);
+      if (last) break;
+    }
+    asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");      // nobody leaves while its sums are being read
+    return;
+  }
   __threadfence();
   __syncthreads();
   if (tid == 0) {
@@ -557,7 +611,7 @@ attn_small_q_ws_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                        const bf16* __restrict__ qkv, int row_stride, const int* __restrict__ block_tables, int bt_stride,
                        const int* __restrict__ cu_q, const int* __restrict__ seq_lens, bf16* __restrict__ out,
                        float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ counters, int nq,
-                       int nkv, int share, int page_size, AttScale sc, float sink, int window, int num_splits) {
+                       int nkv, int share, int page_size, AttScale sc, float sink, int window, int num_splits, int clustered) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int is_last;
   __shared__ uint64_t full_bar[SQ_STAGES], empty_bar[SQ_STAGES];
@@ -656,10 +710,10 @@ attn_small_q_ws_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
   __syncthreads();                                              // every tile has been read; the stages are free
   if (*abort_flag) {                                            // a wait gave up: let copies in flight land, then leave
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-    return;
+    if (!clustered) return;                                     // (a cluster's CTAs meet at its barriers whatever happened)
   }
   small_q_finish(reinterpret_cast<float*>(KV), m, l, o, rows, G, q0, kvh, r, split, num_splits, nq, nkv, out, part_o, part_ml,
-                 counters, &is_last, sink);
+                 counters, &is_last, sink, clustered != 0);
 }
 
 // --------------------------------------------------------------------------------------------
@@ -812,7 +866,7 @@ static size_t small_q_smem(bool tma) {
   const size_t stages = tma ? (size_t)(SQ_STAGES * BN * (D + VD)) * sizeof(bf16) : (size_t)(SQ_STAGES * BN * (DP + VDP)) * sizeof(bf16);
   return stages + (size_t)16 * DP * sizeof(bf16) + (tma ? 1024 : 0);
 }
-static_assert((size_t)SQ_STAGES * BN * (D + VD) * sizeof(bf16) >= (size_t)(4 * 16 * VD + 128) * sizeof(float),
+static_assert((size_t)SQ_STAGES * BN * (D + VD) * sizeof(bf16) >= (size_t)(5 * 16 * VD + 160) * sizeof(float),
               "the merge of the warps' sums must fit in the stages");
 static size_t tile_smem(bool tma) {
   return tma ? (size_t)(2 * BN * (D + VD)) * sizeof(bf16) + 1024 : (size_t)(2 * BN * (DP + VDP)) * sizeof(bf16);
@@ -850,6 +904,33 @@ struct AttArgs {
   float sink;
 };
 
+// How many clusters of `splits` CTAs of the small-q kernel the device holds at a time (0 if it cannot say): clusters that have to
+// wait for a second round cost more than their quicker merge gives.  Only 2, 4 and 8 splits run as clusters: five do not fill the
+// parts of the device that a cluster lies in (seven requests of 2,000 keys, 0.6B sizes: 921 us a step merged through memory, 1,016
+// as clusters of five; three requests of 1,200 keys in four splits 746 against 701, eighteen of 1,400 in two 1,538 against 1,491).
+static int att_max_clusters(int splits) {
+  static int known[IFB_MAX_DEVICES][ATT_MAX_CLUSTER + 1] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= IFB_MAX_DEVICES) return 0;
+  if (!known[dev][splits]) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(splits);
+    cfg.blockDim = dim3(WS_THREADS);
+    cfg.dynamicSmemBytes = small_q_smem(true);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, attn_small_q_ws_kernel, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    known[dev][splits] = n;
+  }
+  return known[dev][splits];
+}
+
 template <bool TMA>
 static int att_launch(const AttArgs& a, cudaStream_t stream) {
   if (TMA) IFB_ALLOW_SMEM(attn_small_q_ws_kernel, small_q_smem(true));
@@ -861,10 +942,31 @@ static int att_launch(const AttArgs& a, cudaStream_t stream) {
     float* part_ml = a.scratch ? a.scratch + (size_t)a.n_tokens * a.nq * a.num_splits * VD : nullptr;
     dim3 grid(a.num_splits, a.nkv, a.n_req);
     int st;
-    if (TMA)
+    if (TMA && a.num_splits > 1 && a.num_splits <= ATT_MAX_CLUSTER && !(a.num_splits & (a.num_splits - 1)) &&
+        (long long)a.nkv * a.n_req <= att_max_clusters(a.num_splits)) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = grid;
+      cfg.blockDim = dim3(WS_THREADS);
+      cfg.dynamicSmemBytes = small_q_smem(true);
+      cfg.stream = stream;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = a.num_splits;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = ifb_pdl_enabled() ? 2 : 1;
+      cudaError_t e = cudaLaunchKernelEx(&cfg, attn_small_q_ws_kernel, a.k_map, a.v_map, a.rows, a.err, (const bf16*)a.qkv, a.row_stride,
+                                         a.block_tables, a.bt_stride, a.cu_q, a.seq_lens, (bf16*)a.out, part_o, part_ml, a.counters, a.nq,
+                                         a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 1);
+      if (e != cudaSuccess) { cudaGetLastError(); return -(int)e; }
+      st = IFB_OK;
+    } else if (TMA)
       st = ifb_launch(attn_small_q_ws_kernel, grid, dim3(WS_THREADS), small_q_smem(true), stream, a.k_map, a.v_map, a.rows, a.err,
                       (const bf16*)a.qkv, a.row_stride, a.block_tables, a.bt_stride, a.cu_q, a.seq_lens, (bf16*)a.out, part_o, part_ml,
-                      a.counters, a.nq, a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits);
+                      a.counters, a.nq, a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 0);
     else
       st = ifb_launch(attn_small_q_kernel<false>, grid, dim3(THREADS), small_q_smem(false), stream, a.k_map, a.v_map, a.rows, a.err,
                       (const bf16*)a.qkv, a.row_stride, a.k, a.v, a.block_tables, a.bt_stride, a.cu_q, a.seq_lens, (bf16*)a.out, part_o,

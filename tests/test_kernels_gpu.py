@@ -683,6 +683,23 @@ def test_linear_with_a_folded_norm_on_prompts(K, n, hidden, inner, gdt, monkeypa
     torch.testing.assert_close(vals.cpu().double(), ref * g.double(), rtol=1e-2, atol=1e-3)
 
 
+# The splits of a context as a thread-block cluster (2, 4, 8) and merged through scratch memory (the others), with splits that get
+# no keys, requests that are not this kernel's and a window.
+@pytest.mark.parametrize("splits", [1, 2, 4, 5, 8, 9])
+@pytest.mark.parametrize("nq,nkv,d,ps,window", [(16, 8, 128, 16, 0), (16, 1, 64, 32, 0), (6, 3, 128, 16, 70)])
+def test_splits_of_a_context_as_a_cluster(K, splits, nq, nkv, d, ps, window):
+    q_lens, seq_lens = [1, 1, 2, 40, 1], [1, 700, 130, 90, 64]
+    qkv, kv, bt, cu, sl = _attention_case(torch.bfloat16, nq, nkv, d, ps, window, q_lens, seq_lens, 29)
+    n = qkv.shape[0]
+    ref = torch.empty((n, nq * d), dtype=torch.bfloat16)
+    REF.paged_attention(qkv, nq, nkv, d, kv, bt, cu, sl, ref, d ** -0.5, window, max(q_lens), max(seq_lens))
+    out = torch.full((n, nq * d), float("nan"), dtype=torch.bfloat16, device="cuda")
+    K._paged_attention_mma(qkv.cuda(), nq, nkv, d, kv.cuda(), bt.cuda(), cu.cuda(), sl.cuda(), out, d ** -0.5, window,
+                           max(q_lens), max(seq_lens), n, len(q_lens), num_splits=splits)
+    torch.testing.assert_close(out.cpu().float(), ref.float(), rtol=1.6e-2, atol=1.6e-2)
+    K.check_device_errors()
+
+
 # The kernel over pairs of SMs: one and several tiles per pair, ragged rows, features and k, both output types and every epilogue.
 @pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,o,k", [(1, 72, 72), (257, 256, 64), (513, 1000, 136), (2048, 4096, 200), (300, 20000, 1032)])
