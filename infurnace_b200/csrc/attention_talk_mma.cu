@@ -226,7 +226,8 @@ attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
       for (int o = 0; o < 4; ++o) { b[o][0] = b[o][1] = b[o][2] = b[o][3] = 0.f; }
       const uint32_t s_at = tm_smem(Ss) + (uint32_t)(pq * 16);
       // four source heads at a time: their scores (from a peer's shared memory, in a cluster) are asked for together
-      for (int h0 = 0; h0 < H; h0 += 4) {
+      // (rows beyond the tile's queries, 15 of 16 for a decoded token, are not mixed: nothing reads them)
+      for (int h0 = 0; h0 < (pq >> 3 < rows ? H : 0); h0 += 4) {
         float4 sv[4], tv[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -346,7 +347,7 @@ attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
 }
 
 // out[t, h, :] = sum_z parts[t, h, z, :D] * exp(m_z - m) / sum_z l_z * exp(m_z - m), m = max_z m_z, times sigmoid(gate):
-// a warp per (token, head), the parts added in ascending z.
+// a warp per (token, head), the parts' rows added in ascending z.
 template <int D>
 __global__ void __launch_bounds__(128)
 attention_talk_merge_kernel(TalkMmaArgs a) {
@@ -361,22 +362,35 @@ attention_talk_merge_kernel(TalkMmaArgs a) {
   while (hi - lo > 1) { const int mid = (lo + hi) >> 1; if (a.cu_q[mid] <= tok) lo = mid; else hi = mid; }
   const bool live = tok < a.cu_q[a.n_req] && a.seq_lens[lo] > 0;
   const float* p = a.parts + (size_t)item * a.splits * (D + 2);
-  float m = -INFINITY;
-  if (live) for (int z = 0; z < a.splits; ++z) m = fmaxf(m, p[(size_t)z * (D + 2) + D]);
+  // a lane holds the maximum and the sum of parts `lane` and `lane + 32`; the rows of four parts are requested at a time
+  float mz[2] = {-INFINITY, -INFINITY}, lz[2] = {0.f, 0.f};
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int z = lane + 32 * u;
+    if (live && z < a.splits) { mz[u] = p[(size_t)z * (D + 2) + D]; lz[u] = p[(size_t)z * (D + 2) + D + 1]; }
+  }
+  const float m = warp_max(fmaxf(mz[0], mz[1]));
   constexpr int PER = (D + 31) / 32;
-  float acc[PER], l = 0.f;
+  float acc[PER], wz[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) wz[u] = mz[u] == -INFINITY ? 0.f : expf(mz[u] - m);      // 0: a part that saw no key
+  const float l = warp_sum((wz[0] != 0.f ? lz[0] * wz[0] : 0.f) + (wz[1] != 0.f ? lz[1] * wz[1] : 0.f));
 #pragma unroll
   for (int j = 0; j < PER; ++j) acc[j] = 0.f;
-  if (live)
-    for (int z = 0; z < a.splits; ++z) {
-      const float* pz = p + (size_t)z * (D + 2);
-      const float mz = pz[D];
-      if (mz == -INFINITY) continue;               // a split that saw no key
-      const float w = expf(mz - m);
-      l += pz[D + 1] * w;
+  for (int z0 = 0; z0 < (live ? a.splits : 0); z0 += 4) {
+    float row[4][PER], w[4];
 #pragma unroll
-      for (int j = 0; j < PER; ++j) { const int c = lane + 32 * j; if (c < D) acc[j] = fmaf(pz[c], w, acc[j]); }
+    for (int u = 0; u < 4; ++u) {
+      const int z = z0 + u;
+      w[u] = z < a.splits ? __shfl_sync(0xffffffffu, z < 32 ? wz[0] : wz[1], z & 31) : 0.f;
+#pragma unroll
+      for (int j = 0; j < PER; ++j) { const int c = lane + 32 * j; row[u][j] = w[u] != 0.f && c < D ? p[(size_t)z * (D + 2) + c] : 0.f; }
     }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int j = 0; j < PER; ++j) acc[j] = w[u] != 0.f ? fmaf(row[u][j], w[u], acc[j]) : acc[j];
+  }
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
     const int c = lane + 32 * j;

@@ -926,7 +926,7 @@ class CudaKernels:
     def _talk_splits(self, n, r, num_heads, head_dim, chunk, max_q_len, max_seq_len):
         """CTAs that share the keys of one query tile of the tensor-core talking attention: 1 unless the step's tiles
         alone leave most SMs idle (few query tokens) and a query may see many keys; then enough to fill the device
-        once, with no fewer than four tiles of 32 keys each.  Up to 4 for a prompt of few tiles (see below)."""
+        once, with no fewer than four tiles of 32 keys each (decoded tokens: one).  Up to 4 for a prompt of few tiles (see below)."""
         if not max_q_len or not max_seq_len:
             return 1
         reach = min(chunk, max_seq_len) if chunk else max_seq_len
@@ -935,6 +935,9 @@ class CudaKernels:
             # a prompt: a tile late in its chunk has many times the keys of an early one, and with less than two CTAs
             # per SM the longest tile is the kernel's time; shares of at most a quarter of the keys even that out
             return max(1, min(4, reach // 128)) if tiles < 2 * self.sm_count else 1
+        if max_q_len == 1:
+            # decoded tokens: a tile of 32 keys is a chain of round trips (some 5 us), so every tile gets a CTA of its own
+            return max(1, min(self.sm_count // max(1, tiles), reach // 32, 32))
         return max(1, min(self.sm_count // max(1, tiles), reach // 128, 32))
 
     # ------------------------------------------------------------------ sandwich-norm blocks, state recurrences, routed experts
