@@ -46,7 +46,7 @@ template <int EPI_, int MH_, int NACC_, int STAGES_> struct GemmCfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int TMEM_COLS = MH * NACC;                 // 128, 256 or 512 columns of 32 bits
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /* alignment */ + 256 /* barriers */;
-  static constexpr bool SHARED_K = MH == 1 && 2 * SMEM_BYTES > 226 * 1024;      // the deep shapes: the k range may be shared by a cluster
+  static constexpr bool SHARED_K = MH == 1 && FO == 128 && 2 * SMEM_BYTES > 226 * 1024;      // the deep shapes: the k range may be shared by a cluster
   // float32 accumulator, bfloat16 a and b, both K-major, M = 128, N = NACC
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NACC >> 3) << 17) | ((uint32_t)(G_BM >> 4) << 24);
 };
@@ -1518,13 +1518,14 @@ static int tc_sm_count() {
   }
   return sm_count;
 }
-// By measurement.  With the silu_gate epilogue: the persistent kernel (its tile already accumulates 256 columns per
+// By measurement.  With the silu_gate epilogue: tiles of 64 features (64 gate and 64 up rows, one tile per CTA, a deep ring) where
+// they are no more than the SMs: twice the SMs of tiles of 128, each with two thirds of the bytes.  Else the persistent kernel (its tile already accumulates 256 columns per
 // product, and the heavy epilogue of one tile runs beside the products of the next).  Otherwise one tile per CTA:
 // the wide shape when there are enough wide tiles to fill the SMs (a 256 x 256 tile reads half the operand bytes
 // per product from shared memory, which is what bounds these kernels), else the deep or the narrow one.
 static int tc_pick_shape(int epi, int n, int o) {
-  if (epi) return 4;
   const int sm_count = tc_sm_count();
+  if (epi) return (long long)((o + 63) / 64) * ((n + G_BM - 1) / G_BM) <= sm_count ? 7 : 4;
   const long long tn = (long long)((o + 127) / 128) * ((n + G_BM - 1) / G_BM);
   const long long tw = (long long)((o + 255) / 256) * ((n + 2 * G_BM - 1) / (2 * G_BM));
   const double cost_narrow = (double)((tn + 2 * sm_count - 1) / (2 * sm_count));
@@ -1583,6 +1584,10 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
     return tc_launch_pair<Pair, TO>(x, w, out, n, o, k, err, s, fold);
   }
   if (fold.res_x && shape > 3) return IFB_ERR_ARG;        // the making side is the one-tile kernel's
+  if (shape == 7) {
+    if constexpr (EPI) return tc_launch_cfg<GemmCfg<1, 1, 128, 6>, TO>(x, w, out, n, o, k, err, s, fold);
+    return IFB_ERR_ARG;
+  }
   if (shape == 5 && !EPI) return tc_launch_persistent<P256, TO>(x, w, out, n, o, k, err, tc_sm_count(), s, fold);
   if (shape == 4 || shape == 5) return tc_launch_persistent<P128, TO>(x, w, out, n, o, k, err, tc_sm_count(), s, fold);
   if (shape == 3) return tc_launch_cfg<Wide, TO>(x, w, out, n, o, k, err, s, fold);
@@ -1594,8 +1599,8 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
 // 1 + 16 * u: gated with u in silu's place.
 // x [n_rows, k] and w [out_features (x2 for the silu_gate epilogue), k] bfloat16, 16-byte aligned, k a multiple of 8;
 // out bfloat16 or float32.  `err` points to a device int that stays 0 unless a bounded wait gave up.  shape: 0 lets the
-// library choose, 1-3 force the one-tile-per-CTA kernel narrow, deep or wide, 6 the kernel over pairs of SMs, 4 and 5 the persistent kernel with tiles
-// of 128 or 256 features.  splits 2 to 8: the k range of a tile of 128 x 128 is shared by a cluster of
+// library choose, 1-3 force the one-tile-per-CTA kernel narrow, deep or wide, 4 and 5 the persistent kernel with tiles of 128
+// or 256 features, 6 the kernel over pairs of SMs, 7 (silu_gate) the one-tile kernel with 64 features.  splits 2 to 8: the k range of a tile of 128 x 128 is shared by a cluster of
 // that many CTAs, whose parts are added in a fixed order; for few tiles of a long k (a step of some tens of tokens).
 // scale_partials (may be null): [scale_parts][n_rows] sums of squares; output row n is multiplied by
 // rsqrt(sum_p partials[p][n] / scale_width + scale_eps) before the epilogue.
@@ -1613,7 +1618,7 @@ IFB_EXPORT int ifb_linear_tcgen05_ex(const void* x, const void* w, void* out, in
   epilogue &= 15;
   if (epilogue > 1 || unary < 0 || unary > IFB_UNARY_LAST || (unary && res_x) || (bias && epilogue))
     return IFB_ERR_ARG;
-  if (shape < 0 || shape > 6 || splits < 0 || splits > 8) return IFB_ERR_ARG;
+  if (shape < 0 || shape > 7 || splits < 0 || splits > 8) return IFB_ERR_ARG;
   if (scale_partials && (scale_parts < 1 || scale_width < 1)) return IFB_ERR_ARG;
   if (res_x && (!res_g || !res_partials || ((uintptr_t)res_x & 15))) return IFB_ERR_ARG;
   TcFold fold = {};

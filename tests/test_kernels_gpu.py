@@ -733,3 +733,21 @@ def test_linear_with_a_folded_norm_over_pairs(K, n, hidden, inner, epilogue, mon
 @pytest.mark.parametrize("norm,rotate,scaled", [(True, True, True), (False, True, False), (True, False, False)])
 def test_qkv_product_over_pairs_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, norm, rotate, scaled):
     test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, 128, 520, 16, norm, rotate, scaled)
+
+
+# Gate and up of a short prompt in tiles of 64 features: ragged rows, features and k, with and without a folded norm's factors.
+@pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,o,k", [(1, 40, 72), (129, 3072, 1024), (200, 1000, 136), (513, 65, 520)])
+@pytest.mark.parametrize("epilogue,scaled", [("silu_gate", False), ("silu_gate", True), ("gelu_gate", False)])
+def test_gated_product_in_tiles_of_64_features(K, od, n, o, k, epilogue, scaled):
+    from infurnace_b200.kernels.cuda import EPILOGUES
+    x, w = rnd((n, k), torch.bfloat16, 4).cuda(), rnd((2 * o, k), torch.bfloat16, 5, scale=k ** -0.5).cuda()
+    partials = torch.rand((3, n)).cuda() * 40 + 1
+    y = x.double() @ w.double().t()
+    if scaled:
+        y = y * torch.rsqrt(partials.double().sum(0) / 55.0 + 1e-5)[:, None]
+    g = torch.nn.functional.silu(y[:, :o]) if epilogue == "silu_gate" else torch.nn.functional.gelu(y[:, :o], approximate="tanh")
+    out = torch.full((n, o), float("nan"), dtype=od, device="cuda")
+    K._linear_tcgen05(x, w, out, n, o, k, EPILOGUES[epilogue], shape=7, row_scale=(partials, 3, 1e-5, 55) if scaled else None)
+    K.check_device_errors()
+    torch.testing.assert_close(out.double(), g * y[:, o:], rtol=1.6e-2 if od == torch.bfloat16 else 4e-3, atol=1e-2 if od == torch.bfloat16 else 2e-3)
