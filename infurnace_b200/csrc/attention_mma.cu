@@ -369,12 +369,17 @@ __device__ __forceinline__ void small_q_finish(float* scratch, float (&m)[2], fl
       sm_m[warp * 16 + rowA] = m[0]; sm_m[warp * 16 + rowB] = m[1];
       sm_l[warp * 16 + rowA] = l[0]; sm_l[warp * 16 + rowB] = l[1];
     }
+    // only the rows that exist (two for a decoded token and a group of two): they lie a multiple of all banks apart, and writing
+    // all sixteen cost a microsecond of a launch's five
+    if (rowA < rows) {
 #pragma unroll
-    for (int n = 0; n < VD / 8; ++n) {
-      const int col = n * 8 + ((lane & 3) << 1);
-      float* pa = sm_o + ((size_t)warp * 16 + rowA) * VD + col;
-      float* pb = sm_o + ((size_t)warp * 16 + rowB) * VD + col;
-      pa[0] = o[n][0]; pa[1] = o[n][1]; pb[0] = o[n][2]; pb[1] = o[n][3];
+      for (int n = 0; n < VD / 8; ++n)
+        *reinterpret_cast<float2*>(sm_o + ((size_t)warp * 16 + rowA) * VD + n * 8 + ((lane & 3) << 1)) = make_float2(o[n][0], o[n][1]);
+    }
+    if (rowB < rows) {
+#pragma unroll
+      for (int n = 0; n < VD / 8; ++n)
+        *reinterpret_cast<float2*>(sm_o + ((size_t)warp * 16 + rowB) * VD + n * 8 + ((lane & 3) << 1)) = make_float2(o[n][2], o[n][3]);
     }
   }
   __syncthreads();
