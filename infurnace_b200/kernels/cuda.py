@@ -335,6 +335,10 @@ class CudaKernels:
     def _tcgen05_splits_rule(self, n, o, k, epi):
         if n > (128 if epi else 512):
             return 1
+        if epi and k <= 1024 and -(-o // 64) <= self.sm_count:
+            # gate and up of a small model: a CTA per 64 features walks the whole k range in less time than a cluster's sum takes
+            # (with the q | k | v product of the same k likewise, 64 decoding requests of the 0.6B sizes 1,647 to 1,503 us)
+            return 1
         tiles = -(-o // 128) * -(-n // 128)
         for splits in range(min(8, k // self.tc_split_min_k), 1, -1):
             if splits not in self._tc_clusters:
@@ -500,8 +504,9 @@ class CudaKernels:
             raise KernelError("linear_qkv_rope_store: no kernel takes these sizes (see can_fuse_qkv)")
         if route == "tcgen05":
             self._err_armed = True
-            # (more than one tile of rows: the cluster's sum would take longer over the heads than the shorter k range saves)
-            splits = self.tcgen05_splits(n, width, k) if n <= 128 else 1
+            # (more than one tile of rows, or a short k: the cluster's sum would take longer over the heads than the shared k
+            # range saves)
+            splits = self.tcgen05_splits(n, width, k) if n <= 128 and k > 1024 else 1
             self.tc_shared_k_calls += splits > 1
             self.tc_folded_calls += partials is not None
             _check(self._tc_lib().ifb_linear_tcgen05_qkv(
