@@ -92,7 +92,7 @@ __device__ __forceinline__ void gv_cluster_barrier() {
 // 2: a warp walks a long k range and keeps the memory pipe full while it multiplies (large models, where the
 // bytes count).
 template <int NB, int EPI, int WARPS, typename TO, int STAGES>
-__global__ void __launch_bounds__(WARPS * 32, (EPI == 4 && WARPS == 8) ? 2 : (EPI == 0 && WARPS == 8 && STAGES == 1 && NB == 1) ? IFB_GV_LM_BLOCKS
+__global__ void __launch_bounds__(WARPS * 32, (EPI == 4 && WARPS == 8) ? (STAGES == 1 ? 3 : 2) : (EPI == 0 && WARPS == 8 && STAGES == 1 && NB == 1) ? IFB_GV_LM_BLOCKS
                                   : (EPI == 2 && NB == 1 && WARPS <= 16 && (WARPS == 16 || STAGES == 2)) ? 2 : 0)
 linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* __restrict__ out, int n_rows, int o_out,
                    int k_dim, GvRowScale rs, GvResidual res, GvQkv qk) {
@@ -435,6 +435,7 @@ static int gv_launch(const void* x, const void* w, void* out, int n, int o, int 
   const int per_cta = EPI == 4 ? 8 : res_f.feat;
   dim3 grid((o + per_cta - 1) / per_cta, (n + NB * 8 - 1) / (NB * 8));
   // matrices beyond GV_EARLY_BYTES are streamed; a launch ahead of the predecessor's end costs them more than it hides
+  // (eight layers of the 8B sizes, all ahead: two requests 909 to 1,130 us, one at 1,000 keys 920 to 1,087)
   const bool early = (size_t)o * k * ((EPI == 1 || EPI == 4) ? 4 : 2) <= GV_EARLY_BYTES;
   return ifb_launch_opt(early, linear_gemv_kernel<NB, EPI, WARPS, TO, STAGES>, grid, dim3(WARPS * 32), smem, s, (const bf16*)x,
                         (const bf16*)w, (TO*)out, n, o, k, rs, res_f, GvQkv{});
@@ -474,12 +475,13 @@ template <int EPI, int WARPS, typename TO, int STAGES = 1>
 static int gv_by_n(int nb, const void* x, const void* w, void* out, int n, int o, int k, const GvRowScale& rs,
                    const GvResidual& res, cudaStream_t s) {
   switch (nb) {
-    // one block of tokens of a long k (two stages): the silu_gate epilogue in its 8-features-per-CTA form, two CTAs per SM
-    // (40 against 35 to 37 us for the 201 MB of the 8B sizes, 90 against 83 to 85 for the 524 MB of the 32B sizes; with more
-    // blocks of tokens it is the slower one, and for a short k it gains in a chain of its own kind but not in the step)
+    // one block of tokens: the silu_gate epilogue in its 8-features-per-CTA form, two CTAs per SM for a long k (40 against 35 to
+    // 37 us for the 201 MB of the 8B sizes, 90 against 83 to 85 for the 524 MB of the 32B sizes; with more blocks of tokens it is
+    // the slower one), three for a short one (3,072 features: 384 CTAs over 148 SMs instead of 192, the fullest SM with 96 KB of
+    // weights instead of 128; held to 80 registers, or the third does not fit: one decoded token of the 0.6B sizes 595 to 576 us)
     case 1:
       if (g_gv_gate_plan < 0) return gv_launch<1, EPI, WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);
-      return gv_launch<1, ((EPI == 1 && STAGES == 2) ? 4 : EPI), WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);
+      return gv_launch<1, (EPI == 1 ? 4 : EPI), WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);
     case 2: return gv_launch<2, EPI, WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);
     case 4: return gv_launch<4, EPI, WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);
     default: return gv_launch<8, EPI, WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);
