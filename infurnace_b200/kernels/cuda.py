@@ -267,8 +267,9 @@ class CudaKernels:
         range in clusters (:meth:`tcgen05_splits`): the tcgen05 kernel in that form, which streams a long k
         faster than the few-rows kernel.  Else up to 8 rows: the few-rows kernel.  Between, by measurement:
         the few-rows kernel re-reads the rows from L2 in every CTA, so for a large weight matrix (from 2^24
-        elements, or from 33 rows and 4,096 features) the tcgen05 kernel, which streams the weights once
-        through its tiles, is the faster one although most of its 128-row tile is empty."""
+        elements, or 4,096 features from 33 rows on, from 17 where a k of at most 1,024 needs no cluster: 17 to 32
+        decoding requests of the 0.6B sizes 1,157 to 1,238 us a step against 1,094 to 1,172) the tcgen05 kernel, which
+        streams the weights once through its tiles, is the faster one although most of its 128-row tile is empty."""
         if n >= self.tc_min_rows:
             return True
         if shared_k and epilogue == "none" and n >= self._shared_k_min_rows(w) and w.dtype == torch.bfloat16 \
@@ -276,7 +277,7 @@ class CudaKernels:
             return True
         if n <= 8:
             return False
-        return w.numel() >= (1 << 24) or (n >= 33 and w.shape[0] >= 4096)
+        return w.numel() >= (1 << 24) or (n >= (17 if w.shape[1] <= 1024 else 33) and w.shape[0] >= 4096)
 
     def _shared_k_min_rows(self, w):
         """From how many rows the tcgen05 kernel with a shared k range beats the few-rows kernel, by
