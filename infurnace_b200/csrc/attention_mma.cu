@@ -604,6 +604,14 @@ attn_small_q_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
 // "full" barrier (armed with the tile's bytes by the producer) and an "empty" barrier (one arrival per consumer warp
 // when it has read the tile), so no warp waits for another at a tile's end: a slow warp holds back only the refill
 // of its own stage.
+//
+// beside: the kernel before this one is the tcgen05 attention kernel over the same step's longer requests, of which
+// this one reads nothing.  Every CTA of that kernel waits for its own predecessor, the kernel that stored this step's
+// queries, keys and values, before it triggers or exits, so by the time a CTA of this grid runs those are complete and it
+// need not wait for its neighbour; the two write different rows of the output.  It waits at its end instead, on every
+// path, so that the kernel after this one, which waits for this grid alone, still comes after both.  The requests that
+// decode then run on the SMs that the prompts' items leave free (a portion of a prompt beside fourteen decoding requests, 0.6B
+// sizes: 4,398 to 4,356 us for two steps; 4,070 with the prompts' kernel by slots).
 // --------------------------------------------------------------------------------------------
 constexpr int WS_THREADS = 160;
 __device__ __forceinline__ void att_mbar_arrive(uint64_t* bar) {
@@ -616,7 +624,8 @@ attn_small_q_ws_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                        const bf16* __restrict__ qkv, int row_stride, const int* __restrict__ block_tables, int bt_stride,
                        const int* __restrict__ cu_q, const int* __restrict__ seq_lens, bf16* __restrict__ out,
                        float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ counters, int nq,
-                       int nkv, int share, int page_size, AttScale sc, float sink, int window, int num_splits, int clustered) {
+                       int nkv, int share, int page_size, AttScale sc, float sink, int window, int num_splits, int clustered,
+                       int beside) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int is_last;
   __shared__ uint64_t full_bar[SQ_STAGES], empty_bar[SQ_STAGES];
@@ -667,7 +676,7 @@ attn_small_q_ws_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
     // The kernel before this one wrote the keys and values of this step's tokens (positions >= p_first) and nothing
     // else that is read here, so tiles of older keys are requested without waiting for it: the first stages fill
     // while it still runs.
-    bool waited = false;
+    bool waited = beside != 0;
     for (int t = 0; t < n_tiles && ok; ++t) {
       const int stage = t % SQ_STAGES;
       if (!waited && T0 + (t + 1) * BN > p_first) {
@@ -681,7 +690,7 @@ attn_small_q_ws_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
     }
   } else {
     // ---- consumers: the query rows (row = token * G + head-in-group), then the tiles
-    ifb_pdl_wait();
+    if (!beside) ifb_pdl_wait();
     ifb_pdl_trigger();
     for (int c = tid; c < 16 * KCH; c += 128) {
       const int row = c / KCH, ch = c % KCH;
@@ -715,10 +724,14 @@ attn_small_q_ws_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
   __syncthreads();                                              // every tile has been read; the stages are free
   if (*abort_flag) {                                            // a wait gave up: let copies in flight land, then leave
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
-    if (!clustered) return;                                     // (a cluster's CTAs meet at its barriers whatever happened)
+    if (!clustered) {
+      ifb_pdl_wait();
+      return;
+    }                                                           // (a cluster's CTAs meet at its barriers whatever happened)
   }
   small_q_finish(reinterpret_cast<float*>(KV), m, l, o, rows, G, q0, kvh, r, split, num_splits, nq, nkv, out, part_o, part_ml,
                  counters, &is_last, sink, clustered != 0);
+  if (beside) ifb_pdl_wait();                                   // see `beside`: this grid ends after the one it ran beside
 }
 
 // --------------------------------------------------------------------------------------------
@@ -965,13 +978,13 @@ static int att_launch(const AttArgs& a, cudaStream_t stream) {
       cfg.numAttrs = ifb_pdl_enabled() ? 2 : 1;
       cudaError_t e = cudaLaunchKernelEx(&cfg, attn_small_q_ws_kernel, a.k_map, a.v_map, a.rows, a.err, (const bf16*)a.qkv, a.row_stride,
                                          a.block_tables, a.bt_stride, a.cu_q, a.seq_lens, (bf16*)a.out, part_o, part_ml, a.counters, a.nq,
-                                         a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 1);
+                                         a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 1, (int)(a.run_small == 2));
       if (e != cudaSuccess) { cudaGetLastError(); return -(int)e; }
       st = IFB_OK;
     } else if (TMA)
       st = ifb_launch(attn_small_q_ws_kernel, grid, dim3(WS_THREADS), small_q_smem(true), stream, a.k_map, a.v_map, a.rows, a.err,
                       (const bf16*)a.qkv, a.row_stride, a.block_tables, a.bt_stride, a.cu_q, a.seq_lens, (bf16*)a.out, part_o, part_ml,
-                      a.counters, a.nq, a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 0);
+                      a.counters, a.nq, a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 0, (int)(a.run_small == 2));
     else
       st = ifb_launch(attn_small_q_kernel<false>, grid, dim3(THREADS), small_q_smem(false), stream, a.k_map, a.v_map, a.rows, a.err,
                       (const bf16*)a.qkv, a.row_stride, a.k, a.v, a.block_tables, a.bt_stride, a.cu_q, a.seq_lens, (bf16*)a.out, part_o,
@@ -991,7 +1004,8 @@ static int att_launch(const AttArgs& a, cudaStream_t stream) {
 // qkv: the q heads are the first nq * d columns of its rows.  k_pages / v_pages: the two streams, pages k_page_stride /
 // v_page_stride elements apart, num_pages of them, each [kv heads][page_size][d or dv].  nkv: groups of query heads, `share`
 // of which read one key/value head.  max_q_len: the most query tokens any request brings.  run_small / run_tiles: which of the
-// two kernels to launch; requests are routed by rows = q_len * (nq / nkv) <= 16.  err: a device int that stays 0 unless a
+// two kernels to launch (run_small 2: the launch before this one on the stream is the tcgen05 attention kernel of this step);
+// requests are routed by rows = q_len * (nq / nkv) <= 16.  err: a device int that stays 0 unless a
 // bounded wait gave up (TMA path).  use_tma 0 forces the cp.async path.  softcap: 0 none (a library compiled with SOFTCAP
 // takes a positive one and no other takes one).  has_sink: exp(sink) joins the denominators.
 IFB_EXPORT int ifb_attention_mma(const void* qkv, int row_stride, const void* k_pages, long long k_page_stride, const void* v_pages,

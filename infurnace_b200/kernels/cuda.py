@@ -712,7 +712,7 @@ class CudaKernels:
         lib = self.attention_library(head_dim, weight_terms, value_head_dim, bool(softcap))
         group = num_heads // num_kv_heads
         page_size = k[2]
-        only_small = max_q_len * group <= 16
+        only_small, behind_tiles = max_q_len * group <= 16, False
         if num_splits is None:
             num_splits = self.attention_splits(r, num_kv_heads, max_seq_len, window)
         need = lib.ifb_attention_mma_scratch_floats(n, num_heads, num_splits)
@@ -734,7 +734,7 @@ class CudaKernels:
                                        kind=2 if score_bound else 1 if softcap else 0)
             if min_q_len * group > 16:
                 return                 # no request of this step is left for the small-q kernel
-            only_small = True          # the tile kernel's requests are done; the small-q kernel takes the rest
+            only_small = behind_tiles = True       # the tile kernel has its requests; the small-q kernel takes the rest beside it
         self.launches += 1 + (0 if only_small else 1)
         self.small_q_calls += 1
         if self.attention_tma and head_dim % 64 == 0 and value_head_dim % 64 == 0 and page_size in (16, 32, 64):
@@ -744,7 +744,7 @@ class CudaKernels:
             qkv.data_ptr(), qkv.stride(0), k[0], k[1], v[0], v[1], num_pages, block_tables.data_ptr(), block_tables.stride(0),
             cu_q.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), _ptr(scratch), _ptr(counters), self._dev_err.data_ptr(), n, r, num_heads,
             num_kv_heads, share, head_dim, value_head_dim, page_size, float(scale), int(window), float(softcap or 0.0),
-            0 if sink is None else 1, float(sink or 0.0), int(max_q_len), int(num_splits), 1, 0 if only_small else 1,
+            0 if sink is None else 1, float(sink or 0.0), int(max_q_len), int(num_splits), 2 if behind_tiles else 1, 0 if only_small else 1,
             1 if self.attention_tma else 0, self._stream()), "paged_attention")
 
     # ------------------------------------------------------------------ post-norm sublayers, recurrence, talking attention

@@ -700,6 +700,42 @@ def test_splits_of_a_context_as_a_cluster(K, splits, nq, nkv, d, ps, window):
     K.check_device_errors()
 
 
+# A prompt's portion beside requests that decode: two kernels that run side by side, behind the one that makes the queries and before
+# one that reads all their rows.  Whatever overlaps, the numbers are those of launches that wait for one another.
+@pytest.mark.parametrize("prompt", [9, 130, 700])
+@pytest.mark.parametrize("splits", [1, 4, 5])
+def test_attention_beside_attention(K, prompt, splits):
+    nq, nkv, d, ps, rounds = 16, 8, 128, 16, 8
+    q_lens = [1, 1, 2, prompt, 1, 8, 1]
+    seq_lens = [1, 900, 130, prompt + 40, 1500, 64, 2000]
+    qkv, kv, bt, cu, sl = (t.cuda() for t in _attention_case(torch.bfloat16, nq, nkv, d, ps, 0, q_lens, seq_lens, 30))
+    n, width = qkv.shape
+    ws = [rnd((width, nq * d), torch.bfloat16, 40 + i, scale=(nq * d) ** -0.5).cuda() for i in range(2)]
+    x0 = rnd((n, nq * d), torch.bfloat16, 39).cuda()
+
+    def run(apart):
+        x = x0.clone()
+        for i in range(rounds):
+            q, out = torch.empty_like(qkv), torch.full((n, nq * d), float("nan"), dtype=torch.bfloat16, device="cuda")
+            K.linear(x, ws[i % 2], q)
+            if apart:
+                torch.cuda.synchronize()
+            K._paged_attention_mma(q, nq, nkv, d, kv, bt, cu, sl, out, d ** -0.5, 0, max(q_lens), max(seq_lens), n, len(q_lens),
+                                   num_splits=splits)
+            if apart:
+                torch.cuda.synchronize()
+            x = torch.empty_like(x0)
+            K.linear(out, ws[0][:nq * d], x)
+        torch.cuda.synchronize()
+        return x
+
+    want = run(True)
+    assert torch.isfinite(want.float()).all()
+    for _ in range(3):
+        assert torch.equal(run(False), want)
+    K.check_device_errors()
+
+
 # The kernel over pairs of SMs: one and several tiles per pair, ragged rows, features and k, both output types and every epilogue.
 @pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,o,k", [(1, 72, 72), (257, 256, 64), (513, 1000, 136), (2048, 4096, 200), (300, 20000, 1032)])
