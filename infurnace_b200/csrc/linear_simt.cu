@@ -2,7 +2,7 @@
 // cores and no reduced-precision mode.  It is the product of the true 32-bit path and the
 // fallback for operand dtypes or sizes that the tensor-core kernels refuse.  Any n, o, k.
 //
-// Three kernels.  Float32 operands: `rows32_kernel` up to 32 rows and `tile32_kernel` beyond; operands of which one is
+// Three kernels.  Float32 operands: `rows32_kernel` up to 16 rows and `tile32_kernel` beyond; operands of which one is
 // bfloat16: `linear_simt_kernel`.  The order in which an output's products are added depends on k alone, never on the
 // number of rows or on the row's place, so a token's values are the same bits in every way of cutting the work:
 // the bfloat16 combinations add them one after the other; float32 operands in S32_GROUPS consecutive parts of the k range,
