@@ -611,7 +611,7 @@ attn_small_q_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
 // need not wait for its neighbour; the two write different rows of the output.  It waits at its end instead, on every
 // path, so that the kernel after this one, which waits for this grid alone, still comes after both.  The requests that
 // decode then run on the SMs that the prompts' items leave free (a portion of a prompt beside fourteen decoding requests, 0.6B
-// sizes: 4,398 to 4,356 us for two steps; 4,070 with the prompts' kernel by slots).
+// sizes: 4,398 to 4,356 us for two steps).
 // --------------------------------------------------------------------------------------------
 constexpr int WS_THREADS = 160;
 __device__ __forceinline__ void att_mbar_arrive(uint64_t* bar) {

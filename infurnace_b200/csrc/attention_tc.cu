@@ -292,73 +292,27 @@ struct TcBars {
   uint64_t q_full, q_empty, o_free, k_full[2], v_full[2], k_empty[2][2], v_empty[2][2], s_full[2][2], p_ready[2][2], o_done[2];
 };
 
-// The requests of a CTA.  Those of the step with more than 16 rows, counted from the first request on, go to the grid's z
-// slots in turn; a slot's CTAs take one after the other, and the barriers' phases run on from request to request.  A z per
-// request would be as right, but in a step that mixes prompts with decoding requests nearly all of its CTAs have nothing to do, and
-// each has to wait for an SM's shared memory to say so: a portion of 400 tokens beside fourteen requests, 0.6B sizes, took 18.1 us a
-// layer with 56 x 15 CTAs and takes 12.5 with 56 x 4.
-constexpr int TC_MAX_LIST = 64;
-struct TcRequest { int r, q0, q_len, p_first, nt, n_rounds; };
-struct TcList { int count; TcRequest of[TC_MAX_LIST]; };      // ceil(n_req / slots) <= TC_MAX_LIST: the launch sees to it
-
-// Whole warps, 32 requests a look; `fill` for one warp, which writes the list.  True: some request has an item for this CTA.
-__device__ __forceinline__ bool tc_list_requests(TcList& list, bool fill, int n_req, int G, int nkv, int tpt, const int* __restrict__ cu_q,
-                                                 const int* __restrict__ seq_lens) {
-  const int lane = threadIdx.x & 31;
-  int rank = 0;
-  bool mine = false;
-  for (int base = 0; base < n_req; base += 32) {
-    const int r = base + lane;
-    const int q0 = r < n_req ? cu_q[r] : 0, q_len = r < n_req ? cu_q[r + 1] - q0 : 0;
-    const bool is_long = q_len * G > 16;
-    const uint32_t longs = __ballot_sync(0xffffffffu, is_long);
-    const int place = rank + __popc(longs & ((1u << lane) - 1));
-    if (is_long && place % (int)gridDim.z == (int)blockIdx.z) {
-      const int nt = (q_len + tpt - 1) / tpt;
-      mine = mine || (int)blockIdx.x < nt * nkv;
-      if (fill) list.of[place / gridDim.z] = {r, q0, q_len, seq_lens[r] - q_len, nt, (nt * nkv + (int)gridDim.x - 1) / (int)gridDim.x};
-    }
-    rank += __popc(longs);
-  }
-  // long requests of places blockIdx.z, blockIdx.z + slots, ...
-  if (fill && lane == 0) list.count = (rank - (int)blockIdx.z + (int)gridDim.z - 1) / (int)gridDim.z;
-  return __any_sync(0xffffffffu, mine) != 0;
-}
-
 // One work item: a query tile of one key/value head.
 struct TcItem {
-  int r, q0, p_first, kvh, t0, t1, lo, hi, T0, n_half, n_tiles;
+  int kvh, t0, t1, lo, hi, T0, n_half, n_tiles;
 };
-// The next item of a CTA's walk; j and k, its place in the list and its round, start as 0.  Within a request (item = tile
-// rank * nkv + head, the tiles with the most keys first) a CTA goes forwards in even rounds, backwards in odd ones, so that
-// the CTAs with the longest items of one round get the shortest of the next.
-__device__ __forceinline__ bool tc_next_item(const TcList& list, int& j, int& k, int nkv, int tpt, int window, TcItem& it) {
-  const int cta = blockIdx.x, ctas = gridDim.x;
-  while (j < list.count) {
-    const TcRequest& q = list.of[j];
-    if (k >= q.n_rounds) {
-      ++j;
-      k = 0;
-      continue;
-    }
-    const int idx = (k & 1) ? (k + 1) * ctas - 1 - cta : k * ctas + cta;
-    ++k;
-    if (idx >= q.nt * nkv) continue;
-    const int rank = idx / nkv;
-    it.r = q.r;
-    it.q0 = q.q0;
-    it.p_first = q.p_first;
-    it.kvh = idx % nkv;
-    it.t0 = (q.nt - 1 - rank) * tpt;
-    it.t1 = min(q.q_len, it.t0 + tpt);
-    it.lo = window > 0 ? max(0, it.p_first + it.t0 - window + 1) : 0;
-    it.hi = it.p_first + it.t1 - 1;
-    it.T0 = (it.lo / BK) * BK;
-    it.n_half = (it.hi + 1 - it.T0 + SUB - 1) / SUB;     // halves of 64 keys; stream x works on half x of every tile of 128
-    it.n_tiles = (it.n_half + 1) / 2;
-    return true;
-  }
-  return false;
+// Round k of a CTA's walk over the request's items (item = tile rank * nkv + head, the tiles with the most keys first):
+// forwards in even rounds, backwards in odd ones, so that the CTAs with the longest items of one round get the
+// shortest of the next.  False: the round has no item for this CTA.
+__device__ __forceinline__ bool tc_item(int k, int cta, int ctas, int nt, int nkv, int tpt, int q_len, int p_first, int window,
+                                        TcItem& it) {
+  const int idx = (k & 1) ? (k + 1) * ctas - 1 - cta : k * ctas + cta;
+  if (idx >= nt * nkv) return false;
+  const int rank = idx / nkv;
+  it.kvh = idx % nkv;
+  it.t0 = (nt - 1 - rank) * tpt;
+  it.t1 = min(q_len, it.t0 + tpt);
+  it.lo = window > 0 ? max(0, p_first + it.t0 - window + 1) : 0;
+  it.hi = p_first + it.t1 - 1;
+  it.T0 = (it.lo / BK) * BK;
+  it.n_half = (it.hi + 1 - it.T0 + SUB - 1) / SUB;       // halves of 64 keys; stream x works on half x of every tile of 128
+  it.n_tiles = (it.n_half + 1) / 2;
+  return true;
 }
 
 // The two streams as matrices of rows: how many rows a page spans and how many rows there are.
@@ -368,11 +322,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                     const __grid_constant__ CUtensorMap v_map, TcRows mrows, int* __restrict__ err,
                     const int* __restrict__ block_tables, int bt_stride, const int* __restrict__ cu_q,
-                    const int* __restrict__ seq_lens, bf16* __restrict__ out, int n_req, int nq, int nkv, int share, int page_size,
+                    const int* __restrict__ seq_lens, bf16* __restrict__ out, int nq, int nkv, int share, int page_size,
                     TcScore score, float sink, int window) {
   extern __shared__ unsigned char tc_smem_raw[];
   __shared__ TcBars bars;
-  __shared__ TcList list;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_word;
   __shared__ float merge_m[2][2][ROWS], merge_l[2][2][ROWS];       // [item parity][stream][row]: maxima and sums, exchanged
@@ -383,11 +336,19 @@ attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
   unsigned char* Ks = smem + K_BYTES;                        // two stages of K tiles, same layout
   unsigned char* Vs = smem + 3 * K_BYTES;                    // two stages of V tiles, [VH][128 rows][128 bytes]
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform
+  const int r = blockIdx.z, cta = blockIdx.x, ctas = gridDim.x;
   const int G = nq / nkv;
-  const int tpt = ROWS / G;                                  // tokens per query tile
+  const int q0 = cu_q[r], q_len = cu_q[r + 1] - q0, L = seq_lens[r];
   // every exit path waits for the predecessor: a grid none of whose threads waited could end before the kernel that
   // stores this step's keys, and its own successor, which waits for this grid alone, would then start too early
-  if (!tc_list_requests(list, warp == 0, n_req, G, nkv, tpt, cu_q, seq_lens)) { ifb_pdl_wait(); return; }
+  if (q_len * G <= 16) { ifb_pdl_wait(); return; }           // the small-q kernel's request
+  const int tpt = ROWS / G;                                  // tokens per query tile
+  const int nt = (q_len + tpt - 1) / tpt;
+  const int n_items = nt * nkv;
+  if (cta >= n_items) { ifb_pdl_wait(); return; }
+  const int n_rounds = (n_items + ctas - 1) / ctas;
+  const int p_first = L - q_len;
+  const int* bt = block_tables + (size_t)r * bt_stride;
   const int ps_shift = __ffs(page_size) - 1;
 
   if (tpt * G < ROWS) {                                      // rows of the tile that no query fills: zeros, once
@@ -433,17 +394,17 @@ attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const int halves = kv ? VH : KH;                         // swizzle rows per key or value
     const int n_ops = ppt * halves;                          // at most 8 x 3 per tile
     bool ok = true;
-    int jt = 0, ic = 0, j_req = 0, round = 0;                // tiles and items so far; the place in the walk
-    TcItem it;
-    while (ok && tc_next_item(list, j_req, round, nkv, tpt, window, it)) {
-      const int* bt = block_tables + (size_t)it.r * bt_stride;
+    int jt = 0, ic = 0;                                      // tiles and items so far
+    for (int k = 0; k < n_rounds && ok; ++k) {
+      TcItem it;
+      if (!tc_item(k, cta, ctas, nt, nkv, tpt, q_len, p_first, window, it)) continue;
       if (!kv) {
         if (ic > 0) ok = tc_mbar_wait(&bars.q_empty, (ic - 1) & 1, abort_flag, err, 10);
         if (!ok) break;
         if (lane == 0) {
           tc_mbar_expect_tx(&bars.q_full, (uint32_t)(KH * tpt * G * 128));
 #pragma unroll
-          for (int hf = 0; hf < KH; ++hf) tc_tma_3d(Qs + hf * HALF_BYTES, &q_map, &bars.q_full, hf * 64, it.kvh * G, it.q0 + it.t0);
+          for (int hf = 0; hf < KH; ++hf) tc_tma_3d(Qs + hf * HALF_BYTES, &q_map, &bars.q_full, hf * 64, it.kvh * G, q0 + it.t0);
         }
         __syncwarp();
       }
@@ -482,9 +443,9 @@ attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const uint32_t tb = tmem + x * COLS_PER_TILE;
     bool ok = true;
     int kc = 0, hc = 0, ic = 0;                              // key tiles, this stream's halves, and items so far
-    int j_req = 0, round = 0;
-    TcItem it;
-    while (ok && tc_next_item(list, j_req, round, nkv, tpt, window, it)) {
+    for (int k = 0; k < n_rounds && ok; ++k) {
+      TcItem it;
+      if (!tc_item(k, cta, ctas, nt, nkv, tpt, q_len, p_first, window, it)) continue;
       const int n_mine = (it.n_half + 1 - x) / 2;
       ok = tc_mbar_wait(&bars.q_full, ic & 1, abort_flag, err, 12);
       auto issue_qk = [&](int i) {
@@ -560,10 +521,10 @@ attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
     const uint32_t lane_addr = tmem + ((uint32_t)(qd * 32) << 16) + x * COLS_PER_TILE;
     uint64_t* o_done = &bars.o_done[x];
     bool ok = true;
-    int hc = 0, ic = 0, j_req = 0, round = 0;                // this stream's halves and the items so far; the place in the walk
-    TcItem it;
-    while (tc_next_item(list, j_req, round, nkv, tpt, window, it)) {
-      const int p_first = it.p_first;
+    int hc = 0, ic = 0;                                      // this stream's halves and the items so far
+    for (int k = 0; k < n_rounds; ++k) {
+      TcItem it;
+      if (!tc_item(k, cta, ctas, nt, nkv, tpt, q_len, p_first, window, it)) continue;
       const int n_mine = (it.n_half + 1 - x) / 2;
       const int t0x = it.t0, t1x = it.t1, T0 = it.T0, kvh = it.kvh;
       const int tok = t0x + row / G;
@@ -756,7 +717,7 @@ attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         const float w0 = a0 * inv, w1 = a1 * inv;
         const bool two = it.n_half > 1;                          // stream 1's accumulator holds something of this item
         const uint32_t o_addr = tmem + ((uint32_t)(qd * 32) << 16) + COL_O;
-        bf16* dst = p != NO_ROW ? out + ((size_t)(it.q0 + tok) * nq + kvh * G + row % G) * VD : nullptr;
+        bf16* dst = p != NO_ROW ? out + ((size_t)(q0 + tok) * nq + kvh * G + row % G) * VD : nullptr;
 #pragma unroll 1
         for (int cc = 0; cc < VN / 64; ++cc) {
           const int col0 = x * (VN / 2) + cc * 32;
@@ -849,7 +810,6 @@ IFB_EXPORT int ifb_attention_tc(const void* qkv, int row_stride, const void* k_p
     if (ifb_tensor_map_bf16(&v_map, v_pages, 2, dims, strides, box)) return IFB_ERR_ARG;
   }
   IFB_ALLOW_SMEM(attn_tile_tc_kernel, SMEM_BYTES);
-  if (max_q_len < 1) return IFB_ERR_ARG;
   const long long items = (long long)((max_q_len + tpt - 1) / tpt) * nkv;      // of the longest request
   static int sm_count = 0;
   if (!sm_count) {
@@ -865,10 +825,7 @@ IFB_EXPORT int ifb_attention_tc(const void* qkv, int row_stride, const void* k_p
     score.limit = scale != 0.f ? TC_TANH_RANGE / fabsf(score.to_y) : INFINITY;
   }
   const TcRows rows = {(int)k_page, (int)v_page, (int)k_rows, (int)v_rows};
-  // a CTA per SM walks a request's items; the z slots are one more than fill the SMs with the longest request's items
-  const long long x = items < sm_count ? items : sm_count, fill = 1 + (sm_count + x - 1) / x;
-  const long long least = (n_req + TC_MAX_LIST - 1) / TC_MAX_LIST, slots = fill > least ? fill : least;
-  dim3 grid((unsigned)x, 1, (unsigned)(slots < n_req ? slots : n_req));
+  dim3 grid((unsigned)(items < sm_count ? items : sm_count), 1, n_req);       // a CTA per SM walks the request's items
   return ifb_launch(attn_tile_tc_kernel, grid, dim3(TC_THREADS), (size_t)SMEM_BYTES, stream, q_map, k_map, v_map, rows, err, block_tables,
-                    bt_stride, cu_q, seq_lens, (bf16*)out, n_req, nq, nkv, share, page_size, score, has_sink ? sink * LOG2E : -INFINITY, window);
+                    bt_stride, cu_q, seq_lens, (bf16*)out, nq, nkv, share, page_size, score, has_sink ? sink * LOG2E : -INFINITY, window);
 }

@@ -736,24 +736,6 @@ def test_attention_beside_attention(K, prompt, splits):
     K.check_device_errors()
 
 
-# Requests by slots in the tcgen05 kernel: a CTA with none, one and several, more requests than a list of 64 per slot takes, requests
-# of the small-q kernel between them.
-@pytest.mark.parametrize("q_lens", [[1, 30, 1], [9, 20, 1, 40, 70, 8] * 24, [17, 1] * 100 + [1300], [400, 1, 200, 1, 600, 130, 90, 9]])
-@pytest.mark.parametrize("nq,nkv,ps,window", [(16, 8, 16, 0), (6, 3, 32, 70)])
-def test_prompts_by_slots(K, q_lens, nq, nkv, ps, window):
-    d, seq_lens = 128, [n + 37 * (i % 3) for i, n in enumerate(q_lens)]
-    qkv, kv, bt, cu, sl = _attention_case(torch.bfloat16, nq, nkv, d, ps, window, q_lens, seq_lens, 31)
-    n, calls = qkv.shape[0], K.tc_attention_calls
-    ref = torch.empty((n, nq * d), dtype=torch.bfloat16)
-    REF.paged_attention(qkv, nq, nkv, d, kv, bt, cu, sl, ref, d ** -0.5, window, max(q_lens), max(seq_lens))
-    out = torch.full((n, nq * d), float("nan"), dtype=torch.bfloat16, device="cuda")
-    K._paged_attention_mma(qkv.cuda(), nq, nkv, d, kv.cuda(), bt.cuda(), cu.cuda(), sl.cuda(), out, d ** -0.5, window,
-                           max(q_lens), max(seq_lens), n, len(q_lens))
-    assert K.tc_attention_calls == calls + 1
-    torch.testing.assert_close(out.cpu().float(), ref.float(), rtol=1.6e-2, atol=1.6e-2)
-    K.check_device_errors()
-
-
 # The kernel over pairs of SMs: one and several tiles per pair, ragged rows, features and k, both output types and every epilogue.
 @pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,o,k", [(1, 72, 72), (257, 256, 64), (513, 1000, 136), (2048, 4096, 200), (300, 20000, 1032)])
