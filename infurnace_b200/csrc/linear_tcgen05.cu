@@ -773,17 +773,21 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
               sum[b][e] = t;
             }
           const bool last = rb + B * WARPS >= r_hi;
-          // this warp has read all it reads of the other CTAs' shared memory (and has stored nothing of its own yet that the
-          // release would have to wait for, where one batch of rows is all)
+          // This warp has read all it reads of the other CTAs' shared memory, and its arrival lets them leave.  What has to hold is
+          // that its reads are complete, that is, their values are in registers: the vote takes a part of every one of them, and the
+          // arrival is predicated on the vote.  The predicate is always true (a count of lanes is above minus the number of rows),
+          // but the number of rows is the launch's, so no compiler can know that and drop what the arrival waits for.  (A release
+          // instead would wait for the stores of the rows before as well: 131 tokens of the 0.6B sizes 1,161 to 1,184 us, with the
+          // sums kept in shared memory until all is read 1,199.)
           if (last) {
-            // (the vote makes the arrival wait for every value read; it needs no release, which would wait for more)
             float all = 0.f;
 #pragma unroll
             for (int b = 0; b < B; ++b)
 #pragma unroll
               for (int e = 0; e < PARTS; ++e) all += sum[b][e].x;
             const int votes = __popc(__ballot_sync(0xffffffffu, all != 0.f));
-            asm volatile("{\n .reg .pred p;\n setp.ge.s32 p, %0, 0;\n @p barrier.cluster.arrive.relaxed.aligned;\n}\n" ::"r"(votes) : "memory");
+            asm volatile("{\n .reg .pred p;\n setp.gt.s32 p, %0, %1;\n @p barrier.cluster.arrive.relaxed.aligned;\n}\n" ::"r"(votes), "r"(-n_rows)
+                         : "memory");
           }
 #pragma unroll
           for (int b = 0; b < B; ++b) {

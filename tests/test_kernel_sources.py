@@ -1,0 +1,21 @@
+"""Rules that the kernels' sources keep and that no run can show reliably."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "infurnace_b200", "csrc")
+
+
+def test_a_relaxed_arrival_at_a_cluster_barrier_waits_for_what_was_read():
+    """A CTA's arrival lets its peers leave or overwrite shared memory that it was reading.  A release orders the reads; a
+    relaxed arrival is held back only by a predicate made of the values, and only one that compares them with an operand
+    (``%1``): a compiler may know the outcome of a comparison with a constant and drop it."""
+    arrivals = 0
+    for path in glob.glob(os.path.join(CSRC, "*.cu*")):
+        with open(path, encoding="utf-8") as f:
+            for line in f:
+                for m in re.finditer(r"(@p )?barrier\.cluster\.arrive(\S*)", line):
+                    arrivals += 1
+                    if ".release" not in m.group(2):
+                        assert m.group(1) and re.search(r"setp\.\w+\.s32 p, %0, %1;", line), (os.path.basename(path), line)
+    assert arrivals
