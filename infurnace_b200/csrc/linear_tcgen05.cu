@@ -1547,8 +1547,10 @@ static int tc_pair_rounds(int n, int o, int features) {
   return (int)((tiles + pairs - 1) / pairs);
 }
 static bool tc_pair_narrow(int n, int o) { return 0.7 * tc_pair_rounds(n, o, 128) < tc_pair_rounds(n, o, 256); }
+// (A device that cannot run the pairs, by the largest of their kernels, or none at all: never.)
+static bool tc_can_pair() { return tc_sm_count() >= 2 && tc_pairs<PairCfg<0, 128, 6, true>, bf16>() > 0; }
 static bool tc_pick_pair(int epi, int n, int o) {
-  if (o % 64 || n <= 512) return false;
+  if (o % 64 || n <= 512 || !tc_can_pair()) return false;
   const int features = epi || tc_pair_narrow(n, o) ? 128 : 256;
   const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
   return tiles * 10 >= (long long)tc_sm_count() / 2 * 8 * tc_pair_rounds(n, o, features);
