@@ -1541,19 +1541,24 @@ static int tc_pick_shape(int epi, int n, int o) {
 // launch): from 513 rows on (up to 512 few tiles share their k range in clusters), where the tiles of its last round, of 256 x 256
 // or 256 x 128, keep most pairs busy (four fifths over all rounds).  Narrow tiles take 0.7 of a wide one's time: an SM gets 24 KB
 // per 64 of k where it gets 32 (2,048 x 1,024 x 2,048: one round of 64 narrow tiles 10.9 us).
-static int tc_pair_rounds(int n, int o, int features) {
-  const int pairs = tc_sm_count() / 2;
+// `pairs`: of SMs; 0 where the device cannot run the largest of their kernels, or there is none: never.
+static int tc_device_pairs() { return tc_pairs<PairCfg<0, 128, 6, true>, bf16>() > 0 ? tc_sm_count() / 2 : 0; }
+static int tc_pair_rounds(int pairs, int n, int o, int features) {
   const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
   return (int)((tiles + pairs - 1) / pairs);
 }
-static bool tc_pair_narrow(int n, int o) { return 0.7 * tc_pair_rounds(n, o, 128) < tc_pair_rounds(n, o, 256); }
-// (A device that cannot run the pairs, by the largest of their kernels, or none at all: never.)
-static bool tc_can_pair() { return tc_sm_count() >= 2 && tc_pairs<PairCfg<0, 128, 6, true>, bf16>() > 0; }
-static bool tc_pick_pair(int epi, int n, int o) {
-  if (o % 64 || n <= 512 || !tc_can_pair()) return false;
-  const int features = epi || tc_pair_narrow(n, o) ? 128 : 256;
+// Features of the tiles of a launch over pairs: 128 with the silu_gate epilogue (their gate and up rows); two whole heads for the
+// fused q | k | v product; else the quicker.
+static int tc_pair_features(int pairs, int epi, bool heads, int n, int o) {
+  if (epi) return 128;
+  if (heads || pairs < 1) return 256;
+  return 0.7 * tc_pair_rounds(pairs, n, o, 128) < tc_pair_rounds(pairs, n, o, 256) ? 128 : 256;
+}
+static bool tc_pick_pair(int pairs, int epi, bool heads, int n, int o) {
+  if (o % 64 || n <= 512 || pairs < 1) return false;
+  const int features = tc_pair_features(pairs, epi, heads, n, o);
   const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
-  return tiles * 10 >= (long long)tc_sm_count() / 2 * 8 * tc_pair_rounds(n, o, features);
+  return tiles * 10 >= (long long)pairs * 8 * tc_pair_rounds(pairs, n, o, features);
 }
 
 template <int EPI, typename TO>
@@ -1571,7 +1576,7 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
   }
   if (shape == 0) {
     shape = tc_pick_shape(EPI, n, o);
-    if (tc_pick_pair(EPI, n, o)) shape = 6;
+    if (tc_pick_pair(tc_device_pairs(), EPI, fold.qk_nq > 0, n, o)) shape = 6;
   }
   if (EPI && fold.res_x) return IFB_ERR_ARG;
   if (shape == 6) {
@@ -1580,7 +1585,7 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
       using Rows256 = PairCfg<0, 256, 4, true>;
       using Rows128 = PairCfg<0, 128, 6, true>;
       using Pair128 = PairCfg<0, 128, 7, false>;
-      const bool narrow = !fold.qk_nq && tc_pair_narrow(n, o);
+      const bool narrow = tc_pair_features(tc_device_pairs(), 0, fold.qk_nq > 0, n, o) == 128;
       if (fold.qk_nq || fold.res_x) {
         if (o % 64) return IFB_ERR_ARG;                              // (a forced shape: the rule asks for it)
         return narrow ? tc_launch_pair<Rows128, TO>(x, w, out, n, o, k, err, s, fold) : tc_launch_pair<Rows256, TO>(x, w, out, n, o, k, err, s, fold);
@@ -1701,10 +1706,17 @@ IFB_EXPORT int ifb_linear_tcgen05_qkv(const void* x, const void* w, void* qkv, i
   return tc_launch<0, bf16>(x, w, qkv, n_rows, (nq + 2 * nkv) * 128, k_dim, err, 0, splits, fold, stream);
 }
 
+// Features of the tiles with which a product of these sizes runs over pairs of SMs (shape 0, splits 1), or 0 where it runs on another
+// kernel.  heads: the fused q | k | v product.  pairs: how many of them to answer for, 0: this device's.
+IFB_EXPORT int ifb_linear_tcgen05_pair_tile(int n_rows, int out_features, int gated, int heads, int pairs) {
+  if (!pairs) pairs = tc_device_pairs();
+  return tc_pick_pair(pairs, gated, heads != 0, n_rows, out_features) ? tc_pair_features(pairs, gated, heads != 0, n_rows, out_features) : 0;
+}
+
 // Parts of sums of squares that a product with res_x writes per row (the launch with shape 0 and these splits).
 IFB_EXPORT int ifb_linear_tcgen05_fold_parts(int n_rows, int out_features, int splits) {
   if (splits > 1) return (out_features + 127) / 128;
-  if (tc_pick_pair(0, n_rows, out_features)) return (out_features + 63) / 64;
+  if (tc_pick_pair(tc_device_pairs(), 0, false, n_rows, out_features)) return (out_features + 63) / 64;
   return tc_pick_shape(0, n_rows, out_features) == 3 ? 2 * ((out_features + 255) / 256) : 2 * ((out_features + 127) / 128);
 }
 

@@ -19,3 +19,25 @@ def _without_a_device(code):
 def test_where_no_pair_of_sms_can_run_the_parts_are_those_of_one_tile_per_cta(n, o):
     got = int(_without_a_device(f"print(lib.ifb_linear_tcgen05_fold_parts({n}, {o}, 1))")[0])
     assert got in (2 * -(-o // 128), 2 * -(-o // 256))
+
+
+@pytest.mark.parametrize("gated,heads", [(0, 0), (0, 1), (1, 0)])
+def test_the_tiles_that_are_launched_keep_the_pairs_busy(gated, heads):
+    """A product runs over pairs of SMs only where its own tiles, two whole heads wide for the fused q | k | v product, keep four
+    fifths of 74 pairs busy over their rounds."""
+    lib = load_library("linear_tcgen05")
+    taken = 0
+    for n in (1, 512, 513, 768, 769, 1000, 1400, 1900, 2048, 5000):
+        for o in (64, 128, 1024, 1088, 2048, 3072, 4096, 5120, 12288):
+            if heads and o % 128:
+                continue
+            f = lib.ifb_linear_tcgen05_pair_tile(n, o, gated, heads, 74)
+            if not f:
+                continue
+            taken += 1
+            assert n > 512 and f in ((256,) if heads else (128,) if gated else (128, 256))
+            tiles = -(-n // 256) * -(-o // f)
+            assert 5 * tiles >= 4 * 74 * -(-tiles // 74), (n, o, f)
+    assert taken
+    assert lib.ifb_linear_tcgen05_pair_tile(1900, 1024, 0, 0, 74) == 128
+    assert lib.ifb_linear_tcgen05_pair_tile(1900, 1024, 0, 1, 74) == 0
