@@ -1537,28 +1537,35 @@ static int tc_pick_shape(int epi, int n, int o) {
   return (n > G_BM && cost_wide < cost_narrow) ? 3 : (tn <= sm_count ? 2 : 1);
 }
 
-// Whether the kernel over pairs of SMs takes a product (a rule on sizes alone, as the parts of a folded norm must agree with the
-// launch): from 513 rows on (up to 512 few tiles share their k range in clusters), where the tiles of its last round, of 256 x 256
-// or 256 x 128, keep most pairs busy (four fifths over all rounds).  Narrow tiles take 0.7 of a wide one's time: an SM gets 24 KB
-// per 64 of k where it gets 32 (2,048 x 1,024 x 2,048: one round of 64 narrow tiles 10.9 us).
+// Whether the kernel over pairs of SMs takes a product (a rule on sizes and on the epilogue's kind alone, as the parts of a folded
+// norm must agree with the launch): from 513 rows on (up to 512 few tiles share their k range in clusters), where its own tiles keep
+// most pairs busy (four fifths over all rounds).
 // `pairs`: of SMs; 0 where the device cannot run the largest of their kernels, or there is none: never.
 static int tc_device_pairs() { return tc_pairs<PairCfg<0, 128, 6, true>, bf16>() > 0 ? tc_sm_count() / 2 : 0; }
 static int tc_pair_rounds(int pairs, int n, int o, int features) {
   const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
   return (int)((tiles + pairs - 1) / pairs);
 }
+enum TcKind { TC_PLAIN, TC_RESIDUAL, TC_HEADS, TC_GATED };     // the epilogues whose weight differs
+static TcKind tc_kind(int epi, const TcFold& f) { return epi ? TC_GATED : f.res_x ? TC_RESIDUAL : f.qk_nq > 0 ? TC_HEADS : TC_PLAIN; }
 // Features of the tiles of a launch over pairs: 128 with the silu_gate epilogue (their gate and up rows); two whole heads for the
-// fused q | k | v product; else the quicker.
-static int tc_pair_features(int pairs, int epi, bool heads, int n, int o) {
-  if (epi) return 128;
-  if (heads || pairs < 1) return 256;
+// fused q | k | v product; else the quicker, a round of narrow tiles taking 0.7 of a wide one's time: an SM gets 24 KB per 64 of k
+// where it gets 32 (2,048 x 1,024 x 2,048: one round of 64 narrow tiles 10.9 us).
+static int tc_pair_features(int pairs, TcKind kind, int n, int o) {
+  if (kind == TC_GATED) return 128;
+  if (kind == TC_HEADS || pairs < 1) return 256;
   return 0.7 * tc_pair_rounds(pairs, n, o, 128) < tc_pair_rounds(pairs, n, o, 256) ? 128 : 256;
 }
-static bool tc_pick_pair(int pairs, int epi, bool heads, int n, int o) {
+// The heads' epilogue is as long as the products of a k of 1,024, and in a single round there are no other tile's products to run
+// it beside: steps of 850 and 1,000 rows of the 0.6B sizes (4,096 x 1,024, one round) 723 and 739 us for eight layers with it over
+// pairs, 687 and 708 without, of 1,800 and 2,048 rows (two rounds) 930 and 978 against 911 and 967; six layers of the 8B sizes
+// (6,144 x 4,096) at 513 rows (one round) 1,739 against 1,695, at 1,500 (two) 3,163 and 3,151, at 2,048 (three) 3,899 against 4,055.
+static bool tc_pick_pair(int pairs, TcKind kind, int n, int o, int k) {
   if (o % 64 || n <= 512 || pairs < 1) return false;
-  const int features = tc_pair_features(pairs, epi, heads, n, o);
+  const int features = tc_pair_features(pairs, kind, n, o), rounds = tc_pair_rounds(pairs, n, o, features);
+  if (kind == TC_HEADS && (rounds < 2 || k < 2048)) return false;
   const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
-  return tiles * 10 >= (long long)pairs * 8 * tc_pair_rounds(pairs, n, o, features);
+  return tiles * 10 >= (long long)pairs * 8 * rounds;
 }
 
 template <int EPI, typename TO>
@@ -1575,8 +1582,7 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
     return tc_launch_cfg<Deep, TO>(x, w, out, n, o, k, err, s, fold, splits);
   }
   if (shape == 0) {
-    shape = tc_pick_shape(EPI, n, o);
-    if (tc_pick_pair(tc_device_pairs(), EPI, fold.qk_nq > 0, n, o)) shape = 6;
+    shape = tc_pick_pair(tc_device_pairs(), tc_kind(EPI, fold), n, o, k) ? 6 : tc_pick_shape(EPI, n, o);
   }
   if (EPI && fold.res_x) return IFB_ERR_ARG;
   if (shape == 6) {
@@ -1585,7 +1591,7 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
       using Rows256 = PairCfg<0, 256, 4, true>;
       using Rows128 = PairCfg<0, 128, 6, true>;
       using Pair128 = PairCfg<0, 128, 7, false>;
-      const bool narrow = tc_pair_features(tc_device_pairs(), 0, fold.qk_nq > 0, n, o) == 128;
+      const bool narrow = tc_pair_features(tc_device_pairs(), tc_kind(0, fold), n, o) == 128;
       if (fold.qk_nq || fold.res_x) {
         if (o % 64) return IFB_ERR_ARG;                              // (a forced shape: the rule asks for it)
         return narrow ? tc_launch_pair<Rows128, TO>(x, w, out, n, o, k, err, s, fold) : tc_launch_pair<Rows256, TO>(x, w, out, n, o, k, err, s, fold);
@@ -1707,16 +1713,18 @@ IFB_EXPORT int ifb_linear_tcgen05_qkv(const void* x, const void* w, void* qkv, i
 }
 
 // Features of the tiles with which a product of these sizes runs over pairs of SMs (shape 0, splits 1), or 0 where it runs on another
-// kernel.  heads: the fused q | k | v product.  pairs: how many of them to answer for, 0: this device's.
-IFB_EXPORT int ifb_linear_tcgen05_pair_tile(int n_rows, int out_features, int gated, int heads, int pairs) {
+// kernel.  kind: 0 plain, 1 with the residual addition, 2 the fused q | k | v product, 3 gated.  pairs: how many of them to answer
+// for, 0: this device's.
+IFB_EXPORT int ifb_linear_tcgen05_pair_tile(int kind, int n_rows, int out_features, int k_dim, int pairs) {
+  if (kind < TC_PLAIN || kind > TC_GATED) return 0;
   if (!pairs) pairs = tc_device_pairs();
-  return tc_pick_pair(pairs, gated, heads != 0, n_rows, out_features) ? tc_pair_features(pairs, gated, heads != 0, n_rows, out_features) : 0;
+  return tc_pick_pair(pairs, (TcKind)kind, n_rows, out_features, k_dim) ? tc_pair_features(pairs, (TcKind)kind, n_rows, out_features) : 0;
 }
 
 // Parts of sums of squares that a product with res_x writes per row (the launch with shape 0 and these splits).
 IFB_EXPORT int ifb_linear_tcgen05_fold_parts(int n_rows, int out_features, int splits) {
   if (splits > 1) return (out_features + 127) / 128;
-  if (tc_pick_pair(tc_device_pairs(), 0, false, n_rows, out_features)) return (out_features + 63) / 64;
+  if (tc_pick_pair(tc_device_pairs(), TC_RESIDUAL, n_rows, out_features, 0)) return (out_features + 63) / 64;       // (whatever the k)
   return tc_pick_shape(0, n_rows, out_features) == 3 ? 2 * ((out_features + 255) / 256) : 2 * ((out_features + 127) / 128);
 }
 

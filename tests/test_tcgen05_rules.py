@@ -21,23 +21,39 @@ def test_where_no_pair_of_sms_can_run_the_parts_are_those_of_one_tile_per_cta(n,
     assert got in (2 * -(-o // 128), 2 * -(-o // 256))
 
 
-@pytest.mark.parametrize("gated,heads", [(0, 0), (0, 1), (1, 0)])
-def test_the_tiles_that_are_launched_keep_the_pairs_busy(gated, heads):
+PLAIN, RESIDUAL, HEADS, GATED = range(4)
+
+
+@pytest.mark.parametrize("kind", [PLAIN, RESIDUAL, HEADS, GATED])
+def test_the_tiles_that_are_launched_keep_the_pairs_busy(kind):
     """A product runs over pairs of SMs only where its own tiles, two whole heads wide for the fused q | k | v product, keep four
-    fifths of 74 pairs busy over their rounds."""
+    fifths of 74 pairs busy over their rounds; and a longer k never sends it back."""
     lib = load_library("linear_tcgen05")
     taken = 0
     for n in (1, 512, 513, 768, 769, 1000, 1400, 1900, 2048, 5000):
         for o in (64, 128, 1024, 1088, 2048, 3072, 4096, 5120, 12288):
-            if heads and o % 128:
+            if kind == HEADS and o % 128:
                 continue
-            f = lib.ifb_linear_tcgen05_pair_tile(n, o, gated, heads, 74)
-            if not f:
-                continue
-            taken += 1
-            assert n > 512 and f in ((256,) if heads else (128,) if gated else (128, 256))
-            tiles = -(-n // 256) * -(-o // f)
-            assert 5 * tiles >= 4 * 74 * -(-tiles // 74), (n, o, f)
+            tile = 0
+            for k in (64, 512, 1024, 2048, 4096, 8192, 25600):
+                f = lib.ifb_linear_tcgen05_pair_tile(kind, n, o, k, 74)
+                if not f:
+                    continue
+                taken += 1
+                assert n > 512 and f in {PLAIN: (128, 256), RESIDUAL: (128, 256), HEADS: (256,), GATED: (128,)}[kind]
+                tiles = -(-n // 256) * -(-o // f)
+                assert 5 * tiles >= 4 * 74 * -(-tiles // 74), (n, o, k, f)
+                assert tile in (0, f)
+                tile = f
     assert taken
-    assert lib.ifb_linear_tcgen05_pair_tile(1900, 1024, 0, 0, 74) == 128
-    assert lib.ifb_linear_tcgen05_pair_tile(1900, 1024, 0, 1, 74) == 0
+    assert lib.ifb_linear_tcgen05_pair_tile(HEADS, 1900, 1024, 25600, 74) == 0        # 64 tiles of one head, 32 of two
+
+
+# Sizes on either side of the lines for the heads' epilogue (rounds, k), and others at which those lines do not hold.
+@pytest.mark.parametrize("kind,n,o,k,tile", [
+    (PLAIN, 2048, 1024, 1024, 128), (PLAIN, 1000, 4096, 1024, 256), (PLAIN, 2048, 4096, 1024, 256),
+    (RESIDUAL, 2048, 1024, 1024, 128), (RESIDUAL, 2048, 4096, 4096, 256),
+    (HEADS, 1000, 4096, 1024, 0), (HEADS, 2048, 4096, 1024, 0), (HEADS, 1000, 4096, 4096, 0), (HEADS, 2048, 4096, 2040, 0), (HEADS, 2048, 4096, 2048, 256), (HEADS, 2048, 6144, 4096, 256),
+    (GATED, 600, 3072, 1024, 128), (GATED, 2048, 12288, 4096, 128)])
+def test_the_heads_of_a_short_product_stay_on_one_tile_per_cta(kind, n, o, k, tile):
+    assert load_library("linear_tcgen05").ifb_linear_tcgen05_pair_tile(kind, n, o, k, 74) == tile
