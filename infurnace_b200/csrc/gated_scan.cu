@@ -242,7 +242,7 @@ gated_scan_carry_kernel(GatedScanArgs a) {
     for (int j = 0; j < 8; ++j) {
       const bool in = b0 + j < blocks;
       z[j] = in ? __ldcg(a.z + (size_t)(first + b0 + j) * per + e) : 0.f;
-      g[j] = in ? __ldg(a.decay + (size_t)(first + b0 + j) * a.heads * a.dim + hi) : 1.f;
+      g[j] = in ? __ldcg(a.decay + (size_t)(first + b0 + j) * a.heads * a.dim + hi) : 1.f;
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {

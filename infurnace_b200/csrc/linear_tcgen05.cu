@@ -235,7 +235,7 @@ __device__ __forceinline__ float tc_row_factor(const TcFold& f, int row, int n_r
   if (!f.rs_partials || row >= n_rows) return 1.f;
   float sum = 0.f;
 #pragma unroll 4
-  for (int p = 0; p < f.rs_parts; ++p) sum += __ldg(f.rs_partials + (size_t)p * n_rows + row);
+  for (int p = 0; p < f.rs_parts; ++p) sum += f.rs_partials[(size_t)p * n_rows + row];
   return rsqrtf(sum * f.rs_inv_width + f.rs_eps);
 }
 // v = x + y for 32 consecutive features of one row (x updated in place), y <- v * g; returns the sum of v^2.
@@ -362,9 +362,9 @@ __device__ __forceinline__ void tc_heads_load(const TcFold& f, int row0, int n_r
     const int row = row0 + a * RPP + lane / LPR;
     const float4* t = reinterpret_cast<const float4*>(f.qk_rope + (size_t)row * 64 + i0 + (lane % LPR) * 4);
     const bool in = rotate && row < n_rows;
-    cs[a][0] = in ? __ldg(t) : make_float4(1.f, 0.f, 1.f, 0.f);
-    cs[a][1] = in ? __ldg(t + 1) : make_float4(1.f, 0.f, 1.f, 0.f);
-    slot[a] = store && row < n_rows ? __ldg(f.qk_slots + row) : -1;
+    cs[a][0] = in ? t[0] : make_float4(1.f, 0.f, 1.f, 0.f);
+    cs[a][1] = in ? t[1] : make_float4(1.f, 0.f, 1.f, 0.f);
+    slot[a] = store && row < n_rows ? f.qk_slots[row] : -1;
   }
 }
 // `cs`, `slot`: the first AHEAD passes' angles and places, requested by the caller before it waited for the product.
@@ -773,9 +773,9 @@ linear_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_c
             if (!EPI && fold.qk_nq) {
               const bool turn = !qk_v && fold.qk_rope && r < r_hi;
               const float4* t = reinterpret_cast<const float4*>(fold.qk_rope + (size_t)(m0 + r) * 64 + (c & 63));
-              cs[b][0] = turn ? __ldg(t) : make_float4(1.f, 0.f, 1.f, 0.f);
-              cs[b][1] = turn ? __ldg(t + 1) : make_float4(1.f, 0.f, 1.f, 0.f);
-              slot[b] = (qk_v || qk_k) && fold.qk_slots && r < r_hi ? __ldg(fold.qk_slots + m0 + r) : -1;
+              cs[b][0] = turn ? t[0] : make_float4(1.f, 0.f, 1.f, 0.f);
+              cs[b][1] = turn ? t[1] : make_float4(1.f, 0.f, 1.f, 0.f);
+              slot[b] = (qk_v || qk_k) && fold.qk_slots && r < r_hi ? fold.qk_slots[m0 + r] : -1;
             }
           }
           float4 sum[B][PARTS];

@@ -19,3 +19,14 @@ def test_a_relaxed_arrival_at_a_cluster_barrier_waits_for_what_was_read():
                     if ".release" not in m.group(2):
                         assert m.group(1) and re.search(r"setp\.\w+\.s32 p, %0, %1;", line), (os.path.basename(path), line)
     assert arrivals
+
+
+def test_only_constants_are_read_through_the_read_only_path():
+    """A kernel may be resident while the one before it still writes, and a load through ``__ldg`` may be moved ahead of the wait
+    for that kernel: it is for what no kernel of a step writes (biases, convolution weights)."""
+    for path in glob.glob(os.path.join(CSRC, "*.cu*")):
+        with open(path, encoding="utf-8") as f:
+            for line in f:
+                for m in re.finditer(r"__ldg\(([^)]*)", line):
+                    if not m.group(0).endswith("(__ldg"):
+                        assert re.search(r"bias|conv_w", m.group(1)), (os.path.basename(path), line)
