@@ -1701,7 +1701,7 @@ IFB_EXPORT int ifb_linear_tcgen05(const void* x, const void* w, void* out, int o
 // The fused q | k | v projection of an attention layer with what follows it (see TcFold) in the epilogue of the one-tile
 // kernel (splits 1) or in the sum over the cluster of the shared-k form (splits 2 to 8): qkv [n_rows, (nq + 2 nkv) * 128] bfloat16 gets the normalised and rotated q heads (and the k and
 // v heads as they are stored), the pages get k and v at slots[n].  Heads of 128, rotated whole in the half-split pairing
-// (rope: [n_rows][64] pairs of cos and sin, or null).  scale_*: as in ifb_linear_tcgen05_ex.
+// (rope: [n_rows][64] pairs of cos and sin, 16-byte aligned, or null).  scale_*: as in ifb_linear_tcgen05_ex.
 IFB_EXPORT int ifb_linear_tcgen05_qkv(const void* x, const void* w, void* qkv, int n_rows, int nq, int nkv, int head_dim, int k_dim,
                                       int splits, const float* scale_partials, int scale_parts, float scale_eps, int scale_width,
                                       const void* q_weight, const void* k_weight, int w_dtype, float eps, const float* rope,

@@ -505,6 +505,10 @@ class CudaKernels:
             raise KernelError("linear_qkv_rope_store: no kernel takes these sizes (see can_fuse_qkv)")
         if route == "tcgen05":
             self._err_armed = True
+            if rope_table is not None and rope_table.data_ptr() % 16 == 8:
+                # the kernel reads two pairs at a time (with a choice in its epilogue a prompt of 2,048 tokens of the 0.6B sizes took 3,151
+                # to 3,202 us for 3,116); the tables of the step function lie on 16 bytes
+                rope_table = rope_table.clone()
             # (more than one tile of rows, or a short k: the cluster's sum would take longer over the heads than the shared k
             # range saves)
             splits = self.tcgen05_splits(n, width, k) if n <= 128 and k > 1024 else 1

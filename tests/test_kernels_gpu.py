@@ -663,6 +663,28 @@ def test_qkv_product_of_a_prompt_with_norm_rotation_and_store_in_its_epilogue(K,
     test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, d, k, ps, norm, rotate, scaled)
 
 
+# Angles that lie at 8 bytes from a 16-byte border, as the kernel always took them: in the cluster's sum (40 rows, long k), in the
+# epilogue of one tile per CTA, and over pairs of SMs (31 heads and a k of 2,048: two rounds).  The same bits as from the border.
+@pytest.mark.parametrize("n,nq,nkv,k", [(40, 5, 1, 2056), (129, 16, 8, 1024), (1300, 16, 8, 520), (2048, 25, 3, 2048)])
+def test_qkv_product_with_angles_aligned_to_one_pair(K, n, nq, nkv, k):
+    width = (nq + 2 * nkv) * 128
+    x, w = rnd((n, k), torch.bfloat16, 1).cuda(), rnd((width, k), torch.bfloat16, 2, scale=k ** -0.5).cuda()
+    kv = torch.zeros((-(-n // 16), 2, nkv, 16, 128), dtype=torch.bfloat16, device="cuda")
+    slots = torch.arange(n, dtype=torch.int32, device="cuda")
+    room = rnd((n * 128 + 2,), torch.float32, 3).cuda()
+    outs = []
+    for off in (0, 2):
+        table = room[off:off + n * 128].view(n, 128)
+        table.copy_(rnd((n, 128), torch.float32, 4).cuda())
+        assert table.data_ptr() % 16 == 4 * off
+        qkv = torch.full((n, width), float("nan"), dtype=torch.bfloat16, device="cuda")
+        K.linear_qkv_rope_store(x, w, qkv, nq, nkv, 128, None, None, 1e-6, table, slots, kv)
+        outs.append((qkv, kv.clone()))
+    K.check_device_errors()
+    assert torch.isfinite(outs[0][0].float()).all()
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 # A prompt's product with the residual addition by whole row segments (one tile per CTA: deep, narrow; wide is tested above), and
 # with rows of features that are not whole (by single features).
 @pytest.mark.parametrize("n,hidden,inner", [(700, 1024, 520), (1300, 2304, 264), (513, 1096, 136), (700, 1026, 136)])
