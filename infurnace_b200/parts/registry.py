@@ -85,9 +85,9 @@ def fold_residual_norm(kernels, ctx, tag, a, w, fold, act_dtype):
         return None
     parts = kernels.fold_parts(o, n, w)
     out = ctx.buffer("folded_" + tag, (n, o), act_dtype)
-    # one flat buffer for the most rows that a step can have (a part covers 64 features or more of the tcgen05 kernels, which
-    # take large steps, 8 or more of the few-rows kernel's), so that its address stays the same from step to step
-    most = max(parts * n, -(-o // 64) * getattr(ctx, "max_rows", n), -(-o // 8) * 64)
+    # one flat buffer for the most rows that a step can have, so that its address stays the same from step to step: of a row the
+    # tcgen05 kernels, which take large steps, write at most two parts per 128 features, the few-rows kernel one per 8
+    most = max(parts * n, 2 * -(-o // 128) * getattr(ctx, "max_rows", n), -(-o // 8) * 64)
     partials = ctx.buffer("folded_partials_" + tag, (parts * n,), __import__("torch").float32, rows=most).view(parts, n)
     kernels.linear_residual_norm(a, w, x, norm.weight, out, partials)
     return Folded(out, (partials, parts, float(norm.spec.eps), o))

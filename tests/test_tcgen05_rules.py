@@ -3,6 +3,7 @@ import subprocess
 import sys
 
 import pytest
+import torch
 
 from infurnace_b200.kernels.build import load_library
 
@@ -57,3 +58,46 @@ def test_the_tiles_that_are_launched_keep_the_pairs_busy(kind):
     (GATED, 600, 3072, 1024, 128), (GATED, 2048, 12288, 4096, 128)])
 def test_the_heads_of_a_short_product_stay_on_one_tile_per_cta(kind, n, o, k, tile):
     assert load_library("linear_tcgen05").ifb_linear_tcgen05_pair_tile(kind, n, o, k, 74) == tile
+
+
+class _Norm:
+    weight = None
+
+    class spec:
+        eps = 1e-6
+
+
+class _Kernels:
+    """Only what the folding of a norm asks for: the parts that the library's kernels write."""
+
+    def can_fold_norm(self, n, dtype, w, epilogue="none"):
+        return True
+
+    def fold_parts(self, o, n=None, w=None):
+        lib = load_library("linear_tcgen05")
+        tile = lib.ifb_linear_tcgen05_pair_tile(RESIDUAL, n, o, w.shape[1], 74) if n > 512 else 0
+        return -(-o // 64) if tile else 2 * -(-o // 128) if n > 64 else -(-o // 16)
+
+    def linear_residual_norm(self, a, w, x, weight, out, partials):
+        pass
+
+
+@pytest.mark.parametrize("o", [64, 192, 320, 1024, 1088, 4160])
+def test_the_buffer_of_partial_sums_never_grows(o):
+    """Its address is part of the steps that were recorded: small steps first, then the largest."""
+    from infurnace_b200.engine.runner import _Arena
+    from infurnace_b200.parts.registry import fold_residual_norm
+
+    class Context:
+        max_rows = 2048
+        arena = _Arena("cpu", 2048)
+
+        def buffer(self, name, shape, dtype, rows=None):
+            return self.arena.get(name, shape, dtype, rows)
+    ctx, w = Context(), torch.empty((o, 64), dtype=torch.bfloat16)
+    for n in (1, 8, 64, 129, 512, 513, 1500, 2047, 2048):
+        x = torch.empty((n, o))
+        fold_residual_norm(_Kernels(), ctx, "mixer", torch.empty((n, 64), dtype=torch.bfloat16), w, (x, _Norm()), torch.bfloat16)
+        if n == 1:
+            first = ctx.arena.generation
+    assert ctx.arena.generation == first
