@@ -179,8 +179,10 @@ paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, c
         const bool seen = q < queries && kp && key <= p && (window <= 0 || key > p - window);
         const float sv = seen ? s[q] * scale : -INFINITY;
         const float m_new = fmaxf(m[q], warp_max(sv));
-        const float pj = seen ? expf(sv - m_new) : 0.f;
-        const float corr = m_new == -INFINITY ? 1.f : expf(m[q] - m_new);      // nothing seen so far: nothing to rescale
+        // nothing seen so far, or scores of minus infinity alone (a block of them may be all that this warp sees): no weight, nothing
+        // to rescale
+        const float pj = seen && (sv != -INFINITY || m_new != -INFINITY) ? expf(sv - m_new) : 0.f;
+        const float corr = m_new == -INFINITY ? 1.f : expf(m[q] - m_new);
         l[q] = l[q] * corr + warp_sum(pj);
         m[q] = m_new;
 #pragma unroll

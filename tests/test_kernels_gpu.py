@@ -663,6 +663,33 @@ def test_qkv_product_of_a_prompt_with_norm_rotation_and_store_in_its_epilogue(K,
     test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, d, k, ps, norm, rotate, scaled)
 
 
+# Whole blocks of 32 keys whose scores are minus infinity (products beyond the range of float32) count for nothing, wherever they
+# stand but at the start, and a NaN among the scores still reaches the output.
+@pytest.mark.parametrize("nq,nkv,d", [(4, 2, 16), (6, 1, 128), (2, 2, 256)])
+def test_plain_attention_with_blocks_of_infinite_scores(K, nq, nkv, d):
+    q_lens, seq_lens, ps = [2, 1, 5], [400, 300, 70], 16
+    qkv, kv, bt, cu, sl = _attention_case(torch.float32, nq, nkv, d, ps, 0, q_lens, seq_lens, 23)
+    qkv[:, :nq * d] = 1.0 + 0.1 * qkv[:, :nq * d].abs()
+    far = [(0, 32, 96), (0, 160, 352), (1, 64, 288), (2, 32, 64)]
+    for r, lo, hi in far:
+        for p in range(lo, hi):
+            kv[int(bt[r, p // ps]), 0, :, p % ps] = -3e38
+    args = (nq, nkv, d)
+
+    def run(pages):
+        out = torch.empty((qkv.shape[0], nq * d), device="cuda")
+        K.paged_attention(qkv.cuda(), *args, pages.cuda(), bt.cuda(), cu.cuda(), sl.cuda(), out, d ** -0.5, 0, max(q_lens), max(seq_lens))
+        return out.cpu()
+    ref = torch.empty((qkv.shape[0], nq * d), dtype=torch.float64)
+    ReferenceKernels(torch.float64).paged_attention(qkv.double(), *args, kv.double(), bt, cu, sl, ref, d ** -0.5, 0, max(q_lens), max(seq_lens))
+    assert torch.isfinite(ref).all()
+    torch.testing.assert_close(run(kv).double(), ref, rtol=1e-4, atol=1e-5)
+    bad = kv.clone()
+    bad[int(bt[1, 200 // ps]), 0, :, 200 % ps] = float("nan")
+    out = run(bad)
+    assert torch.isnan(out[2]).all() and torch.isfinite(out[:2]).all() and torch.isfinite(out[3:]).all()
+
+
 # Angles that lie at 8 bytes from a 16-byte border, as the kernel always took them: in the cluster's sum (40 rows, long k), in the
 # epilogue of one tile per CTA, and over pairs of SMs (31 heads and a k of 2,048: two rounds).  The same bits as from the border.
 @pytest.mark.parametrize("n,nq,nkv,k", [(40, 5, 1, 2056), (129, 16, 8, 1024), (1300, 16, 8, 520), (2048, 25, 3, 2048)])
