@@ -402,8 +402,10 @@ class ParallelBlock:
         last = self.ffn if self.ffn is not None else self.mixer
         if next_layer is not None and all(getattr(p, "can_fold_output", False) for p in (self.mixer, last)) and next_layer.takes_folded(n):
             norm = next_layer.mixer_norm
-            d = self.mixer.forward(h, ctx, call, fold=(x, norm))
-            if isinstance(d, Folded):                # x holds the mixer's result; the half norm of that sum is not used
+            # x then holds the mixer's result; the half norm of that sum is not used, and lies apart, since h, which the feed-forward
+            # reads too, may be what the mixer of a block without feed-forward left in a mixer's buffers
+            d = self.mixer.forward(h, ctx, call, fold=(x, norm) if self.ffn is None else (x, norm, "unread"))
+            if isinstance(d, Folded):
                 if self.ffn is None:
                     return d
                 return self.ffn.forward(h, ctx, fold=(x, norm))      # a Folded, or the feed-forward's plain delta

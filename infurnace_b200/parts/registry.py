@@ -76,10 +76,11 @@ def unfolded(h):
 def fold_residual_norm(kernels, ctx, tag, a, w, fold, act_dtype):
     """The last product of a mixer or feed-forward with the residual addition and the next
     norm folded in, if the kernels can do it for these sizes: returns a :class:`Folded`,
-    or None (then the caller runs the plain product).  ``fold`` = (x, norm)."""
+    or None (then the caller runs the plain product).  ``fold`` = (x, norm), or (x, norm, tag) for buffers
+    other than the part's own."""
     if fold is None or not getattr(kernels, "can_fold_norm", None):
         return None
-    x, norm = fold
+    x, norm, tag = fold if len(fold) == 3 else (*fold, tag)
     n, o = a.shape[0], w.shape[0]
     if a.dtype != act_dtype or x.shape != (n, o) or not kernels.can_fold_norm(n, a.dtype, w):
         return None

@@ -330,6 +330,10 @@ VARIANTS = {
         TM.layer(5, 5, 8, 4, 0.4, 3.0, TM.moe(16, 5, 8, groups=(8, 4), shared=12)),
         TM.layer(5, 1, 4, 8, 0.6, 2.0, TM.moe(9, 3, 12, groups=(3, 1))), TM.layer(5, 1, 4, 8, 0.5, 3.0, None, kv_from=1),
         TM.layer(10, 5, 8, 4, 0.5, 4.0, TM.dense(30), kv_from=0), TM.layer(2, 2, 3, 5, 0.8, None, TM.moe(2, 1, 6))], logit=0.3),
+    # layers without feed-forward before dense ones: both sublayers read a norm that the mixer before left half done
+    "bare_before_dense": TM.config(37, 24, 1e-5, [
+        TM.layer(2, 1, 6, 8, 0.5, 3.0, None), TM.layer(2, 2, 6, 4, 0.6, 2.0, TM.dense(20)), TM.layer(2, 1, 5, 4, 0.7, 2.5, None),
+        TM.layer(2, 1, 6, 8, 0.5, 3.0, TM.dense(28), kv_from=0), TM.layer(3, 1, 4, 4, 0.5, None, TM.dense(16))], emb=2.0),
 }
 
 
