@@ -373,8 +373,9 @@ attention_talk_merge_kernel(TalkMmaArgs a) {
   constexpr int PER = (D + 31) / 32;
   float acc[PER], wz[2];
 #pragma unroll
-  for (int u = 0; u < 2; ++u) wz[u] = mz[u] == -INFINITY ? 0.f : expf(mz[u] - m);      // 0: a part that saw no key
-  const float l = warp_sum((wz[0] != 0.f ? lz[0] * wz[0] : 0.f) + (wz[1] != 0.f ? lz[1] * wz[1] : 0.f));
+  for (int u = 0; u < 2; ++u) wz[u] = mz[u] == -INFINITY ? -1.f : expf(mz[u] - m);      // -1: a part that saw no key
+  // (a weight that is 0 counts: an infinity or a NaN among the values of far keys reaches the output, as in one softmax)
+  const float l = warp_sum((wz[0] != -1.f ? lz[0] * wz[0] : 0.f) + (wz[1] != -1.f ? lz[1] * wz[1] : 0.f));
 #pragma unroll
   for (int j = 0; j < PER; ++j) acc[j] = 0.f;
   for (int z0 = 0; z0 < (live ? a.splits : 0); z0 += 4) {
@@ -382,14 +383,15 @@ attention_talk_merge_kernel(TalkMmaArgs a) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int z = z0 + u;
-      w[u] = z < a.splits ? __shfl_sync(0xffffffffu, z < 32 ? wz[0] : wz[1], z & 31) : 0.f;
+      const float wu = __shfl_sync(0xffffffffu, z < 32 ? wz[0] : wz[1], z & 31);
+      w[u] = z < a.splits ? wu : -1.f;
 #pragma unroll
-      for (int j = 0; j < PER; ++j) { const int c = lane + 32 * j; row[u][j] = w[u] != 0.f && c < D ? p[(size_t)z * (D + 2) + c] : 0.f; }
+      for (int j = 0; j < PER; ++j) { const int c = lane + 32 * j; row[u][j] = w[u] != -1.f && c < D ? p[(size_t)z * (D + 2) + c] : 0.f; }
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u)
 #pragma unroll
-      for (int j = 0; j < PER; ++j) acc[j] = w[u] != 0.f ? fmaf(row[u][j], w[u], acc[j]) : acc[j];
+      for (int j = 0; j < PER; ++j) acc[j] = w[u] != -1.f ? fmaf(row[u][j], w[u], acc[j]) : acc[j];
   }
 #pragma unroll
   for (int j = 0; j < PER; ++j) {

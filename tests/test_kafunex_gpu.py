@@ -150,7 +150,7 @@ def test_gated_recurrence_kernel(K, heads, dim, vdim):
     close(out_bf[rows], want[rows], 0.05, "bfloat16 outputs")
 
 
-def _attention_case(K, H, G, d, ps, chunk, dtype, lens_and_new, seed, talk=True, gate=True, slope=8.0, plant=None):
+def _attention_case(K, H, G, d, ps, chunk, dtype, lens_and_new, seed, talk=True, gate=True, slope=8.0, plant=None, nan_at=None):
     """Requests of (length after the step, new tokens) over a shuffled page pool; compares kernel and statement."""
     g = gen(seed)
     R = len(lens_and_new)
@@ -174,6 +174,8 @@ def _attention_case(K, H, G, d, ps, chunk, dtype, lens_and_new, seed, talk=True,
         for h in range(H):
             pages[page, 0, h // (H // G), off] = q[new - 1, h * d:(h + 1) * d] * size / d
         pages[page, 1, :, off] = 9.0
+    if nan_at is not None:                # the values of one key of request 0
+        pages[int(bt[0, nan_at // ps]), 1, :, nan_at % ps] = float("nan")
     tk = (torch.eye(H) + 0.5 * torch.randn(H, H, generator=g)) if talk else None
     gt = torch.randn(n, H * d + 7, generator=g) if gate else None
     seq = torch.tensor([L for L, _ in lens_and_new], dtype=torch.int32)
@@ -220,6 +222,16 @@ def test_talking_attention_with_the_keys_split_over_ctas(K, chunk):
         got, want = _attention_case(K, H, G, d, 16, chunk, torch.bfloat16, cases, seed=chunk + H)
         assert K.talk_split_calls == before + 1
         close(got, want, 0.06, f"split keys, {H} heads")
+
+
+def test_a_nan_among_the_values_of_far_keys_reaches_the_output_of_split_keys(K):
+    """Where one key's score is so far above the others that their weights are 0, their values still count: 0 times NaN."""
+    for key, d in ((40, 64), (200, 16)):
+        before = K.talk_split_calls
+        got, want = _attention_case(K, 8, 2, d, 16, 0, torch.bfloat16, [(700, 1), (400, 1)], seed=key, talk=False, gate=False, slope=0.0,
+                                    plant=(690, 400.0), nan_at=key)
+        assert K.talk_split_calls == before + 1
+        assert bool(torch.isnan(want[0]).all()) and bool(torch.isnan(got[0].cpu()).all()) and bool(torch.isfinite(got[1].cpu()).all())
 
 
 def test_talking_attention_variants(K):
