@@ -250,10 +250,8 @@ paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, c
       if (top != -INFINITY) {
 #pragma unroll
         for (int w = 0; w < W; ++w) {
-          const float lw = ml[(w * QT + q) * 2 + 1];
-          if (lw == 0.f) continue;                              // this warp saw no key of the query
-          const float f = expf(ml[(w * QT + q) * 2] - top);
-          total = fmaf(f, lw, total);
+          const float f = expf(ml[(w * QT + q) * 2] - top);      // 0 for a warp that saw no key, whose sums are 0
+          total = fmaf(f, ml[(w * QT + q) * 2 + 1], total);
           sum = fmaf(f, keys[(size_t)(w * QT + q) * d + i % d], sum);
         }
       }

@@ -664,7 +664,7 @@ def test_qkv_product_of_a_prompt_with_norm_rotation_and_store_in_its_epilogue(K,
 
 
 # Whole blocks of 32 keys whose scores are minus infinity (products beyond the range of float32) count for nothing, wherever they
-# stand but at the start, and a NaN among the scores still reaches the output.
+# stand but at the start, and a NaN among the scores or their values still reaches the output.
 @pytest.mark.parametrize("nq,nkv,d", [(4, 2, 16), (6, 1, 128), (2, 2, 256)])
 def test_plain_attention_with_blocks_of_infinite_scores(K, nq, nkv, d):
     q_lens, seq_lens, ps = [2, 1, 5], [400, 300, 70], 16
@@ -684,10 +684,11 @@ def test_plain_attention_with_blocks_of_infinite_scores(K, nq, nkv, d):
     ReferenceKernels(torch.float64).paged_attention(qkv.double(), *args, kv.double(), bt, cu, sl, ref, d ** -0.5, 0, max(q_lens), max(seq_lens))
     assert torch.isfinite(ref).all()
     torch.testing.assert_close(run(kv).double(), ref, rtol=1e-4, atol=1e-5)
-    bad = kv.clone()
-    bad[int(bt[1, 200 // ps]), 0, :, 200 % ps] = float("nan")
-    out = run(bad)
-    assert torch.isnan(out[2]).all() and torch.isfinite(out[:2]).all() and torch.isfinite(out[3:]).all()
+    for what in (0, 1):                                          # among the keys, or the values of a key without weight
+        bad = kv.clone()
+        bad[int(bt[1, 100 // ps]), what, :, 100 % ps] = float("nan")
+        out = run(bad)
+        assert torch.isnan(out[2]).all() and torch.isfinite(out[:2]).all() and torch.isfinite(out[3:]).all(), what
 
 
 # Angles that lie at 8 bytes from a 16-byte border, as the kernel always took them: in the cluster's sum (40 rows, long k), in the
