@@ -196,14 +196,14 @@ def test_qk_norm_rope_store_for_many_tokens_of_head_size_128(K, nq, nkv, ps, nor
 
 @pytest.mark.parametrize("n", [1, 5, 8, 13, 16, 40, 100, 128])
 @pytest.mark.parametrize("nq,nkv,d,k,ps", [(16, 8, 128, 1024, 16), (4, 2, 64, 2048, 8), (2, 1, 256, 4096, 32), (3, 3, 128, 136, 16),
-                                           (5, 1, 128, 2056, 32)])
+                                           (5, 1, 128, 2056, 32), (16, 8, 128, 2048, 16)])
 @pytest.mark.parametrize("norm,rotate,scaled", [(True, True, False), (True, True, True), (False, True, False), (True, False, False)])
 def test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, d, k, ps, norm, rotate, scaled):
     """The one-launch form of a step's q | k | v projection against its three steps in float64: the
     product (with the row factors of a folded norm before it, when ``scaled``), the RMSNorm of the q and k
     heads, the rotation, and k and v in the pages at the tokens' slots (one token stores nothing).  Up to 16
-    rows on the few-rows kernel (a cluster per head), more rows of heads of 128 on the tcgen05 kernel whose
-    clusters share the k range of a head."""
+    rows on the few-rows kernel (a cluster per head), more rows of heads of 128 on the tcgen05 kernel: up to 128
+    with a k above 1,024 in the form whose clusters share the k range of a head, else in one tile per head."""
     width = (nq + 2 * nkv) * d
     if n > 16:
         w_probe = torch.empty((width, k), dtype=torch.bfloat16, device="cuda")
@@ -242,9 +242,11 @@ def test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv,
     if norm:
         with pytest.raises(Exception, match="differ in dtype"):
             K.linear_qkv_rope_store(x.cuda(), w.cuda(), qkv, nq, nkv, d, qw.cuda(), kw.cuda(), 1e-6, table, slots.cuda(), kv)
+    shared = K.tc_shared_k_calls
     K.linear_qkv_rope_store(x.cuda(), w.cuda(), qkv, nq, nkv, d, qw.cuda() if norm else None, kw_used.cuda() if norm else None,
                             1e-6, table, slots.cuda(), kv,
                             row_scale=(partials.cuda(), parts, 1e-5, 77) if scaled else None)
+    assert K.tc_shared_k_calls - shared == (16 < n <= 128 and k > 1024)
     t = dict(rtol=1.6e-2, atol=2e-2)
     torch.testing.assert_close(qkv.cpu().double(), qkv_ref, **t)
     torch.testing.assert_close(kv.cpu().double(), kv_ref, **t)
@@ -654,8 +656,8 @@ def test_plain_attention_of_a_query_is_the_same_in_every_step(K, nq, nkv, d, ps,
         assert torch.equal(alone[0], out[row])
 
 
-# More than one tile of rows: the shared-k form again (129), then the epilogue of the one-tile kernel with one head per tile
-# (deep stages, then two CTAs per SM) and with two, the last tile's second one missing where the heads are odd.
+# More than one tile of rows: the epilogue of the one-tile kernel with one head per tile (deep stages, then two CTAs per SM) and
+# with two, the last tile's second one missing where the heads are odd.
 @pytest.mark.parametrize("n", [129, 300, 700, 1300])
 @pytest.mark.parametrize("nq,nkv,d,k,ps", [(16, 8, 128, 1024, 16), (25, 1, 128, 520, 32)])
 @pytest.mark.parametrize("norm,rotate,scaled", [(True, True, False), (True, True, True), (False, True, False), (True, False, False)])
@@ -808,17 +810,29 @@ def test_linear_tcgen05_over_pairs(K, od, n, o, k, epilogue):
     torch.testing.assert_close(out.double(), ref, rtol=1.6e-2 if od == torch.bfloat16 else 2e-3, atol=1e-2 if od == torch.bfloat16 else 1e-3)
 
 
-# Folded norms and heads on pairs of SMs: tiles of 256 x 128 (1,900 rows of 1,024 features) and of 256 x 256, the reading side behind them.
-@pytest.mark.parametrize("n,hidden,inner,epilogue", [(1900, 1024, 520, "silu_gate"), (1300, 4160, 264, "none"), (4000, 2048, 72, "silu_gate")])
-def test_linear_with_a_folded_norm_over_pairs(K, n, hidden, inner, epilogue, monkeypatch):
+def _pair_tile(K, kind, n, o, k):
+    """Features of the pairs' tiles that the rule gives a product of these sizes, 0 where another kernel takes it."""
+    return K._tc_lib().ifb_linear_tcgen05_pair_tile(kind, n, o, k, 0)
+
+
+# Folded norms on pairs of SMs: tiles of 256 x 128 and of 256 x 256, whole and with 64 features in the last, ragged rows, and behind them
+# the reading side; beside them a size that the rule leaves to one tile per CTA.  (The tiles hold for 74 pairs.)
+@pytest.mark.parametrize("n,hidden,inner,epilogue,tile", [(1900, 1024, 520, "silu_gate", 128), (1300, 4160, 264, "none", 0),
+                                                          (4000, 2048, 72, "silu_gate", 256), (1900, 1088, 520, "silu_gate", 128),
+                                                          (2000, 2112, 136, "silu_gate", 256)])
+def test_linear_with_a_folded_norm_over_pairs(K, n, hidden, inner, epilogue, tile, monkeypatch):
+    assert _pair_tile(K, 1, n, hidden, inner) == tile and (not tile or _pair_tile(K, 3, n, 1024, hidden) == 128)
     monkeypatch.setattr(K, "tc_fold_max_rows", 1 << 20)
     _folded_norm_case(K, n, hidden, inner, 1024, epilogue, torch.bfloat16)
 
 
-@pytest.mark.parametrize("n,nq,nkv", [(1500, 17, 4), (2500, 16, 8)])
+# The heads' epilogue over pairs of SMs: ragged rows with an odd number of heads (the last tile holds one), whole tiles; and sizes that
+# the rule leaves to one tile per CTA (a short k).
+@pytest.mark.parametrize("n,nq,nkv,k,tile", [(1500, 17, 4, 520, 0), (2500, 16, 8, 520, 0), (1900, 27, 4, 2056, 256), (2048, 16, 8, 2048, 256)])
 @pytest.mark.parametrize("norm,rotate,scaled", [(True, True, True), (False, True, False), (True, False, False)])
-def test_qkv_product_over_pairs_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, norm, rotate, scaled):
-    test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, 128, 520, 16, norm, rotate, scaled)
+def test_qkv_product_over_pairs_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, k, tile, norm, rotate, scaled):
+    assert _pair_tile(K, 2, n, (nq + 2 * nkv) * 128, k) == tile
+    test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, 128, k, 16, norm, rotate, scaled)
 
 
 # Gate and up of a short prompt in tiles of 64 features: ragged rows, features and k, with and without a folded norm's factors.

@@ -74,7 +74,7 @@ def test_real_layer_sizes(model, dtype, tolerance):
 # Every way of cutting the work where the product's own kernels meet: head size 128 and pages of 16, so that prompt
 # portions run on the tcgen05 attention kernel beside decoded tokens on the TMA-fed small-q kernel in one step,
 # products of more than 64 rows on tcgen05 beside few-row ones (and, from 17 rows, o and down on tcgen05 with their k
-# range shared by a cluster), norms folded into the products of steps up to 128 rows and run as kernels above.  The layer sizes are Qwen3-0.6B's, with two layers and a vocabulary of 4,096.
+# range shared by a cluster), norms folded into the products around them.  The layer sizes are Qwen3-0.6B's, with two layers and a vocabulary of 4,096.
 # ----------------------------------------------------------------------------------------------------------------
 CUT_LENS = [137, 300, 64, 19, 285, 150, 1, 2, 328]
 
@@ -204,4 +204,63 @@ def test_a_long_context_in_the_benchmarks_regime(small_06b, dtype, tolerance):
     assert worst[2] <= tolerance * max(1.0, scale), worst
     if dtype == "bfloat16":
         assert K.tc_attention_calls > 0 and K.small_q_tma_calls > 0
+    K.check_device_errors()
+
+
+# ----------------------------------------------------------------------------------------------------------------
+# Norms folded into the products of prompts (matrices of 2^20 elements, any number of rows) in the other designs whose blocks
+# fold: the delta rule, latent attention and joint mixers, and parallel blocks, each also without a feed-forward before
+# blocks that have one.  Sample sizes of those designs, steps of 300 rows (one tile per CTA) and of 620 (over pairs of SMs
+# where the rule says so).
+# ----------------------------------------------------------------------------------------------------------------
+def _tigelorn(root):
+    import plain_tigelorn as plain
+    import tiny_tigelorn as T
+    with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "configs", "tigelorn-s.json")) as f:
+        d = json.load(f)
+    delta, latent, joint = d["layers"][:3]
+    bare = [dict(layer, mlp=None) for layer in (delta, latent, joint)]
+    d.update(vocab=1000, layers=[delta, bare[1], joint, bare[0], latent, bare[2], delta])
+    d["embedding"]["bigram"]["buckets"] = 4095
+    return plain, T, T.make_model_dir("T_wide", root, config=d, seed=5, store="bfloat16", sharpen=1.0)
+
+
+def _mubutar(root):
+    import plain_mubutar as plain
+    import tiny_mubutar as T
+    sizes = (16, 4, 64, 64, 0.125, 40.0)
+    layers = [T.layer(*sizes, mlp) for mlp in (None, T.dense(2048), T.dense(2048), None, T.dense(2048), T.dense(2048))]
+    return plain, T, T.make_model_dir("M_wide", root, config=T.config(1000, 1024, 1e-6, layers, emb=32.0), seed=6, store="bfloat16", sharpen=1.0)
+
+
+@pytest.mark.parametrize("design", [_tigelorn, _mubutar], ids=["tigelorn", "mubutar"])
+def test_prompts_of_other_designs_with_folded_norms(tmp_path, design):
+    """Against the plain implementation (nine tenths of the positions within 4 % of the largest logit, the median within 2 %: 8 bits
+    between kernels), and beside the same steps with the norms' own kernels, which round as often at another place."""
+    from infurnace_b200.engine.loading import EngineOptions, build_runner
+    plain, T, path = design(str(tmp_path))
+    cfg, w = T.load_model_dir(path)
+    reqs = {"a": tiny.random_tokens(1000, 300, 1), "b": tiny.random_tokens(1000, 620, 2)}
+    steps = [{"step": i, "entries": [{"id": r, "tokens": t, "want": list(range(len(t)))}], "end": [r]} for i, (r, t) in enumerate(reqs.items())]
+    want = torch.cat([plain.forward(cfg, w, t).double() for t in reqs.values()])
+    top = max(1.0, float(want.abs().max()))
+    runner = build_runner(path, EngineOptions(dtype="bfloat16", device="cuda", page_size=16, num_pages=64, max_num_seqs=2, max_num_batched_tokens=640,
+                                              max_model_len=640))[2]
+    K = runner.rt.kernels
+    runner.use_graphs = False
+    medians = {}
+    large = K.tc_fold_large
+    try:
+        for fold in (True, False):
+            K.tc_fold_large = large if fold else 1 << 62
+            before = K.tc_folded_calls
+            out = tiny.collect(steps, tiny.run_inprocess(runner, steps), 1000)
+            calls = K.tc_folded_calls - before
+            assert calls >= 2 * len(cfg["layers"]) if fold else calls == 0, calls
+            err = (torch.cat([out[r] for r in reqs]).double() - want).abs().max(dim=-1).values
+            medians[fold] = float(err.median())
+            assert float((err <= 0.04 * top).double().mean()) >= 0.9 and medians[fold] <= 0.02 * top, (fold, float(err.max()), medians, top)
+    finally:
+        K.tc_fold_large = large
+    assert medians[True] <= 1.5 * medians[False], medians
     K.check_device_errors()
