@@ -37,6 +37,8 @@ static inline int ifb_launch_status() {
 // L2 cache to fetch them.  ifb_pdl_trigger() lets the next kernel in the stream start being
 // scheduled; it is called right after the wait, so that one kernel, not the rest of the graph, runs
 // ahead and sits on the SMs.  IFB_PDL=0 in the environment turns the launch attribute off.
+// One kernel keeps the rule at its end instead of its start: the decode attention that runs beside the prompts' of the same step
+// (attention_mma.cu, `beside`).  It needs a predecessor whose every CTA waits before it triggers or exits, and of which it reads nothing.
 // A kernel may thus be resident while its predecessor still writes: only constants are read through the read-only path (__ldg), whose
 // loads a compiler may move ahead of the wait.
 __device__ __forceinline__ void ifb_pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }

@@ -479,6 +479,8 @@ static int gv_by_n(int nb, const void* x, const void* w, void* out, int n, int o
     // 37 us for the 201 MB of the 8B sizes, 90 against 83 to 85 for the 524 MB of the 32B sizes; with more blocks of tokens it is
     // the slower one), three for a short one (3,072 features: 384 CTAs over 148 SMs instead of 192, the fullest SM with 96 KB of
     // weights instead of 128; held to 80 registers, or the third does not fit: one decoded token of the 0.6B sizes 595 to 576 us)
+    // (a k of 1,025 to 2,048, 16 warps: 64 registers without spills, so two CTAs per SM where the form of 16 features, with 128, has one:
+    // the same weights in flight, in CTAs half as large; not timed apart)
     case 1:
       if (g_gv_gate_plan < 0) return gv_launch<1, EPI, WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);
       return gv_launch<1, (EPI == 1 ? 4 : EPI), WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);

@@ -1146,7 +1146,8 @@ linear_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, con
 // count both CTAs' bytes, the "empty" and "accumulator ready" barriers are each CTA's own and get a multicast commit, and the
 // "accumulator read" barriers are the first CTA's and count both CTAs' epilogue warps.
 // Measured at 2,048 rows against the best shape of one CTA: gate and up of 12,288 x 4,096 338 to 257 us (1.6 PFLOP/s),
-// q | k | v of 6,144 x 4,096 82 to 70, gate and up of 3,072 x 1,024 22.4 to 20.3, 1,024 x 3,072 14.9 to 13.8.
+// q | k | v of 6,144 x 4,096 82 to 70, gate and up of 3,072 x 1,024 22.4 to 20.3 (each alone, repeated; in a step it adds 23.3),
+// 1,024 x 3,072 14.9 to 13.8.
 // ROWS32: the epilogue stages 64 float32 features of a row at a time (tc_finish_residual, tc_finish_heads).
 // ---------------------------------------------------------------------------------------------------
 template <int EPI_, int NACC_, int STAGES_, bool ROWS32_> struct PairCfg {
@@ -1632,7 +1633,7 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
 // that many CTAs, whose parts are added in a fixed order; for few tiles of a long k (a step of some tens of tokens).
 // scale_partials (may be null): [scale_parts][n_rows] sums of squares; output row n is multiplied by
 // rsqrt(sum_p partials[p][n] / scale_width + scale_eps) before the epilogue.
-// res_x (may be null; plain epilogue, shape 0-3): the residual stream [n_rows][out_features] float32: v = x + y is
+// res_x (may be null; plain epilogue, shapes 0-3 and, with out_features a multiple of 64, 6): the residual stream [n_rows][out_features] float32: v = x + y is
 // written back to it, out = v * res_g, and res_partials [ifb_linear_tcgen05_fold_parts(...)][n_rows] gets sums of v^2.
 // bias (may be null; plain epilogue): float32 [out_features], added to the (scaled) product.
 IFB_EXPORT int ifb_linear_tcgen05_ex(const void* x, const void* w, void* out, int out_dtype, int n_rows, int out_features,
@@ -1699,7 +1700,7 @@ IFB_EXPORT int ifb_linear_tcgen05(const void* x, const void* w, void* out, int o
 }
 
 // The fused q | k | v projection of an attention layer with what follows it (see TcFold) in the epilogue of the one-tile
-// kernel (splits 1) or in the sum over the cluster of the shared-k form (splits 2 to 8): qkv [n_rows, (nq + 2 nkv) * 128] bfloat16 gets the normalised and rotated q heads (and the k and
+// kernel or of the pairs' (splits 1) or in the sum over the cluster of the shared-k form (splits 2 to 8): qkv [n_rows, (nq + 2 nkv) * 128] bfloat16 gets the normalised and rotated q heads (and the k and
 // v heads as they are stored), the pages get k and v at slots[n].  Heads of 128, rotated whole in the half-split pairing
 // (rope: [n_rows][64] pairs of cos and sin, 16-byte aligned, or null).  scale_*: as in ifb_linear_tcgen05_ex.
 IFB_EXPORT int ifb_linear_tcgen05_qkv(const void* x, const void* w, void* qkv, int n_rows, int nq, int nkv, int head_dim, int k_dim,

@@ -452,7 +452,8 @@ class CudaKernels:
     def can_fuse_qkv(self, n, dtype, w_qkv, head_dim, rotary_dim, interleaved, kv_pages):
         """Whether :meth:`linear_qkv_rope_store` takes a step of ``n`` rows: bfloat16, heads rotated whole in
         the half-split pairing (or not rotated); up to 16 rows on the few-rows kernel (heads of 64, 128 or
-        256), or on the tcgen05 kernel (heads of 128; up to 128 rows in its shared-k form only)."""
+        256), or on the tcgen05 kernel (heads of 128; up to 128 rows only where its clusters could share the
+        k range, although a k of at most 1,024 then runs in one tile per head)."""
         if not (self.fused_qkv and n > 0 and dtype == torch.bfloat16 and w_qkv.dtype == torch.bfloat16
                 and w_qkv.shape[1] % 8 == 0 and (rotary_dim == 0 or (rotary_dim == head_dim and not interleaved))
                 and (kv_pages is None or kv_pages.dtype == torch.bfloat16)):
