@@ -480,7 +480,8 @@ static int gv_by_n(int nb, const void* x, const void* w, void* out, int n, int o
     // the slower one), three for a short one (3,072 features: 384 CTAs over 148 SMs instead of 192, the fullest SM with 96 KB of
     // weights instead of 128; held to 80 registers, or the third does not fit: one decoded token of the 0.6B sizes 595 to 576 us)
     // (a k of 1,025 to 2,048, 16 warps: 64 registers without spills, so two CTAs per SM where the form of 16 features, with 128, has one:
-    // the same weights in flight, in CTAs half as large; not timed apart)
+    // the same weights in flight, in CTAs half as large: 6,144 x 2,048 14.4 to 12.8 us for one row and 14.3 to 13.8 for eight, 3,072 x
+    // 2,048 6.6 to 6.4 and 6.6 to 7.1)
     case 1:
       if (g_gv_gate_plan < 0) return gv_launch<1, EPI, WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);
       return gv_launch<1, (EPI == 1 ? 4 : EPI), WARPS, TO, STAGES>(x, w, out, n, o, k, rs, res, s);

@@ -338,7 +338,9 @@ class CudaKernels:
             return 1
         if epi and k <= 1024 and -(-o // 64) <= self.sm_count:
             # gate and up of a small model: a CTA per 64 features walks the whole k range in less time than a cluster's sum takes
-            # (with the q | k | v product of the same k likewise, 64 decoding requests of the 0.6B sizes 1,647 to 1,503 us)
+            # (with the q | k | v product of the same k likewise, 64 decoding requests of the 0.6B sizes 1,647 to 1,503 us).  Alone, 3,072
+            # features: 64 rows at k 1,024 6.7 us whole and 7.9 shared, at 1,536 8.3 and 8.7, at 2,048 10.0 and 9.8; 20 rows 7.3
+            # and 6.6, 9.7 and 7.9; 128 rows whole to 2,560 at least (11.8 and 13.0)
             return 1
         tiles = -(-o // 128) * -(-n // 128)
         for splits in range(min(8, k // self.tc_split_min_k), 1, -1):
@@ -511,7 +513,7 @@ class CudaKernels:
                 # to 3,202 us for 3,116); the tables of the step function lie on 16 bytes
                 rope_table = rope_table.clone()
             # (more than one tile of rows, or a short k: the cluster's sum would take longer over the heads than the shared k
-            # range saves)
+            # range saves; 32 heads at k 1,280: 64 rows 8.7 us whole and 7.3 shared, 128 rows 8.9 and 8.8)
             splits = self.tcgen05_splits(n, width, k) if n <= 128 and k > 1024 else 1
             self.tc_shared_k_calls += splits > 1
             self.tc_folded_calls += partials is not None
