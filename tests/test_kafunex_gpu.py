@@ -150,6 +150,47 @@ def test_gated_recurrence_kernel(K, heads, dim, vdim):
     close(out_bf[rows], want[rows], 0.05, "bfloat16 outputs")
 
 
+# The tiled form of the recurrence in blocks (heads of 33 to 64 rows and 65 to 128 columns): the corners of its sizes, aligned
+# rows and not, blocks of one token, of 63, 64 and 65, and several; gates that are 0, 1 and tiny.
+@pytest.mark.parametrize("heads,dim,vdim,pad", [(8, 64, 128, 4), (3, 33, 65, 3), (2, 64, 100, 0), (1, 47, 128, 1), (2, 36, 127, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_recurrence_in_tiles(K, heads, dim, vdim, pad, dtype):
+    lens = [1, 63, 64, 65, 0, 290, 17]
+    cu = [0]
+    for ql in lens:
+        cu.append(cu[-1] + max(1, ql))                          # padding has a row too
+    n, hd, hv = cu[-1], heads * dim, heads * vdim
+    proj, bias, lower, nw = _scan_inputs(heads, dim, vdim, n, heads + dim + vdim)
+    proj = torch.cat((proj[:, :2 * hd + hv], torch.zeros(n, pad)), dim=1).contiguous()
+    proj[100:140, hd:hd + hd // 2] = -200.0                     # gates at their lower bounds ...
+    lower[: hd // 4] = 0.0                                      # ... of which some are 0
+    proj[150:200, hd + hd // 2:2 * hd] = 200.0                  # gates of 1
+    slots = torch.tensor([6, 0, 5, 1, 0, 3, 2], dtype=torch.int32)
+    state0 = torch.randn(7, heads, dim, vdim, generator=gen(1))
+    seq = torch.tensor([100, 63, 64, 70, 0, 290, 40], dtype=torch.int32)
+    want_state, want = state0.clone().double(), torch.zeros(n, hv, dtype=torch.float64)
+    REF.gated_scan(proj, 0, hd, 2 * hd, bias, lower, nw, 1e-5, want_state, slots, torch.tensor(cu, dtype=torch.int32), seq, want,
+                   heads, dim, vdim)
+    rows = [i for i in range(n) if i != cu[4]]
+
+    def run(x, y):
+        state, got, before = y.cuda(), torch.full((n, hv), 7.0, device="cuda", dtype=dtype), K.scan_blocked_calls
+        K.gated_scan(x.cuda(), 0, hd, 2 * hd, bias.cuda(), lower.cuda(), nw.cuda(), 1e-5, state, slots.cuda(),
+                     torch.tensor(cu, dtype=torch.int32).cuda(), seq.cuda(), got, heads, dim, vdim, max_q_len=290)
+        assert K.scan_blocked_calls == before + 1
+        return got, state
+    got, state = run(proj, state0)
+    close(got[rows], want[rows], 2e-5 if dtype == torch.float32 else 0.05, "outputs"), close(state, want_state, 2e-5, "states")
+    assert torch.equal(state[4].cpu(), state0[4]) and bool((got[cu[4]] == 7.0).all())          # a slot of nobody, a row of padding
+    # what a later token holds never reaches an earlier one, whatever it is
+    for value in (float("nan"), float("inf")):
+        bad = proj.clone()
+        bad[cu[5] + 133] = value
+        again, _ = run(bad, state0)
+        keep = [i for i in rows if i < cu[5] + 133 or i >= cu[6]]
+        assert torch.equal(again[keep], got[keep])
+
+
 def _attention_case(K, H, G, d, ps, chunk, dtype, lens_and_new, seed, talk=True, gate=True, slope=8.0, plant=None, nan_at=None):
     """Requests of (length after the step, new tokens) over a shuffled page pool; compares kernel and statement."""
     g = gen(seed)
