@@ -31,6 +31,7 @@ pages that a window has passed.  ``free_request`` gives everything back, once.
 """
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional, Tuple
 
@@ -73,6 +74,7 @@ class StateGroup:
     need: StateNeed
     cache_ids: List[int]
     tensors: Dict[int, object] = field(default_factory=dict)      # cache id -> [slots, *shape]
+    store: object = None      # [entries, numbers of an entry, to a multiple of 64]: the memory that the tensors are views of
 
 
 class CacheLayout:
@@ -155,8 +157,11 @@ class CacheManager:
                         g.streams[cid] = {x.name: torch.zeros((g.pool.num_pages, x.heads, page_size, x.width),
                                                               dtype=dtype, device=device) for x in st}
             for g in self.state_groups:
-                for cid in g.cache_ids:
-                    g.tensors[cid] = torch.zeros((max_requests, *g.need.shape), dtype=torch.float32, device=device)
+                # one allocation, so that a new request's slot is cleared in all entries by one launch; an entry starts
+                # at a multiple of 256 bytes, as an allocation of its own would
+                size = max_requests * math.prod(g.need.shape)
+                g.store = torch.zeros((len(g.cache_ids), -(-size // 64) * 64), dtype=torch.float32, device=device)
+                g.tensors = {cid: g.store[i, :size].view(max_requests, *g.need.shape) for i, cid in enumerate(g.cache_ids)}
 
     # ------------------------------------------------------------------ lookups
     def kv_group_of(self, cache_id: int) -> int:
@@ -217,8 +222,9 @@ class CacheManager:
         for g in self.kv_groups:
             g.tables[rid] = []
         for g in self.state_groups:
-            for t in g.tensors.values():
-                t[slot].zero_()
+            if g.store is not None:
+                per = math.prod(g.need.shape)
+                g.store[:, slot * per:(slot + 1) * per].zero_()
         return slot
 
     def pages_needed(self, rid: str, num_new_tokens: int) -> List[int]:
