@@ -23,8 +23,8 @@ __host__ __device__ __forceinline__ int s32_group(int k_dim) {
 __device__ __forceinline__ float s32_total(const float (&p)[S32_GROUPS]) {
   return (((p[0] + p[1]) + (p[2] + p[3])) + (p[4] + p[5])) + (p[6] + p[7]);
 }
-// Two multiply-adds in one instruction (a and b: two neighbouring floats each): the device's full float32 rate, which
-// single multiply-adds reach half of.
+// Two multiply-adds in one instruction (a and b: two neighbouring floats each): half the instructions at the rate of single ones
+// (a warp's takes 2.2 cycles of a scheduler, a single one's 1.02).
 __device__ __forceinline__ void s32_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(acc) : "l"(a), "l"(b));
 }
@@ -155,37 +155,49 @@ rows32_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __re
 }
 
 // ---------------------------------------------------------------------------------------------------
-// Many rows: bound by shared-memory reads (two of 16 bytes per 32 multiply-adds), which is why the tile per thread is as large as
-// the registers hold: 32 TFLOP/s at 2,048 rows, 25 at 193; the single chain per output had 22.5 and, where 1,024 features
-// leave most SMs without a tile, 4 (193 rows, k = 2,048: 202 to 35 us).  A cluster of two CTAs owns a tile of 64 rows of x by 64 rows of w; each of
+// Many rows: bound by the multiply-adds, of which two warps per scheduler keep one going every 3.5 cycles (2.5 is the least with
+// operands in registers; four warps with half the outputs each, or single multiply-adds, are no faster).  The tile per thread is as large as
+// the registers hold (a single chain per output had 22.5 TFLOP/s at 2,048 rows and, where 1,024 features
+// leave most SMs without a tile, 4).  A cluster of two CTAs owns a tile of up to 64 rows of x by 64 rows of w; each of
 // the eight slices of 64 threads (four per CTA) runs one group of the k range through its own ring of stages, a
-// thread summing 8 x 8 outputs (16 16-byte reads of shared memory, free of bank conflicts, per 256 multiply-adds).  The
+// thread summing up to 8 x 8 outputs (16 16-byte reads of shared memory, free of bank conflicts, per 256 multiply-adds).  The
 // groups' tiles then meet in the two CTAs' shared memory, each CTA adding half of the tile's rows.  EPI 1: the tile's first 32 rows of w are gate rows, the others the up rows of the same features.
+// ALONE: where tiles are more than the pairs of SMs, a CTA takes a whole tile, each slice two groups one after the other in one run
+// through its ring (of three stages; the first group's tile waits beside it).  Filling the ring and the sum at the end cost a CTA
+// of a pair 17,000 of 37,000 cycles at a k of 1,024: 2,048 rows of 4,096 x 1,024 535 to 424 us (40 TFLOP/s), 193 rows of the LM head 2,371 to 1,830.
+// RT: rows per thread, and an eighth of a tile's (tile32_form).
 // ---------------------------------------------------------------------------------------------------
 constexpr int T32 = 64, T32_SLICES = S32_GROUPS / 2, T32_PITCH = S32_BK + 4;      // 20 floats: conflict-free 16-byte reads
 constexpr int T32_STAGE = 2 * T32 * T32_PITCH;                                    // floats: the rows of x, then those of w
-constexpr int T32_STAGES = 4;
+constexpr int T32_LANES = 64, T32_TO = 8, T32_J = T32 / T32_TO;                   // threads of a slice, across features; features per thread
+constexpr int T32_SMS = 148;                                                     // of the device that the choice of a form is for
 constexpr int T32_RED = T32 + 8;                                                  // floats per row of a group's tile
-constexpr size_t T32_SMEM = (size_t)T32_SLICES * T32_STAGES * T32_STAGE * sizeof(float);
-static_assert(T32 * T32_RED <= T32_STAGES * T32_STAGE, "a group's tile goes where its stages were");
+template <bool ALONE> struct Tile32 {
+  static constexpr int STAGES = ALONE ? 3 : 4;
+  static constexpr int RING = STAGES * T32_STAGE;                                 // floats of a slice's stages, then those of a first group's tile
+  static constexpr int SLICE = RING + (ALONE ? T32 * T32_RED : 0);
+  static constexpr size_t SMEM = (size_t)T32_SLICES * SLICE * sizeof(float);
+  static_assert(T32 * T32_RED <= RING, "a group's tile goes where its stages were");
+};
 
-template <int EPI, bool VEC, typename TO>
-__global__ void __launch_bounds__(T32_SLICES * 64, 1)
+template <int EPI, bool VEC, bool ALONE, int RT, typename TO>
+__global__ void __launch_bounds__(T32_SLICES * T32_LANES, 1)
 tile32_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __restrict__ out, int n_rows, int o_out, int k_dim,
               int unary, const float* __restrict__ bias) {
-  constexpr int STEP = VEC ? 4 : 1, PER = S32_BK / STEP, FO = EPI ? T32 / 2 : T32;
+  constexpr int STEP = VEC ? 4 : 1, PER = S32_BK / STEP, FO = EPI ? T32 / 2 : T32, T32_STAGES = Tile32<ALONE>::STAGES, ROWS = 8 * RT;
   extern __shared__ __align__(16) float s32_smem[];
-  const int slice = threadIdx.x >> 6, t = threadIdx.x & 63, to = t & 7, tn = t >> 3;
-  float* buf = s32_smem + (size_t)slice * T32_STAGES * T32_STAGE;
-  uint32_t rank;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
-  const int o0 = (blockIdx.x >> 1) * FO, n0 = blockIdx.y * T32;
-  const int gl = s32_group(k_dim), kbeg = min(k_dim, ((int)rank * T32_SLICES + slice) * gl), kend = min(k_dim, kbeg + gl);
+  const int slice = threadIdx.x / T32_LANES, t = threadIdx.x % T32_LANES, to = t % T32_TO, tn = t / T32_TO;
+  float* buf = s32_smem + (size_t)slice * Tile32<ALONE>::SLICE;
+  uint32_t rank = 0;
+  if (!ALONE) asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(rank));
+  const int o0 = (ALONE ? blockIdx.x : blockIdx.x >> 1) * FO, n0 = blockIdx.y * ROWS;
+  const int gl = s32_group(k_dim), per = ALONE ? 2 : 1;           // groups of a slice
+  const int kbeg = min(k_dim, ((int)rank * T32_SLICES + slice) * per * gl), kend = min(k_dim, kbeg + per * gl);
   const int steps = (kend - kbeg + S32_BK - 1) / S32_BK;
   auto load_w = [&](int st) {
     float* dst = buf + (st % T32_STAGES) * T32_STAGE + T32 * T32_PITCH;
 #pragma unroll
-    for (int i = t; i < T32 * PER; i += 64) {
+    for (int i = t; i < T32 * PER; i += T32_LANES) {
       const int r = i / PER, k = kbeg + st * S32_BK + (i % PER) * STEP;
       const int o = o0 + (EPI ? r % FO : r);
       const bool in = o < o_out && k < kend;
@@ -196,13 +208,13 @@ tile32_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __re
   auto load_x = [&](int st) {
     float* dst = buf + (st % T32_STAGES) * T32_STAGE;
 #pragma unroll
-    for (int i = t; i < T32 * PER; i += 64) {
+    for (int i = t; i < ROWS * PER; i += T32_LANES) {
       const int r = i / PER, k = kbeg + st * S32_BK + (i % PER) * STEP;
       const bool in = n0 + r < n_rows && k < kend;
       s32_copy<VEC>(dst + r * T32_PITCH + (i % PER) * STEP, in ? x + (size_t)(n0 + r) * k_dim + k : x, in);
     }
   };
-  auto slice_sync = [&]() { asm volatile("bar.sync %0, 64;\n" ::"r"(slice + 1) : "memory"); };
+  auto slice_sync = [&]() { asm volatile("bar.sync %0, %1;\n" ::"r"(slice + 1), "n"(T32_LANES) : "memory"); };
 #pragma unroll 1
   for (int st = 0; st < T32_STAGES - 1; ++st)
     if (st < steps) load_w(st);
@@ -213,11 +225,20 @@ tile32_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __re
     if (st < steps) load_x(st);
     s32_commit();
   }
-  unsigned long long acc[8][8];                                   // sums over even and over odd k
+  unsigned long long acc[RT][T32_J];                                   // sums over even and over odd k
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < RT; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0;
+    for (int j = 0; j < T32_J; ++j) acc[i][j] = 0;
+  auto keep = [&](float* tile) {                                  // a group's sums, and from zero again
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int j = 0; j < T32_J; ++j) {
+        tile[(tn + 8 * i) * T32_RED + to + T32_TO * j] = s32_pair_sum(acc[i][j]);
+        acc[i][j] = 0;
+      }
+  };
 #pragma unroll 1
   for (int st = 0; st < steps; ++st) {
     s32_wait<T32_STAGES - 2>();
@@ -228,25 +249,47 @@ tile32_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __re
     const float* ws = buf + (st % T32_STAGES) * T32_STAGE + (T32 + to) * T32_PITCH;
 #pragma unroll
     for (int k = 0; k < S32_BK; k += 4) {
-      ulonglong2 wv[8];
+      ulonglong2 wv[T32_J];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(ws + 8 * j * T32_PITCH + k);
+      for (int j = 0; j < T32_J; ++j) wv[j] = *reinterpret_cast<const ulonglong2*>(ws + T32_TO * j * T32_PITCH + k);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < RT; ++i) {
         const ulonglong2 xv = *reinterpret_cast<const ulonglong2*>(xs + 8 * i * T32_PITCH + k);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) s32_fma2(acc[i][j], xv.x, wv[j].x);
+        for (int j = 0; j < T32_J; ++j) s32_fma2(acc[i][j], xv.x, wv[j].x);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) s32_fma2(acc[i][j], xv.y, wv[j].y);
+        for (int j = 0; j < T32_J; ++j) s32_fma2(acc[i][j], xv.y, wv[j].y);
       }
     }
+    if (ALONE && (st + 1) * S32_BK == gl) keep(buf + Tile32<ALONE>::RING);       // the first group is complete
   }
   s32_wait<0>();
   slice_sync();                                                   // no copy into the slice's stages is left, none is read
+  if (ALONE && steps * S32_BK < gl) keep(buf + Tile32<ALONE>::RING);             // it was the last, and cut short
+  keep(buf);
+  if constexpr (ALONE) {
+    __syncthreads();
+    // the first groups of the slices, then the second ones
+    auto total = [&](int r, int c) {
+      float p[S32_GROUPS];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) buf[(tn + 8 * i) * T32_RED + to + 8 * j] = s32_pair_sum(acc[i][j]);
+      for (int g = 0; g < S32_GROUPS; ++g) p[g] = s32_smem[(g / 2) * Tile32<ALONE>::SLICE + (g % 2 ? 0 : Tile32<ALONE>::RING) + r * T32_RED + c];
+      return s32_total(p);
+    };
+#pragma unroll 2
+    for (int i = threadIdx.x; i < ROWS * FO; i += T32_SLICES * T32_LANES) {
+      const int r = i / FO, c = i % FO, o = o0 + c, n = n0 + r;
+      if (n >= n_rows || o >= o_out) continue;
+      float y = total(r, c);
+      if (EPI) y = ifb_gate_act(y, unary) * total(r, FO + c);
+      else {
+        if (bias) y += bias[o];
+        if (unary) y = ifb_unary(y, unary);
+      }
+      out[(size_t)n * o_out + o] = from_f32<TO>(y);
+    }
+    return;
+  }
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
   // the tiles of groups 0-3 lie in CTA 0, those of 4-7 in CTA 1; this CTA adds the rows [32 * rank, 32 * rank + 32)
@@ -258,14 +301,14 @@ tile32_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __re
     float p[S32_GROUPS];
 #pragma unroll
     for (int g = 0; g < S32_GROUPS; ++g) {
-      const uint32_t a = base[g / T32_SLICES] + (uint32_t)(((g % T32_SLICES) * T32_STAGES * T32_STAGE + r * T32_RED + c) * 4);
+      const uint32_t a = base[g / T32_SLICES] + (uint32_t)(((g % T32_SLICES) * Tile32<ALONE>::SLICE + r * T32_RED + c) * 4);
       asm volatile("ld.shared::cluster.f32 %0, [%1];\n" : "=f"(p[g]) : "r"(a) : "memory");
     }
     return s32_total(p);
   };
 #pragma unroll 2
-  for (int i = threadIdx.x; i < (T32 / 2) * FO; i += T32_SLICES * 64) {
-    const int r = (int)rank * (T32 / 2) + i / FO, c = i % FO, o = o0 + c, n = n0 + r;
+  for (int i = threadIdx.x; i < (ROWS / 2) * FO; i += T32_SLICES * T32_LANES) {
+    const int r = (int)rank * (ROWS / 2) + i / FO, c = i % FO, o = o0 + c, n = n0 + r;
     if (n >= n_rows || o >= o_out) continue;
     float y = total(r, c);
     if (EPI) y = ifb_gate_act(y, unary) * total(r, FO + c);
@@ -288,32 +331,69 @@ static int rows32_launch(const float* x, const float* w, TO* out, int n, int o, 
                     unary, bias);
 }
 
-template <int EPI, bool VEC, typename TO>
-static int tile32_launch(const float* x, const float* w, TO* out, int n, int o, int k, int unary, const float* bias, cudaStream_t s) {
-  IFB_ALLOW_SMEM((tile32_kernel<EPI, VEC, TO>), T32_SMEM);
-  const int fo = EPI ? T32 / 2 : T32;
+template <int EPI, bool VEC, bool ALONE, int RT, typename TO>
+static int tile32_launch_as(const float* x, const float* w, TO* out, int n, int o, int k, int unary, const float* bias, cudaStream_t s) {
+  constexpr size_t smem = Tile32<ALONE>::SMEM;
+  constexpr int fo = EPI ? T32 / 2 : T32;
+  IFB_ALLOW_SMEM((tile32_kernel<EPI, VEC, ALONE, RT, TO>), smem);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * ((o + fo - 1) / fo), (n + T32 - 1) / T32);
-  cfg.blockDim = dim3(T32_SLICES * 64);
-  cfg.dynamicSmemBytes = T32_SMEM;
+  cfg.gridDim = dim3((ALONE ? 1 : 2) * ((o + fo - 1) / fo), (n + 8 * RT - 1) / (8 * RT));
+  cfg.blockDim = dim3(T32_SLICES * T32_LANES);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = ifb_pdl_enabled() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = ifb_pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, tile32_kernel<EPI, VEC, TO>, x, w, out, n, o, k, unary, bias);
+  cfg.numAttrs = ALONE ? 1 : 2;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, tile32_kernel<EPI, VEC, ALONE, RT, TO>, x, w, out, n, o, k, unary, bias);
   if (e != cudaSuccess) { cudaGetLastError(); return -(int)e; }
   return IFB_OK;
 }
 
+// Rows per thread (a tile has eight times as many) and whether a CTA takes a tile alone: the form whose waves should take least
+// time, by the time of one wave at a k of 1,024 (in tenths of a microsecond, measured over matrices of 1,024 to 40,000 features, 17 to 193
+// rows; a longer k scales them alike).  17 rows 18.8 to 11.5 us for 4,096 x 1,024 and 31.9 to 16.4 for 1,024 x 2,048 against tiles of 64
+// rows by pairs, 193 rows 72 to 59 and 33.5 to 31.3.  The sums are the same in every form.
+static void tile32_form(int n, int tiles, int* rows, bool* alone) {
+  static const int wave[2][9] = {{0, 0, 98, 117, 127, 148, 168, 180, 196}, {0, 0, 146, 201, 218, 240, 295, 289, 310}};
+  long long least = 0;
+  for (int rt = 8; rt >= 2; --rt) {
+    const long long all = (long long)tiles * ((n + 8 * rt - 1) / (8 * rt));
+    for (int a = 0; a < 2; ++a) {
+      const int slots = a ? T32_SMS : T32_SMS / 2;
+      const long long time = (all + slots - 1) / slots * wave[a][rt];
+      if (!least || time < least) { least = time; *rows = rt; *alone = a; }
+    }
+  }
+}
+template <int EPI, bool VEC, typename TO>
+static int tile32_launch(const float* x, const float* w, TO* out, int n, int o, int k, int unary, const float* bias, cudaStream_t s) {
+  const int fo = EPI ? T32 / 2 : T32;
+  int rows = 8;
+  bool alone = false;
+  tile32_form(n, (o + fo - 1) / fo, &rows, &alone);
+#define IFB_T32(RT) \
+  case RT: return alone ? tile32_launch_as<EPI, VEC, true, RT, TO>(x, w, out, n, o, k, unary, bias, s) \
+                        : tile32_launch_as<EPI, VEC, false, RT, TO>(x, w, out, n, o, k, unary, bias, s);
+  if constexpr (VEC && sizeof(TO) == 4) {                        // rows not at 16 bytes, and bfloat16 outputs, are rare: eight rows per thread
+    if (n <= 65535 * 16)                                         // tiles of rows that a grid holds
+      switch (rows) {
+        IFB_T32(2) IFB_T32(3) IFB_T32(4) IFB_T32(5) IFB_T32(7)
+        case 6: return tile32_launch_as<EPI, VEC, false, 6, TO>(x, w, out, n, o, k, unary, bias, s);      // alone, seven take less
+      }
+  }
+  switch (8) { IFB_T32(8) }
+#undef IFB_T32
+  return IFB_ERR_ARG;
+}
+
 // Float32 operands.  Up to S32_FEW_ROWS rows the weights are streamed once per eight rows (from the second time on out of
-// L2); beyond, a tile of 64 rows, however few of them exist, is the cheaper one (4,096 x 1,024: 8 rows 9.6 us, 32 rows as four
-// times eight 26 us, 48 rows as a tile 20 us).
+// L2); beyond, tiles are the cheaper ones (4,096 x 1,024: 8 rows 9.6 us, 32 rows as four times eight 26 us, as a tile 12.8).
 constexpr int S32_FEW_ROWS = 16;
 template <int EPI, bool VEC, typename TO>
 static int launch32_vec(const float* x, const float* w, TO* out, int n, int o, int k, int unary, const float* bias, cudaStream_t s) {

@@ -632,6 +632,16 @@ def test_plain_product_of_a_row_is_the_same_in_every_batch(K, n, o, k, epilogue)
         assert torch.equal(alone[0], out[row])
 
 
+# The product of many rows in all its forms: tiles of 16 to 64 rows (every number of rows per thread, full and with one row of the
+# last tile), by pairs of CTAs and by one (from 2,000 features on), k ranges that end in a slice's first group, in its
+# second and in a later slice.
+@pytest.mark.parametrize("n", [17, 18, 24, 25, 33, 41, 49, 57, 65, 113, 193])
+@pytest.mark.parametrize("o,k", [(65, 272), (2000, 24), (4800, 136), (9600, 36), (4760, 16)])
+@pytest.mark.parametrize("epilogue", ["none", "silu_gate"])
+def test_plain_product_of_many_rows(K, n, o, k, epilogue):
+    test_plain_product_of_a_row_is_the_same_in_every_batch(K, n, o, k, epilogue)
+
+
 # Plain attention in float32 storage: a query's bits do not depend on the other queries of the step, and rows that it may
 # not see (stale pages, later tokens, here NaN) never reach it.
 @pytest.mark.parametrize("nq,nkv,d,ps,window", [(16, 8, 128, 16, 0), (4, 2, 16, 16, 0), (9, 1, 36, 8, 33), (20, 1, 4, 1, 0), (6, 3, 200, 5, 40),
