@@ -441,7 +441,7 @@ def time_e2e(engine, vocab, batch, context, steps, warmup):
     while not engine.is_done():
         engine.step()
     run = engine.runner
-    h2d = run._small_len * 4 + batch * run.max_pages * 4 * max(1, len(run.cache.kv_groups))
+    h2d = run._tables_at * 4 + batch * run.max_pages * 4 * max(1, len(run.cache.kv_groups))
     return {"value": n / wall, "unit": "tokens/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": batch * 4,
             "ms_per_step": wall * 1000 / steps, "device_ms_per_step": s.elapsed_time(e) / steps}
 

@@ -30,10 +30,16 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional, Sequence
 
+import numpy as np
 import torch
 
 from ..cache import CacheManager, RELEASED
 from ..errors import BatchError, OutOfPages
+
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+if _raw_stream is None:                       # an older torch: the public, slower way
+    def _raw_stream(device_index):
+        return torch.cuda.current_stream(device_index).cuda_stream
 
 
 @dataclass
@@ -67,6 +73,22 @@ class KVView:
     page_size: int
     window: Optional[int]
     streams: Optional[Dict[str, torch.Tensor]] = None
+
+
+@dataclass
+class _Staged:
+    """A step that is on its way to the device: what its launches take from the host."""
+    num_tokens: int
+    num_requests: int
+    num_logit_rows: int
+    num_real_logit_rows: int
+    max_q_len: int
+    min_q_len: int
+    max_seq_len: int
+    cu_q: List[int]
+    seq_lens: List[int]
+    state_slots: List[int]
+    first_portion: List[int]
 
 
 class _Arena:
@@ -153,18 +175,21 @@ class ModelRunner:
         n, r, g = self._n_cap, self.max_requests, len(cache.kv_groups)
         # one staging area: [ids n][pos n][req n][logit_rows n][cu_q r+1][seq r][slot r][first r] + g * [slots n]
         self._small_len = 4 * n + 4 * r + 1 + g * n + 2 * r      # the last 2r words: temperatures, uniforms (float32)
+        # behind it, from a multiple of 256 bytes on, the block tables [g][r][pages]: with one group one copy brings a step's share of both
+        self._tables_at = -(-self._small_len // 64) * 64
         # two host staging sets used in turn: a set is rewritten only after the copy that
         # read it last has finished (its event), so the host may run a step ahead
-        self._stage = [
-            (torch.zeros(self._small_len, dtype=torch.int32, pin_memory=self._pin),
-             torch.full((max(g, 1), r, self.max_pages), RELEASED, dtype=torch.int32, pin_memory=self._pin))
-            for _ in range(2)]
+        self._stage = [self._staging(torch.zeros, pin_memory=self._pin) for _ in range(2)]
         self._stage_events = [None, None]
-        self._stage_np = [(a.numpy(), b.numpy()) for a, b in self._stage]      # the same memory, for cheap list writes
+        self._stage_np = [(b.numpy(), c.numpy()) for _, b, c in self._stage]      # the same memory, for cheap list writes
+        # whose table a row of a staging set holds, and how much of it: (rid, epoch, length) by (group, row)
+        self._stage_rows = [{}, {}]
         # block tables of live requests as arrays that grow with the tables: (epoch, synced length, array) by (rid, group)
         self._table_rows: Dict[tuple, list] = {}
-        self._dev_small = torch.zeros(self._small_len, dtype=torch.int32, device=dev)
-        self._dev_tables = torch.full((max(g, 1), r, self.max_pages), RELEASED, dtype=torch.int32, device=dev)
+        self._dev_all, self._dev_small, self._dev_tables = self._staging(torch.zeros, device=dev)
+        self._event_pool: Dict[tuple, object] = {}
+        self._parts: Dict[tuple, list] = {}
+        self._stream_held = (None, None)                         # (raw handle, torch's object) of the stream that events go to
         self.steps_run = 0
         self.sampled = torch.zeros(max(r, 1), dtype=torch.int32, device=dev)
         # the sampled ids of the last two steps (a step in flight may feed the next one from the device)
@@ -178,6 +203,35 @@ class ModelRunner:
         self.max_graphs = 64
         self.graph_replays = 0
         self.launches_per_graph_step = 0
+
+    def _staging(self, make, **kw):
+        """A staging area and its two parts: what a step's tokens and requests are, and the block tables."""
+        shape = (max(len(self.cache.kv_groups), 1), self.max_requests, self.max_pages)
+        whole = make(self._tables_at + shape[0] * shape[1] * shape[2], dtype=torch.int32, **kw)
+        tables = whole[self._tables_at:].view(shape)
+        tables.fill_(RELEASED)
+        return whole, whole[:self._small_len], tables
+
+    def _part(self, name, n, *tensors):
+        """The first ``n`` elements of tensors that live as long as the runner (``name`` stands for them), without slicing them anew
+        in every step."""
+        parts = self._parts.get((name, n))
+        if parts is None:
+            if len(self._parts) > 4096:
+                self._parts.clear()
+            parts = self._parts[(name, n)] = [t[:n] for t in tensors]
+        return parts
+
+    def _record(self, name):
+        """The event ``name`` (one object for the runner's life), recorded on the current stream."""
+        event = self._event_pool.get(name)
+        if event is None:
+            event = self._event_pool[name] = torch.cuda.Event()
+        raw = _raw_stream(torch._C._cuda_getDevice())
+        if raw != self._stream_held[0]:
+            self._stream_held = (raw, torch.cuda.current_stream())
+        event.record(self._stream_held[1])
+        return event
 
     # ------------------------------------------------------------------ the step
     def validate(self, entries: Sequence[StepEntry], placeholders: bool = False, sampled: bool = False) -> None:
@@ -268,12 +322,10 @@ class ModelRunner:
         slot = self._sampled_steps % 2
         self._sampled_steps += 1
         dev, host = self._hist[slot], self._hist_host[slot]
-        dev[:wanted].copy_(self.sampled[:wanted])
-        host[:wanted].copy_(dev[:wanted], non_blocking=True)
-        event = None
-        if self._pin:
-            event = torch.cuda.Event()
-            event.record()
+        dev_part, host_part, sampled_part = self._part(("hist", slot), wanted, dev, host, self.sampled)
+        dev_part.copy_(sampled_part)
+        host_part.copy_(dev_part, non_blocking=True)
+        event = self._record(("sampled", slot)) if self._pin else None
         return SampledTokens(dev, host, event, wanted, slot)
 
     def _run_reserved(self, entries, temperatures, uniforms, feed, sample: bool):
@@ -283,22 +335,25 @@ class ModelRunner:
         try:
             return self._execute(entries, temperatures, uniforms, feed, sample=sample)
         except BaseException:
+            self._table_rows.clear()               # the tables get shorter, and may grow again with other pages
+            for held in self._stage_rows:
+                held.clear()
             for e in entries:
                 if self.cache.has_request(e.request_id):
                     self.cache.release_allocation(e.request_id)
             raise
 
-    def _apply_feed(self, ctx, feed) -> None:
+    def _apply_feed(self, feed) -> None:
         """Overwrite the step's token ids on the device with rows of the previous step's sampled ids."""
         if feed is None:
             return
         prev, rows = feed
         n = len(rows)
         if list(rows) == list(range(n)):
-            ctx.token_ids[:n].copy_(prev.device[:n])
+            self._part("ids", n, self._dev_small)[0].copy_(prev.device[:n])          # the ids come first in the staging area
         else:
             idx = torch.tensor(list(rows), dtype=torch.int64, device=prev.device.device)
-            ctx.token_ids[:n].copy_(prev.device.index_select(0, idx))
+            self._dev_small[:n].copy_(prev.device.index_select(0, idx))
 
     def _forward(self, ctx, sample: bool, greedy: bool):
         logits = self.model.forward(ctx)
@@ -322,7 +377,7 @@ class ModelRunner:
         portions of one size, a benchmark's repeated prompt), so that one-off shapes cost no
         recording.  A graph is dropped when a buffer it points at has moved."""
         greedy = sample and all(t == 0.0 for t in temperatures)
-        build = dict(temperatures=temperatures, uniforms=uniforms) if sample else {}
+        build = dict(temperatures=temperatures, uniforms=uniforms) if sample and not greedy else {}      # nothing reads them then
         # The padding and the length bucket are the same whether graphs are used or not, so that a step launches
         # the same kernels with the same parameters either way (the split of a context over CTAs follows the bucket).
         longest = max(self.cache.num_computed(e.request_id) + len(e.tokens) for e in entries)
@@ -338,16 +393,15 @@ class ModelRunner:
             r_bucket = min(r_bucket, self.max_requests)      # <= _n_cap, which the staging regions are sized by
         if not self.use_graphs:
             ctx = self._build_context(entries, pad_to=r_bucket, seq_bucket=seq_bucket, **build)
-            self._apply_feed(ctx, feed)
+            self._apply_feed(feed)
             return self._forward(ctx, sample, greedy)
+        staged = self._stage_step(entries, pad_to=r_bucket, seq_bucket=seq_bucket, **build)
         if decode_only:
             key = ("decode", r_bucket, seq_bucket, greedy)
-            ctx = self._build_context(entries, pad_to=r_bucket, seq_bucket=seq_bucket, **build)
         else:
-            ctx = self._build_context(entries, seq_bucket=seq_bucket, **build)
-            key = ("any", ctx.num_tokens, ctx.num_requests, ctx.num_logit_rows, ctx.max_q_len, ctx.min_q_len, seq_bucket,
-                   sample, greedy)
-        self._apply_feed(ctx, feed)
+            key = ("any", staged.num_tokens, staged.num_requests, staged.num_logit_rows, staged.max_q_len, staged.min_q_len,
+                   seq_bucket, sample, greedy)
+        self._apply_feed(feed)
         stamp = (self.arena.generation, getattr(self.rt.kernels, "scratch_generation", 0))
         held = self._graphs.get(key)
         if held is not None and held[1] == stamp:
@@ -358,6 +412,7 @@ class ModelRunner:
             self._shapes_seen.clear()
         seen = self._shapes_seen.get(key, 0) + 1
         self._shapes_seen[key] = seen
+        ctx = self._context(staged)
         # run once as it is (which also makes every allocation) ...
         logits = self._forward(ctx, sample, greedy)
         if not decode_only and seen < 2:
@@ -386,7 +441,6 @@ class ModelRunner:
     def _table_row(self, rid, gi):
         """The block table of (request, group) as an int32 array, extended by the pages taken since last
         time.  Entries of pages that a window released are left as they were: nothing reads them."""
-        import numpy as np
         cache = self.cache
         table = cache.block_table(rid, gi)
         epoch = cache.epoch_of(rid)
@@ -404,14 +458,19 @@ class ModelRunner:
 
     # ------------------------------------------------------------------ metadata
     def _build_context(self, entries, temperatures=None, uniforms=None, pad_to=0, seq_bucket=0) -> StepContext:
+        return self._context(self._stage_step(entries, temperatures, uniforms, pad_to, seq_bucket))
+
+    def _stage_step(self, entries, temperatures=None, uniforms=None, pad_to=0, seq_bucket=0) -> _Staged:
+        """Write what the kernels see of a step into a staging set and start its copy to the device.  A replayed step needs no more
+        than this: the views that a StepContext is made of cost a third of a small model's step."""
         cache = self.cache
         n_max, r_max = self._n_cap, self.max_requests
         turn = self.steps_run % 2
         if self._stage_events[turn] is not None:
             self._stage_events[turn].synchronize()
-        host_small, host_tables = self._stage[turn]
-        np_small, np_tables = self._stage_np[turn]
-        import numpy as np
+        host_all, host_small, host_tables = self._stage[turn]
+        h, np_tables = self._stage_np[turn]
+        held_rows = self._stage_rows[turn]
         n_groups = len(cache.kv_groups)
         o_ids, o_pos, o_req, o_rows = 0, n_max, 2 * n_max, 3 * n_max
         o_cu = 4 * n_max
@@ -419,26 +478,49 @@ class ModelRunner:
         o_slot = o_seq + r_max
         o_first = o_slot + r_max
         o_g = o_first + r_max
-        h = np_small
-        total = sum(len(e.tokens) for e in entries) + max(0, pad_to - len(entries))
-        wanted = sum(len(e.want) for e in entries) + max(0, pad_to - len(entries))
+        pad = max(0, pad_to - len(entries))
+        total = sum(len(e.tokens) for e in entries) + pad
+        wanted = sum(len(e.want) for e in entries) + pad
         if total > n_max or max(len(entries), pad_to) > r_max or wanted > n_max:
             raise BatchError(f"a step of {total} rows, {max(len(entries), pad_to)} requests and {wanted} wanted rows does not "
                              f"fit the staging regions ({n_max} rows, {r_max} requests)")
         cu, seq, slots, first = [0], [], [], []
         max_q, min_q = 0, 1 << 30
         base = n_rows = 0
-        for r, e in enumerate(entries):            # whole spans at a time: a prompt portion costs no Python loop over its tokens
-            start = cache.num_computed(e.request_id)
+        # runs of decoded tokens are gathered in lists and written at once; a portion is written as a span (no Python loop over its tokens)
+        ids, positions, owners, rows, places, run_at, rows_at = [], [], [], [], [[] for _ in range(n_groups)], 0, 0
+
+        def flush():
+            n = len(ids)
+            if n:
+                h[o_ids + run_at:o_ids + run_at + n] = ids
+                h[o_pos + run_at:o_pos + run_at + n] = positions
+                h[o_req + run_at:o_req + run_at + n] = owners
+                for gi in range(n_groups):
+                    at = o_g + gi * n_max + run_at
+                    h[at:at + n] = places[gi]
+                    places[gi].clear()
+            if rows:
+                h[o_rows + rows_at:o_rows + rows_at + len(rows)] = rows
+            ids.clear(), positions.clear(), owners.clear(), rows.clear()
+
+        for r, e in enumerate(entries):
+            rid = e.request_id
+            start = cache.num_computed(rid)
             n = len(e.tokens)
-            if n == 1:                              # a decoded token: plain scalar writes beat array calls
-                h[o_ids + base] = max(0, int(e.tokens[0]))
-                h[o_pos + base] = start
-                h[o_req + base] = r
+            if n == 1:
+                if not ids:
+                    run_at, rows_at = base, n_rows
+                ids.append(max(0, int(e.tokens[0])))
+                positions.append(start)
+                owners.append(r)
+                for gi in range(n_groups):
+                    places[gi].append(cache.slots_for(rid, gi, 1)[0])
                 for w in e.want:
-                    h[o_rows + n_rows] = base + int(w)
+                    rows.append(base + int(w))
                     n_rows += 1
             else:
+                flush()
                 h[o_ids + base:o_ids + base + n] = np.maximum(np.asarray(e.tokens, dtype=np.int64), 0)
                 h[o_pos + base:o_pos + base + n] = np.arange(start, start + n, dtype=np.int32)
                 h[o_req + base:o_req + base + n] = r
@@ -446,33 +528,40 @@ class ModelRunner:
                 if k:
                     h[o_rows + n_rows:o_rows + n_rows + k] = np.asarray(e.want, dtype=np.int64) + base
                     n_rows += k
+                for gi in range(n_groups):
+                    at = o_g + gi * n_max + base
+                    h[at:at + n] = cache.slots_array(rid, gi, n)
             cu.append(base + n)
             seq.append(start + n)
-            slots.append(cache.slot_of(e.request_id))
+            slots.append(cache.slot_of(rid))
             first.append(1 if start == 0 else 0)
             max_q, min_q = max(max_q, n), min(min_q, n)
+            epoch = cache.epoch_of(rid)
             for gi in range(n_groups):
-                if n == 1:
-                    h[o_g + gi * n_max + base] = cache.slots_for(e.request_id, gi, 1)[0]
-                else:
-                    h[o_g + gi * n_max + base:o_g + gi * n_max + base + n] = cache.slots_array(e.request_id, gi, n)
-                row = self._table_row(e.request_id, gi)
-                np_tables[gi, r, : len(row)] = row
+                row = self._table_row(rid, gi)
+                held = held_rows.get((gi, r))
+                done = held[2] if held is not None and held[0] == rid and held[1] == epoch and held[2] <= len(row) else 0
+                if len(row) > done:
+                    np_tables[gi, r, done:len(row)] = row[done:]
+                if held is None or done == 0 or len(row) > done:
+                    held_rows[(gi, r)] = (rid, epoch, len(row))
             base += n
         real_rows = n_rows
         for j in range(len(entries), pad_to):      # padding of a graph bucket: tokens that store and see nothing
-            h[o_ids + base] = 0; h[o_pos + base] = 0; h[o_req + base] = j; h[o_rows + n_rows] = 0
+            if not ids:
+                run_at, rows_at = base, n_rows
+            ids.append(0), positions.append(0), owners.append(j), rows.append(0)
             for gi in range(n_groups):
-                h[o_g + gi * n_max + base] = -1
+                places[gi].append(-1)
             cu.append(cu[-1] + 1); seq.append(0); slots.append(0); first.append(0)
             base += 1; n_rows += 1
+        flush()
         N, R, M = base, len(cu) - 1, n_rows
         h[o_cu:o_cu + R + 1] = cu
         h[o_seq:o_seq + R] = seq
         h[o_slot:o_slot + R] = slots
         h[o_first:o_first + R] = first
-        group_slots = cache.kv_groups
-        o_f = o_g + len(group_slots) * n_max
+        o_f = o_g + n_groups * n_max
         if temperatures is not None:
             hf = h.view("float32")
             k = len(temperatures)
@@ -480,28 +569,42 @@ class ModelRunner:
             if k:
                 hf[o_f:o_f + k] = temperatures
                 hf[o_f + r_max:o_f + r_max + k] = uniforms
-        h = host_small
-        d = self._dev_small
-        d.copy_(h, non_blocking=True)
-        if cache.kv_groups:
-            self._dev_tables[:, :R].copy_(host_tables[:, :R], non_blocking=True)
+        if n_groups == 1:
+            end = self._tables_at + R * self.max_pages
+            to, source = self._part(("staged", turn), end, self._dev_all, host_all)
+            to.copy_(source, non_blocking=True)
+        else:
+            self._dev_small.copy_(host_small, non_blocking=True)
+            if n_groups:
+                self._dev_tables[:, :R].copy_(host_tables[:, :R], non_blocking=True)
         if self._pin:
-            ev = torch.cuda.Event()
-            ev.record()
-            self._stage_events[turn] = ev
+            self._stage_events[turn] = self._record(("staged", turn))
+        return _Staged(N, R, M, real_rows, max_q, 1 if pad_to > len(entries) else max(1, min(min_q, max_q)),
+                       max(max(seq), seq_bucket), cu, seq, slots, first)
+
+    def _context(self, staged: _Staged) -> StepContext:
+        """The step as the parts see it: views of the device's copy."""
+        cache, d = self.cache, self._dev_small
+        n_max, r_max = self._n_cap, self.max_requests
+        N, R, M = staged.num_tokens, staged.num_requests, staged.num_logit_rows
+        o_pos, o_req, o_rows, o_cu = n_max, 2 * n_max, 3 * n_max, 4 * n_max
+        o_seq = o_cu + r_max + 1
+        o_slot = o_seq + r_max
+        o_first = o_slot + r_max
+        o_g = o_first + r_max
+        o_f = o_g + len(cache.kv_groups) * n_max
         ctx = StepContext(self)
         ctx.num_tokens, ctx.num_requests, ctx.num_logit_rows = N, R, M
-        ctx.max_q_len, ctx.max_seq_len = max_q, max(max(seq), seq_bucket)
-        ctx.min_q_len = 1 if pad_to > len(entries) else max(1, min(min_q, max_q))
+        ctx.max_q_len, ctx.min_q_len, ctx.max_seq_len = staged.max_q_len, staged.min_q_len, staged.max_seq_len
         df = d.view(torch.float32)
         ctx.temperatures, ctx.uniforms = df[o_f:o_f + r_max], df[o_f + r_max:o_f + 2 * r_max]
-        ctx.num_real_logit_rows = real_rows
-        ctx.token_ids, ctx.positions = d[o_ids:o_ids + N], d[o_pos:o_pos + N]
+        ctx.num_real_logit_rows = staged.num_real_logit_rows
+        ctx.token_ids, ctx.positions = d[:N], d[o_pos:o_pos + N]
         ctx.req_index, ctx.logit_rows = d[o_req:o_req + N], d[o_rows:o_rows + M]
         ctx.cu_q, ctx.seq_lens = d[o_cu:o_cu + R + 1], d[o_seq:o_seq + R]
         ctx.state_slots, ctx.first_portion = d[o_slot:o_slot + R], d[o_first:o_first + R]
         ctx.group_slot_mapping = [d[o_g + gi * n_max: o_g + gi * n_max + N] for gi in range(len(cache.kv_groups))]
         ctx.group_block_tables = [self._dev_tables[gi, :R] for gi in range(len(cache.kv_groups))]
-        ctx.host_cu_q, ctx.host_seq_lens = cu, seq
-        ctx.host_state_slots, ctx.host_first_portion = slots, [bool(f) for f in first]
+        ctx.host_cu_q, ctx.host_seq_lens = staged.cu_q, staged.seq_lens
+        ctx.host_state_slots, ctx.host_first_portion = staged.state_slots, [bool(f) for f in staged.first_portion]
         return ctx

@@ -12,6 +12,7 @@ import plain_qwen3 as P
 import tiny
 from kernel_refs import ReferenceKernels
 from infurnace_b200.engine import Engine, EngineOptions, Request, RequestState, SamplingParams, StepEntry, generate
+from infurnace_b200.cache import RELEASED
 from infurnace_b200.errors import BatchError, KernelError, OutOfPages
 
 
@@ -331,3 +332,50 @@ def test_a_fault_recorded_on_the_device_fails_the_requests_that_ran(models):
     assert eng.is_done() and eng.runner.cache.free_pages() == [40]
     eng.runner.cache.check()
     assert len(eng.generate([[7, 8, 9]], SamplingParams(max_tokens=4))[0]) == 4
+
+
+def test_staged_tables_follow_their_requests(models):
+    """A staging set keeps the block tables that its rows held two steps ago and writes only what is new: requests that change rows,
+    end, start again under an old id, or lose the pages of a step that failed and get others must all be seen as they are."""
+    import random
+    eng = engine(models["B"], "B", max_num_batched_tokens=64, max_num_seqs=4)
+    run, cache, rng = eng.runner, eng.runner.cache, random.Random(3)
+    real = run.model.forward
+
+    def fails(ctx):
+        raise RuntimeError("planted")
+    for step in range(120):
+        live = [rid for rid in "abcde" if cache.has_request(rid)]
+        if live and rng.random() < 0.2:
+            cache.free_request(live.pop(rng.randrange(len(live))))
+        if len(live) < 4 and rng.random() < 0.5:
+            rid = rng.choice([r for r in "abcde" if not cache.has_request(r)])
+            cache.add_request(rid)
+            live.append(rid)
+        rng.shuffle(live)
+        entries = [StepEntry(rid, [1] * rng.choice([1, 1, 1, 2, 5]), [0]) for rid in live if cache.num_computed(rid) < 80]
+        if not entries:
+            continue
+        bad = rng.random() < 0.25
+        run.model.forward = fails if bad else real
+        held = {}
+
+        def look(ctx, forward=run.model.forward):
+            for gi in range(len(cache.kv_groups)):
+                for r, e in enumerate(entries):
+                    want = cache.block_table(e.request_id, gi)
+                    got = ctx.group_block_tables[gi][r, :len(want)].tolist()
+                    held[gi, r] = all(w == RELEASED or w == g for w, g in zip(want, got))
+            return forward(ctx)
+        run.model.forward = look
+        try:
+            run.step(entries)
+            assert not bad
+        except RuntimeError as e:
+            assert bad and "planted" in str(e)
+        except OutOfPages:
+            for rid in live:
+                cache.free_request(rid)
+        assert all(held.values()), (step, held)
+        cache.check()
+    run.model.forward = real
