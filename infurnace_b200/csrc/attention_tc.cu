@@ -315,6 +315,25 @@ __device__ __forceinline__ bool tc_item(int k, int cta, int ctas, int nt, int nk
   return true;
 }
 
+// The request of a row of the grid, where the grid has a row for each of the step's long requests (those with more than 16 rows) only:
+// the `place`-th of them, or -1.  In a step that mixes a prompt with decoding requests a row for every request means that nearly all
+// CTAs have nothing to do, and each waits for 160 KB of an SM's shared memory to say so (15 requests beside a portion of 446
+// tokens, 0.6B sizes: 784 of 840; the kernel takes 17.6 us a layer with them and @US without).  Whole warps, 32 requests a look, which costs a round trip: a step without
+// short requests has its rows numbered as the requests are.
+__device__ __forceinline__ int tc_long_request(int place, int n_req, int G, const int* __restrict__ cu_q) {
+  const int lane = threadIdx.x & 31;
+  for (int base = 0; base < n_req; base += 32) {
+    const int r = base + lane;
+    const bool is_long = r < n_req && (cu_q[r + 1] - cu_q[r]) * G > 16;
+    const uint32_t longs = __ballot_sync(0xffffffffu, is_long);
+    const int count = __popc(longs);
+    if (place < count)
+      return base + __ffs(__ballot_sync(0xffffffffu, is_long && __popc(longs & ((1u << lane) - 1)) == place)) - 1;
+    place -= count;
+  }
+  return -1;
+}
+
 // The two streams as matrices of rows: how many rows a page spans and how many rows there are.
 struct TcRows { int k_page, v_page, k_total, v_total; };
 
@@ -322,7 +341,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                     const __grid_constant__ CUtensorMap v_map, TcRows mrows, int* __restrict__ err,
                     const int* __restrict__ block_tables, int bt_stride, const int* __restrict__ cu_q,
-                    const int* __restrict__ seq_lens, bf16* __restrict__ out, int nq, int nkv, int share, int page_size,
+                    const int* __restrict__ seq_lens, bf16* __restrict__ out, int n_req, int nq, int nkv, int share, int page_size,
                     TcScore score, float sink, int window) {
   extern __shared__ unsigned char tc_smem_raw[];
   __shared__ TcBars bars;
@@ -336,8 +355,10 @@ attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
   unsigned char* Ks = smem + K_BYTES;                        // two stages of K tiles, same layout
   unsigned char* Vs = smem + 3 * K_BYTES;                    // two stages of V tiles, [VH][128 rows][128 bytes]
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform
-  const int r = blockIdx.z, cta = blockIdx.x, ctas = gridDim.x;
+  const int cta = blockIdx.x, ctas = gridDim.x;
   const int G = nq / nkv;
+  const int r = (int)gridDim.z < n_req ? tc_long_request(blockIdx.z, n_req, G, cu_q) : (int)blockIdx.z;
+  if (r < 0) { ifb_pdl_wait(); return; }                     // fewer long requests than the launch allowed for
   const int q0 = cu_q[r], q_len = cu_q[r + 1] - q0, L = seq_lens[r];
   // every exit path waits for the predecessor: a grid none of whose threads waited could end before the kernel that
   // stores this step's keys, and its own successor, which waits for this grid alone, would then start too early
@@ -770,12 +791,12 @@ attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
 // nkv: groups of query heads (at most 128 each), `share` of which read one key/value head.  Takes the requests with
 // q_len * (nq / nkv) > 16.  page_size must be 16, 32 or 64.  softcap: 0 none (a library compiled with SOFTCAP takes a positive
 // one, or with SOFTCAP=2 the scores' bound, of at most 60 and no other takes one).  has_sink: exp(sink) joins the denominators (with SOFTCAP, sink at most 60).
-// err: a device int that stays 0 unless a bounded wait gave up.
+// err: a device int that stays 0 unless a bounded wait gave up.  max_long: at most so many requests are the kernel's (0: any may be).
 IFB_EXPORT int ifb_attention_tc(const void* qkv, int row_stride, const void* k_pages, long long k_page_stride, const void* v_pages,
                                 long long v_page_stride, long long num_pages, const int* block_tables, int bt_stride, const int* cu_q,
                                 const int* seq_lens, void* out, int* err, int n_tokens, int n_req, int nq, int nkv, int share, int d,
                                 int dv, int page_size, float scale, int window, float softcap, int has_sink, float sink, int max_q_len,
-                                cudaStream_t stream) {
+                                int max_long, cudaStream_t stream) {
   if (n_tokens <= 0 || n_req <= 0) return IFB_OK;
   if (d != D || dv != VD) return IFB_ERR_SIZE;
   if (nkv < 1 || nq % nkv || share < 1 || nkv % share || window < 0 || !err || num_pages < 1) return IFB_ERR_ARG;
@@ -825,7 +846,8 @@ IFB_EXPORT int ifb_attention_tc(const void* qkv, int row_stride, const void* k_p
     score.limit = scale != 0.f ? TC_TANH_RANGE / fabsf(score.to_y) : INFINITY;
   }
   const TcRows rows = {(int)k_page, (int)v_page, (int)k_rows, (int)v_rows};
-  dim3 grid((unsigned)(items < sm_count ? items : sm_count), 1, n_req);       // a CTA per SM walks the request's items
+  // a CTA per SM walks the request's items
+  dim3 grid((unsigned)(items < sm_count ? items : sm_count), 1, max_long > 0 && max_long < n_req ? max_long : n_req);
   return ifb_launch(attn_tile_tc_kernel, grid, dim3(TC_THREADS), (size_t)SMEM_BYTES, stream, q_map, k_map, v_map, rows, err, block_tables,
-                    bt_stride, cu_q, seq_lens, (bf16*)out, nq, nkv, share, page_size, score, has_sink ? sink * LOG2E : -INFINITY, window);
+                    bt_stride, cu_q, seq_lens, (bf16*)out, n_req, nq, nkv, share, page_size, score, has_sink ? sink * LOG2E : -INFINITY, window);
 }

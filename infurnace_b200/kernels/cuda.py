@@ -63,6 +63,7 @@ def _dense(t, name, dtype=None):
 
 class CudaKernels:
     name = "cuda"
+    takes_exact_lens = True        # paged_attention's ``exact_lens``
 
     def __init__(self, progress=None):
         if not torch.cuda.is_available():
@@ -580,8 +581,9 @@ class CudaKernels:
 
     # ------------------------------------------------------------------ attention
     def paged_attention(self, qkv, num_heads, num_kv_heads, head_dim, kv_pages, block_tables, cu_q, seq_lens, out,
-                        scale, window, max_q_len, max_seq_len, min_q_len=1, weight_terms=1, score_bound=None):
-        """``weight_terms`` 2 (tensor-core route only): a softmax weight enters the weighted sum as two bfloat16 terms, its
+                        scale, window, max_q_len, max_seq_len, min_q_len=1, weight_terms=1, score_bound=None, exact_lens=False):
+        """``exact_lens``: some request brings ``max_q_len`` tokens, none fewer than ``min_q_len``, and qkv has a row for each token of
+        theirs and no other, which bounds how many are long.  ``weight_terms`` 2 (tensor-core route only): a softmax weight enters the weighted sum as two bfloat16 terms, its
         rounding and what the rounding left out, so that 16 bits of the float32 weight count; the tcgen05 prompt kernel for
         plain scores, which has one term, is then not taken.  ``score_bound``: what no scaled score exceeds in size, if the
         caller knows it; up to ``TC_CAP_LIMIT`` prompts then run on the tcgen05 kernel for bounded scores."""
@@ -601,7 +603,8 @@ class CudaKernels:
                 and num_heads % num_kv_heads == 0:
             return self._paged_attention_mma(qkv, num_heads, num_kv_heads, head_dim, kv_pages, block_tables, cu_q,
                                              seq_lens, out, scale, window, max_q_len, max_seq_len, n, r,
-                                             min_q_len=min_q_len, weight_terms=weight_terms, score_bound=score_bound)      # keys and values in one tensor
+                                             min_q_len=min_q_len, weight_terms=weight_terms, score_bound=score_bound,
+                                             exact_lens=exact_lens)      # keys and values in one tensor
         self.launches += 1
         _check(self.core.ifb_paged_attention_simt(
             qkv.data_ptr(), _code(qkv), qkv.stride(0), kv_pages.data_ptr(), block_tables.data_ptr(),
@@ -618,7 +621,8 @@ class CudaKernels:
             lib = self._attn_tc[key] = load_library("attention_tc", defines or None, progress=self._progress)
             lib.ifb_attention_tc.argtypes = [
                 c_void_p, c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-                c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_float, c_int, c_float, c_int, c_void_p]
+                c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_float, c_int, c_float, c_int, c_int,
+                c_void_p]
         return lib
 
     TC_CAP_LIMIT = 60.0       # soft caps (and sinks beside them) up to here: 2^(cap log2 e) summed over any context is a float32 number
@@ -635,8 +639,9 @@ class CudaKernels:
                 and one_tensor.data_ptr() % 128 == 0)
 
     def _attention_tc_streams(self, qkv, num_heads, num_kv_heads, share, head_dim, value_head_dim, k, v, num_pages, block_tables, cu_q,
-                              seq_lens, out, scale, window, max_q_len, n, r, weight_terms, softcap, sink, kind):
-        """``kind``: 0 plain scores, 1 capped at ``softcap``, 2 no larger than ``softcap`` as they are."""
+                              seq_lens, out, scale, window, max_q_len, n, r, weight_terms, softcap, sink, kind, max_long=0):
+        """``kind``: 0 plain scores, 1 capped at ``softcap``, 2 no larger than ``softcap`` as they are.  ``max_long``: at most so many
+        requests have more than 16 rows of a key/value head (0: any may)."""
         self._err_armed = True
         self.launches += 1
         self.tc_attention_calls += 1
@@ -645,7 +650,7 @@ class CudaKernels:
             qkv.data_ptr(), qkv.stride(0), k[0], k[1], v[0], v[1], num_pages, block_tables.data_ptr(), block_tables.stride(0),
             cu_q.data_ptr(), seq_lens.data_ptr(), out.data_ptr(), self._dev_err.data_ptr(), n, r, num_heads, num_kv_heads, share,
             head_dim, value_head_dim, k[2], float(scale), int(window), float(softcap or 0.0), 0 if sink is None else 1,
-            float(sink or 0.0), int(max_q_len), self._stream()), "paged_attention")
+            float(sink or 0.0), int(max_q_len), int(max_long), self._stream()), "paged_attention")
 
     @staticmethod
     def attention_defines(head_dim, weight_terms=1, value_head_dim=None, softcap=False):
@@ -693,14 +698,26 @@ class CudaKernels:
 
     def _paged_attention_mma(self, qkv, num_heads, num_kv_heads, head_dim, kv_pages, block_tables, cu_q, seq_lens, out,
                              scale, window, max_q_len, max_seq_len, n, r, num_splits=None, min_q_len=1, weight_terms=1,
-                             score_bound=None):
+                             score_bound=None, exact_lens=False):
         """Keys and values of one width in one tensor [pages, 2, kv_heads, page_size, head_dim]: two streams of a common stride."""
         esize, ps = kv_pages.element_size(), kv_pages.shape[3]
         k = (kv_pages.data_ptr(), kv_pages.stride(0), ps)
         v = (kv_pages.data_ptr() + esize * num_kv_heads * ps * head_dim, kv_pages.stride(0), ps)
         self._attention_mma_streams(qkv, num_heads, num_kv_heads, head_dim, head_dim, k, v, kv_pages.shape[0], block_tables, cu_q, seq_lens,
                                     out, scale, window, max_q_len, max_seq_len, n, r, num_splits, min_q_len, weight_terms,
-                                    one_tensor=kv_pages, score_bound=score_bound)
+                                    one_tensor=kv_pages, score_bound=score_bound, exact_lens=exact_lens)
+
+    @staticmethod
+    def long_requests(tokens, requests, group, max_q_len, min_q_len):
+        """How many requests at most have more than 16 rows of a key/value head with ``group`` query heads, where one brings
+        ``max_q_len`` tokens, none fewer than ``min_q_len``, and all together ``tokens``."""
+        least = 16 // group + 1                                  # tokens of a long request
+        if max_q_len < least:
+            return 0
+        if min_q_len >= least:
+            return requests
+        spare = tokens - max_q_len - (requests - 1) * min_q_len  # beside the longest, above the fewest that each brings
+        return min(requests, 1 + max(0, spare) // (least - min_q_len))
 
     ATTENTION_GROUP = 16      # query heads that share a key/value head's rows in one CTA of the small-q kernel
 
@@ -711,7 +728,7 @@ class CudaKernels:
 
     def _attention_mma_streams(self, qkv, num_heads, num_kv_heads, head_dim, value_head_dim, k, v, num_pages, block_tables, cu_q,
                                seq_lens, out, scale, window, max_q_len, max_seq_len, n, r, num_splits=None, min_q_len=1,
-                               weight_terms=1, softcap=None, sink=None, one_tensor=None, score_bound=None):
+                               weight_terms=1, softcap=None, sink=None, one_tensor=None, score_bound=None, exact_lens=False):
         """The tensor-core attention kernels over key and value streams ``k`` and ``v`` = (address, elements between pages, page
         size).  ``one_tensor``: the tensor that holds both, where there is one (what the tcgen05 kernel for plain attention takes)."""
         share = self.attention_share(num_heads // num_kv_heads)
@@ -738,7 +755,8 @@ class CudaKernels:
                                                       one_tensor):
             self._attention_tc_streams(qkv, num_heads, num_kv_heads, share, head_dim, value_head_dim, k, v, num_pages, block_tables, cu_q,
                                        seq_lens, out, scale, window, max_q_len, n, r, weight_terms, softcap or score_bound, sink,
-                                       kind=2 if score_bound else 1 if softcap else 0)
+                                       kind=2 if score_bound else 1 if softcap else 0,
+                                       max_long=self.long_requests(n, r, group, max_q_len, min_q_len) if exact_lens else 0)
             if min_q_len * group > 16:
                 return                 # no request of this step is left for the small-q kernel
             only_small = behind_tiles = True       # the tile kernel has its requests; the small-q kernel takes the rest beside it

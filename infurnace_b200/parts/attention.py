@@ -69,7 +69,7 @@ class PagedAttention:
         attn = ctx.buffer("attn", (n, s.num_heads * s.head_dim), self.rt.act_dtype)
         k.paged_attention(qkv, s.num_heads, s.num_kv_heads, s.head_dim, kv.pages, kv.block_tables,
                           ctx.cu_q, ctx.seq_lens, attn, s.scale, s.window or 0, ctx.max_q_len, ctx.max_seq_len,
-                          min_q_len=ctx.min_q_len)
+                          min_q_len=ctx.min_q_len, **({"exact_lens": True} if getattr(k, "takes_exact_lens", False) else {}))
         folded = fold_residual_norm(k, ctx, "mixer", attn, self.w_o, fold, self.rt.act_dtype)
         if folded is not None:
             return folded

@@ -158,6 +158,7 @@ class RotaryValueAttention:
             # the framework's tensor-core attention over the entry's one tensor of keys and values, then the turn back
             k.paged_attention(q, s.num_heads, s.num_kv_heads, s.head_dim, kv.pages, kv.block_tables, ctx.cu_q, ctx.seq_lens, attn,
                               s.scale, s.window or 0, ctx.max_q_len, ctx.max_seq_len, min_q_len=ctx.min_q_len,
+                              **({"exact_lens": True} if getattr(k, "takes_exact_lens", False) else {}),
                               **{key: self.extra[key] for key in ("weight_terms", "score_bound") if key in self.extra})
             if v_table is not None:
                 k.rotate_rows(attn, v_table, s.num_heads, s.value_head_dim, s.value_head_dim, bool(s.value_position.interleaved),
