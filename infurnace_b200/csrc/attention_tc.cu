@@ -318,7 +318,7 @@ __device__ __forceinline__ bool tc_item(int k, int cta, int ctas, int nt, int nk
 // The request of a row of the grid, where the grid has a row for each of the step's long requests (those with more than 16 rows) only:
 // the `place`-th of them, or -1.  In a step that mixes a prompt with decoding requests a row for every request means that nearly all
 // CTAs have nothing to do, and each waits for 160 KB of an SM's shared memory to say so (15 requests beside a portion of 446
-// tokens, 0.6B sizes: 784 of 840; the kernel takes 17.6 us a layer with them and @US without).  Whole warps, 32 requests a look, which costs a round trip: a step without
+// tokens, 0.6B sizes: 784 of 840; the kernel takes 17.6 us a layer with them and 13.5 without).  Whole warps, 32 requests a look, which costs a round trip: a step without
 // short requests has its rows numbered as the requests are.
 __device__ __forceinline__ int tc_long_request(int place, int n_req, int G, const int* __restrict__ cu_q) {
   const int lane = threadIdx.x & 31;

@@ -580,6 +580,34 @@ def test_attention_on_tcgen05_with_more_items_than_sms(K, q_lens, seq_lens, wind
         torch.testing.assert_close(out.cpu().float(), ref.float(), rtol=1.6e-2, atol=1.6e-2)
 
 
+@pytest.mark.parametrize("nq,nkv", [(16, 8), (16, 2)])
+@pytest.mark.parametrize("longs,shorts", [([70], 15), ([9, 500, 17], 40), ([64], 1), ([100, 30], 32), ([200], 63), ([65, 65], 70)])
+def test_attention_of_mixed_steps(K, nq, nkv, longs, shorts):
+    """Prompts beside decoding requests, with lengths that bound how many requests are long: the prompts' grid has a row for each of
+    these (more, where the bound allows more) and finds it among the others, and the decoding requests run in the order of their
+    keys (up to 64 requests), ties, a request of one key and the edges of 32 and 64 requests included."""
+    d, ps = 128, 16
+    g = torch.Generator().manual_seed(shorts)
+    q_lens, seq_lens = [1] * shorts, torch.randint(1, 400, (shorts,), generator=g).tolist()
+    seq_lens[0] = 1
+    seq_lens[shorts // 2] = seq_lens[-1]
+    for i, q in enumerate(longs):
+        at = (shorts * (i + 1)) // (len(longs) + 1)
+        q_lens.insert(at, q), seq_lens.insert(at, q + 37 * i)
+    qkv, kv, bt, cu, sl = _attention_case(torch.bfloat16, nq, nkv, d, ps, 0, q_lens, seq_lens, 5)
+    n = qkv.shape[0]
+    ref = torch.empty((n, nq * d), dtype=torch.bfloat16)
+    REF.paged_attention(qkv, nq, nkv, d, kv, bt, cu, sl, ref, d ** -0.5, 0, max(q_lens), max(seq_lens))
+    least = 16 // (nq // nkv) + 1
+    assert sum(q >= least for q in q_lens) <= K.long_requests(n, len(q_lens), nq // nkv, max(q_lens), 1) <= len(q_lens)
+    for exact in (True, False):
+        out = torch.full((n, nq * d), float("nan"), dtype=torch.bfloat16, device="cuda")
+        K.paged_attention(qkv.cuda(), nq, nkv, d, kv.cuda(), bt.cuda(), cu.cuda(), sl.cuda(), out, d ** -0.5, 0, max(q_lens),
+                          max(seq_lens), exact_lens=exact)
+        K.check_device_errors()
+        torch.testing.assert_close(out.cpu().float(), ref.float(), rtol=1.6e-2, atol=1.6e-2)
+
+
 @pytest.mark.parametrize("q_len", [65, 100, 105, 127, 128, 200])
 def test_attention_on_tcgen05_waits_for_its_products(K, q_len):
     """A stream that works through exactly two halves of keys reads its accumulator after a wait by parity on the

@@ -101,3 +101,16 @@ def test_the_buffer_of_partial_sums_never_grows(o):
         if n == 1:
             first = ctx.arena.generation
     assert ctx.arena.generation == first
+
+
+def test_the_bound_of_long_requests_holds():
+    """Rows of the prompts' attention grid: never fewer than the requests with more than 16 rows, never more than the requests."""
+    import itertools
+    from infurnace_b200.kernels.cuda import CudaKernels
+    for group in (1, 2, 4, 8, 16):
+        least = 16 // group + 1
+        for count in (1, 2, 3, 4):
+            for lens in itertools.product((1, 2, 3, 5, 8, 9, 10, 17, 18, 30), repeat=count):
+                bound = CudaKernels.long_requests(sum(lens), count, group, max(lens), min(lens))
+                assert sum(q >= least for q in lens) <= bound <= count, (group, lens)
+                assert CudaKernels.long_requests(sum(lens), count, group, max(lens), 1) >= bound
