@@ -15,6 +15,7 @@
 
 typedef __nv_bfloat16 bf16;
 constexpr int GV_ROWS = 16;
+constexpr int GV_SMS = 148;
 // CTAs per SM asked of the compiler for the plain one-stage kernel of 8 warps and one block of tokens (the LM head of a
 // small model, 9,496 CTAs): with 80 registers three fit and the 311 MB stream at 5.8 to 6.3 TB/s; with the 103 the
 // compiler took unasked two fit (4.8 to 5.0 TB/s), with four (64 registers, spills) it is slower again.
@@ -87,29 +88,32 @@ __device__ __forceinline__ void gv_cluster_barrier() {
 // out = act(gate) * up, act = silu or rs.unary.  EPI 2: v = x + y is written back to x, out = v * g.  EPI 4: as EPI 1 with 8 features per
 // CTA, whose 8 gate rows and 8 up rows are the two halves of one 16-row tile (half the registers of EPI 1, so two CTAs
 // per SM where EPI 1 with two stages has one).  WARPS: warps of a CTA (they split k).
+// EPI 5: as EPI 3 with 8 feature pairs per CTA, likewise the two halves of one tile.
 // STAGES: steps of 128 of k whose weights (and, for one block of tokens, activations) a warp has requested at any
 // time.  1: every warp's k range is one step (the sizes of small models, where the chain of round trips counts);
 // 2: a warp walks a long k range and keeps the memory pipe full while it multiplies (large models, where the
 // bytes count).
 template <int NB, int EPI, int WARPS, typename TO, int STAGES>
-__global__ void __launch_bounds__(WARPS * 32, (EPI == 4 && WARPS == 8) ? (STAGES == 1 ? 3 : 2) : (EPI == 0 && WARPS == 8 && STAGES == 1 && NB == 1) ? IFB_GV_LM_BLOCKS
+__global__ void __launch_bounds__(WARPS * 32, ((EPI == 4 || EPI == 5) && WARPS == 8) ? (STAGES == 1 ? 3 : 2) : (EPI == 0 && WARPS == 8 && STAGES == 1 && NB == 1) ? IFB_GV_LM_BLOCKS
                                   : (EPI == 2 && NB == 1 && WARPS <= 16 && (WARPS == 16 || STAGES == 2)) ? 2 : 0)
 linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* __restrict__ out, int n_rows, int o_out,
                    int k_dim, GvRowScale rs, GvResidual res, GvQkv qk) {
   extern __shared__ float gv_red[];                 // [WARPS][NE][NB*8][GV_ROWS], then [NB*8] row factors
   constexpr int NE = (EPI == 1 || EPI == 3) ? 2 : 1;
-  static_assert(EPI != 3 || (NB <= 2 && WARPS * 32 >= NB * 8 * GV_ROWS), "the fused qkv epilogue keeps one (token, feature pair) per thread");
+  constexpr bool QK = EPI == 3 || EPI == 5;
+  constexpr int PAIRS = EPI == 5 ? 8 : GV_ROWS;      // feature pairs of a CTA
+  static_assert(!QK || (NB <= 2 && WARPS * 32 >= NB * 8 * PAIRS), "the fused qkv epilogue keeps one (token, feature pair) per thread");
   constexpr bool STAGE_X = STAGES > 1 && NB == 1;    // activations requested ahead with the weights
   float* row_factor = gv_red + (size_t)WARPS * NE * NB * 8 * GV_ROWS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane & 3, rr = lane >> 2;
-  // EPI 3: blockIdx.x = head * (head_dim / 32) + c; the first 16 features are the head's [c*16, c*16+16), the second 16
+  // QK: blockIdx.x = head * (head_dim / (2 PAIRS)) + c; the first features are the head's [c*PAIRS, c*PAIRS+PAIRS), the others
   // their rotation partners head_dim/2 further on
-  const int qk_per_head = EPI == 3 ? qk.head_dim / 32 : 1;
-  const int qk_head = EPI == 3 ? blockIdx.x / qk_per_head : 0, qk_c = EPI == 3 ? blockIdx.x % qk_per_head : 0;
+  const int qk_per_head = QK ? qk.head_dim / (2 * PAIRS) : 1;
+  const int qk_head = QK ? blockIdx.x / qk_per_head : 0, qk_c = QK ? blockIdx.x % qk_per_head : 0;
   const bool half_tile = (EPI == 0 || EPI == 2) && res.feat == 8;     // 8 features per CTA: no weight rows for the tile's second half
   const int feat = (EPI == 4 || half_tile) ? 8 : GV_ROWS;
-  const int o0 = EPI == 3 ? qk_head * qk.head_dim + qk_c * GV_ROWS : blockIdx.x * feat, n0 = blockIdx.y * (NB * 8);
-  const int second = EPI == 3 ? qk.head_dim / 2 : o_out;      // distance of the second set of 16 weight rows from the first
+  const int o0 = QK ? qk_head * qk.head_dim + qk_c * PAIRS : blockIdx.x * feat, n0 = blockIdx.y * (NB * 8);
+  const int second = QK ? qk.head_dim / 2 : o_out;            // distance of the second set of weight rows from the first
   const int kw = ((k_dim + WARPS - 1) / WARPS + 127) / 128 * 128;      // k per warp, whole 128-wide steps
   const int kbeg = warp * kw, kend = min(k_dim, kbeg + kw);
   const int w_rows = (EPI == 1 || EPI == 4) ? 2 * o_out : o_out;
@@ -123,6 +127,7 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
     wrow[0][0] = w + (size_t)min(o0 + rr, o_out - 1) * k_dim;
     wrow[0][1] = w + (size_t)min(o_out + o0 + rr, w_rows - 1) * k_dim;
   }
+  if (EPI == 5) wrow[0][1] = w + (size_t)(second + o0 + rr) * k_dim;      // rows 0-7: features; rows 8-15: their partners
   const bf16* xrow[NB];
   bool xok[NB];
 #pragma unroll
@@ -140,24 +145,24 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
   // What the epilogue reads for this thread's (first) item is requested with the operands, not after the products: norm
   // weights (constants, which come from memory behind the weights of this and the next kernel) before the wait, the
   // stream's element, the angles and the place in the pages after it.
-  const int item_n = tid / GV_ROWS, item_m = tid % GV_ROWS, item_tok = n0 + item_n, item_o = o0 + item_m;
-  const bool item = tid < NB * 8 * GV_ROWS && item_tok < n_rows;
+  const int item_n = tid / PAIRS, item_m = tid % PAIRS, item_tok = n0 + item_n, item_o = o0 + item_m;
+  const bool item = tid < NB * 8 * PAIRS && item_tok < n_rows;
   float pre_a = 1.f, pre_b = 1.f, pre_x = 0.f;
   float2 pre_cs = make_float2(1.f, 0.f);
   int pre_slot = -1;
-  const bool qk_is_v = EPI == 3 && qk_head >= qk.nq + qk.nkv, qk_is_k = EPI == 3 && qk_head >= qk.nq && !qk_is_v;
-  const void* qk_nw = EPI != 3 || qk_is_v ? nullptr : qk_is_k ? qk.kw : qk.qw;
+  const bool qk_is_v = QK && qk_head >= qk.nq + qk.nkv, qk_is_k = QK && qk_head >= qk.nq && !qk_is_v;
+  const void* qk_nw = !QK || qk_is_v ? nullptr : qk_is_k ? qk.kw : qk.qw;
   auto request_constants = [&]() {
     if (EPI == 2 && item && item_o < o_out && (!half_tile || item_m < 8)) pre_a = load_as_f32(res.g, res.g_dtype, item_o);
-    if (EPI == 3 && item && qk_nw) {
-      pre_a = load_as_f32(qk_nw, qk.w_dtype, qk_c * GV_ROWS + item_m);
-      pre_b = load_as_f32(qk_nw, qk.w_dtype, qk_c * GV_ROWS + item_m + qk.head_dim / 2);
+    if (QK && item && qk_nw) {
+      pre_a = load_as_f32(qk_nw, qk.w_dtype, qk_c * PAIRS + item_m);
+      pre_b = load_as_f32(qk_nw, qk.w_dtype, qk_c * PAIRS + item_m + qk.head_dim / 2);
     }
   };
   auto request_item = [&]() {
     if (EPI == 2 && item && item_o < o_out && (!half_tile || item_m < 8)) pre_x = res.x[(size_t)item_tok * o_out + item_o];
-    if (EPI == 3 && item) {
-      if (!qk_is_v && qk.rope) pre_cs = qk.rope[(size_t)item_tok * (qk.head_dim / 2) + qk_c * GV_ROWS + item_m];
+    if (QK && item) {
+      if (!qk_is_v && qk.rope) pre_cs = qk.rope[(size_t)item_tok * (qk.head_dim / 2) + qk_c * PAIRS + item_m];
       if ((qk_is_v || qk_is_k) && qk.slots) pre_slot = qk.slots[item_tok];
     }
   };
@@ -318,7 +323,16 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
   // NB * 8 * GV_ROWS is a multiple of 32 and so is the stride: whole warps walk this loop together, and the 16
   // features of a token sit in 16 neighbouring lanes
   float qk_y0 = 0.f, qk_y1 = 0.f;
-  for (int idx = tid; idx < NB * 8 * GV_ROWS; idx += WARPS * 32) {
+  if (EPI == 5 && tid < NB * 8 * PAIRS) {
+#pragma unroll
+    for (int wv = 0; wv < WARPS; ++wv) {
+      const float* row = gv_red + ((size_t)wv * NB * 8 + item_n) * GV_ROWS + item_m;
+      qk_y0 += row[0];
+      qk_y1 += row[8];
+    }
+    if (rs.partials) { qk_y0 *= row_factor[item_n]; qk_y1 *= row_factor[item_n]; }
+  }
+  for (int idx = tid; EPI != 5 && idx < NB * 8 * GV_ROWS; idx += WARPS * 32) {
     const int n = idx / GV_ROWS, m = idx % GV_ROWS;
     const int o = o0 + m, tok = n0 + n;
     const bool valid = o < o_out && tok < n_rows && (!half_tile || m < 8);
@@ -360,14 +374,14 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
       out[(size_t)tok * o_out + o] = from_f32<TO>((EPI == 0 && rs.unary) ? ifb_unary(r, rs.unary) : r);
     }
   }
-  if (EPI == 3) {
-    __shared__ float qk_ssq[8][NB * 8];                 // [CTA of the head][token]: sums of squares over 32 features
-    const bool mine = tid < NB * 8 * GV_ROWS;           // this thread holds the pair (m, m + head_dim/2) of token n
+  if (QK) {
+    __shared__ float qk_ssq[8][NB * 8];                 // [CTA of the head][token]: sums of squares over its features
+    const bool mine = tid < NB * 8 * PAIRS;             // this thread holds the pair (m, m + head_dim/2) of token n
     const int n = item_n, m = item_m, tok = item_tok;
     const bool is_v = qk_is_v;
     const uint32_t rank = gv_cluster_rank(), peers = gv_cluster_size();
     float sq = mine ? qk_y0 * qk_y0 + qk_y1 * qk_y1 : 0.f;
-    sq += __shfl_xor_sync(0xffffffffu, sq, 8);
+    if (EPI == 3) sq += __shfl_xor_sync(0xffffffffu, sq, 8);
     sq += __shfl_xor_sync(0xffffffffu, sq, 4);
     sq += __shfl_xor_sync(0xffffffffu, sq, 2);
     sq += __shfl_xor_sync(0xffffffffu, sq, 1);
@@ -375,7 +389,7 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
       for (uint32_t p = 0; p < peers; ++p) gv_store_to_peer(&qk_ssq[rank][n], p, sq);
     gv_cluster_barrier();                               // every thread of every CTA of the head, on every path
     if (!mine || tok >= n_rows) return;
-    const int D = qk.head_dim, half = D / 2, i = qk_c * GV_ROWS + m;
+    const int D = qk.head_dim, half = D / 2, i = qk_c * PAIRS + m;
     float a = qk_y0, b = qk_y1;
     if (qk_nw) {
       float total = 0.f;
@@ -427,7 +441,7 @@ static int gv_features_per_cta(int o, int n_rows) {
 template <int NB, int EPI, int WARPS, typename TO, int STAGES = 1>
 static int gv_launch(const void* x, const void* w, void* out, int n, int o, int k, const GvRowScale& rs, const GvResidual& res,
                      cudaStream_t s) {
-  static_assert(EPI != 3, "the fused qkv epilogue is launched by gv_launch_qkv");
+  static_assert(EPI != 3 && EPI != 5, "the fused qkv epilogue is launched by gv_launch_qkv");
   const size_t smem = ((size_t)WARPS * (EPI == 1 ? 2 : 1) * NB * 8 * GV_ROWS + NB * 8) * sizeof(float);
   IFB_ALLOW_SMEM((linear_gemv_kernel<NB, EPI, WARPS, TO, STAGES>), smem);
   GvResidual res_f = res;
@@ -441,13 +455,13 @@ static int gv_launch(const void* x, const void* w, void* out, int n, int o, int 
                         (const bf16*)w, (TO*)out, n, o, k, rs, res_f, GvQkv{});
 }
 
-// The fused q | k | v product: one CTA per (head, 16 feature pairs), the CTAs of a head as a thread-block cluster.
-template <int NB, int WARPS, int STAGES>
+// The fused q | k | v product: one CTA per (head, 16 or 8 feature pairs), the CTAs of a head as a thread-block cluster.
+template <int NB, int WARPS, int STAGES, int EPI = 3>
 static int gv_launch_qkv(const void* x, const void* w, void* out, int n, int k, const GvRowScale& rs, const GvQkv& qk,
                          cudaStream_t s) {
-  const size_t smem = ((size_t)WARPS * 2 * NB * 8 * GV_ROWS + NB * 8) * sizeof(float);
-  IFB_ALLOW_SMEM((linear_gemv_kernel<NB, 3, WARPS, bf16, STAGES>), smem);
-  const int per_head = qk.head_dim / 32, heads = qk.nq + 2 * qk.nkv;
+  const size_t smem = ((size_t)WARPS * (EPI == 5 ? 1 : 2) * NB * 8 * GV_ROWS + NB * 8) * sizeof(float);
+  IFB_ALLOW_SMEM((linear_gemv_kernel<NB, EPI, WARPS, bf16, STAGES>), smem);
+  const int per_head = qk.head_dim / (EPI == 5 ? 16 : 32), heads = qk.nq + 2 * qk.nkv;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(heads * per_head, 1, 1);
   cfg.blockDim = dim3(WARPS * 32);
@@ -462,7 +476,7 @@ static int gv_launch_qkv(const void* x, const void* w, void* out, int n, int k, 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = (ifb_pdl_enabled() && (size_t)heads * qk.head_dim * k * 2 <= GV_EARLY_BYTES) ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, linear_gemv_kernel<NB, 3, WARPS, bf16, STAGES>, (const bf16*)x, (const bf16*)w, (bf16*)out, n,
+  cudaError_t e = cudaLaunchKernelEx(&cfg, linear_gemv_kernel<NB, EPI, WARPS, bf16, STAGES>, (const bf16*)x, (const bf16*)w, (bf16*)out, n,
                                      heads * qk.head_dim, k, rs, GvResidual{nullptr, nullptr, 0, nullptr}, qk);
   if (e != cudaSuccess) { cudaGetLastError(); return -(int)e; }
   return IFB_OK;
@@ -573,6 +587,10 @@ IFB_EXPORT int ifb_linear_gemv_qkv(const void* x, const void* w, void* qkv, int 
   GvQkv qk{nq, nkv, head_dim, q_weight, k_weight, w_dtype, eps, reinterpret_cast<const float2*>(rope), slots,
            reinterpret_cast<bf16*>(pages), page_size};
   const int nb = n_rows <= 8 ? 1 : 2;
+  // A long k, one block of tokens, and more CTAs of 16 pairs (of which an SM holds one) than SMs: 8 pairs, two CTAs per SM (48 heads of
+  // 4,096, 192 CTAs: 19.1 to 16.7 us for eight rows, 18.5 to 15.5 for one; 56 of 5,120 23.4 to 20.1; 28 of 3,072, 112 CTAs, 7.1 to 7.7: not).
+  if (k_dim > 2048 && nb == 1 && head_dim <= 128 && (long long)(nq + 2 * nkv) * (head_dim / 32) > GV_SMS)
+    return gv_launch_qkv<1, 8, 2, 5>(x, w, qkv, n_rows, k_dim, rs, qk, stream);
   if (k_dim <= 1024) return nb == 1 ? gv_launch_qkv<1, 8, 1>(x, w, qkv, n_rows, k_dim, rs, qk, stream)
                                     : gv_launch_qkv<2, 8, 1>(x, w, qkv, n_rows, k_dim, rs, qk, stream);
   if (k_dim <= 2048) return nb == 1 ? gv_launch_qkv<1, 16, 1>(x, w, qkv, n_rows, k_dim, rs, qk, stream)
