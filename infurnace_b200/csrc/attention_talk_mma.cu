@@ -90,22 +90,36 @@ template <int D, int NW, bool CL>
 __global__ void __launch_bounds__(NW * 32, 1)
 attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
   extern __shared__ __align__(16) unsigned char tm_raw[];
-  ifb_pdl_wait();
-  ifb_pdl_trigger();
   constexpr int LD = D + 8;                               // row pitch in elements: 16-byte aligned, no bank conflicts
   const int H = a.H, G = a.G, rep = H / G;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
-  // which (request, tile) this CTA is
+  // Which (request, tile) this CTA is: a lane per request, 32 at a time (a loop over them was a chain of round trips in every CTA).
+  // What the step's lengths are was written at its start, not by the kernel before this one: it may be read before the wait.
   int r = -1, tile = 0;
   {
     int left = blockIdx.x;
-    for (int i = 0; i < a.n_req; ++i) {
-      const int ql = a.seq_lens[i] > 0 ? a.cu_q[i + 1] - a.cu_q[i] : 0;     // a request of length 0 is padding
+    for (int base = 0; base < a.n_req && r < 0; base += 32) {
+      const int i = base + lane;
+      const int ql = i < a.n_req && a.seq_lens[i] > 0 ? a.cu_q[i + 1] - a.cu_q[i] : 0;     // a request of length 0 is padding
       const int tiles = (ql + TM_ROWS - 1) / TM_ROWS;
-      if (left < tiles) { r = i; tile = left; break; }
-      left -= tiles;
+      int upto = tiles;                                             // tiles of the requests up to this lane's
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int before = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= d) upto += before;
+      }
+      const unsigned past = __ballot_sync(0xffffffffu, upto > left);
+      if (past) {
+        const int l = __ffs(past) - 1;
+        r = base + l;
+        tile = left - __shfl_sync(0xffffffffu, upto - tiles, l);
+      } else {
+        left -= __shfl_sync(0xffffffffu, upto, 31);
+      }
     }
   }
+  ifb_pdl_wait();
+  ifb_pdl_trigger();
   if (r < 0) return;
   const int q_len = a.cu_q[r + 1] - a.cu_q[r];
   const int q0 = a.cu_q[r] + tile * TM_ROWS;
@@ -114,6 +128,17 @@ attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
   const int p_last = p0 + rows - 1;
   const int o0 = blockIdx.y * NW;                                   // first head of the group
   const int heads_here = min(NW, H - o0);
+  const int chunk = a.chunk;
+  const int first = chunk > 0 ? (p0 / chunk) * chunk : 0;           // the first key any row of the tile sees
+  const int k_first = first + (int)blockIdx.z * TM_KEYS, k_step = TM_KEYS * a.splits;
+  if (k_first > p_last && a.splits > 1) {                           // no keys for this share (all groups of the tile leave together)
+    for (int i = tid; i < rows * heads_here; i += NW * 32) {
+      float* part = a.parts + (((size_t)(q0 + i / heads_here) * H + o0 + i % heads_here) * a.splits + blockIdx.z) * (D + 2);
+      part[D] = -INFINITY;
+      part[D + 1] = 0.f;
+    }
+    return;
+  }
   const int g_lo = o0 / rep, g_hi = (o0 + heads_here - 1) / rep, GV = g_hi - g_lo + 1;
 
   bf16* Qs = reinterpret_cast<bf16*>(tm_raw);
@@ -136,9 +161,7 @@ attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
       Tt[idx] = o < heads_here ? load_as_f32(a.talk, a.talk_dtype, (size_t)(o0 + o) * H + h) : 0.f;
     }
 
-  const int chunk = a.chunk;
   const int ps_shift = (a.page_size & (a.page_size - 1)) == 0 ? __ffs(a.page_size) - 1 : -1;
-  const int first = chunk > 0 ? (p0 / chunk) * chunk : 0;           // the first key any row of the tile sees
   const int* bt = a.block_tables + (size_t)r * a.bt_stride;
   const size_t head_stride = (size_t)a.page_size * D, page_stride = 2 * (size_t)G * head_stride;
   const int rl = lane >> 2, cl = (lane & 3) * 2;                    // this lane's row and first column in an 8-wide tile
@@ -172,7 +195,6 @@ attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
       }
     }
   };
-  const int k_first = first + (int)blockIdx.z * TM_KEYS, k_step = TM_KEYS * a.splits;
   if (k_first <= p_last) load_tile(k_first, false);
   tm_cp_commit();
   if (k_first <= p_last) load_tile(k_first, true);
