@@ -72,6 +72,42 @@ def test_residual_update_with_norm_and_layer_scale(K, rows, width):
     close(xb, want, 3e-6, "residual update, bfloat16 weights")
 
 
+# Four features at a time: one to eight groups per thread and their edges (1,024, 2,048, 4,096, 8,192), blocks of one warp and more, and
+# rows that do not start at 16 bytes, which are taken feature by feature.
+@pytest.mark.parametrize("rows,width", [(3, 4), (9, 36), (5, 132), (70, 1024), (3, 1028), (2, 2048), (3, 2052), (2, 4096), (2, 4100), (2, 8192), (2, 8196)])
+def test_residual_update_in_groups_of_four(K, rows, width):
+    test_residual_update_with_norm_and_layer_scale(K, rows, width)
+    g = gen(width)
+    x, y, ls = torch.randn(rows, width, generator=g), torch.randn(rows, width, generator=g), torch.ones(width)
+    want = x.clone().double()
+    REF.residual_postnorm(want, y, torch.tensor(1.0), ls, 1e-5)
+    moved = torch.zeros(rows * width + 1, device="cuda")[1:].view(rows, width).copy_(x)
+    K.residual_postnorm(moved, y.cuda(), torch.tensor(1.0).cuda(), ls.cuda(), 1e-5)
+    close(moved, want, 3e-6, "rows at 4 bytes")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,kv,d,ps,own_v,weights", [(16, 4, 64, 16, False, True), (3, 1, 24, 8, True, True), (2, 2, 4, 3, True, False),
+                                                         (16, 8, 128, 16, True, True), (32, 32, 64, 16, False, True), (40, 8, 128, 32, True, True)])
+def test_whole_projection_norm_and_store_in_groups_of_four(K, heads, kv, d, ps, own_v, weights, dtype):
+    """Rows of whole groups of four: q and k of 16 to 6,144 features in all, values of their own and the keys, no weights; a slot of
+    nobody.  A page holds what the statement says and nothing else changes."""
+    g = gen(heads * d + kv)
+    n, qw, kw = 11, heads * d, kv * d
+    ld = qw + kw + (kw if own_v else 0) + 4
+    proj = torch.randn(n, ld, generator=g) * 3
+    wq, wk = (1 + 0.2 * torch.randn(qw, generator=g), 1 + 0.2 * torch.randn(kw, generator=g)) if weights else (None, None)
+    slots = torch.tensor([17, 3, -1, 40, 41, 42, 0, 9, 63, 25, 31], dtype=torch.int32)
+    pages = torch.full((-(-64 // ps), 2, kv, ps, d), 7.0)
+    want_q, want_p = torch.zeros(n, qw, dtype=torch.float64), pages.clone().double()
+    REF.wide_norm_store(proj, qw, kw, qw + kw if own_v else -1, d, wq, wk, 1e-5, want_q, slots, want_p)
+    got_q, got_p = torch.zeros(n, qw, device="cuda", dtype=dtype), pages.to(dtype).cuda()
+    K.wide_norm_store(proj.cuda(), qw, kw, qw + kw if own_v else -1, d, wq.cuda() if weights else None, wk.cuda() if weights else None, 1e-5,
+                      got_q, slots.cuda(), got_p)
+    tol = 1e-5 if dtype == torch.float32 else 0.06
+    close(got_q, want_q, tol, "q"), close(got_p, want_p, tol, "pages")
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("heads,kv,d,ps,own_v", [(4, 2, 16, 16, False), (3, 1, 24, 8, True), (6, 6, 8, 4, False)])
 def test_whole_projection_norm_and_store(K, heads, kv, d, ps, own_v, dtype):
