@@ -1149,10 +1149,14 @@ linear_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap tmap_x, con
 // q | k | v of 6,144 x 4,096 82 to 70, gate and up of 3,072 x 1,024 22.4 to 20.3 (each alone, repeated; in a step it adds 23.3),
 // 1,024 x 3,072 14.9 to 13.8.
 // ROWS32: the epilogue stages 64 float32 features of a row at a time (tc_finish_residual, tc_finish_heads).
+// HALVES: the tiles of a last round that has no more of them than half the pairs are halved, so that the round takes twice the pairs
+// and 0.6 of a round's time (an SM gets 24 KB per 64 of k where it gets 32, and its epilogue is half as long).
+// (Gate and up of 12,288 x 4,096 at 2,048 rows, 768 tiles for 74 pairs, 249 to 241 us; 3,072 x 1,024 at 2,048, 96 tiles, float32,
+// 18.9 on one tile per CTA, 14.9 so.)
 // ---------------------------------------------------------------------------------------------------
-template <int EPI_, int NACC_, int STAGES_, bool ROWS32_> struct PairCfg {
+template <int EPI_, int NACC_, int STAGES_, bool ROWS32_, bool HALVES_ = false> struct PairCfg {
   static constexpr int EPI = EPI_, NACC = NACC_, STAGES = STAGES_;
-  static constexpr bool ROWS32 = ROWS32_;
+  static constexpr bool ROWS32 = ROWS32_, HALVES = HALVES_;
   static constexpr int FO = EPI ? NACC / 2 : NACC;            // output features per tile
   static constexpr int W_ROWS = NACC / 2;                     // rows of w of a CTA's stage
   static constexpr int A_BYTES = G_TILE_BYTES, B_BYTES = W_ROWS * G_BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
@@ -1160,8 +1164,9 @@ template <int EPI_, int NACC_, int STAGES_, bool ROWS32_> struct PairCfg {
   static constexpr int STAGING_PITCH = (ROWS32 ? 256 : 128) + 16;
   static constexpr int STAGING_BYTES = 8 * 32 * STAGING_PITCH;
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STAGING_BYTES + 1024 /* alignment */ + 256 /* barriers */;
-  // float32 accumulator, bfloat16 a and b, both K-major, M = 256 over the pair, N = NACC
-  static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NACC >> 3) << 17) | ((uint32_t)(2 * G_BM >> 4) << 24);
+  // float32 accumulator, bfloat16 a and b, both K-major, M = 256 over the pair, N = NACC, or half of it
+  static constexpr uint32_t IDESC_N0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(2 * G_BM >> 4) << 24);
+  static constexpr uint32_t IDESC = IDESC_N0 | ((uint32_t)(NACC >> 3) << 17), IDESC_HALF = IDESC_N0 | ((uint32_t)(NACC >> 4) << 17);
   static_assert(SMEM_BYTES <= 227 * 1024, "stages and staging rows must fit in shared memory");
 };
 
@@ -1185,11 +1190,22 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                ::"r"(g_smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
+// Tile t of a launch over pairs: its tile of rows, and its first feature.  The first `whole` are whole, then come the two halves of
+// tile `whole`, of the next, ...
+template <bool HALVES>
+__device__ __forceinline__ int tc_pair_place(int t, int whole, int tiles_m, int fo, int& n0) {
+  if (!HALVES) { n0 = t / tiles_m * fo; return t % tiles_m; }
+  const int half = t < whole ? 0 : (t - whole) & 1, tile = t < whole ? t : whole + ((t - whole) >> 1);
+  n0 = tile / tiles_m * fo + half * (fo / 2);
+  return tile % tiles_m;
+}
+
+// tiles_total: whole tiles and halves.  tmap_half: w in boxes of half a tile's rows (HALVES).
 template <typename Cfg, typename TO>
 __global__ void __launch_bounds__(G_THREADS, 1)
 linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
-                           TO* __restrict__ out, int n_rows, int o_out, int k_dim, int tiles_m, int tiles_total,
-                           int* __restrict__ err, TcFold fold) {
+                           const __grid_constant__ CUtensorMap tmap_half, TO* __restrict__ out, int n_rows, int o_out, int k_dim,
+                           int tiles_m, int tiles_whole, int tiles_total, int* __restrict__ err, TcFold fold) {
   constexpr int EPI = Cfg::EPI, NACC = Cfg::NACC, FO = Cfg::FO, STAGES = Cfg::STAGES;
   extern __shared__ unsigned char g_smem_raw[];
   const uint32_t raw = g_smem_u32(g_smem_raw);
@@ -1204,7 +1220,7 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;     // warp-uniform
   const int rank = blockIdx.x & 1;                             // the cluster is two neighbours along x
   const int kblocks = (k_dim + G_BK - 1) / G_BK;
-  // this pair's tiles: first, first + step, ...; tile t covers tokens (t % tiles_m) * 256 and features (t / tiles_m) * FO
+  // this pair's tiles: first, first + step, ... (tc_pair_place)
   const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
@@ -1229,16 +1245,18 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
     int g = 0;                                                  // k blocks issued so far, over all tiles
     bool waited = false, ok = true;
     for (int t = first; t < tiles_total && ok; t += step) {
-      const int m0 = (t % tiles_m) * (2 * G_BM) + rank * G_BM, n0 = (t / tiles_m) * FO;
-      const int w0 = EPI ? rank * o_out + n0 : n0 + rank * Cfg::W_ROWS;
+      int n0;
+      const int m0 = tc_pair_place<Cfg::HALVES>(t, tiles_whole, tiles_m, FO, n0) * (2 * G_BM) + rank * G_BM;
+      const bool half = Cfg::HALVES && t >= tiles_whole;
+      const int w0 = EPI ? rank * o_out + n0 : n0 + rank * (half ? Cfg::W_ROWS / 2 : Cfg::W_ROWS);
       for (int kb = 0; kb < kblocks; ++kb, ++g) {
         const int s = g % STAGES;
         if (g >= STAGES && !mbar_wait(&empty[s], ((g / STAGES) - 1) & 1, abort_flag, err, 1)) { ok = false; break; }
         unsigned char* stage = smem + s * Cfg::STAGE_BYTES;
         const uint32_t bar = cluster_addr(&full[s], 0);
         if (elect_one()) {
-          if (rank == 0) mbar_expect_tx(&full[s], 2 * Cfg::STAGE_BYTES);
-          tma_load_2d_pair(stage + Cfg::A_BYTES, &tmap_w, bar, kb * G_BK, w0);
+          if (rank == 0) mbar_expect_tx(&full[s], half ? 2 * Cfg::A_BYTES + Cfg::B_BYTES : 2 * Cfg::STAGE_BYTES);
+          tma_load_2d_pair(stage + Cfg::A_BYTES, half ? &tmap_half : &tmap_w, bar, kb * G_BK, w0);
         }
         __syncwarp();
         if (!waited && (g == STAGES - 1 || (kb == kblocks - 1 && t + step >= tiles_total))) {
@@ -1247,13 +1265,15 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
           ifb_pdl_trigger();
           waited = true;
           int gg = 0;
-          for (int tt = first; tt < tiles_total && gg <= g; tt += step)
+          for (int tt = first; tt < tiles_total && gg <= g; tt += step) {
+            int nn;
+            const int mm = tc_pair_place<Cfg::HALVES>(tt, tiles_whole, tiles_m, FO, nn) * (2 * G_BM) + rank * G_BM;
             for (int kk = 0; kk < kblocks && gg <= g; ++kk, ++gg) {
               const uint32_t bb = cluster_addr(&full[gg % STAGES], 0);
-              if (elect_one())
-                tma_load_2d_pair(smem + (gg % STAGES) * Cfg::STAGE_BYTES, &tmap_x, bb, kk * G_BK, (tt % tiles_m) * (2 * G_BM) + rank * G_BM);
+              if (elect_one()) tma_load_2d_pair(smem + (gg % STAGES) * Cfg::STAGE_BYTES, &tmap_x, bb, kk * G_BK, mm);
               __syncwarp();
             }
+          }
         } else if (waited) {
           if (elect_one()) tma_load_2d_pair(stage, &tmap_x, bar, kb * G_BK, m0);
           __syncwarp();
@@ -1281,7 +1301,7 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
 #pragma unroll
           for (int k = 0; k < G_BK / G_UK; ++k) {
             const uint64_t kstep = (uint64_t)((k * G_UK * 2) >> 4);          // 32 bytes per k step, in 16-byte units
-            umma_bf16_pair(tmem_base + b * NACC, a_desc + kstep, b_desc + kstep, Cfg::IDESC, (kb | k) != 0);
+            umma_bf16_pair(tmem_base + b * NACC, a_desc + kstep, b_desc + kstep, Cfg::HALVES && t >= tiles_whole ? Cfg::IDESC_HALF : Cfg::IDESC, (kb | k) != 0);
           }
           umma_commit_pair(&empty[s]);
           if (kb == kblocks - 1) umma_commit_pair(&acc_full[b]);
@@ -1301,7 +1321,8 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
     if (fold.rs_partials || Cfg::ROWS32) ifb_pdl_wait();         // what the predecessors wrote is read here directly
     for (int t = first; t < tiles_total && ok; t += step, ++it) {
       const int b = it & 1;
-      const int row0 = (t % tiles_m) * (2 * G_BM) + rank * G_BM + q * 32, n0 = (t / tiles_m) * FO;
+      int n0;
+      const int row0 = tc_pair_place<Cfg::HALVES>(t, tiles_whole, tiles_m, FO, n0) * (2 * G_BM) + rank * G_BM + q * 32;
       const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16) + b * NACC;
       float rfac = tc_row_factor(fold, row0 + lane, n_rows);
       if constexpr (Cfg::ROWS32) {
@@ -1358,19 +1379,22 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
           }
         }
       } else {
-        constexpr int PW = 128 / (int)sizeof(TO);                // features per staged row segment
-        static_assert(CW % PW == 0, "a warp's features are whole row segments");
+        constexpr int LEAST = Cfg::HALVES ? CW / 2 : CW;         // features of a warp's piece of a half
+        constexpr int PW = 128 / (int)sizeof(TO) < LEAST ? 128 / (int)sizeof(TO) : LEAST, SEG = PW * (int)sizeof(TO);   // per staged row segment
+        static_assert(LEAST % PW == 0, "a warp's features are whole row segments");
         ok = mbar_wait(&acc_full[b], (it >> 1) & 1, abort_flag, err, 3);
         if (!ok) break;
         tc_fence_after();
-        const bool vec = ((size_t)o_out * sizeof(TO)) % 16 == 0 && (((uintptr_t)out) & 15) == 0 && n0 + c_lo + CW <= o_out;
+        const bool half = Cfg::HALVES && t >= tiles_whole;
+        const int cw = half ? CW / 2 : CW, c_at = half ? c_lo / 2 : c_lo, fo = half ? FO / 2 : FO;
+        const bool vec = ((size_t)o_out * sizeof(TO)) % 16 == 0 && (((uintptr_t)out) & 15) == 0 && n0 + c_at + cw <= o_out;
 #pragma unroll 1
-        for (int p0 = c_lo; p0 < c_lo + CW; p0 += PW) {
+        for (int p0 = c_at; p0 < c_at + cw; p0 += PW) {
           if (n0 + p0 >= o_out || row0 >= n_rows) break;         // warp-uniform
 #pragma unroll
           for (int c0 = p0; c0 < p0 + PW; c0 += 32) {
             float y[32];
-            tc_epilogue_row<EPI>(fold, lane_base + c0, FO, rfac, n0 + c0, o_out, y);
+            tc_epilogue_row<EPI>(fold, lane_base + c0, fo, rfac, n0 + c0, o_out, y);
             if (vec) tc_pack_row<TO>(buf + lane * PITCH + (c0 - p0) * (int)sizeof(TO), y);
             else if (row0 + lane < n_rows) {
               TO* dst = out + (size_t)(row0 + lane) * o_out + n0 + c0;
@@ -1383,8 +1407,8 @@ linear_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __g
             __syncwarp();
             unsigned char* obase = reinterpret_cast<unsigned char*>(out + (size_t)row0 * o_out + n0 + p0);
 #pragma unroll
-            for (int off = lane * 16; off < 32 * 128; off += 512) {
-              const int r = off >> 7, cb = off & 127;
+            for (int off = lane * 16; off < 32 * SEG; off += 512) {
+              const int r = off / SEG, cb = off % SEG;
               if (row0 + r < n_rows)
                 *reinterpret_cast<uint4*>(obase + (size_t)r * o_out * sizeof(TO) + cb) = *reinterpret_cast<const uint4*>(buf + r * PITCH + cb);
             }
@@ -1440,6 +1464,14 @@ static int tc_pairs() {
   return known[dev];
 }
 
+// Tiles of the last round that are halved: all of them, where whole rounds come before it and its halves find a pair each.  From a k of
+// 512: below it the products of a round are shorter than its epilogue (gate and up of 3,072 features at 818 rows: k 256 7.3 us on the
+// persistent kernel and 8.5 so, k 512 10.1 and 9.8; plain 2,304 x 256 at 5,000 rows 11.3 whole, 11.7 halved).
+static int tc_pair_halved(int pairs, long long tiles, int k) {
+  const int rest = (int)(tiles % pairs);
+  return k >= 512 && tiles > pairs && 2 * rest <= pairs ? rest : 0;
+}
+
 template <typename Cfg, typename TO>
 static int tc_launch_pair(const void* x, const void* w, void* out, int n, int o, int k, int* err, cudaStream_t s, const TcFold& fold) {
   CUtensorMap mx, mw;
@@ -1451,8 +1483,17 @@ static int tc_launch_pair(const void* x, const void* w, void* out, int n, int o,
   if (!pairs) return IFB_ERR_ARG;
   IFB_ALLOW_SMEM((linear_tcgen05_pair_kernel<Cfg, TO>), Cfg::SMEM_BYTES);
   const long long tiles_m = (n + 2 * G_BM - 1) / (2 * G_BM), tiles_n = (o + Cfg::FO - 1) / Cfg::FO;
-  if (tiles_m * tiles_n > 0x7fffffffLL) return IFB_ERR_SIZE;
-  const int total = (int)(tiles_m * tiles_n);
+  if (tiles_m * tiles_n > 0x3fffffffLL) return IFB_ERR_SIZE;
+  int total = (int)(tiles_m * tiles_n);
+  const int halved = tc_pair_halved(pairs, total, k), whole = total - (Cfg::HALVES ? halved : 0);
+  CUtensorMap mh = mw;
+  if constexpr (Cfg::HALVES) {
+    total += halved;
+    st = make_map(&mh, w, Cfg::EPI ? 2 * o : o, k, Cfg::W_ROWS / 2);
+    if (st) return st;
+  } else if constexpr (!Cfg::ROWS32 && Cfg::NACC == 256) {        // (a kernel of its own: the second epilogue costs the first registers)
+    if (halved) return tc_launch_pair<PairCfg<Cfg::EPI, 256, Cfg::STAGES, false, true>, TO>(x, w, out, n, o, k, err, s, fold);
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2 * (total < pairs ? total : pairs));
   cfg.blockDim = dim3(G_THREADS);
@@ -1467,7 +1508,7 @@ static int tc_launch_pair(const void* x, const void* w, void* out, int n, int o,
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = ifb_pdl_enabled() ? 2 : 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, linear_tcgen05_pair_kernel<Cfg, TO>, mx, mw, (TO*)out, n, o, k, (int)tiles_m, total, err, fold);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, linear_tcgen05_pair_kernel<Cfg, TO>, mx, mw, mh, (TO*)out, n, o, k, (int)tiles_m, whole, total, err, fold);
   if (e != cudaSuccess) { cudaGetLastError(); return -(int)e; }
   return IFB_OK;
 }
@@ -1579,6 +1620,15 @@ static bool tc_pick_pair(int pairs, TcKind kind, int n, int o, int k) {
   const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
   return tiles * 10 >= (long long)pairs * 8 * rounds;
 }
+// Tiles of the last round that are halved, 0 for none.  A product with such a round takes the pairs even where whole tiles would leave
+// more than a fifth of them idle: everywhere the quickest (gate and up of 3,072 x 1,024 at 818 rows 16.1 us on the
+// persistent kernel, 12.9 so, at 1,600 rows 21.8 and 17.4; 6,144 x 2,048 at 818 rows 27.8 and 21.7, at 1,600 50 and 31).
+static int tc_pick_halves(int pairs, TcKind kind, int n, int o, int k) {
+  if (o % 64 || n <= 512 || pairs < 1 || (kind != TC_PLAIN && kind != TC_GATED)) return 0;
+  const int features = tc_pair_features(pairs, kind, n, o);
+  if (features != (kind == TC_GATED ? 128 : 256)) return 0;
+  return tc_pair_halved(pairs, (long long)((n + 255) / 256) * ((o + features - 1) / features), k);
+}
 
 template <int EPI, typename TO>
 static int tc_launch(const void* x, const void* w, void* out, int n, int o, int k, int* err, int shape, int splits, const TcFold& fold,
@@ -1594,7 +1644,9 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
     return tc_launch_cfg<Deep, TO>(x, w, out, n, o, k, err, s, fold, splits);
   }
   if (shape == 0) {
-    shape = tc_pick_pair(tc_device_pairs(), tc_kind(EPI, fold), n, o, k) ? 6 : tc_pick_shape(EPI, n, o);
+    const int pairs = tc_device_pairs();
+    const TcKind kind = tc_kind(EPI, fold);
+    shape = tc_pick_pair(pairs, kind, n, o, k) || tc_pick_halves(pairs, kind, n, o, k) > 0 ? 6 : tc_pick_shape(EPI, n, o);
   }
   if (EPI && fold.res_x) return IFB_ERR_ARG;
   if (shape == 6) {
@@ -1725,12 +1777,18 @@ IFB_EXPORT int ifb_linear_tcgen05_qkv(const void* x, const void* w, void* qkv, i
 }
 
 // Features of the tiles with which a product of these sizes runs over pairs of SMs (shape 0, splits 1), or 0 where it runs on another
-// kernel.  kind: 0 plain, 1 with the residual addition, 2 the fused q | k | v product, 3 gated.  pairs: how many of them to answer
+// kernel or over pairs for its halved tiles' sake alone.  kind: 0 plain, 1 with the residual addition, 2 the fused q | k | v product, 3 gated.  pairs: how many of them to answer
 // for, 0: this device's.
 IFB_EXPORT int ifb_linear_tcgen05_pair_tile(int kind, int n_rows, int out_features, int k_dim, int pairs) {
   if (kind < TC_PLAIN || kind > TC_GATED) return 0;
   if (!pairs) pairs = tc_device_pairs();
   return tc_pick_pair(pairs, (TcKind)kind, n_rows, out_features, k_dim) ? tc_pair_features(pairs, (TcKind)kind, n_rows, out_features) : 0;
+}
+
+// Tiles of a product's last round over pairs of SMs that are halved (shape 0, splits 1): 0 where none is, or another kernel takes it.
+IFB_EXPORT int ifb_linear_tcgen05_pair_halved(int kind, int n_rows, int out_features, int k_dim, int pairs) {
+  if (kind < TC_PLAIN || kind > TC_GATED) return 0;
+  return tc_pick_halves(pairs ? pairs : tc_device_pairs(), (TcKind)kind, n_rows, out_features, k_dim);
 }
 
 // Parts of sums of squares that a product with res_x writes per row (the launch with shape 0 and these splits).

@@ -882,6 +882,32 @@ def test_qkv_product_over_pairs_with_norm_rotation_and_store_in_its_epilogue(K, 
     test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, 128, k, 16, norm, rotate, scaled)
 
 
+# A last round of halved tiles: one and two whole rounds before it, ragged rows, the last tile whole, three quarters and one quarter full,
+# float32 and bfloat16, a function and a bias, gates and a folded norm's factors.  (The halves hold for 74 pairs.)  Every feature is the
+# sum that a whole tile forms, in the same order: the halves leave the bits of the forced whole-tile kernel of one CTA.
+@pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,o,k,kind,epilogue", [(2043, 3072, 520, 0, "relu2"), (1280, 4096, 512, 0, "none"), (4600, 2240, 584, 0, "none"), (2043, 2368, 520, 0, "none"),
+                                                 (818, 3072, 512, 3, "silu_gate"), (700, 3264, 584, 3, "gelu_gate"), (1600, 3136, 520, 3, "silu_gate"), (5000, 1024, 1032, 3, "silu_gate")])
+def test_product_over_pairs_with_halved_tiles(K, od, n, o, k, kind, epilogue):
+    from infurnace_b200.kernels.cuda import EPILOGUES
+    assert K._tc_lib().ifb_linear_tcgen05_pair_halved(kind, n, o, k, 0) > 0
+    x, w = rnd((n, k), torch.bfloat16, 4).cuda(), rnd(((2 if kind else 1) * o, k), torch.bfloat16, 5, scale=k ** -0.5).cuda()
+    partials, bias = torch.rand((3, n)).cuda() * 40 + 1, torch.randn(o).cuda() if epilogue == "none" else None
+    kw = dict(row_scale=(partials, 3, 1e-5, 55), bias=bias)
+    y = (x.double() @ w.double().t()) * torch.rsqrt(partials.double().sum(0) / 55.0 + 1e-5)[:, None]
+    if kind:
+        g = torch.nn.functional.silu(y[:, :o]) if epilogue == "silu_gate" else torch.nn.functional.gelu(y[:, :o], approximate="tanh")
+        y = g * y[:, o:]
+    else:
+        y = y + bias.double() if bias is not None else y.relu() ** 2
+    out, same = (torch.full((n, o), float("nan"), dtype=od, device="cuda") for _ in range(2))
+    K._linear_tcgen05(x, w, out, n, o, k, EPILOGUES[epilogue], **kw)
+    K._linear_tcgen05(x, w, same, n, o, k, EPILOGUES[epilogue], shape=4, **kw)
+    K.check_device_errors()
+    torch.testing.assert_close(out.double(), y, rtol=1.6e-2 if od == torch.bfloat16 else 4e-3, atol=1e-2 if od == torch.bfloat16 else 2e-3)
+    assert torch.equal(out, same)
+
+
 # Gate and up of a short prompt in tiles of 64 features: ragged rows, features and k, with and without a folded norm's factors.
 @pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,o,k", [(1, 40, 72), (129, 3072, 1024), (200, 1000, 136), (513, 65, 520)])

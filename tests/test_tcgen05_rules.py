@@ -60,6 +60,23 @@ def test_the_heads_of_a_short_product_stay_on_one_tile_per_cta(kind, n, o, k, ti
     assert load_library("linear_tcgen05").ifb_linear_tcgen05_pair_tile(kind, n, o, k, 74) == tile
 
 
+def test_only_a_last_round_that_leaves_half_the_pairs_idle_is_halved():
+    lib = load_library("linear_tcgen05")
+    taken = 0
+    for kind in (PLAIN, RESIDUAL, HEADS, GATED):
+        for n in (1, 512, 513, 768, 1000, 1400, 1900, 2048, 5000):
+            for o in (64, 1000, 1024, 1088, 2304, 3072, 4096, 6144, 12288):
+                rest = lib.ifb_linear_tcgen05_pair_halved(kind, n, o, 512, 74)
+                assert lib.ifb_linear_tcgen05_pair_halved(kind, n, o, 511, 74) == 0
+                tiles = -(-n // 256) * -(-o // (128 if kind == GATED else 256))
+                if kind in (RESIDUAL, HEADS) or n <= 512 or o % 64 or tiles <= 74:
+                    assert rest == 0, (kind, n, o)
+                else:
+                    assert rest == (tiles % 74 if tiles % 74 <= 37 else 0), (kind, n, o)
+                    taken += rest > 0
+    assert taken > 20
+
+
 class _Norm:
     weight = None
 
