@@ -38,7 +38,7 @@ struct TalkMmaArgs {
   bf16* out;                // [tokens][H * D]
   int n_tokens, n_req, H, G, page_size, chunk;
   float scale, slope_exp;
-  int splits;               // > 1: CTA z takes every splits-th tile of keys and leaves its part in `parts` for the merge
+  int splits;               // > 1: share z takes every splits-th tile of keys and leaves its part in `parts` for the merge
   float* parts;             // [tokens][H][splits][D + 2]: the unnormalised output row, then the maximum and the sum
 };
 
@@ -84,6 +84,57 @@ __device__ __forceinline__ float4 tm_ld_cluster_f4(uint32_t addr, int rank) {
   return v;
 }
 
+// The i-th tile of the step, its request in `r` (-1: there are fewer), found by a whole warp.  A CTA has an SM to itself and a prompt's tile
+// has up to 32 times the keys of another, so the tiles with the most keys come first and short ones fill the SMs at the end: of every
+// chunk of every request the last tile of a whole chunk, then the ones before, by a search over the place within the chunk
+// (16 heads of 64, chunks of 512, with the merge: 2,048 tokens 83 to 63 us, prompts of 147, 681 and 1,215 tokens 79 to 58, both then
+// in two shares instead of four).  Chunks are counted from a request's first tile: where it continues a prompt the order is less
+// good.  More than 32 requests are taken one after the other, the last tile first.
+__device__ __forceinline__ int tm_find_tile(const TalkMmaArgs& a, int i, int lane, int& r) {
+  r = -1;
+  if (a.n_req <= 32) {
+    const int ql = lane < a.n_req && a.seq_lens[lane] > 0 ? a.cu_q[lane + 1] - a.cu_q[lane] : 0;    // a request of length 0 is padding
+    const int tiles = (ql + TM_ROWS - 1) / TM_ROWS, most = __reduce_max_sync(0xffffffffu, tiles);
+    if (i >= __reduce_add_sync(0xffffffffu, tiles)) return 0;
+    const int per = a.chunk >= TM_ROWS ? min(a.chunk / TM_ROWS, most) : most;
+    const int whole = tiles ? (tiles - 1) / per : 0, last = tiles - whole * per;     // whole chunks, and the tiles of the one after them
+    int lo = 0, hi = per;                                                            // the place: tiles at lo or behind it > i >= at hi or behind it
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (__reduce_add_sync(0xffffffffu, whole * (per - mid) + max(0, last - mid)) > i) lo = mid; else hi = mid;
+    }
+    const int left = i - __reduce_add_sync(0xffffffffu, whole * (per - lo - 1) + max(0, last - lo - 1));
+    const int here = whole + (lo < last ? 1 : 0);                                    // this request's tiles at that place
+    int upto = here;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int before = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto += before;
+    }
+    r = __ffs(__ballot_sync(0xffffffffu, upto > left)) - 1;
+    return (left - __shfl_sync(0xffffffffu, upto - here, r)) * per + lo;
+  }
+  for (int base = 0; base < a.n_req; base += 32) {
+    const int at = base + lane;
+    const int ql = at < a.n_req && a.seq_lens[at] > 0 ? a.cu_q[at + 1] - a.cu_q[at] : 0;
+    const int tiles = (ql + TM_ROWS - 1) / TM_ROWS;
+    int upto = tiles;                                                                // tiles of the requests up to this lane's
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int before = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto += before;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, upto > i);
+    if (past) {
+      const int l = __ffs(past) - 1;
+      r = base + l;
+      return __shfl_sync(0xffffffffu, upto, l) - 1 - i;
+    }
+    i -= __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return 0;
+}
+
 // Shared memory, in this order: Q [NW][16][D + 8] bf16, K and V [GV][32][D + 8] bf16 each (GV: key/value heads of the
 // group), S [NW][16][32] float, M [NW][16][32] float, talk^T [H][NW] float.  CL: the groups form a cluster.
 template <int D, int NW, bool CL>
@@ -93,31 +144,11 @@ attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
   constexpr int LD = D + 8;                               // row pitch in elements: 16-byte aligned, no bank conflicts
   const int H = a.H, G = a.G, rep = H / G;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
-  // Which (request, tile) this CTA is: a lane per request, 32 at a time (a loop over them was a chain of round trips in every CTA).
+  // Which (request, tile) and share of its keys this CTA is: the shares of a tile are neighbours, as the next shorter tile comes after them.
   // What the step's lengths are was written at its start, not by the kernel before this one: it may be read before the wait.
-  int r = -1, tile = 0;
-  {
-    int left = blockIdx.x;
-    for (int base = 0; base < a.n_req && r < 0; base += 32) {
-      const int i = base + lane;
-      const int ql = i < a.n_req && a.seq_lens[i] > 0 ? a.cu_q[i + 1] - a.cu_q[i] : 0;     // a request of length 0 is padding
-      const int tiles = (ql + TM_ROWS - 1) / TM_ROWS;
-      int upto = tiles;                                             // tiles of the requests up to this lane's
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int before = __shfl_up_sync(0xffffffffu, upto, d);
-        if (lane >= d) upto += before;
-      }
-      const unsigned past = __ballot_sync(0xffffffffu, upto > left);
-      if (past) {
-        const int l = __ffs(past) - 1;
-        r = base + l;
-        tile = left - __shfl_sync(0xffffffffu, upto - tiles, l);
-      } else {
-        left -= __shfl_sync(0xffffffffu, upto, 31);
-      }
-    }
-  }
+  const int share = blockIdx.x % a.splits;
+  int r;
+  const int tile = tm_find_tile(a, blockIdx.x / a.splits, lane, r);
   ifb_pdl_wait();
   ifb_pdl_trigger();
   if (r < 0) return;
@@ -130,10 +161,10 @@ attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
   const int heads_here = min(NW, H - o0);
   const int chunk = a.chunk;
   const int first = chunk > 0 ? (p0 / chunk) * chunk : 0;           // the first key any row of the tile sees
-  const int k_first = first + (int)blockIdx.z * TM_KEYS, k_step = TM_KEYS * a.splits;
+  const int k_first = first + share * TM_KEYS, k_step = TM_KEYS * a.splits;
   if (k_first > p_last && a.splits > 1) {                           // no keys for this share (all groups of the tile leave together)
     for (int i = tid; i < rows * heads_here; i += NW * 32) {
-      float* part = a.parts + (((size_t)(q0 + i / heads_here) * H + o0 + i % heads_here) * a.splits + blockIdx.z) * (D + 2);
+      float* part = a.parts + (((size_t)(q0 + i / heads_here) * H + o0 + i % heads_here) * a.splits + share) * (D + 2);
       part[D] = -INFINITY;
       part[D + 1] = 0.f;
     }
@@ -332,8 +363,8 @@ attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
   if (warp >= heads_here) return;
   const int head = o0 + warp;
   if (a.splits > 1) {                       // this CTA's part: rows as they are, with their maxima and sums
-    float* pr0p = a.parts + (((size_t)(q0 + rl) * H + head) * a.splits + blockIdx.z) * (D + 2);
-    float* pr1p = a.parts + (((size_t)(q0 + rl + 8) * H + head) * a.splits + blockIdx.z) * (D + 2);
+    float* pr0p = a.parts + (((size_t)(q0 + rl) * H + head) * a.splits + share) * (D + 2);
+    float* pr1p = a.parts + (((size_t)(q0 + rl + 8) * H + head) * a.splits + share) * (D + 2);
 #pragma unroll
     for (int n = 0; n < D / 8; ++n) {
       if (row0) *reinterpret_cast<float2*>(pr0p + n * 8 + cl) = make_float2(O[n][0], O[n][1]);
@@ -371,7 +402,7 @@ attention_talk_mma_kernel(TalkMmaArgs a, int gv_max) {
 // out[t, h, :] = sum_z parts[t, h, z, :D] * exp(m_z - m) / sum_z l_z * exp(m_z - m), m = max_z m_z, times sigmoid(gate):
 // a warp per (token, head), the parts' rows added in ascending z.  A warp's time is its chain of round trips to memory, so
 // the token's request is found by all lanes and before the wait (the step's lengths were written at its start), and the maxima, the first four
-// rows and the gate are requested together, whether or not those parts saw a key (16 heads of 64: 2,043 tokens in 3 parts 15.4 to 12.5 us,
+// rows and the gate are requested together, whether or not those parts saw a key (16 heads of 64: 2,043 tokens in four parts 15.4 to 12.5 us,
 // eight tokens 5.7 to 3.2).
 template <int D>
 __global__ void __launch_bounds__(128)
@@ -494,7 +525,9 @@ static int tm_launch(const TalkMmaArgs& a, cudaStream_t s) {
   const int gv_max = tm_gv_max(a.H, a.G, NW);
   const size_t smem = tm_smem_bytes(a.H, a.G, D, NW, gv_max);
   const int groups = (a.H + NW - 1) / NW;
-  dim3 grid((a.n_tokens + TM_ROWS - 1) / TM_ROWS + a.n_req, groups, a.splits);
+  const long long ctas = ((long long)(a.n_tokens + TM_ROWS - 1) / TM_ROWS + a.n_req) * a.splits;
+  if (ctas > 0x7fffffffLL) return IFB_ERR_SIZE;
+  dim3 grid((unsigned)ctas, groups);
   int st;
   if (groups == 1) {
     IFB_ALLOW_SMEM((attention_talk_mma_kernel<D, NW, false>), smem);

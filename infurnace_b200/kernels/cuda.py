@@ -955,17 +955,23 @@ class CudaKernels:
             self._stream()), "attention_talk")
 
     def _talk_splits(self, n, r, num_heads, head_dim, chunk, max_q_len, max_seq_len):
-        """CTAs that share the keys of one query tile of the tensor-core talking attention: 1 unless the step's tiles
-        alone leave most SMs idle (few query tokens) and a query may see many keys; then enough to fill the device
-        once, with no fewer than four tiles of 32 keys each (decoded tokens: one).  Up to 4 for a prompt of few tiles (see below)."""
+        """CTAs that share the keys of one query tile of the tensor-core talking attention: for few query tokens enough to fill
+        the device once, with no fewer than four tiles of 32 keys each (decoded tokens: one); for prompts see below."""
         if not max_q_len or not max_seq_len:
             return 1
         reach = min(chunk, max_seq_len) if chunk else max_seq_len
         tiles = (-(-n // 16) + r) * -(-num_heads // 16)
         if max_q_len > 64:
-            # a prompt: a tile late in its chunk has many times the keys of an early one, and with less than two CTAs
-            # per SM the longest tile is the kernel's time; shares of at most a quarter of the keys even that out
-            return max(1, min(4, reach // 128)) if tiles < 2 * self.sm_count else 1
+            # a prompt: tiles have 1 to `trips` tiles of 32 keys, the longest first, a CTA per SM.  The time is the longest share's or the
+            # sum of all over the SMs, whichever is more, and the merge's, in trips of some 5 us: a CTA takes 1.6 to begin
+            # and end, the merge 0.8 and what it reads.  Over 25 sets of lengths within 8 % of the best of 1 to 12 (16 heads of 64, us: 2,048
+            # tokens, chunks of 512, two shares 63, one 90, four 74; 4,096 one 96, two 120, four 140; 300 five 20, two 33)
+            trips = -(-reach // 32)
+
+            def cost(s):
+                longest, work = 1.6 + -(-trips // s), tiles * s / self.sm_count * (1.6 + (trips + 1) / (2 * s))
+                return max(longest, work) + (0.8 + n * num_heads * head_dim * s / 5.12e6 if s > 1 else 0)
+            return min(range(1, min(8, trips) + 1), key=cost)
         if max_q_len == 1:
             # decoded tokens: a tile of 32 keys is a chain of round trips (some 5 us), so every tile gets a CTA of its own
             return max(1, min(self.sm_count // max(1, tiles), reach // 32, 32))

@@ -301,6 +301,25 @@ def test_talking_attention_with_the_keys_split_over_ctas(K, chunk):
         close(got, want, 0.06, f"split keys, {H} heads")
 
 
+# Every tile of every request is taken once, whatever its place in the order: chunks that are no whole tiles, longer than the prompts, and
+# none; whole and ragged last chunks, prompts that continue, decoded tokens and padding beside them; 32 requests and one more.
+@pytest.mark.parametrize("chunk", [0, 8, 64, 300, 512])
+@pytest.mark.parametrize("cases", [[(700, 700), (33, 20), (0, 3), (130, 130), (1, 1)], [(64, 64), (128, 128), (129, 100), (16, 16), (17, 17)],
+                                   [(20 + 3 * i, 1 + i % 19) for i in range(32)], [(20 + 3 * i, 17 + i % 19) for i in range(33)]])
+@pytest.mark.parametrize("H,G,splits", [(8, 2, 1), (8, 2, 3), (32, 4, 2)])
+def test_talking_attention_takes_the_longest_tiles_first(K, H, G, splits, cases, chunk, monkeypatch):
+    monkeypatch.setattr(K, "_talk_splits", lambda *sizes: splits)
+    got, want = _attention_case(K, H, G, 32, 16, chunk, torch.bfloat16, cases, seed=chunk + H)
+    close(got, want, 0.06, f"{H} heads, {len(cases)} requests")
+
+
+def test_shares_of_a_prompts_keys(K):
+    """More shares for fewer tiles, never more than tiles of keys or eight; a prompt that fills the device takes its tiles whole."""
+    rule = lambda n, chunk, length, r=1: K._talk_splits(n, r, 16, 64, chunk, length, length)
+    assert [rule(n, 512, n) for n in (80, 300, 600, 1100, 1400, 2048, 4096, 8192)] == [3, 5, 6, 4, 3, 2, 1, 1]
+    assert rule(2048, 128, 2048) == 1 and rule(1600, 512, 100, 16) == 1 and rule(512, 0, 30000) == 8
+
+
 def test_a_nan_among_the_values_of_far_keys_reaches_the_output_of_split_keys(K):
     """Where one key's score is so far above the others that their weights are 0, their values still count: 0 times NaN."""
     for key, d in ((40, 64), (200, 16)):
