@@ -9,6 +9,7 @@
 // `first` may be stale (-1): they are never read.
 #include "common.cuh"
 #include <math.h>
+#include <type_traits>
 
 #define ATT_MAX_D 256
 
@@ -94,9 +95,15 @@ paged_attention_simt_kernel(const T* __restrict__ qkv, int row_stride, const T* 
 // of values.  What bounds it is the chain of round trips of a block for few keys, and shared-memory reads for many.
 // Measured in a step of the 0.6B sizes at 195 keys: one token 155 to about 10 us per layer, 193 tokens 156 to 60 us, against a warp
 // per query and head that read keys with a stride of a row.
+// Eight queries (a prompt): the keys of a block come in pieces of 32 features, one piece ahead of the one that is being used, which takes a
+// third of whole rows' shared memory and lets two CTAs share an SM, and which queries see a row is a bit each, found with the scores (193 tokens, 392 CTAs: 52 to 34 us; 1,000
+// tokens 546 to 292).  Two queries and a CTA to an SM (AHEAD; a decoded token): whole rows at once, and all of a block's values are requested
+// before its scores are formed, as a warp has one block or two and its time is that chain (9.8 to 8.2 us).
 // ---------------------------------------------------------------------------------------------------
-template <int QT, int DC, int W>
-__global__ void __launch_bounds__(W * 32)
+constexpr int S32_SMS = 148;                                    // SMs of a B200
+constexpr int S32_PITCH = 36;                                   // floats of a row of a piece: 16-byte reads without conflicts
+template <int QT, int DC, int W, bool AHEAD>
+__global__ void __launch_bounds__(W * 32, AHEAD ? 1 : W == 8 ? 2 : QT == 8 ? 3 : 4)
 paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, const float* __restrict__ pages,
                                 const int* __restrict__ block_tables, int bt_stride, const int* __restrict__ cu_q,
                                 const int* __restrict__ seq_lens, float* __restrict__ out, int n_tokens, int n_req, int nq,
@@ -105,12 +112,14 @@ paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, c
   ifb_pdl_wait();
   ifb_pdl_trigger();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr bool PIECES = QT == 8;
+  constexpr int VB = AHEAD ? 32 : 8 / DC;                          // rows of values requested at a time
   const int pitch = d + 4, d4 = d / 4, row_step = 32 / d4, c_step = 32 % d4;
   float* qs = sm;                                               // [QT][d]
   float* ps = qs + QT * d;                                      // [W][QT][32]: a block's weights
   float* ml = ps + W * QT * 32;                                 // [W][QT][2]: maximum and sum of a warp, then its factor
-  float* keys = ml + W * QT * 2;                                // [W][32][pitch], later [W][QT][d]: the warps' sums
-  float* kr = keys + (size_t)warp * 32 * pitch;
+  float* keys = ml + W * QT * 2;                                // [W][32][pitch] (PIECES: [W][2][32][S32_PITCH]), later [W][QT][d]: the warps' sums
+  float* kr = keys + (size_t)warp * (PIECES ? 64 * S32_PITCH : 32 * pitch);
   const int rep = nq / nkv, chunks = (rep + heads_per_cta - 1) / heads_per_cta;
   const int kvh = blockIdx.y / chunks, hlo = (blockIdx.y % chunks) * heads_per_cta;
   const int nh = min(heads_per_cta, rep - hlo), h0 = kvh * rep + hlo;
@@ -146,24 +155,25 @@ paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, c
       const float* kp = nullptr;
       if (key >= first && key <= last)
         kp = pages + (size_t)bt[key / page_size] * page_stride + (size_t)kvh * head_stride + (size_t)(key % page_size) * d;
-      // 16 bytes per lane, row by row; lane's place moves on by 32 pieces at a time
-      for (int it = 0, row = lane / d4, c = lane % d4; it < d4; ++it) {
-        const float* src = (const float*)__shfl_sync(0xffffffffu, (unsigned long long)kp, row);
-        if (src) {
-          const uint32_t dst = (uint32_t)__cvta_generic_to_shared(kr + row * pitch + c * 4);
-          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src + c * 4) : "memory");
+      const unsigned long long vp = (unsigned long long)(kp ? kp + (size_t)nkv * head_stride : nullptr);
+      float4 v[VB][DC];
+      auto values = [&](int j0) {
+#pragma unroll
+        for (int jj = 0; jj < VB; ++jj) {
+          const float* row = (const float*)__shfl_sync(0xffffffffu, vp, j0 + jj);      // warp-uniform
+#pragma unroll
+          for (int c = 0; c < DC; ++c) {
+            const int dim = (c * 32 + lane) * 4;
+            v[jj][c] = row && dim < d ? *reinterpret_cast<const float4*>(row + dim) : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
         }
-        row += row_step; c += c_step;
-        if (c >= d4) { c -= d4; ++row; }
-      }
-      asm volatile("cp.async.wait_all;\n" ::: "memory");
-      __syncwarp();
+      };
       float s[QT];
 #pragma unroll
       for (int q = 0; q < QT; ++q) s[q] = 0.f;
-#pragma unroll 4
-      for (int c = 0; c < d4; ++c) {
-        const float4 k4 = *reinterpret_cast<const float4*>(kr + lane * pitch + c * 4);
+      // 16 bytes of this lane's key, at `at`, for all queries
+      auto scores = [&](const float* at, int c) {
+        const float4 k4 = *reinterpret_cast<const float4*>(at);
 #pragma unroll
         for (int q = 0; q < QT; ++q) {
           const float4 q4 = *reinterpret_cast<const float4*>(qs + q * d + c * 4);
@@ -172,11 +182,63 @@ paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, c
           s[q] = fmaf(q4.z, k4.z, s[q]);
           s[q] = fmaf(q4.w, k4.w, s[q]);
         }
+      };
+      if constexpr (PIECES) {
+        const int pieces = (d4 + 7) / 8;
+        auto piece = [&](int i) {                               // 8 lanes bring 128 bytes of a row, four rows at a time
+          float* to = kr + (i & 1) * 32 * S32_PITCH + (lane & 7) * 4;
+          const int c = i * 8 + (lane & 7);
+#pragma unroll
+          for (int it = 0; it < 8; ++it) {
+            const int row = it * 4 + (lane >> 3);
+            const float* src = (const float*)__shfl_sync(0xffffffffu, (unsigned long long)kp, row);
+            if (src && c < d4) {
+              const uint32_t dst = (uint32_t)__cvta_generic_to_shared(to + row * S32_PITCH);
+              asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src + c * 4) : "memory");
+            }
+          }
+          asm volatile("cp.async.commit_group;\n" ::: "memory");
+        };
+        piece(0);
+#pragma unroll 1
+        for (int i = 0; i < pieces; ++i) {
+          if (i + 1 < pieces) {
+            piece(i + 1);
+            asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+          } else {
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+          }
+          __syncwarp();
+          const float* at = kr + (i & 1) * 32 * S32_PITCH + lane * S32_PITCH;
+          const int n = min(8, d4 - i * 8);
+#pragma unroll 4
+          for (int c = 0; c < n; ++c) scores(at + c * 4, i * 8 + c);
+          __syncwarp();                                         // the piece after the next overwrites this one
+        }
+      } else {
+        // 16 bytes per lane, row by row; lane's place moves on by 32 pieces at a time
+        for (int it = 0, row = lane / d4, c = lane % d4; it < d4; ++it) {
+          const float* src = (const float*)__shfl_sync(0xffffffffu, (unsigned long long)kp, row);
+          if (src) {
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(kr + row * pitch + c * 4);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src + c * 4) : "memory");
+          }
+          row += row_step; c += c_step;
+          if (c >= d4) { c -= d4; ++row; }
+        }
+        if (AHEAD) values(0);
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncwarp();
+#pragma unroll 4
+        for (int c = 0; c < d4; ++c) scores(kr + lane * pitch + c * 4, c);
       }
+      uint32_t sees = 0;                                        // the queries that see this lane's key
+      int p = p0, of = 0;
 #pragma unroll
       for (int q = 0; q < QT; ++q) {
-        const int p = p0 + q / nh;
         const bool seen = q < queries && kp && key <= p && (window <= 0 || key > p - window);
+        sees |= (seen ? 1u : 0u) << q;
+        if (++of == nh) { of = 0; ++p; }
         const float sv = seen ? s[q] * scale : -INFINITY;
         const float m_new = fmaxf(m[q], warp_max(sv));
         // nothing seen so far, or scores of minus infinity alone (a block of them may be all that this warp sees): no weight, nothing
@@ -190,40 +252,44 @@ paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, c
         ps[(warp * QT + q) * 32 + lane] = pj;
       }
       __syncwarp();
-      const int lo = max(first, b * 32), hi = min(last, b * 32 + 31);
-      // a row that some query does not see is left out of that query's sum, not added with weight 0
-      const bool all_see = hi <= p0 && (window <= 0 || lo > last - window);
-      const unsigned long long vp = (unsigned long long)(kp ? kp + (size_t)nkv * head_stride : nullptr);
-      constexpr int VB = 8 / DC;                                // rows of values requested at a time
 #pragma unroll 1
       for (int j0 = 0; j0 < 32; j0 += VB) {
-        float4 v[VB][DC];
+        if (!AHEAD) values(j0);
+        constexpr int G = VB < 4 ? VB : 4;                      // rows whose weights are read at once
 #pragma unroll
-        for (int jj = 0; jj < VB; ++jj) {
-          const float* row = (const float*)__shfl_sync(0xffffffffu, vp, j0 + jj);      // warp-uniform
+        for (int g = 0; g < VB; g += G) {
+          uint32_t row[G], any = 0, all = (1u << queries) - 1;
 #pragma unroll
-          for (int c = 0; c < DC; ++c) {
-            const int dim = (c * 32 + lane) * 4;
-            v[jj][c] = row && dim < d ? *reinterpret_cast<const float4*>(row + dim) : make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int jj = 0; jj < G; ++jj) {
+            row[jj] = __shfl_sync(0xffffffffu, sees, j0 + g + jj);
+            any |= row[jj];
+            all &= row[jj];
           }
-        }
+          if (!any) continue;                                   // warp-uniform
+          // a row that some query does not see is left out of that query's sum, not added with weight 0
+          auto add = [&](auto every) {
 #pragma unroll
-        for (int jj = 0; jj < VB; ++jj) {
-          const int kj = b * 32 + j0 + jj;
-          if (kj < lo || kj > hi) continue;                     // warp-uniform
+            for (int q = 0; q < QT; ++q) {
+              float pv[G];
+              const float* at = ps + (warp * QT + q) * 32 + j0 + g;
+              if constexpr (G == 4) *reinterpret_cast<float4*>(pv) = *reinterpret_cast<const float4*>(at);
+              else *reinterpret_cast<float2*>(pv) = *reinterpret_cast<const float2*>(at);
 #pragma unroll
-          for (int q = 0; q < QT; ++q) {
-            const int p = p0 + q / nh;
-            if (!all_see && (kj > p || (window > 0 && kj <= p - window))) continue;
-            const float pv = ps[(warp * QT + q) * 32 + j0 + jj];
+              for (int jj = 0; jj < G; ++jj) {
+                if (!decltype(every)::value && !((row[jj] >> q) & 1)) continue;
 #pragma unroll
-            for (int c = 0; c < DC; ++c) {
-              acc[q][c * 4] = fmaf(pv, v[jj][c].x, acc[q][c * 4]);
-              acc[q][c * 4 + 1] = fmaf(pv, v[jj][c].y, acc[q][c * 4 + 1]);
-              acc[q][c * 4 + 2] = fmaf(pv, v[jj][c].z, acc[q][c * 4 + 2]);
-              acc[q][c * 4 + 3] = fmaf(pv, v[jj][c].w, acc[q][c * 4 + 3]);
+                for (int c = 0; c < DC; ++c) {
+                  const float4 x = v[g + jj][c];
+                  acc[q][c * 4] = fmaf(pv[jj], x.x, acc[q][c * 4]);
+                  acc[q][c * 4 + 1] = fmaf(pv[jj], x.y, acc[q][c * 4 + 1]);
+                  acc[q][c * 4 + 2] = fmaf(pv[jj], x.z, acc[q][c * 4 + 2]);
+                  acc[q][c * 4 + 3] = fmaf(pv[jj], x.w, acc[q][c * 4 + 3]);
+                }
+              }
             }
-          }
+          };
+          if (all == (1u << queries) - 1) add(std::true_type());
+          else add(std::false_type());
         }
       }
       __syncwarp();                                             // the next block overwrites the keys and the weights
@@ -262,14 +328,21 @@ paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, c
   }
 }
 
-template <int QT, int DC, int W>
+template <int QT, int DC, int W, bool AHEAD = false>
 static int shared32_launch(const float* qkv, int row_stride, const float* pages, const int* block_tables, int bt_stride, const int* cu_q,
                            const int* seq_lens, float* out, int n_tokens, int n_req, int nq, int nkv, int d, int page_size, float scale,
                            int window, int tokens, int heads, cudaStream_t stream) {
-  const size_t smem = ((size_t)QT * d + W * QT * 34 + (size_t)W * 32 * (d + 4)) * sizeof(float);
-  IFB_ALLOW_SMEM((paged_attention_shared32_kernel<QT, DC, W>), smem);
+  const size_t keys = QT == 8 ? 64 * S32_PITCH : 32 * (size_t)(d + 4), sums = (size_t)QT * d;      // of a warp, in the same place
+  const size_t smem = ((size_t)QT * d + W * QT * 34 + W * (keys > sums ? keys : sums)) * sizeof(float);
+  IFB_ALLOW_SMEM((paged_attention_shared32_kernel<QT, DC, W, AHEAD>), smem);
   const int chunks = (nq / nkv + heads - 1) / heads;
-  return ifb_launch(paged_attention_shared32_kernel<QT, DC, W>, dim3((n_tokens + tokens - 1) / tokens, nkv * chunks), dim3(W * 32), smem,
+  // the values ahead take the registers of a second CTA per SM: where one has an SM to itself, for want of CTAs or of shared memory
+  // (16 heads of 64: 64 tokens at 300 keys, 1,024 CTAs, 73 us without, 111 so)
+  if constexpr (QT == 2 && DC == 1 && !AHEAD)
+    if ((long long)((n_tokens + tokens - 1) / tokens) * nkv * chunks <= S32_SMS || smem > 113 * 1024)
+      return shared32_launch<QT, DC, W, true>(qkv, row_stride, pages, block_tables, bt_stride, cu_q, seq_lens, out, n_tokens, n_req, nq, nkv, d,
+                                              page_size, scale, window, tokens, heads, stream);
+  return ifb_launch(paged_attention_shared32_kernel<QT, DC, W, AHEAD>, dim3((n_tokens + tokens - 1) / tokens, nkv * chunks), dim3(W * 32), smem,
                     stream, qkv, row_stride, pages, block_tables, bt_stride, cu_q, seq_lens, out, n_tokens, n_req, nq, nkv, d,
                     page_size, scale, window, tokens, heads);
 }

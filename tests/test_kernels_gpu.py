@@ -694,6 +694,14 @@ def test_plain_attention_of_a_query_is_the_same_in_every_step(K, nq, nkv, d, ps,
         assert torch.equal(alone[0], out[row])
 
 
+# Keys in pieces of 32 features (eight queries to a CTA) against whole rows (a single token's one, two and four): heads of one piece, of
+# whole pieces and of 4 features more or fewer, to four and eight pieces.
+@pytest.mark.parametrize("nq,nkv,d,ps,window", [(8, 2, 28, 16, 0), (8, 8, 32, 16, 40), (8, 4, 36, 8, 0), (16, 2, 64, 16, 33), (4, 4, 124, 16, 0),
+                                                (8, 2, 132, 16, 0), (4, 2, 160, 5, 31), (8, 1, 252, 16, 0)])
+def test_plain_attention_with_keys_in_pieces(K, nq, nkv, d, ps, window):
+    test_plain_attention_of_a_query_is_the_same_in_every_step(K, nq, nkv, d, ps, window)
+
+
 # Eight feature pairs per CTA: a k over 2,048 and more CTAs of sixteen pairs than SMs (38 heads of 128, 75 of 64); 37 heads and 74 lie
 # just below.  A last step of k of 8, rows 1 to 8.
 @pytest.mark.parametrize("n", [1, 3, 8])
