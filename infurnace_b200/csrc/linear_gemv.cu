@@ -380,7 +380,10 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
     const int n = item_n, m = item_m, tok = item_tok;
     const bool is_v = qk_is_v;
     const uint32_t rank = gv_cluster_rank(), peers = gv_cluster_size();
-    float sq = mine ? qk_y0 * qk_y0 + qk_y1 * qk_y1 : 0.f;
+    // (which product of a sum of two is rounded first is written out, here and in the rotation: left to the compiler it changed with
+    // code around it, and with it some bits of a step's keys)
+    float sq = 0.f;
+    if (mine) sq = STAGES > 1 ? fmaf(qk_y0, qk_y0, __fmul_rn(qk_y1, qk_y1)) : fmaf(qk_y1, qk_y1, __fmul_rn(qk_y0, qk_y0));
     if (EPI == 3) sq += __shfl_xor_sync(0xffffffffu, sq, 8);
     sq += __shfl_xor_sync(0xffffffffu, sq, 4);
     sq += __shfl_xor_sync(0xffffffffu, sq, 2);
@@ -400,7 +403,7 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
     }
     if (!is_v && qk.rope) {
       const float2 cs = pre_cs;
-      const float ra = a * cs.x - b * cs.y, rb = b * cs.x + a * cs.y;
+      const float ra = fmaf(a, cs.x, -__fmul_rn(b, cs.y)), rb = fmaf(a, cs.y, __fmul_rn(b, cs.x));
       a = ra; b = rb;
     }
     const bf16 oa = __float2bfloat16_rn(a), ob = __float2bfloat16_rn(b);

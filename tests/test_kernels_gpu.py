@@ -711,6 +711,48 @@ def test_qkv_product_of_eight_pairs_per_cta(K, n, nq, nkv, d, k, ps, norm, rotat
     test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, d, k, ps, norm, rotate, scaled)
 
 
+# The fused product's head norm and rotation, bit for bit by the order of operations that the kernel states: of two products that are
+# added, one is rounded first.  Rows of x with two powers of two make every feature an exact sum, squares that need rounding, and so many
+# values that another choice (it was once the compiler's) shows in several of them: 20 of 12.6 million.
+@pytest.mark.parametrize("n", [8, 16])
+@pytest.mark.parametrize("k", [1024, 2048, 3072])
+def test_qkv_product_rounds_the_products_that_it_states(K, n, k):
+    nq, nkv, d, rows, eps = 16, 8, 128, 4096, 1e-6
+    heads = nq + 2 * nkv
+    w = rnd((heads * d, k), torch.bfloat16, 41).cuda()
+    w = torch.where(w.abs() < 2.0 ** -4, 0.5, w.float()).clamp(-3, 3).bfloat16()
+    g = torch.Generator().manual_seed(42)
+    i = torch.randint(0, k, (rows,), generator=g)
+    j = (i + torch.randint(1, k, (rows,), generator=g)) % k
+    x = torch.zeros(rows, k)
+    x[torch.arange(rows), i], x[torch.arange(rows), j] = 1.0, 2.0 ** -7
+    x, qw, kw = x.bfloat16().cuda(), rnd((d,), torch.bfloat16, 43).cuda(), rnd((d,), torch.bfloat16, 44).cuda()
+    angles = rnd((rows, d // 2), torch.float32, 45, 3.0).cuda()
+    rope = torch.stack([angles.cos(), angles.sin()], -1).reshape(rows, d).contiguous()
+    got = torch.empty(rows, heads * d, dtype=torch.bfloat16, device="cuda")
+    for at in range(0, rows, n):
+        K.linear_qkv_rope_store(x[at:at + n], w, got[at:at + n], nq, nkv, d, qw, kw, eps, rope[at:at + n], None, None)
+
+    def fma(a, b, c):                                              # the product is exact in 64 bits
+        return (a.double() * b.double() + c.double()).float()
+    wf = w.double()
+    y = (wf[:, i] + wf[:, j] * 2.0 ** -7).t().float().view(rows, heads, 2, d // 2)      # exact
+    a, b = y[:, :nq + nkv, 0], y[:, :nq + nkv, 1]
+    sq = fma(a, a, b * b) if k > 2048 else fma(b, b, a * a)
+    sq = sq.view(rows, nq + nkv, d // 32, 16)                      # the 16 pairs of a CTA, then its peers in order
+    for step in (8, 4, 2, 1):
+        sq = sq[..., :step] + sq[..., step:]
+    total = sq[:, :, 0, 0]
+    for c in range(1, d // 32):
+        total = total + sq[:, :, c, 0]
+    rn = torch.rsqrt(total / d + eps)[:, :, None]
+    wt = torch.cat([qw.float().view(1, 1, 2, -1).expand(1, nq, 2, -1), kw.float().view(1, 1, 2, -1).expand(1, nkv, 2, -1)], 1)
+    a, b = a * (rn * wt[:, :, 0]), b * (rn * wt[:, :, 1])
+    cos, sin = angles.cos()[:, None], angles.sin()[:, None]
+    want = torch.stack([fma(a, cos, -(b * sin)), fma(a, sin, b * cos)], 2).bfloat16()
+    assert torch.equal(got.view(rows, heads, 2, d // 2)[:, :nq + nkv], want)
+
+
 # More than one tile of rows: the epilogue of the one-tile kernel with one head per tile (deep stages, then two CTAs per SM) and
 # with two, the last tile's second one missing where the heads are odd.
 @pytest.mark.parametrize("n", [129, 300, 700, 1300])
