@@ -962,15 +962,24 @@ class CudaKernels:
         reach = min(chunk, max_seq_len) if chunk else max_seq_len
         tiles = (-(-n // 16) + r) * -(-num_heads // 16)
         if max_q_len > 64:
-            # a prompt: tiles have 1 to `trips` tiles of 32 keys, the longest first, a CTA per SM.  The time is the longest share's or the
-            # sum of all over the SMs, whichever is more, and the merge's, in trips of some 5 us: a CTA takes 1.6 to begin
-            # and end, the merge 0.8 and what it reads.  Over 25 sets of lengths within 8 % of the best of 1 to 12 (16 heads of 64, us: 2,048
-            # tokens, chunks of 512, two shares 63, one 90, four 74; 4,096 one 96, two 120, four 140; 300 five 20, two 33)
-            trips = -(-reach // 32)
+            # A prompt, the tiles with the most keys first.  The time is the longest share's or all shares' over the places of the device,
+            # whichever is more, and the merge's, in trips of 32 keys: a CTA takes 2 to begin and end, a request has one tile with
+            # as many trips as there are and 0.45 of them in each 16 of its tokens (half of them where they are its own).  CTAs of four warps
+            # (up to 4 heads) share an SM by three.  A trip takes some 2.4, 3.3 and 5.1 us with 4, 8 and 16 warps, the merge 1 us for a
+            # million numbers.  ``max_seq_len`` is a power of two in the step function; a lone prompt that brings half of it or more is taken
+            # to be new.  Over 464 sets, 2 to 32 heads of 16 to 128, 1 to 16 prompts of 66 to 2,048 tokens, some continued or beside decoding
+            # requests: within 1.7 % of the best of 1 to 8 on average.  Us at 16 heads of 64, chunks of 512: 2,048 tokens two shares 63, one
+            # 91, four 74; 400 tokens seven 21, four 29.  4 heads: 2,048 tokens four 22, two 31.  32 heads, 200 tokens beside 7 decoding: four
+            # 41, six 47
+            if r == 1 and 2 * max_q_len >= max_seq_len:
+                reach = min(reach, max_q_len)
+            trips, groups = -(-reach // 32), -(-num_heads // 16)
+            places, trip_us = (3 * self.sm_count, 2.4) if num_heads <= 4 else (self.sm_count, 3.3 if num_heads <= 8 else 5.1)
 
             def cost(s):
-                longest, work = 1.6 + -(-trips // s), tiles * s / self.sm_count * (1.6 + (trips + 1) / (2 * s))
-                return max(longest, work) + (0.8 + n * num_heads * head_dim * s / 5.12e6 if s > 1 else 0)
+                longest = 2 + -(-trips // s)
+                work = groups * s / places * (-(-n // 16) * (2 + 0.45 * (trips + 1) / s) + r * (2 + trips / s))
+                return max(longest, work) + (n * num_heads * head_dim * s / (1e6 * trip_us) if s > 1 else 0)
             return min(range(1, min(8, trips) + 1), key=cost)
         if max_q_len == 1:
             # decoded tokens: a tile of 32 keys is a chain of round trips (some 5 us), so every tile gets a CTA of its own

@@ -228,3 +228,22 @@ def test_the_new_parts_in_another_arrangement():
     got = torch.cat([runner.step([StepEntry("a", toks[:13], list(range(13)))]).clone(),
                      runner.step([StepEntry("a", toks[13:], list(range(len(toks) - 13)))]).clone()]).double()
     assert (got - want).abs().max() < TOL
+
+
+def test_shares_of_a_prompts_keys():
+    """The rule as the step function asks it, which knows the longest request as a power of two of at least 256: more shares for fewer
+    tiles, never more than tiles of keys or eight; more where several CTAs share an SM; a prompt that fills the device takes its tiles
+    whole; a lone prompt's own length counts and not the power of two; requests that decode beside a prompt bring whole tiles of keys."""
+    from types import SimpleNamespace
+    from infurnace_b200.kernels.cuda import CudaKernels
+
+    def shares(heads, lens, new=None, chunk=512):
+        new, bucket = new or lens, 256
+        while bucket < max(lens):
+            bucket *= 2
+        return CudaKernels._talk_splits(SimpleNamespace(sm_count=148), sum(new), len(lens), heads, 64, chunk, max(new), bucket)
+    assert [shares(16, [n]) for n in (130, 300, 400, 600, 1100, 1400, 2048, 4096, 8192)] == [5, 5, 7, 6, 4, 3, 2, 1, 1]
+    assert [shares(4, [n]) for n in (512, 1215, 2048)] == [8, 8, 4] and shares(4, [147, 681, 1215]) == 4
+    assert shares(16, [147, 681, 1215]) == 2 and shares(16, [100] * 16) == 2
+    assert shares(32, [200] + [400] * 7, [200] + [1] * 7) == 4 and shares(32, [70] + [700] * 15, [70] + [1] * 15, 0) == 4
+    assert shares(16, [2048], chunk=128) == 1 and shares(16, [30000], [512], 0) == 8 and shares(16, [66], chunk=32) == 1

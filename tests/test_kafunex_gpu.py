@@ -313,13 +313,6 @@ def test_talking_attention_takes_the_longest_tiles_first(K, H, G, splits, cases,
     close(got, want, 0.06, f"{H} heads, {len(cases)} requests")
 
 
-def test_shares_of_a_prompts_keys(K):
-    """More shares for fewer tiles, never more than tiles of keys or eight; a prompt that fills the device takes its tiles whole."""
-    rule = lambda n, chunk, length, r=1: K._talk_splits(n, r, 16, 64, chunk, length, length)
-    assert [rule(n, 512, n) for n in (80, 300, 600, 1100, 1400, 2048, 4096, 8192)] == [3, 5, 6, 4, 3, 2, 1, 1]
-    assert rule(2048, 128, 2048) == 1 and rule(1600, 512, 100, 16) == 1 and rule(512, 0, 30000) == 8
-
-
 def test_a_nan_among_the_values_of_far_keys_reaches_the_output_of_split_keys(K):
     """Where one key's score is so far above the others that their weights are 0, their values still count: 0 times NaN."""
     for key, d in ((40, 64), (200, 16)):
