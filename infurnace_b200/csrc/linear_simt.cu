@@ -164,7 +164,7 @@ rows32_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __re
 // groups' tiles then meet in the two CTAs' shared memory, each CTA adding half of the tile's rows.  EPI 1: the tile's first 32 rows of w are gate rows, the others the up rows of the same features.
 // ALONE: where tiles are more than the pairs of SMs, a CTA takes a whole tile, each slice two groups one after the other in one run
 // through its ring (of three stages; the first group's tile waits beside it).  Filling the ring and the sum at the end cost a CTA
-// of a pair 17,000 of 37,000 cycles at a k of 1,024: 2,048 rows of 4,096 x 1,024 535 to 424 us (40 TFLOP/s), 193 rows of the LM head 2,371 to 1,830.
+// of a pair 17,000 of 37,000 cycles at a k of 1,024: 2,048 rows of 4,096 x 1,024 535 to 424 us (40 TFLOP/s), 193 rows of the LM head 2,371 to 1,837.
 // RT: rows per thread, and an eighth of a tile's (tile32_form).
 // ---------------------------------------------------------------------------------------------------
 constexpr int T32 = 64, T32_SLICES = S32_GROUPS / 2, T32_PITCH = S32_BK + 4;      // 20 floats: conflict-free 16-byte reads
@@ -356,40 +356,56 @@ static int tile32_launch_as(const float* x, const float* w, TO* out, int n, int 
 }
 
 // Rows per thread (a tile has eight times as many) and whether a CTA takes a tile alone: the form whose waves should take least
-// time, by the time of one wave at a k of 1,024 (in tenths of a microsecond, measured over matrices of 1,024 to 40,000 features, 17 to 193
-// rows; a longer k scales them alike).  17 rows 18.8 to 11.5 us for 4,096 x 1,024 and 31.9 to 16.4 for 1,024 x 2,048 against tiles of 64
-// rows by pairs, 193 rows 72 to 59 and 33.5 to 31.3.  The sums are the same in every form.
-static void tile32_form(int n, int tiles, int* rows, bool* alone) {
-  static const int wave[2][9] = {{0, 0, 98, 117, 127, 148, 168, 180, 196}, {0, 0, 146, 201, 218, 240, 295, 289, 310}};
-  long long least = 0;
-  for (int rt = 8; rt >= 2; --rt) {
+// time, a wave taking so many tenths of a microsecond and so many more for each 1,024 of k: what two CTAs share of a tile, filling the rings and
+// the sum at the end, is most of a short k and little of a long one.  Over 66 products of 17 to 2,048 rows at each k of 256 to 4,096 within 0.2 % of the best
+// form on average (0.6 to 2.5 % by the times of a k of 1,024 alone, which gave 300 rows of 2,500 x 4,096 203 us, now 182).  17 rows 18.8
+// to 11.5 us for 4,096 x 1,024 and 31.9 to 16.4 for 1,024 x 2,048 against tiles of 64 rows by pairs, 193 rows 72 to 59 and 33.5 to 31.3.  The sums
+// are the same in every form.  least: the fewest rows per thread that are compiled; vec: rows at 16 bytes.
+static void tile32_form(int n, int k, int tiles, int sms, bool vec, int least, int* rows, bool* alone) {
+  struct Wave { int begin, per_k; };                             // (six rows alone never take less than seven)
+  static const Wave waves[2][9] = {{{0, 0}, {0, 0}, {30, 59}, {34, 74}, {35, 81}, {41, 100}, {40, 118}, {48, 127}, {47, 142}},
+                                   {{0, 0}, {0, 0}, {26, 113}, {24, 166}, {27, 184}, {33, 205}, {0, 0}, {42, 252}, {49, 266}}};
+  static const Wave scalar[2] = {{56, 222}, {44, 462}};
+  long long best = 0;
+  for (int rt = 8; rt >= least; --rt) {
     const long long all = (long long)tiles * ((n + 8 * rt - 1) / (8 * rt));
     for (int a = 0; a < 2; ++a) {
-      const int slots = a ? T32_SMS : T32_SMS / 2;
-      const long long time = (all + slots - 1) / slots * wave[a][rt];
-      if (!least || time < least) { least = time; *rows = rt; *alone = a; }
+      const Wave w = vec ? waves[a][rt] : scalar[a];
+      if (!w.per_k) continue;
+      const int slots = a ? sms : sms / 2 > 1 ? sms / 2 : 1;
+      const long long time = (all + slots - 1) / slots * (w.begin * 1024LL + (long long)w.per_k * k);
+      if (!best || time < best) { best = time; *rows = rt; *alone = a; }
     }
   }
 }
+// Rows not at 16 bytes and bfloat16 outputs are rare: eight rows per thread.  So are more tiles of 16 rows than a grid holds.
+static int tile32_least(int n, bool vec, size_t out_size) { return vec && out_size == 4 && n <= 65535 * 16 ? 2 : 8; }
 template <int EPI, bool VEC, typename TO>
 static int tile32_launch(const float* x, const float* w, TO* out, int n, int o, int k, int unary, const float* bias, cudaStream_t s) {
   const int fo = EPI ? T32 / 2 : T32;
   int rows = 8;
   bool alone = false;
-  tile32_form(n, (o + fo - 1) / fo, &rows, &alone);
+  tile32_form(n, k, (o + fo - 1) / fo, T32_SMS, VEC, tile32_least(n, VEC, sizeof(TO)), &rows, &alone);
 #define IFB_T32(RT) \
   case RT: return alone ? tile32_launch_as<EPI, VEC, true, RT, TO>(x, w, out, n, o, k, unary, bias, s) \
                         : tile32_launch_as<EPI, VEC, false, RT, TO>(x, w, out, n, o, k, unary, bias, s);
-  if constexpr (VEC && sizeof(TO) == 4) {                        // rows not at 16 bytes, and bfloat16 outputs, are rare: eight rows per thread
-    if (n <= 65535 * 16)                                         // tiles of rows that a grid holds
-      switch (rows) {
-        IFB_T32(2) IFB_T32(3) IFB_T32(4) IFB_T32(5) IFB_T32(7)
-        case 6: return tile32_launch_as<EPI, VEC, false, 6, TO>(x, w, out, n, o, k, unary, bias, s);      // alone, seven take less
-      }
-  }
-  switch (8) { IFB_T32(8) }
+  if constexpr (VEC && sizeof(TO) == 4)
+    switch (rows) {
+      IFB_T32(2) IFB_T32(3) IFB_T32(4) IFB_T32(5) IFB_T32(7)
+      case 6: return tile32_launch_as<EPI, VEC, false, 6, TO>(x, w, out, n, o, k, unary, bias, s);      // alone, seven take less
+    }
+  switch (rows) { IFB_T32(8) }
 #undef IFB_T32
   return IFB_ERR_ARG;
+}
+// The form of a product of more than S32_FEW_ROWS rows, for tests: twice the rows per thread, and 1 more where a CTA takes a tile alone.
+// vec: rows at 16 bytes; sms: of the device.
+IFB_EXPORT int ifb_linear_float32_form(int n_rows, int out_features, int k_dim, int epilogue, int vec, int out_dtype, int sms) {
+  const int fo = (epilogue & 15) ? T32 / 2 : T32;
+  int rows = 0;
+  bool alone = false;
+  tile32_form(n_rows, k_dim, (out_features + fo - 1) / fo, sms, vec != 0, tile32_least(n_rows, vec != 0, out_dtype == IFB_F32 ? 4 : 2), &rows, &alone);
+  return 2 * rows + alone;
 }
 
 // Float32 operands.  Up to S32_FEW_ROWS rows the weights are streamed once per eight rows (from the second time on out of

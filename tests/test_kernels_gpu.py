@@ -662,12 +662,35 @@ def test_plain_product_of_a_row_is_the_same_in_every_batch(K, n, o, k, epilogue)
 
 # The product of many rows in all its forms: tiles of 16 to 64 rows (every number of rows per thread, full and with one row of the
 # last tile), by pairs of CTAs and by one (from 2,000 features on), k ranges that end in a slice's first group, in its
-# second and in a later slice.
-@pytest.mark.parametrize("n", [17, 18, 24, 25, 33, 41, 49, 57, 65, 113, 193])
-@pytest.mark.parametrize("o,k", [(65, 272), (2000, 24), (4800, 136), (9600, 36), (4760, 16)])
+# second and in a later slice.  The forms that only a longer k takes are in LONGER; tests/test_float32_forms.py holds that none is missing.
+MANY_ROWS, MANY_ROWS_OF = [17, 18, 24, 25, 33, 41, 49, 57, 65, 113, 193], [(65, 272), (2000, 24), (4800, 136), (9600, 36), (4760, 16)]
+LONGER = [(17, 3600, 1044), (33, 2500, 1044), (25, 3600, 1044), (33, 3600, 1044), (41, 3600, 1044), (49, 3600, 1044), (57, 3600, 1044)]
+
+
+@pytest.mark.parametrize("n", MANY_ROWS)
+@pytest.mark.parametrize("o,k", MANY_ROWS_OF)
 @pytest.mark.parametrize("epilogue", ["none", "silu_gate"])
 def test_plain_product_of_many_rows(K, n, o, k, epilogue):
     test_plain_product_of_a_row_is_the_same_in_every_batch(K, n, o, k, epilogue)
+
+
+@pytest.mark.parametrize("n,o,k", LONGER)
+@pytest.mark.parametrize("epilogue", ["none", "silu_gate"])
+def test_plain_product_of_many_rows_and_a_longer_k(K, n, o, k, epilogue):
+    test_plain_product_of_a_row_is_the_same_in_every_batch(K, n, o, k, epilogue)
+
+
+# Eight rows per thread alone: rows not at 16 bytes, by pairs of CTAs and by one, and bfloat16 outputs, which are the float32 ones rounded.
+@pytest.mark.parametrize("n,o,k", [(49, 2500, 1041), (41, 9600, 37)])
+@pytest.mark.parametrize("epilogue", ["none", "silu_gate"])
+def test_plain_product_of_many_rows_by_single_copies_and_to_bfloat16(K, n, o, k, epilogue):
+    test_plain_product_of_a_row_is_the_same_in_every_batch(K, n, o, k, epilogue)
+    k -= 1
+    x, w = rnd((n, k), torch.float32, 91).cuda(), rnd((2 * o if epilogue != "none" else o, k), torch.float32, 92).cuda()
+    out, half = torch.empty((n, o), device="cuda"), torch.empty((n, o), dtype=torch.bfloat16, device="cuda")
+    K.linear(x, w, out, epilogue)
+    K.linear(x, w, half, epilogue)
+    assert torch.equal(half, out.bfloat16())
 
 
 # Plain attention in float32 storage: a query's bits do not depend on the other queries of the step, and rows that it may
