@@ -100,7 +100,6 @@ paged_attention_simt_kernel(const T* __restrict__ qkv, int row_stride, const T* 
 // tokens 546 to 292).  Two queries and a CTA to an SM (AHEAD; a decoded token): whole rows at once, and all of a block's values are requested
 // before its scores are formed, as a warp has one block or two and its time is that chain (9.8 to 8.2 us).
 // ---------------------------------------------------------------------------------------------------
-constexpr int S32_SMS = 148;                                    // SMs of a B200
 constexpr int S32_PITCH = 36;                                   // floats of a row of a piece: 16-byte reads without conflicts
 template <int QT, int DC, int W, bool AHEAD>
 __global__ void __launch_bounds__(W * 32, AHEAD ? 1 : W == 8 ? 2 : QT == 8 ? 3 : 4)
@@ -339,7 +338,7 @@ static int shared32_launch(const float* qkv, int row_stride, const float* pages,
   // the values ahead take the registers of a second CTA per SM: where one has an SM to itself, for want of CTAs or of shared memory
   // (16 heads of 64: 64 tokens at 300 keys, 1,024 CTAs, 73 us without, 111 so)
   if constexpr (QT == 2 && DC == 1 && !AHEAD)
-    if ((long long)((n_tokens + tokens - 1) / tokens) * nkv * chunks <= S32_SMS || smem > 113 * 1024)
+    if ((long long)((n_tokens + tokens - 1) / tokens) * nkv * chunks <= ifb_sm_count() || smem > 113 * 1024)
       return shared32_launch<QT, DC, W, true>(qkv, row_stride, pages, block_tables, bt_stride, cu_q, seq_lens, out, n_tokens, n_req, nq, nkv, d,
                                               page_size, scale, window, tokens, heads, stream);
   return ifb_launch(paged_attention_shared32_kernel<QT, DC, W, AHEAD>, dim3((n_tokens + tokens - 1) / tokens, nkv * chunks), dim3(W * 32), smem,

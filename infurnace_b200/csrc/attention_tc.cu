@@ -832,12 +832,7 @@ IFB_EXPORT int ifb_attention_tc(const void* qkv, int row_stride, const void* k_p
   }
   IFB_ALLOW_SMEM(attn_tile_tc_kernel, SMEM_BYTES);
   const long long items = (long long)((max_q_len + tpt - 1) / tpt) * nkv;      // of the longest request
-  static int sm_count = 0;
-  if (!sm_count) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sm_count = 1;
-  }
+  const int sm_count = ifb_sm_count();
   constexpr float LOG2E = 1.4426950408889634f;
   TcScore score = {scale * LOG2E, 0.f, 0.f, 0.f};
   if (SOFTCAP) {

@@ -78,6 +78,18 @@ static inline bool ifb_pdl_enabled() {
     }                                                                                                                   \
   } while (0)
 
+// SMs of the current device, which the rules that spread work go by (1 where it cannot be asked).
+static inline int ifb_sm_count() {
+  static int known[IFB_MAX_DEVICES] = {};
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= IFB_MAX_DEVICES) return 1;
+  if (!known[dev]) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) return 1;
+    known[dev] = n;
+  }
+  return known[dev];
+}
+
 // early: whether this launch may be scheduled before its predecessor has finished.  A kernel that lives on its bytes in
 // flight is better off without: launched early, its CTAs sit on registers and shared memory of SMs where the
 // predecessor still has CTAs to place, and at these sizes the launch latency that the overlap hides is small change.

@@ -15,7 +15,6 @@
 
 typedef __nv_bfloat16 bf16;
 constexpr int GV_ROWS = 16;
-constexpr int GV_SMS = 148;
 // CTAs per SM asked of the compiler for the plain one-stage kernel of 8 warps and one block of tokens (the LM head of a
 // small model, 9,496 CTAs): with 80 registers three fit and the 311 MB stream at 5.8 to 6.3 TB/s; with the 103 the
 // compiler took unasked two fit (4.8 to 5.0 TB/s), with four (64 registers, spills) it is slower again.
@@ -429,16 +428,10 @@ linear_gemv_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, TO* _
 // 0.802 to 0.787 ms at one row; with 2, 4 and 8 rows the 128 CTAs' reads of the rows outweigh it (0.894 to 0.948,
 // 1.020 to 1.117, 1.314 to 1.374 ms), so those keep 16.
 static int gv_features_per_cta(int o, int n_rows) {
-  static int sm_count = 0;
-  if (!sm_count) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sm_count = 1;
-  }
   static int forced = -1;                    // IFB_GV_FEAT=16 keeps tiles of 16 (for measurements)
   if (forced < 0) { const char* v = getenv("IFB_GV_FEAT"); forced = v ? atoi(v) : 0; }
   if (forced == 16 || n_rows > 1) return GV_ROWS;
-  return 2 * ((o + GV_ROWS - 1) / GV_ROWS) <= sm_count ? 8 : GV_ROWS;
+  return 2 * ((o + GV_ROWS - 1) / GV_ROWS) <= ifb_sm_count() ? 8 : GV_ROWS;
 }
 
 template <int NB, int EPI, int WARPS, typename TO, int STAGES = 1>
@@ -592,7 +585,7 @@ IFB_EXPORT int ifb_linear_gemv_qkv(const void* x, const void* w, void* qkv, int 
   const int nb = n_rows <= 8 ? 1 : 2;
   // A long k, one block of tokens, and more CTAs of 16 pairs (of which an SM holds one) than SMs: 8 pairs, two CTAs per SM (48 heads of
   // 4,096, 192 CTAs: 19.1 to 16.7 us for eight rows, 18.5 to 15.5 for one; 56 of 5,120 23.4 to 20.1; 28 of 3,072, 112 CTAs, 7.1 to 7.7: not).
-  if (k_dim > 2048 && nb == 1 && head_dim <= 128 && (long long)(nq + 2 * nkv) * (head_dim / 32) > GV_SMS)
+  if (k_dim > 2048 && nb == 1 && head_dim <= 128 && (long long)(nq + 2 * nkv) * (head_dim / 32) > ifb_sm_count())
     return gv_launch_qkv<1, 8, 2, 5>(x, w, qkv, n_rows, k_dim, rs, qk, stream);
   if (k_dim <= 1024) return nb == 1 ? gv_launch_qkv<1, 8, 1>(x, w, qkv, n_rows, k_dim, rs, qk, stream)
                                     : gv_launch_qkv<2, 8, 1>(x, w, qkv, n_rows, k_dim, rs, qk, stream);

@@ -170,7 +170,6 @@ rows32_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __re
 constexpr int T32 = 64, T32_SLICES = S32_GROUPS / 2, T32_PITCH = S32_BK + 4;      // 20 floats: conflict-free 16-byte reads
 constexpr int T32_STAGE = 2 * T32 * T32_PITCH;                                    // floats: the rows of x, then those of w
 constexpr int T32_LANES = 64, T32_TO = 8, T32_J = T32 / T32_TO;                   // threads of a slice, across features; features per thread
-constexpr int T32_SMS = 148;                                                     // of the device that the choice of a form is for
 constexpr int T32_RED = T32 + 8;                                                  // floats per row of a group's tile
 template <bool ALONE> struct Tile32 {
   static constexpr int STAGES = ALONE ? 3 : 4;
@@ -385,7 +384,7 @@ static int tile32_launch(const float* x, const float* w, TO* out, int n, int o, 
   const int fo = EPI ? T32 / 2 : T32;
   int rows = 8;
   bool alone = false;
-  tile32_form(n, k, (o + fo - 1) / fo, T32_SMS, VEC, tile32_least(n, VEC, sizeof(TO)), &rows, &alone);
+  tile32_form(n, k, (o + fo - 1) / fo, ifb_sm_count(), VEC, tile32_least(n, VEC, sizeof(TO)), &rows, &alone);
 #define IFB_T32(RT) \
   case RT: return alone ? tile32_launch_as<EPI, VEC, true, RT, TO>(x, w, out, n, o, k, unary, bias, s) \
                         : tile32_launch_as<EPI, VEC, false, RT, TO>(x, w, out, n, o, k, unary, bias, s);

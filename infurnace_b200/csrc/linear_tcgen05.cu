@@ -1566,22 +1566,13 @@ static int tc_launch_cfg(const void* x, const void* w, void* out, int n, int o, 
 // The shape of the tiles: a wave of wide tiles does four 128 x 128 products per SM in little more time than a wave of
 // narrow tiles (two CTAs per SM) does two, but only if there are enough wide tiles to fill the SMs.  shape: 0 chooses
 // (see below), 1 narrow, 2 deep, 3 wide, 4 and 5 persistent, 6 the pairs (for tests and measurements).
-static int tc_sm_count() {
-  static int sm_count = 0;
-  if (!sm_count) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sm_count = 1;
-  }
-  return sm_count;
-}
 // By measurement.  With the silu_gate epilogue: tiles of 64 features (64 gate and 64 up rows, one tile per CTA, a deep ring) where
 // they are no more than the SMs: twice the SMs of tiles of 128, each with two thirds of the bytes.  Else the persistent kernel (its tile already accumulates 256 columns per
 // product, and the heavy epilogue of one tile runs beside the products of the next).  Otherwise one tile per CTA:
 // the wide shape when there are enough wide tiles to fill the SMs (a 256 x 256 tile reads half the operand bytes
 // per product from shared memory, which is what bounds these kernels), else the deep or the narrow one.
 static int tc_pick_shape(int epi, int n, int o) {
-  const int sm_count = tc_sm_count();
+  const int sm_count = ifb_sm_count();
   if (epi) return (long long)((o + 63) / 64) * ((n + G_BM - 1) / G_BM) <= sm_count ? 7 : 4;
   const long long tn = (long long)((o + 127) / 128) * ((n + G_BM - 1) / G_BM);
   const long long tw = (long long)((o + 255) / 256) * ((n + 2 * G_BM - 1) / (2 * G_BM));
@@ -1594,7 +1585,7 @@ static int tc_pick_shape(int epi, int n, int o) {
 // norm must agree with the launch): from 513 rows on (up to 512 few tiles share their k range in clusters), where its own tiles keep
 // most pairs busy (four fifths over all rounds).
 // `pairs`: of SMs; 0 where the device cannot run the largest of their kernels, or there is none: never.
-static int tc_device_pairs() { return tc_pairs<PairCfg<0, 128, 6, true>, bf16>() > 0 ? tc_sm_count() / 2 : 0; }
+static int tc_device_pairs() { return tc_pairs<PairCfg<0, 128, 6, true>, bf16>() > 0 ? ifb_sm_count() / 2 : 0; }
 static int tc_pair_rounds(int pairs, int n, int o, int features) {
   const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
   return (int)((tiles + pairs - 1) / pairs);
@@ -1669,8 +1660,8 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
     if constexpr (EPI) return tc_launch_cfg<GemmCfg<1, 1, 128, 6>, TO>(x, w, out, n, o, k, err, s, fold);
     return IFB_ERR_ARG;
   }
-  if (shape == 5 && !EPI) return tc_launch_persistent<P256, TO>(x, w, out, n, o, k, err, tc_sm_count(), s, fold);
-  if (shape == 4 || shape == 5) return tc_launch_persistent<P128, TO>(x, w, out, n, o, k, err, tc_sm_count(), s, fold);
+  if (shape == 5 && !EPI) return tc_launch_persistent<P256, TO>(x, w, out, n, o, k, err, ifb_sm_count(), s, fold);
+  if (shape == 4 || shape == 5) return tc_launch_persistent<P128, TO>(x, w, out, n, o, k, err, ifb_sm_count(), s, fold);
   if (shape == 3) return tc_launch_cfg<Wide, TO>(x, w, out, n, o, k, err, s, fold);
   if (shape == 2) return tc_launch_cfg<Deep, TO>(x, w, out, n, o, k, err, s, fold);
   return tc_launch_cfg<Narrow, TO>(x, w, out, n, o, k, err, s, fold);

@@ -30,3 +30,12 @@ def test_only_constants_are_read_through_the_read_only_path():
                 for m in re.finditer(r"__ldg\(([^)]*)", line):
                     if not m.group(0).endswith("(__ldg"):
                         assert re.search(r"bias|conv_w", m.group(1)), (os.path.basename(path), line)
+
+
+def test_the_number_of_sms_is_asked_of_the_device_in_one_place():
+    """A rule that spreads work goes by the SMs of the device it runs on, not by a number written down."""
+    for path in glob.glob(os.path.join(CSRC, "*.c*")) + glob.glob(os.path.join(CSRC, "*.h")):
+        with open(path, encoding="utf-8") as f:
+            text = f.read()
+        assert not re.search(r"\w*SMS?\w*\s*=\s*1\d\d\b", text), os.path.basename(path)
+        assert ("cudaDevAttrMultiProcessorCount" in text) == (os.path.basename(path) == "common.cuh"), os.path.basename(path)
