@@ -93,12 +93,15 @@ paged_attention_simt_kernel(const T* __restrict__ qkv, int row_stride, const T* 
 // lane owns a key: the block goes through shared memory (rows padded by 16 bytes: conflict-free 16-byte reads) and each
 // 16 bytes of it serve all queries; for the weighted sum a lane owns 4 (or 8) elements of the head and reads whole rows
 // of values.  What bounds it is the chain of round trips of a block for few keys, and shared-memory reads for many.
-// Measured in a step of the 0.6B sizes at 195 keys: one token 155 to about 10 us per layer, 193 tokens 156 to 60 us, against a warp
-// per query and head that read keys with a stride of a row.
-// Eight queries (a prompt): the keys of a block come in pieces of 32 features, one piece ahead of the one that is being used, which takes a
-// third of whole rows' shared memory and lets two CTAs share an SM, and which queries see a row is a bit each, found with the scores (193 tokens, 392 CTAs: 52 to 34 us; 1,000
-// tokens 546 to 292).  Two queries and a CTA to an SM (AHEAD; a decoded token): whole rows at once, and all of a block's values are requested
-// before its scores are formed, as a warp has one block or two and its time is that chain (9.8 to 8.2 us).
+// Eight queries (a prompt): the keys of a block come in pieces of 32 features, one piece ahead of the one that is being used: 9 KB of a warp
+// whatever the head (whole rows take 16.5 KB at 128, 33 at 256, and 8.5 at 64 and less), so that two CTAs share an SM, and which queries see a
+// row is a bit each, found with the scores.  Heads of 64 and less gain nothing in memory and as much in time by it.  Two queries and a CTA to an
+// SM (AHEAD; a decoded token): whole rows at once, and all of a block's values are requested before its scores are formed, as a warp has one block or
+// two and its time is that chain.  The registers that the CTAs of an SM leave do not hold all: eight queries spill 76 bytes (128 registers), with
+// heads above 128 104 bytes (168), four queries with such heads 12.
+// Us, 16 heads over 8, whole rows and now: 193 tokens 43 to 26 at heads of 64, 52 to 34 at 128, 83 to 44 at 192, 129 to 51 at 256; 1,000 tokens 446
+// to 222, 540 to 291, 801 to 450, 1,444 to 524; one token at 195 keys 8.7 to 7.1, 10.0 to 8.3, 22.8 to 17.9, 24.8 to 20.1.  (A warp per query and
+// head that read keys with a stride of a row took 156 for the 193 tokens and 155 for the one, at 128.)
 // ---------------------------------------------------------------------------------------------------
 constexpr int S32_PITCH = 36;                                   // floats of a row of a piece: 16-byte reads without conflicts
 template <int QT, int DC, int W, bool AHEAD>
@@ -254,7 +257,8 @@ paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, c
 #pragma unroll 1
       for (int j0 = 0; j0 < 32; j0 += VB) {
         if (!AHEAD) values(j0);
-        constexpr int G = VB < 4 ? VB : 4;                      // rows whose weights are read at once
+        constexpr int G = 4;                                    // rows whose weights are read at once
+        static_assert(VB % G == 0, "whole groups of rows");
 #pragma unroll
         for (int g = 0; g < VB; g += G) {
           uint32_t row[G], any = 0, all = (1u << queries) - 1;
@@ -271,8 +275,7 @@ paged_attention_shared32_kernel(const float* __restrict__ qkv, int row_stride, c
             for (int q = 0; q < QT; ++q) {
               float pv[G];
               const float* at = ps + (warp * QT + q) * 32 + j0 + g;
-              if constexpr (G == 4) *reinterpret_cast<float4*>(pv) = *reinterpret_cast<const float4*>(at);
-              else *reinterpret_cast<float2*>(pv) = *reinterpret_cast<const float2*>(at);
+              *reinterpret_cast<float4*>(pv) = *reinterpret_cast<const float4*>(at);
 #pragma unroll
               for (int jj = 0; jj < G; ++jj) {
                 if (!decltype(every)::value && !((row[jj] >> q) & 1)) continue;
