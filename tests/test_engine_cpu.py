@@ -334,11 +334,14 @@ def test_a_fault_recorded_on_the_device_fails_the_requests_that_ran(models):
     assert len(eng.generate([[7, 8, 9]], SamplingParams(max_tokens=4))[0]) == 4
 
 
-def test_staged_tables_follow_their_requests(models):
+# B has two key/value groups, B0 one: its tables reach the device in one copy with the step's tokens.
+@pytest.mark.parametrize("name", ["B0", "B"])
+def test_staged_tables_follow_their_requests(models, name):
     """A staging set keeps the block tables that its rows held two steps ago and writes only what is new: requests that change rows,
     end, start again under an old id, or lose the pages of a step that failed and get others must all be seen as they are."""
     import random
-    eng = engine(models["B"], "B", max_num_batched_tokens=64, max_num_seqs=4)
+    eng = engine(models[name], name, max_num_batched_tokens=64, max_num_seqs=4)
+    assert len(eng.runner.cache.kv_groups) == {"B0": 1, "B": 2}[name]
     run, cache, rng = eng.runner, eng.runner.cache, random.Random(3)
     real = run.model.forward
 
