@@ -993,6 +993,16 @@ static int att_max_clusters(int splits) {
   return known[dev][splits];
 }
 
+// Whether the decoding requests of a step with prompts run the longest contexts first: where their CTAs are more than the SMs that the prompts'
+// items leave hold, two each, so that some wait for others to end.  Where all find a place finding the request costs half a microsecond a
+// layer for nothing (3 requests beside a portion of 65 tokens, 256 CTAs for 264 places: two steps of the 0.6B sizes 2,350 us in order, 2,324 not).
+// (A grid of decoding requests alone that is more than the SMs hold gains nothing by it: 64 requests of 129 to 383 keys 1,387 to
+// 1,435 us a step.)
+IFB_EXPORT int ifb_attention_mma_ordered(int n_req, int nq, int nkv, int num_splits, int max_q_len, int sms) {
+  const long long items = ((long long)max_q_len * (nq / nkv) + 127) / 128 * nkv, left = items < sms ? sms - items : 0;
+  return n_req > 1 && n_req <= WS_ORDERED && (long long)num_splits * nkv * n_req > 2 * left;
+}
+
 template <bool TMA>
 static int att_launch(const AttArgs& a, cudaStream_t stream) {
   if (TMA) IFB_ALLOW_SMEM(attn_small_q_ws_kernel, small_q_smem(true));
@@ -1003,9 +1013,7 @@ static int att_launch(const AttArgs& a, cudaStream_t stream) {
     float* part_o = a.scratch;
     float* part_ml = a.scratch ? a.scratch + (size_t)a.n_tokens * a.nq * a.num_splits * VD : nullptr;
     dim3 grid(a.num_splits, a.nkv, a.n_req);
-    // the longest contexts first where the grid shares the SMs with the prompts' items.  (A grid of decoding requests alone that is more than
-    // the SMs hold, two CTAs each, gains nothing by it: 64 requests of 129 to 383 keys 1,387 to 1,435 us a step.)
-    const int ordered = a.run_small == 2 && a.n_req > 1 && a.n_req <= WS_ORDERED;
+    const int ordered = a.run_small == 2 && ifb_attention_mma_ordered(a.n_req, a.nq, a.nkv, a.num_splits, a.max_q_len, ifb_sm_count());
     int st;
     if (TMA && a.num_splits > 1 && a.num_splits <= ATT_MAX_CLUSTER && !(a.num_splits & (a.num_splits - 1)) &&
         (long long)a.nkv * a.n_req <= att_max_clusters(a.num_splits)) {

@@ -788,6 +788,14 @@ attn_tile_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
 // ---------------------------------------------------------------------------------------------------
 // qkv [n_tokens, row_stride] bfloat16 (the q heads are the first nq * d columns), k_pages / v_pages: the two streams, pages
 // k_page_stride / v_page_stride elements apart, num_pages of them, each [kv heads][page_size][d or dv]; out [n_tokens, nq * dv].
+// Rows of the grid of `ctas` CTAs each: one per request, or where that is more CTAs than SMs one for each that may be long.  Rows that look
+// their request up cost a round trip, half a microsecond a layer; CTAs without work cost nothing where they find an SM at once (a
+// portion of 65 tokens beside 3 decoding requests, 64 CTAs: two steps of the 0.6B sizes 2,353 us by looking up, 2,324 so; one of 100 beside 5,
+// 192 CTAs to the first portion's 144: 2,503 and 2,460).
+IFB_EXPORT int ifb_attention_tc_rows(int ctas, int n_req, int max_long, int sms) {
+  return max_long > 0 && max_long < n_req && (long long)ctas * n_req > sms ? max_long : n_req;
+}
+
 // nkv: groups of query heads (at most 128 each), `share` of which read one key/value head.  Takes the requests with
 // q_len * (nq / nkv) > 16.  page_size must be 16, 32 or 64.  softcap: 0 none (a library compiled with SOFTCAP takes a positive
 // one, or with SOFTCAP=2 the scores' bound, of at most 60 and no other takes one).  has_sink: exp(sink) joins the denominators (with SOFTCAP, sink at most 60).
@@ -841,8 +849,8 @@ IFB_EXPORT int ifb_attention_tc(const void* qkv, int row_stride, const void* k_p
     score.limit = scale != 0.f ? TC_TANH_RANGE / fabsf(score.to_y) : INFINITY;
   }
   const TcRows rows = {(int)k_page, (int)v_page, (int)k_rows, (int)v_rows};
-  // a CTA per SM walks the request's items
-  dim3 grid((unsigned)(items < sm_count ? items : sm_count), 1, max_long > 0 && max_long < n_req ? max_long : n_req);
+  const unsigned ctas = (unsigned)(items < sm_count ? items : sm_count);
+  dim3 grid(ctas, 1, ifb_attention_tc_rows(ctas, n_req, max_long, sm_count));
   return ifb_launch(attn_tile_tc_kernel, grid, dim3(TC_THREADS), (size_t)SMEM_BYTES, stream, q_map, k_map, v_map, rows, err, block_tables,
                     bt_stride, cu_q, seq_lens, (bf16*)out, n_req, nq, nkv, share, page_size, score, has_sink ? sink * LOG2E : -INFINITY, window);
 }

@@ -581,11 +581,11 @@ def test_attention_on_tcgen05_with_more_items_than_sms(K, q_lens, seq_lens, wind
 
 
 @pytest.mark.parametrize("nq,nkv", [(16, 8), (16, 2)])
-@pytest.mark.parametrize("longs,shorts", [([70], 15), ([9, 500, 17], 40), ([64], 1), ([100, 30], 32), ([200], 63), ([65, 65], 70)])
+@pytest.mark.parametrize("longs,shorts", [([70], 15), ([9, 500, 17], 40), ([64], 1), ([100, 30], 32), ([200], 63), ([65, 65], 70), ([500], 15), ([40], 2)])
 def test_attention_of_mixed_steps(K, nq, nkv, longs, shorts):
     """Prompts beside decoding requests, with lengths that bound how many requests are long: the prompts' grid has a row for each of
-    these (more, where the bound allows more) and finds it among the others, and the decoding requests run in the order of their
-    keys (up to 64 requests), ties, a request of one key and the edges of 32 and 64 requests included."""
+    these (more, where the bound allows more) and finds it among the others, or a row for every request, and the decoding requests run in
+    the order of their keys (up to 64 requests) or the step's (tests/test_tcgen05_rules.py has the lines), ties, a request of one key and the edges of 32 and 64 requests included."""
     d, ps = 128, 16
     g = torch.Generator().manual_seed(shorts)
     q_lens, seq_lens = [1] * shorts, torch.randint(1, 400, (shorts,), generator=g).tolist()

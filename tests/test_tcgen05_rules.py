@@ -131,3 +131,15 @@ def test_the_bound_of_long_requests_holds():
                 bound = CudaKernels.long_requests(sum(lens), count, group, max(lens), min(lens))
                 assert sum(q >= least for q in lens) <= bound <= count, (group, lens)
                 assert CudaKernels.long_requests(sum(lens), count, group, max(lens), 1) >= bound
+
+
+def test_few_requests_beside_a_prompt_are_taken_as_they_come():
+    """Looking a request up, or its place by the number of keys, costs every CTA a round trip: only where CTAs have to wait for an SM."""
+    rows = load_library("attention_tc").ifb_attention_tc_rows
+    assert [rows(16, n, 1, 148) for n in (1, 4, 9, 10, 40)] == [1, 4, 9, 1, 1]
+    assert rows(56, 16, 3, 148) == 3 and rows(56, 16, 0, 148) == 16 and rows(56, 16, 16, 148) == 16 and rows(56, 2, 1, 148) == 2
+    ordered = load_library("attention_mma", {"HEAD_DIM": 128}).ifb_attention_mma_ordered
+    # a portion of 65 tokens leaves 132 SMs, one of 446 tokens 92
+    assert not ordered(4, 16, 8, 8, 65, 148) and ordered(16, 16, 8, 2, 446, 148) and not ordered(16, 16, 8, 2, 65, 148)
+    assert ordered(64, 16, 8, 1, 65, 148) and not ordered(65, 16, 8, 1, 65, 148) and not ordered(1, 16, 8, 32, 2048, 148)
+    assert ordered(2, 16, 8, 1, 2048, 148) and ordered(4, 16, 8, 8, 65, 74)
