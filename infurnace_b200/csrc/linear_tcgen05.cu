@@ -1571,8 +1571,7 @@ static int tc_launch_cfg(const void* x, const void* w, void* out, int n, int o, 
 // product, and the heavy epilogue of one tile runs beside the products of the next).  Otherwise one tile per CTA:
 // the wide shape when there are enough wide tiles to fill the SMs (a 256 x 256 tile reads half the operand bytes
 // per product from shared memory, which is what bounds these kernels), else the deep or the narrow one.
-static int tc_pick_shape(int epi, int n, int o) {
-  const int sm_count = ifb_sm_count();
+static int tc_pick_shape(int epi, int n, int o, int sm_count) {
   if (epi) return (long long)((o + 63) / 64) * ((n + G_BM - 1) / G_BM) <= sm_count ? 7 : 4;
   const long long tn = (long long)((o + 127) / 128) * ((n + G_BM - 1) / G_BM);
   const long long tw = (long long)((o + 255) / 256) * ((n + 2 * G_BM - 1) / (2 * G_BM));
@@ -1612,13 +1611,22 @@ static bool tc_pick_pair(int pairs, TcKind kind, int n, int o, int k) {
   return tiles * 10 >= (long long)pairs * 8 * rounds;
 }
 // Tiles of the last round that are halved, 0 for none.  A product with such a round takes the pairs even where whole tiles would leave
-// more than a fifth of them idle: everywhere the quickest (gate and up of 3,072 x 1,024 at 818 rows 16.1 us on the
-// persistent kernel, 12.9 so, at 1,600 rows 21.8 and 17.4; 6,144 x 2,048 at 818 rows 27.8 and 21.7, at 1,600 50 and 31).
+// more than a fifth of them idle, if the kernel it would go to needs a round more than the whole ones here: plain products that go to the wide
+// tiles (0.62 to 0.92 of their time over 144 products of 512 to 12,288 features, k 512 to 4,096, 513 to 3,000 rows; against narrow tiles 0.92 to
+// 1.31, most of them one round, 1,100 rows of 4,096 x 1,024 13.0 us and 16.3 so), gated ones from a k of 1,024 on with more rounds of the persistent kernel
+// (0.71 to 1.0; with as many 0.93 to 1.36, 1,100 rows of 2,048 x 4,096 27.8 and 36.5, and below that k up to 1.12).  Gate and up of 3,072 x 1,024 at 818 rows
+// 16.1 us on the persistent kernel, 12.9 so, at 1,600 rows 21.8 and 17.4; 6,144 x 2,048 at 818 rows 27.8 and 21.7, at 1,600 50 and 31.
 static int tc_pick_halves(int pairs, TcKind kind, int n, int o, int k) {
   if (o % 64 || n <= 512 || pairs < 1 || (kind != TC_PLAIN && kind != TC_GATED)) return 0;
-  const int features = tc_pair_features(pairs, kind, n, o);
+  const int features = tc_pair_features(pairs, kind, n, o), sms = 2 * pairs;
   if (features != (kind == TC_GATED ? 128 : 256)) return 0;
-  return tc_pair_halved(pairs, (long long)((n + 255) / 256) * ((o + features - 1) / features), k);
+  const long long tiles = (long long)((n + 255) / 256) * ((o + features - 1) / features);
+  const int halved = tc_pair_halved(pairs, tiles, k);
+  if (!halved || tc_pick_pair(pairs, kind, n, o, k)) return halved;
+  const int shape = tc_pick_shape(kind == TC_GATED, n, o, sms);
+  if (kind == TC_PLAIN) return shape == 3 ? halved : 0;
+  const long long alone = (long long)((n + G_BM - 1) / G_BM) * ((o + 127) / 128);
+  return shape == 4 && k >= 1024 && (alone + sms - 1) / sms > tiles / pairs ? halved : 0;
 }
 
 template <int EPI, typename TO>
@@ -1637,7 +1645,7 @@ static int tc_launch(const void* x, const void* w, void* out, int n, int o, int 
   if (shape == 0) {
     const int pairs = tc_device_pairs();
     const TcKind kind = tc_kind(EPI, fold);
-    shape = tc_pick_pair(pairs, kind, n, o, k) || tc_pick_halves(pairs, kind, n, o, k) > 0 ? 6 : tc_pick_shape(EPI, n, o);
+    shape = tc_pick_pair(pairs, kind, n, o, k) || tc_pick_halves(pairs, kind, n, o, k) > 0 ? 6 : tc_pick_shape(EPI, n, o, ifb_sm_count());
   }
   if (EPI && fold.res_x) return IFB_ERR_ARG;
   if (shape == 6) {
@@ -1786,7 +1794,7 @@ IFB_EXPORT int ifb_linear_tcgen05_pair_halved(int kind, int n_rows, int out_feat
 IFB_EXPORT int ifb_linear_tcgen05_fold_parts(int n_rows, int out_features, int splits) {
   if (splits > 1) return (out_features + 127) / 128;
   if (tc_pick_pair(tc_device_pairs(), TC_RESIDUAL, n_rows, out_features, 0)) return (out_features + 63) / 64;       // (whatever the k)
-  return tc_pick_shape(0, n_rows, out_features) == 3 ? 2 * ((out_features + 255) / 256) : 2 * ((out_features + 127) / 128);
+  return tc_pick_shape(0, n_rows, out_features, ifb_sm_count()) == 3 ? 2 * ((out_features + 255) / 256) : 2 * ((out_features + 127) / 128);
 }
 
 using SplitCfg = GemmCfg<0, 1, 128, 6>;

@@ -960,7 +960,7 @@ def test_qkv_product_over_pairs_with_norm_rotation_and_store_in_its_epilogue(K, 
 # sum that a whole tile forms, in the same order: the halves leave the bits of the forced whole-tile kernel of one CTA.
 @pytest.mark.parametrize("od", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,o,k,kind,epilogue", [(2043, 3072, 520, 0, "relu2"), (1280, 4096, 512, 0, "none"), (4600, 2240, 584, 0, "none"), (2043, 2368, 520, 0, "none"),
-                                                 (818, 3072, 512, 3, "silu_gate"), (700, 3264, 584, 3, "gelu_gate"), (1600, 3136, 520, 3, "silu_gate"), (5000, 1024, 1032, 3, "silu_gate")])
+                                                 (818, 3072, 1024, 3, "silu_gate"), (700, 3264, 1096, 3, "gelu_gate"), (1600, 3136, 1032, 3, "silu_gate"), (5000, 1024, 1032, 3, "silu_gate")])
 def test_product_over_pairs_with_halved_tiles(K, od, n, o, k, kind, epilogue):
     from infurnace_b200.kernels.cuda import EPILOGUES
     assert K._tc_lib().ifb_linear_tcgen05_pair_halved(kind, n, o, k, 0) > 0

@@ -61,20 +61,36 @@ def test_the_heads_of_a_short_product_stay_on_one_tile_per_cta(kind, n, o, k, ti
 
 
 def test_only_a_last_round_that_leaves_half_the_pairs_idle_is_halved():
+    """And a product that would not run over pairs with whole tiles takes them for the halves' sake only where the kernel it would go to needs
+    a round more than the whole ones: the wide tiles, or the persistent kernel for gates from a k of 1,024 on."""
     lib = load_library("linear_tcgen05")
-    taken = 0
+    whole, halves, left = 0, 0, 0
     for kind in (PLAIN, RESIDUAL, HEADS, GATED):
-        for n in (1, 512, 513, 768, 1000, 1400, 1900, 2048, 5000):
-            for o in (64, 1000, 1024, 1088, 2304, 3072, 4096, 6144, 12288):
-                rest = lib.ifb_linear_tcgen05_pair_halved(kind, n, o, 512, 74)
+        for n in (1, 512, 513, 768, 818, 1000, 1100, 1400, 1900, 2048, 5000):
+            for o in (64, 1000, 1024, 1088, 2048, 2304, 3072, 4096, 6144, 12288):
+                rest = lib.ifb_linear_tcgen05_pair_halved(kind, n, o, 1024, 74)
                 assert lib.ifb_linear_tcgen05_pair_halved(kind, n, o, 511, 74) == 0
-                tiles = -(-n // 256) * -(-o // (128 if kind == GATED else 256))
-                if kind in (RESIDUAL, HEADS) or n <= 512 or o % 64 or tiles <= 74:
+                tiles, lone = -(-n // 256) * -(-o // (128 if kind == GATED else 256)), -(-n // 128) * -(-o // 128)
+                if kind in (RESIDUAL, HEADS) or n <= 512 or o % 64 or tiles <= 74 or tiles % 74 > 37:
                     assert rest == 0, (kind, n, o)
+                elif lib.ifb_linear_tcgen05_pair_tile(kind, n, o, 1024, 74):
+                    assert rest == tiles % 74, (kind, n, o)
+                    whole += rest > 0
+                elif kind == GATED:
+                    assert rest == (tiles % 74 if -(-lone // 148) > tiles // 74 else 0), (kind, n, o)
+                    assert lib.ifb_linear_tcgen05_pair_halved(kind, n, o, 1016, 74) == 0
                 else:
-                    assert rest == (tiles % 74 if tiles % 74 <= 37 else 0), (kind, n, o)
-                    taken += rest > 0
-    assert taken > 20
+                    narrow, wide = -(-lone // 296), -(-tiles // 148)
+                    assert rest == (tiles % 74 if 1.15 * wide < narrow else 0), (kind, n, o)
+                    assert lib.ifb_linear_tcgen05_pair_halved(kind, n, o, 512, 74) == rest
+                halves, left = halves + (rest > 0), left + (rest == 0 and 0 < tiles % 74 <= 37 < tiles)
+    assert whole > 5 and halves > 15 and left > 10
+
+
+# Measured on both sides: 80 tiles for 74 pairs against one round of 144 or 288 tiles, and against two of 216 or 320.
+@pytest.mark.parametrize("kind,n,o,k,halved", [(GATED, 1100, 2048, 4096, 0), (PLAIN, 1100, 4096, 1024, 0), (GATED, 1280, 2048, 4096, 6), (PLAIN, 1280, 4096, 1024, 6)])
+def test_halves_are_not_worth_a_round_that_the_other_kernels_do_not_need(kind, n, o, k, halved):
+    assert load_library("linear_tcgen05").ifb_linear_tcgen05_pair_halved(kind, n, o, k, 74) == halved
 
 
 class _Norm:
