@@ -210,9 +210,11 @@ IFB_EXPORT int ifb_cast_rows(const float* x, void* out, long long count, cudaStr
 // stores nothing.  A null weight leaves that projection unnormalised.  proj is float32; T is the cache's type.
 // Widths, columns and rows of whole groups of four at 16 bytes, up to 8,192 q and k features: q and k (neighbours in the row) stay in
 // registers, requested with the values at once, both sums share a barrier (q 1,024, k 256: 2,043 rows 12.2 to 6.3 us, eight 4.9 to 2.1).
+// Rows of more than 4,096 (NV 8) are held to the 128 registers with which two blocks share an SM: 32 bytes spill, and at 134 blocks of more than 192
+// threads had an SM each (2,043 rows of q 6,144, k 1,024: 47 us feature by feature, 58 with one block, 33 so).
 // ------------------------------------------------------------------------------------------
 template <typename T, int NV>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, NV == 8 ? 2 : 0)
 wide_norm_store_vec_kernel(const float* proj, int ld, int q_width, int k_width, int v_col, int head_dim, const void* __restrict__ qw,
                            const void* __restrict__ kw, int w_dtype, float eps, T* q_out, const int* slots, T* pages, int page_size) {
   const int n = blockIdx.x, both = q_width + k_width;
