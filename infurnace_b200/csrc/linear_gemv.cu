@@ -584,8 +584,10 @@ IFB_EXPORT int ifb_linear_gemv_qkv(const void* x, const void* w, void* qkv, int 
            reinterpret_cast<bf16*>(pages), page_size};
   const int nb = n_rows <= 8 ? 1 : 2;
   // A long k, one block of tokens, and more CTAs of 16 pairs (of which an SM holds one) than SMs: 8 pairs, two CTAs per SM (48 heads of
-  // 4,096, 192 CTAs: 19.1 to 16.7 us for eight rows, 18.5 to 15.5 for one; 56 of 5,120 23.4 to 20.1; 28 of 3,072, 112 CTAs, 7.1 to 7.7: not).
-  if (k_dim > 2048 && nb == 1 && head_dim <= 128 && (long long)(nq + 2 * nkv) * (head_dim / 32) > ifb_sm_count())
+  // 4,096, 192 CTAs: 19.1 to 16.7 us for eight rows, 18.5 to 15.5 for one; 56 of 5,120 23.4 to 20.1; 28 of 3,072, 112 CTAs, 7.1 to 7.7: not; a k of
+  // 2,304 44 heads, 176 CTAs, 0.86 to 0.88 of the time, of 2,056 as many 1.02 to 1.06, 48 0.86 to 0.90).
+  const long long ctas = (long long)(nq + 2 * nkv) * (head_dim / 32);
+  if (k_dim > 2048 && nb == 1 && head_dim <= 128 && (k_dim >= 2304 ? ctas > ifb_sm_count() : 4 * ctas >= 5LL * ifb_sm_count()))
     return gv_launch_qkv<1, 8, 2, 5>(x, w, qkv, n_rows, k_dim, rs, qk, stream);
   if (k_dim <= 1024) return nb == 1 ? gv_launch_qkv<1, 8, 1>(x, w, qkv, n_rows, k_dim, rs, qk, stream)
                                     : gv_launch_qkv<2, 8, 1>(x, w, qkv, n_rows, k_dim, rs, qk, stream);

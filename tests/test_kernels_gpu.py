@@ -725,10 +725,10 @@ def test_plain_attention_with_keys_in_pieces(K, nq, nkv, d, ps, window):
     test_plain_attention_of_a_query_is_the_same_in_every_step(K, nq, nkv, d, ps, window)
 
 
-# Eight feature pairs per CTA: a k over 2,048 and more CTAs of sixteen pairs than SMs (38 heads of 128, 75 of 64); 37 heads and 74 lie
-# just below.  A last step of k of 8, rows 1 to 8.
+# Eight feature pairs per CTA: a k from 2,304 on and more CTAs of sixteen pairs than SMs (38 heads of 128, 75 of 64; 37 heads and 74 lie
+# just below), or over 2,048 and a quarter more (48 heads; 46 lie below).  A last step of k of 8, rows 1 to 8.
 @pytest.mark.parametrize("n", [1, 3, 8])
-@pytest.mark.parametrize("nq,nkv,d,k,ps", [(32, 3, 128, 2056, 16), (31, 3, 128, 2056, 16), (61, 7, 64, 2176, 8), (60, 7, 64, 2176, 8)])
+@pytest.mark.parametrize("nq,nkv,d,k,ps", [(32, 3, 128, 2312, 16), (31, 3, 128, 2312, 16), (61, 7, 64, 2312, 8), (60, 7, 64, 2312, 8), (40, 4, 128, 2056, 16), (38, 4, 128, 2056, 16)])
 @pytest.mark.parametrize("norm,rotate,scaled", [(True, True, True), (False, True, False), (True, False, False)])
 def test_qkv_product_of_eight_pairs_per_cta(K, n, nq, nkv, d, k, ps, norm, rotate, scaled):
     test_qkv_product_with_norm_rotation_and_store_in_its_epilogue(K, n, nq, nkv, d, k, ps, norm, rotate, scaled)
