@@ -619,6 +619,8 @@ constexpr int WS_ORDERED = 64;         // requests, two per lane, up to which th
 // grid's tail is short work (those that are not the kernel's come last).  What was read of it comes back with it.  Whole warps; one round trip, as
 // without, and some 150 instructions.  Fifteen requests of 77 to 1,500 keys beside a prompt's items: in the order of the step the longest came last,
 // when 184 CTAs had taken the SMs that the items leave, and ended the kernel 14 us after the items; now 6.6 us (3,954 to 3,522 us for two steps).
+// (ORDERED, a form of the kernel of its own: the code alone cost the others 0.05 to 0.25 us a launch; 32 requests of 80 to 200 keys, 0.6B
+// sizes, 1,082 us a step without, 1,094 with it in one kernel, 48 1,256 and 1,263.)
 struct SqRequest { int r, q0, q_len, L; };
 __device__ __forceinline__ SqRequest sq_request(int place, int n_req, int G, const int* __restrict__ cu_q, const int* __restrict__ seq_lens) {
   const int lane = threadIdx.x & 31;
@@ -656,6 +658,7 @@ __device__ __forceinline__ void att_mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 
+template <bool ORDERED>
 __global__ void __launch_bounds__(WS_THREADS)
 attn_small_q_ws_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, AttRows mrows,
                        int* __restrict__ err,
@@ -663,7 +666,7 @@ attn_small_q_ws_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                        const int* __restrict__ cu_q, const int* __restrict__ seq_lens, bf16* __restrict__ out,
                        float* __restrict__ part_o, float* __restrict__ part_ml, int* __restrict__ counters, int nq,
                        int nkv, int share, int page_size, AttScale sc, float sink, int window, int num_splits, int clustered,
-                       int beside, int ordered) {
+                       int beside) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int is_last;
   __shared__ uint64_t full_bar[SQ_STAGES], empty_bar[SQ_STAGES];
@@ -679,7 +682,7 @@ attn_small_q_ws_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = nq / nkv;
   int r = blockIdx.z, q0, q_len, L;
-  if (ordered) {
+  if constexpr (ORDERED) {
     const SqRequest q = sq_request(blockIdx.z, gridDim.z, G, cu_q, seq_lens);
     r = q.r; q0 = q.q0; q_len = q.q_len; L = q.L;
   } else {
@@ -987,7 +990,7 @@ static int att_max_clusters(int splits) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, attn_small_q_ws_kernel, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (cudaOccupancyMaxActiveClusters(&n, attn_small_q_ws_kernel<false>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
     known[dev][splits] = n;
   }
   return known[dev][splits];
@@ -1005,15 +1008,20 @@ IFB_EXPORT int ifb_attention_mma_ordered(int n_req, int nq, int nkv, int num_spl
 
 template <bool TMA>
 static int att_launch(const AttArgs& a, cudaStream_t stream) {
-  if (TMA) IFB_ALLOW_SMEM(attn_small_q_ws_kernel, small_q_smem(true));
-  else IFB_ALLOW_SMEM(attn_small_q_kernel<false>, small_q_smem(false));
+  if (TMA) {
+    IFB_ALLOW_SMEM(attn_small_q_ws_kernel<false>, small_q_smem(true));
+    IFB_ALLOW_SMEM(attn_small_q_ws_kernel<true>, small_q_smem(true));
+  } else {
+    IFB_ALLOW_SMEM(attn_small_q_kernel<false>, small_q_smem(false));
+  }
   IFB_ALLOW_SMEM(attn_tile_kernel<TMA>, tile_smem(TMA));
   const int G = a.nq / a.nkv;
   if (a.run_small) {
     float* part_o = a.scratch;
     float* part_ml = a.scratch ? a.scratch + (size_t)a.n_tokens * a.nq * a.num_splits * VD : nullptr;
     dim3 grid(a.num_splits, a.nkv, a.n_req);
-    const int ordered = a.run_small == 2 && ifb_attention_mma_ordered(a.n_req, a.nq, a.nkv, a.num_splits, a.max_q_len, ifb_sm_count());
+    const bool ordered = a.run_small == 2 && ifb_attention_mma_ordered(a.n_req, a.nq, a.nkv, a.num_splits, a.max_q_len, ifb_sm_count());
+    const auto ws_kernel = ordered ? attn_small_q_ws_kernel<true> : attn_small_q_ws_kernel<false>;
     int st;
     if (TMA && a.num_splits > 1 && a.num_splits <= ATT_MAX_CLUSTER && !(a.num_splits & (a.num_splits - 1)) &&
         (long long)a.nkv * a.n_req <= att_max_clusters(a.num_splits)) {
@@ -1031,15 +1039,15 @@ static int att_launch(const AttArgs& a, cudaStream_t stream) {
       attr[1].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       cfg.numAttrs = ifb_pdl_enabled() ? 2 : 1;
-      cudaError_t e = cudaLaunchKernelEx(&cfg, attn_small_q_ws_kernel, a.k_map, a.v_map, a.rows, a.err, (const bf16*)a.qkv, a.row_stride,
+      cudaError_t e = cudaLaunchKernelEx(&cfg, ws_kernel, a.k_map, a.v_map, a.rows, a.err, (const bf16*)a.qkv, a.row_stride,
                                          a.block_tables, a.bt_stride, a.cu_q, a.seq_lens, (bf16*)a.out, part_o, part_ml, a.counters, a.nq,
-                                         a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 1, (int)(a.run_small == 2), ordered);
+                                         a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 1, (int)(a.run_small == 2));
       if (e != cudaSuccess) { cudaGetLastError(); return -(int)e; }
       st = IFB_OK;
     } else if (TMA)
-      st = ifb_launch(attn_small_q_ws_kernel, grid, dim3(WS_THREADS), small_q_smem(true), stream, a.k_map, a.v_map, a.rows, a.err,
+      st = ifb_launch(ws_kernel, grid, dim3(WS_THREADS), small_q_smem(true), stream, a.k_map, a.v_map, a.rows, a.err,
                       (const bf16*)a.qkv, a.row_stride, a.block_tables, a.bt_stride, a.cu_q, a.seq_lens, (bf16*)a.out, part_o, part_ml,
-                      a.counters, a.nq, a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 0, (int)(a.run_small == 2), ordered);
+                      a.counters, a.nq, a.nkv, a.share, a.page_size, a.sc, a.sink, a.window, a.num_splits, 0, (int)(a.run_small == 2));
     else
       st = ifb_launch(attn_small_q_kernel<false>, grid, dim3(THREADS), small_q_smem(false), stream, a.k_map, a.v_map, a.rows, a.err,
                       (const bf16*)a.qkv, a.row_stride, a.k, a.v, a.block_tables, a.bt_stride, a.cu_q, a.seq_lens, (bf16*)a.out, part_o,
