@@ -87,7 +87,8 @@ __device__ __forceinline__ void gv_cluster_barrier() {
 // out = act(gate) * up, act = silu or rs.unary.  EPI 2: v = x + y is written back to x, out = v * g.  EPI 4: as EPI 1 with 8 features per
 // CTA, whose 8 gate rows and 8 up rows are the two halves of one 16-row tile (half the registers of EPI 1, so two CTAs
 // per SM where EPI 1 with two stages has one).  WARPS: warps of a CTA (they split k).
-// EPI 5: as EPI 3 with 8 feature pairs per CTA, likewise the two halves of one tile.
+// EPI 5: as EPI 3 with 8 feature pairs per CTA, likewise the two halves of one tile (held to 128 registers for the second CTA of an SM, 32 bytes
+// spill).
 // STAGES: steps of 128 of k whose weights (and, for one block of tokens, activations) a warp has requested at any
 // time.  1: every warp's k range is one step (the sizes of small models, where the chain of round trips counts);
 // 2: a warp walks a long k range and keeps the memory pipe full while it multiplies (large models, where the

@@ -165,7 +165,8 @@ rows32_kernel(const float* __restrict__ x, const float* __restrict__ w, TO* __re
 // ALONE: where tiles are more than the pairs of SMs, a CTA takes a whole tile, each slice two groups one after the other in one run
 // through its ring (of three stages; the first group's tile waits beside it).  Filling the ring and the sum at the end cost a CTA
 // of a pair 17,000 of 37,000 cycles at a k of 1,024: 2,048 rows of 4,096 x 1,024 535 to 424 us (40 TFLOP/s), 193 rows of the LM head 2,371 to 1,837.
-// RT: rows per thread, and an eighth of a tile's (tile32_form).
+// RT: rows per thread, and an eighth of a tile's (tile32_form).  Eight take all 255 registers: a lone CTA spills 28 bytes (gated 128), single
+// copies 188 to 592.
 // ---------------------------------------------------------------------------------------------------
 constexpr int T32 = 64, T32_SLICES = S32_GROUPS / 2, T32_PITCH = S32_BK + 4;      // 20 floats: conflict-free 16-byte reads
 constexpr int T32_STAGE = 2 * T32 * T32_PITCH;                                    // floats: the rows of x, then those of w
